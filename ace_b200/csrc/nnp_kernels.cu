@@ -374,7 +374,11 @@ __device__ void sort_cell(int c, int lane, unsigned *keys, int kcap, const Struc
                           int4 *__restrict__ items, int *__restrict__ items_n)
 {
     const int n = cell_cnt[c];
-    if (n == 0) return;                                          // uniform over the warp
+    if (n == 0) {                                                // uniform over the warp
+        // the search reads the counts of every neighbouring cell, empty ones too
+        for (int t = lane; t < ntypes; t += 32) cell_tcnt[(size_t)c * ntypes + t] = 0;
+        return;
+    }
     const int cs = cell_start[c];
     int *a = cell_atoms + cs;
     unsigned *k = (n <= kcap) ? keys : tmp + cs;

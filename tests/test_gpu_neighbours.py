@@ -58,3 +58,34 @@ def test_neighbour_counts_match_oracle(tmp_path, name):
     assert got.shape == want.shape
     bad = np.argwhere(got != want)
     assert bad.size == 0, "first mismatches (atom, element): %s" % bad[:5].tolist()
+
+
+def slab(n, vacuum, seed):
+    """n atoms in the lower part of a cell whose upper part, `vacuum` times as high, is empty"""
+    b = synth.batch_random(seed, [n], 3, shear=0.0)
+    cell = b.cell.copy()
+    cell[0, 2, 2] *= 1.0 + vacuum
+    return synth.Batch(b.atom_off, b.pos, b.type, cell, True)
+
+
+@pytest.mark.parametrize("n, free", [(600, False), (3000, False), (2600, True)])
+def test_empty_cells_have_no_candidates(tmp_path, n, free):
+    """Cells without atoms, in the one-block prologue (600 atoms), the launch
+    sequence and the grid over a large free structure's box, on a handle whose
+    previous batch had atoms in every cell: the counts of the earlier batch
+    must not be seen."""
+    pot = synth.potential_config(2)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    nn = NNP.read(path)
+    full = synth.batch_random(5, [4 * n], 3)
+    nn.compute_batch(full.atom_off, full.pos, full.type, full.cell)
+    b = slab(n, 2.0, 6)
+    if free:
+        b = synth.Batch(b.atom_off, b.pos, b.type, b.cell, pbc=False)
+        nn.compute_batch(b.atom_off, b.pos, b.type, None, pbc=False)
+    else:
+        nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    got = nn.neighbor_counts(b.n_atoms)
+    nn.close()
+    assert np.array_equal(got, oracle_counts(pot.rc, b, 3))
