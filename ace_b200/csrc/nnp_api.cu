@@ -122,6 +122,7 @@ void Engine::free_all()
 {
     rpar.release(); apar.release(); wpar.release(); vac.release();
     rpar64.release(); apar64.release(); cut64.release();
+    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release();
     atom_off.release(); pos.release(); cell.release(); xw.release();
     type.release(); atom_struct.release(); atom_cell.release(); grid.release(); bbox.release();
     cell_cnt.release(); cell_start.release(); cell_fill.release(); cell_atoms.release(); scan_tmp.release();
@@ -284,7 +285,98 @@ std::string Engine::build_tables()
     wpar_host = wp;
     vac_host = vc;
     dpot = d;
+    build_moments();
     return "";
+}
+
+// Coefficients of (1/2 + lf x)^zeta in Legendre polynomials P_0 .. P_L, zeta <= L:
+// x^k = sum over l = k, k-2, .. of (2l+1) k! / (2^((k-l)/2) ((k-l)/2)! (k+l+1)!!) P_l.
+static void legendre_power(double lf, int zeta, int L, double *c)
+{
+    for (int l = 0; l <= L; ++l) c[l] = 0.0;
+    for (int k = 0; k <= zeta; ++k) {
+        double x = std::pow(0.5, zeta - k) * std::pow(lf, k);          // binomial term of x^k
+        for (int q = 0; q < k; ++q) x *= (double)(zeta - q) / (q + 1);
+        for (int l = k; l >= 0; l -= 2) {
+            double t = 2 * l + 1;
+            for (int q = 2; q <= k; ++q) t *= q;
+            for (int q = 1; q <= (k - l) / 2; ++q) t /= 2.0 * q;
+            for (int q = k + l + 1; q > 1; q -= 2) t /= q;
+            c[l] += x * t;
+        }
+    }
+}
+
+// Whether the angular functions have the moment form, and its table (MomTab).
+void Engine::build_moments()
+{
+    const DevPot &d = dpot;
+    const int T = d.ntypes, TT = T * (T + 1) / 2;
+    mom_ok = false;
+    mom_L = mom_ND = mom_NR = mom_fmax = 1;
+    bool any = false;
+    for (int II = 0; II < T; ++II) {
+        int fn = 0;
+        for (int J = 0; J < T; ++J) mom_NR = std::max(mom_NR, d.t[II].br[J].n);
+        for (int tt = 0; tt < TT; ++tt) {
+            const DevBlockA &b = d.t[II].ba[tt];
+            fn += b.n;
+            for (int f = 0; f < b.n; ++f) {
+                const float4 q = apar_host[b.par + f];
+                int pk;
+                std::memcpy(&pk, &q.w, sizeof pk);
+                const int iz = (pk >> 8) - 1;
+                if (b.form != ANG_GAUSS || iz < 0 || iz > NNP_MOM_MAXL || !(std::fabs(q.x) <= 0.5f)) return;
+                mom_L = std::max(mom_L, iz);
+                any = true;
+            }
+        }
+        mom_fmax = std::max(mom_fmax, fn);
+        mom_ND = std::max(mom_ND, d.t[II].ndamp);
+    }
+    // more factors or elements: the moment set outgrows the registers of one pass
+    if (!any || mom_ND > NNP_MOM_MAXD || T * ((mom_ND + 1) / 2) > 8) return;
+    mom_ok = true;
+    const int L = mom_L;
+    std::vector<float> tab(mom_tab_floats(T, L, mom_fmax), 0.f);
+    float *p = tab.data();
+    const int NC = mom_comps(L), TT1 = L + 2;
+    auto put = [&](int c, int l, int m) {
+        double n = (m ? 2.0 : 1.0), lead = 1.0;
+        for (int q = l - m + 1; q <= l + m; ++q) n /= q;               // (2 - delta) (l-m)!/(l+m)!
+        for (int q = 1; q <= l; ++q) lead *= (2.0 * q - 1.0) / q;      // (2l)!/(2^l l!^2)
+        for (int q = l - m + 1; q <= l; ++q) lead *= q;                // l!/(l-m)!
+        p[c] = (float)(std::sqrt(n) * lead);
+        p[NC + c] = (float)std::sqrt(n);
+        std::memcpy(&p[2 * NC + c], &l, sizeof l);
+    };
+    for (int l = 0; l <= L; ++l) put(l, l, 0);
+    for (int m = 1; m <= L; ++m)
+        for (int l = m; l <= L; ++l)
+            for (int s = 0; s < 2; ++s) put(mom_base(L, m) + 2 * (l - m) + s, l, m);
+    p += 3 * NC;
+    float *coef = p + T * NNP_MOM_MAXD, *fun = coef + (size_t)T * TT1 * mom_fmax;
+    for (int II = 0; II < T; ++II)
+        for (int K = 0, tt = 0; K < T; ++K)
+            for (int J = 0; J <= K; ++J, ++tt) {
+                const DevBlockA &b = d.t[II].ba[tt];
+                for (int f = 0; f < b.n; ++f) {
+                    const double4 q = apar64_host[b.par + f];
+                    int pk;
+                    std::memcpy(&pk, &apar_host[b.par + f].w, sizeof pk);
+                    const int dmp = pk & 0xff, fu = tt | dmp << 8 | J << 16 | K << 24;
+                    p[II * NNP_MOM_MAXD + dmp] = (float)(q.z - (double)d.t[II].damp_a[dmp]);
+                    double c[NNP_MOM_MAXL + 1];
+                    legendre_power(q.x, (int)q.y, L, c);
+                    const size_t o = b.off_g - d.t[II].n_input_r + f;
+                    float *cf = coef + (size_t)II * TT1 * mom_fmax + o;
+                    const double half = J == K ? 0.5 : 1.0;
+                    for (int l = 0; l <= L; ++l) cf[(size_t)l * mom_fmax] = (float)(half * c[l]);
+                    cf[(size_t)(L + 1) * mom_fmax] = J == K ? (float)(0.5 * std::pow(0.5 + q.x, q.y)) : 0.f;
+                    std::memcpy(&fun[(size_t)II * mom_fmax + o], &fu, sizeof fu);
+                }
+            }
+    mom_tab_host = tab;
 }
 
 std::string Engine::upload()
@@ -305,6 +397,8 @@ std::string Engine::upload()
     if (rp64.empty()) rp64.push_back(make_double2(0.0, 0.0));
     if (ap64.empty()) ap64.push_back(make_double4(0.0, 0.0, 0.0, 0.0));
     if (c64.empty()) c64.push_back(0.0);
+    std::vector<float> mt = mom_tab_host;
+    if (mt.empty()) mt.push_back(0.f);
     cudaError_t e = cudaSuccess;
     auto r = [&](cudaError_t x) { if (x != cudaSuccess && e == cudaSuccess) e = x; };
     if (!d_pot) r(cudaMalloc((void **)&d_pot, sizeof(DevPot)));
@@ -315,6 +409,7 @@ std::string Engine::upload()
     r(rpar64.reserve(rp64.size()));
     r(apar64.reserve(ap64.size()));
     r(cut64.reserve(c64.size()));
+    r(mom_tab.reserve(mt.size()));
     if (e != cudaSuccess) return std::string("device allocation failed: ") + cudaGetErrorString(e);
     r(cudaMemcpy(d_pot, &d, sizeof d, cudaMemcpyHostToDevice));
     r(cudaMemcpy(rpar.p, rp.data(), rp.size() * sizeof(float2), cudaMemcpyHostToDevice));
@@ -324,6 +419,7 @@ std::string Engine::upload()
     r(cudaMemcpy(rpar64.p, rp64.data(), rp64.size() * sizeof(double2), cudaMemcpyHostToDevice));
     r(cudaMemcpy(apar64.p, ap64.data(), ap64.size() * sizeof(double4), cudaMemcpyHostToDevice));
     r(cudaMemcpy(cut64.p, c64.data(), c64.size() * sizeof(double), cudaMemcpyHostToDevice));
+    r(cudaMemcpy(mom_tab.p, mt.data(), mt.size() * sizeof(float), cudaMemcpyHostToDevice));
     if (e != cudaSuccess) return std::string("potential upload failed: ") + cudaGetErrorString(e);
     return "";
 }
@@ -830,7 +926,8 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
     std::vector<int64_t> key;
     if (graphs)
         key = {N, S, b->pbc, n_ghost, E.cap, (int64_t)flags, (int64_t)(atom_energy != nullptr), (int64_t)(virial != nullptr),
-               E.precision, (int64_t)(intptr_t)(E.use_jit ? E.jit_symm : nullptr), (int64_t)E.acc64 + 2 * E.symm64,
+               E.precision, (int64_t)(intptr_t)(E.use_jit ? E.jit_module : nullptr), (int64_t)E.acc64 + 2 * E.symm64,
+               (int64_t)(intptr_t)E.mom.p, E.mom_rows,
                (int64_t)(intptr_t)E.atom_off.p,
                (int64_t)(intptr_t)E.pos.p, (int64_t)(intptr_t)E.type.p, (int64_t)(intptr_t)E.cell.p,
                (int64_t)(intptr_t)E.nbr.p, (int64_t)(intptr_t)E.G.p, (int64_t)(intptr_t)E.force.p,

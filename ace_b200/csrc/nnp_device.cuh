@@ -103,6 +103,7 @@ struct DevErr {
     int bad_type;     // an atom type was outside [0, ntypes)
     int bad_cell;     // a periodic cell had no volume (1) or was thinner than rc / NNP_MAX_IMAGES (2)
     int nonfinite;    // a non-finite energy or force
+    int few;          // (atom, angular block) entries of few pairs (nnp_moments.cuh); not an error
 };
 
 #if defined(__CUDACC__)

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "nnp_internal.h"
+#include "nnp_moments.cuh"
 
 namespace nnp {
 
@@ -98,7 +99,22 @@ struct Engine {
     bool use_jit = true;
     void *jit_module = nullptr;   // cudaLibrary_t
     void *jit_symm = nullptr, *jit_force = nullptr, *jit_tangent = nullptr;   // cudaKernel_t
+    // cudaKernel_t, moment form: warp or thread per atom; one or two atoms per warp
+    void *jit_symm_mom = nullptr, *jit_symm_momt = nullptr, *jit_force_mom1 = nullptr, *jit_force_mom2 = nullptr;
+    void *jit_symm_few = nullptr;                                            // and the blocks of few pairs
     std::string jit_source, jit_error;
+
+    // moment form of the angular functions (nnp_moments.cuh)
+    bool mom_ok = false;          // every angular block is GAUSS with integer zeta <= NNP_MOM_MAXL
+    int mom_L = 1, mom_ND = 1, mom_NR = 1, mom_fmax = 1;
+    std::vector<float> mom_tab_host;
+    float mom_a_lo(int II, int d) const { return mom_tab_host[3 * mom_comps(mom_L) + II * NNP_MOM_MAXD + d]; }
+    DBuf<float> mom_tab;          // MomTab
+    DBuf<float2> mom;             // moments of atoms order[0 .. mom_rows) (mom_at)
+    DBuf<unsigned short> mom_cnt; // their neighbour counts by element [row][8]
+    DBuf<int2> mom_items;         // (row, block) of the blocks of few pairs (number: DevErr::few)
+    int64_t mom_rows = 0;         // rows of `mom` the current batch uses (0: not reserved)
+    bool mom_valid = false;       // they hold the whole batch's moments
 
     // stream / events
     cudaStream_t stream = nullptr;
@@ -179,6 +195,14 @@ struct Engine {
 
     // device tables of the potential from `host` (host-side only), and their upload
     std::string build_tables();
+    void build_moments();
+    // whether a thread's registers (moments of one element, radial sums) and
+    // its block's shared memory hold the thread-per-atom form
+    bool mom_thread() const
+    {
+        return dpot.ntypes <= NNP_MOM_THREAD_T && 2 * mom_comps(mom_L) + mom_NR <= 184 &&
+               mom_thread_floats(dpot.ntypes, mom_ND, mom_L) * (int)sizeof(float) <= 110 * 1024;
+    }
     std::string upload();
     void free_all();
 };

@@ -34,7 +34,8 @@
 
 namespace nnp {
 
-extern const char *const kDeviceHeaderSource;   // nnp_device.cuh, embedded at build time
+extern const char *const kDeviceHeaderSource;    // nnp_device.cuh, embedded at build time
+extern const char *const kMomentsHeaderSource;   // nnp_moments.cuh
 
 namespace {
 
@@ -106,6 +107,18 @@ std::vector<Fn> block_fns(const Engine &E, const DevBlockA &B)
     return fs;
 }
 
+// bases x_b = |1/2 + lambda/2 cos| of a block's functions
+void gen_bases(std::ostringstream &os, const std::vector<Fn> &fs, std::vector<float> &bases)
+{
+    for (const Fn &f : fs) {
+        bool seen = false;
+        for (float x : bases) seen |= (x == f.lf);
+        if (!seen) bases.push_back(f.lf);
+    }
+    for (size_t b = 0; b < bases.size(); ++b)
+        os << "            const float x" << b << " = fabsf(fmaf(" << flit(bases[b]) << ", cs, 0.5f));\n";
+}
+
 // common per-pair prologue: geometry, bases, damping factors of the used groups
 void pair_prologue(std::ostringstream &os, const std::vector<Fn> &fs, std::vector<float> &bases,
                    std::set<int> &damps, bool force)
@@ -114,14 +127,8 @@ void pair_prologue(std::ostringstream &os, const std::vector<Fn> &fs, std::vecto
           "            pit_slots(k, it, a, b);\n"
           "            const float4 ua = v.u[a], ub = v.u[b];\n"
           "            const float cs = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;\n";
-    for (const Fn &f : fs) {
-        bool seen = false;
-        for (float x : bases) seen |= (x == f.lf);
-        if (!seen) bases.push_back(f.lf);
-        damps.insert(f.damp);
-    }
-    for (size_t b = 0; b < bases.size(); ++b)
-        os << "            const float x" << b << " = fabsf(fmaf(" << flit(bases[b]) << ", cs, 0.5f));\n";
+    gen_bases(os, fs, bases);
+    for (const Fn &f : fs) damps.insert(f.damp);
     // damping factors: groups 2m and 2m+1 of a neighbour are one float2 (wix)
     std::set<int> pairs;
     for (int d : damps) pairs.insert(d >> 1);
@@ -285,6 +292,103 @@ std::string gen_radial_force_body(const Engine &E, const DevBlockR &B)
     return os.str();
 }
 
+// One pair's values of a block's functions: acc[f] += x^zeta w[d] (w: products
+// of the damping factors of the two neighbours).
+std::string gen_few_symm_body(const Engine &E, const DevBlockA &B)
+{
+    std::ostringstream os, body;
+    const std::vector<Fn> fs = block_fns(E, B);
+    std::vector<float> bases;
+    gen_bases(body, fs, bases);
+    Powers P(body);
+    for (size_t f = 0; f < fs.size(); ++f) {
+        const std::string x = P.power(base_of(bases, fs[f].lf), fs[f].zeta, fs[f].iz);
+        body << "            acc[" << f << "] = fmaf(" << x << ", w[" << fs[f].damp << "], acc[" << f << "]);\n";
+    }
+    os << "        {\n" << body.str() << "            return;\n        }\n";
+    return os.str();
+}
+
+// One pair's dE/dcos and dE/dr of both neighbours from e = dE/dG of the block.
+std::string gen_few_force_body(const Engine &E, const DevBlockA &B)
+{
+    std::ostringstream os, body;
+    const std::vector<Fn> fs = block_fns(E, B);
+    std::vector<float> bases;
+    gen_bases(body, fs, bases);
+    Powers P(body);
+    std::set<int> damps;
+    for (const Fn &f : fs) damps.insert(f.damp);
+    for (int d : damps) body << "            float c" << d << " = 0.f, s" << d << " = 0.f;\n";
+    for (size_t f = 0; f < fs.size(); ++f) {
+        const int b = base_of(bases, fs[f].lf);
+        const std::string d = std::to_string(fs[f].damp), F = std::to_string(f);
+        const std::string pz = P.pw(b, fs[f].iz);
+        body << "            s" << d << " = fmaf(e[" << F << "], " << pz << ", s" << d << ");\n";
+        if (fs[f].iz >= 1) {
+            const std::string pm1 = P.pw(b, fs[f].iz - 1);
+            body << "            c" << d << " = fmaf(e[" << F << "] * " << flit(fs[f].zeta * fs[f].lf) << ", " << pm1 << ", c"
+                 << d << ");\n";
+        }
+    }
+    for (int d : damps)
+        body << "            hc = fmaf(c" << d << ", wa[" << d << "] * wb[" << d << "], hc);\n"
+             << "            ha = fmaf(s" << d << ", wda[" << d << "] * wb[" << d << "], ha);\n"
+             << "            hb = fmaf(s" << d << ", wa[" << d << "] * wdb[" << d << "], hb);\n";
+    os << "        {\n" << body.str() << "            return;\n        }\n";
+    return os.str();
+}
+
+// The potential's cutoffs and, when every centre element has the same ones,
+// its damping factors as literals of the moment kernels (class M of
+// nnp_moments.cuh).
+std::string gen_moment_constants(const Engine &E)
+{
+    std::ostringstream os;
+    const DevPot &d = E.dpot;
+    auto pick = [&](const char *type, const char *name, int n, const std::function<std::string(int)> &v) {
+        os << "    __device__ static constexpr " << type << " " << name << "(int k) { return ";
+        for (int k = 0; k + 1 < n; ++k) os << "k == " << k << " ? " << v(k) << " : ";
+        os << v(n - 1) << "; }\n";
+    };
+    pick("DevCut", "cut", d.ncut, [&](int c) {
+        return "DevCut{" + std::to_string(d.cut[c].name) + ", " + flit(d.cut[c].rc) + ", " + flit(d.cut[c].rci) + ", " +
+               flit(d.cut[c].pirci) + "}";
+    });
+    pick("float", "rci_lo", d.ncut, [&](int c) { return flit((float)(1.0 / E.cut64_host[c] - (double)d.cut[c].rci)); });
+    bool same = true;
+    for (int II = 1; II < d.ntypes; ++II) {
+        same = same && d.t[II].ndamp == d.t[0].ndamp;
+        for (int k = 0; same && k < d.t[0].ndamp; ++k)
+            same = d.t[II].damp_a[k] == d.t[0].damp_a[k] && d.t[II].damp_cut[k] == d.t[0].damp_cut[k] &&
+                   E.mom_a_lo(II, k) == E.mom_a_lo(0, k);
+    }
+    os << "    static constexpr bool SAME = " << (same ? "true" : "false") << ";\n";
+    pick("float", "damp_a", E.mom_ND, [&](int k) { return flit(d.t[0].damp_a[k]); });
+    pick("float", "damp_lo", E.mom_ND, [&](int k) { return flit(E.mom_a_lo(0, k)); });
+    pick("int", "damp_cut", E.mom_ND, [&](int k) { return std::to_string(d.t[0].damp_cut[k]); });
+    return os.str();
+}
+
+// Values of one radial block's functions at a neighbour, (rs, eta) as
+// literals: row[f] = G_f(r) with the block's cutoff value.
+std::string gen_radial_row_body(const Engine &E, const DevBlockR &B)
+{
+    std::ostringstream os;
+    os << "        {\n            const float c = fc[" << B.cut << "];\n";
+    for (int f = 0; f < B.n; ++f) {
+        const float2 q = E.rpar_host[B.par + f];
+        if (B.form == RAD_GAUSSIAN)
+            os << "            { const float g = " << flit(q.y) << " * (r - " << flit(q.x) << "); row[" << f
+               << "] = expf(-g * g) * c; }\n";
+        else
+            os << "            { float d; radial_fd(" << B.form << ", r, " << flit(q.x) << ", " << flit(q.y)
+               << ", c, 0.f, row[" << f << "], d); }\n";
+    }
+    os << "            return;\n        }\n";
+    return os.str();
+}
+
 // Tangent of one GAUSS block's symmetry functions along the displacement
 // field (see tangent_body): per pair dG_f = zeta lf x^(zeta-1) w_a w_b dcos
 // + x^zeta (w'_a w_b rr_a + w_a w'_b rr_b), relative to the block's first
@@ -373,20 +477,28 @@ std::string make_source(const Engine &E, const TuneParams &tp)
     // pairs per chunk of the force kernel; small values split the pair rows
     // between many chunks (used by a test)
     if (tp.force_chunk != NNP_PCH) os << "#define NNP_FORCE_CHUNK " << tp.force_chunk << "\n";
-    os << "#include \"nnp_device.cuh\"\nnamespace nnp {\nstruct JitBlocks {\n";
-    std::vector<std::pair<int, std::string>> sy, fo, ta, ra;
+    os << "#include \"nnp_moments.cuh\"\nnamespace nnp {\nstruct JitBlocks {\n";
+    std::vector<std::pair<int, std::string>> sy, fo, ta, ra, rr, fy, ff;
+    int na = 1;   // angular functions of the largest block
     const int T = E.dpot.ntypes, TT = T * (T + 1) / 2;
     for (int II = 0; II < T; ++II)
         for (int J = 0; J < T; ++J) {
             const DevBlockR &B = E.dpot.t[II].br[J];
             if (B.n > 0 && B.form == RAD_GAUSSIAN) ra.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_force_body(E, B));
+            if (B.n > 0 && E.mom_ok) rr.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_row_body(E, B));
         }
     for (int II = 0; II < T; ++II)
         for (int tt = 0; tt < TT; ++tt) {
             const DevBlockA &B = E.dpot.t[II].ba[tt];
             if (B.n == 0 || B.form != ANG_GAUSS) continue;
-            sy.emplace_back(II * NNP_MAX_TT + tt, gen_symm_body(E, B));
-            fo.emplace_back(II * NNP_MAX_TT + tt, gen_force_body(E, B));
+            na = std::max(na, B.n);
+            if (E.mom_ok) {
+                fy.emplace_back(II * NNP_MAX_TT + tt, gen_few_symm_body(E, B));
+                ff.emplace_back(II * NNP_MAX_TT + tt, gen_few_force_body(E, B));
+            } else {
+                sy.emplace_back(II * NNP_MAX_TT + tt, gen_symm_body(E, B));
+                fo.emplace_back(II * NNP_MAX_TT + tt, gen_force_body(E, B));
+            }
             ta.emplace_back(II * NNP_MAX_TT + tt, gen_tangent_body(E, B));
         }
     os << "    template <typename Acc>\n"
@@ -428,8 +540,79 @@ std::string make_source(const Engine &E, const TuneParams &tp)
     }
     os << "    __device__ static bool tangent(const NbrView &v, int II, int tt, const Blk &k, int cap, int lane, float *Cb)\n"
           "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
-       << group_cases(ta) << "        default: return false;\n        }\n    }\n};\n}  // namespace nnp\n";
-    os << R"(
+       << group_cases(ta) << "        default: return false;\n        }\n    }\n};\n";
+    if (E.mom_ok)
+        os << "struct JitMoments : JitBlocks {\n"
+              "    static constexpr int T = " << T << ", L = " << E.mom_L << ", ND = " << E.mom_ND << ", NR = " << E.mom_NR
+           << ", NA = " << na << ", NCUT = " << E.dpot.ncut << ";\n"
+           << gen_moment_constants(E)
+           << "    __device__ static void radial_row(int II, int t, float r, const float *fc, float *row)\n"
+              "    {\n        switch (II * NNP_MAX_TYPES + t) {\n"
+           << group_cases(rr) << "        default: return;\n        }\n    }\n"
+              "    __device__ static void few_symm(int II, int tt, float cs, const float *w, float *acc)\n"
+              "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
+           << group_cases(fy) << "        default: return;\n        }\n    }\n"
+              "    __device__ static void few_force(int II, int tt, float cs, const float *e, const float *wa, const float *wda,\n"
+              "                                     const float *wb, const float *wdb, float &hc, float &ha, float &hb)\n"
+              "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
+           << group_cases(ff) << "        default: return;\n        }\n    }\n};\n";
+    os << "}  // namespace nnp\n";
+    if (E.mom_ok)
+        os << R"(
+extern "C" __global__ void __launch_bounds__(NNP_MOM_SYMM_WARPS * 32)
+k_symm_jit(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+   const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
+   const int *__restrict__ nbr_cnt, int cap, int gstride, float *__restrict__ G, float2 *mom,
+   unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems)
+{
+    extern __shared__ float4 smem4[];
+    nnp::mom_symm_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, items, nitems,
+        reinterpret_cast<float *>(smem4));
+}
+#define NNP_FORCE_KERNEL(name, na) \
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FORCE_WARPS * 32) \
+name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, \
+     const float2 *__restrict__ rpar, const int *__restrict__ type, const int *__restrict__ order, \
+     const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride, \
+     const float *__restrict__ dEdG, const float2 *__restrict__ mom, const unsigned short *__restrict__ mom_cnt, \
+     const int2 *__restrict__ items, const int *__restrict__ nitems, double *__restrict__ F, nnp::DevErr *err, \
+     const int *__restrict__ atom_struct, double *__restrict__ vir) \
+{ \
+    extern __shared__ float4 smem4[]; \
+    if ((int)blockIdx.x >= nmain) \
+        nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x - nmain, (int)gridDim.x - nmain, \
+            NNP_MOM_FORCE_WARPS * 32, items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, \
+            err, atom_struct, vir); \
+    else \
+        nnp::mom_force_body<nnp::JitMoments, na>(nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr, nbr_cnt, cap, \
+            gstride, dEdG, mom, mom_cnt, F, err, atom_struct, vir, reinterpret_cast<float *>(smem4)); \
+}
+NNP_FORCE_KERNEL(k_force_jit, 1)
+NNP_FORCE_KERNEL(k_force_jit2, 2)
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
+k_symm_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
+           const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+           const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+           const unsigned short *__restrict__ mom_cnt, float *__restrict__ G)
+{
+    nnp::mom_few_symm_body<nnp::JitMoments>(items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, G);
+}
+)";
+    if (E.mom_ok && E.mom_thread())
+        os << R"(
+extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
+k_symm_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+   const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
+   const int *__restrict__ nbr_cnt, int cap, int gstride, float *__restrict__ G, float2 *mom,
+   unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems)
+{
+    extern __shared__ float4 smem4[];
+    nnp::mom_symm_thread_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, items, nitems,
+        reinterpret_cast<float *>(smem4));
+}
+)";
+    if (!E.mom_ok)
+        os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_WARPS * 32, NNP_SYMM_MINB)
 k_symm_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__restrict__ rpar,
            const float4 *__restrict__ apar, const int *__restrict__ type, const int *__restrict__ order,
@@ -454,6 +637,8 @@ k_force_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__re
                                     F, err, reinterpret_cast<float *>(smem4), atom_struct, vir);
 }
 
+)";
+    os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_WARPS * 32, 1)
 k_tangent_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__restrict__ rpar,
               const float4 *__restrict__ apar, const int *__restrict__ type, const int *__restrict__ order,
@@ -477,6 +662,8 @@ void jit_release(Engine &E)
     if (E.jit_module) cudaLibraryUnload((cudaLibrary_t)E.jit_module);
     E.jit_module = nullptr;
     E.jit_symm = E.jit_force = E.jit_tangent = nullptr;
+    E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = nullptr;
+    E.jit_symm_few = nullptr;
 }
 
 std::string &jit_last_log()
@@ -529,7 +716,7 @@ std::string jit_compile_params(const Engine &E, const TuneParams &tp, std::strin
     static std::mutex mu;
     static std::map<uint64_t, std::vector<char>> memo;
     source = make_source(E, tp);
-    const uint64_t key = source_hash(source + kDeviceHeaderSource);
+    const uint64_t key = source_hash(source + kDeviceHeaderSource + kMomentsHeaderSource);
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = memo.find(key);
@@ -552,9 +739,9 @@ std::string jit_compile_params(const Engine &E, const TuneParams &tp, std::strin
         }
     }
     nvrtcProgram prog;
-    const char *hdr_src[1] = {kDeviceHeaderSource};
-    const char *hdr_name[1] = {"nnp_device.cuh"};
-    if (nvrtcCreateProgram(&prog, source.c_str(), "nnp_jit.cu", 1, hdr_src, hdr_name) != NVRTC_SUCCESS)
+    const char *hdr_src[2] = {kDeviceHeaderSource, kMomentsHeaderSource};
+    const char *hdr_name[2] = {"nnp_device.cuh", "nnp_moments.cuh"};
+    if (nvrtcCreateProgram(&prog, source.c_str(), "nnp_jit.cu", 2, hdr_src, hdr_name) != NVRTC_SUCCESS)
         return "nvrtcCreateProgram failed";
     const char *opts[] = {"--gpu-architecture=sm_100a", "-std=c++17", "-lineinfo", "--fmad=true",
                           "--ptxas-options=-v"};
@@ -605,25 +792,30 @@ std::string jit_build(Engine &E)
         cudaGetLastError();
         return "cudaLibraryLoadData failed";
     }
-    cudaKernel_t ks, kf, kt;
-    if (cudaLibraryGetKernel(&ks, lib, "k_symm_jit") != cudaSuccess ||
-        cudaLibraryGetKernel(&kf, lib, "k_force_jit") != cudaSuccess ||
-        cudaLibraryGetKernel(&kt, lib, "k_tangent_jit") != cudaSuccess) {
-        cudaGetLastError();
-        cudaLibraryUnload(lib);
-        return "run-time kernels not found";
-    }
     E.jit_module = (void *)lib;
-    E.jit_symm = (void *)ks;
-    E.jit_force = (void *)kf;
-    E.jit_tangent = (void *)kt;
-    if (std::getenv("NNP_JIT_VERBOSE")) {        // registers and local memory of the compiled kernels
-        const char *names[3] = {"k_symm_jit", "k_force_jit", "k_tangent_jit"};
-        const void *fns[3] = {(const void *)ks, (const void *)kf, (const void *)kt};
-        for (int q = 0; q < 3; ++q) {
+    std::vector<std::pair<const char *, void **>> fns = {{"k_tangent_jit", &E.jit_tangent}};
+    if (E.mom_ok) {
+        fns.push_back({"k_symm_jit", &E.jit_symm_mom});
+        if (E.mom_thread()) fns.push_back({"k_symm_jit_t", &E.jit_symm_momt});
+        fns.push_back({"k_force_jit", &E.jit_force_mom1});
+        fns.push_back({"k_force_jit2", &E.jit_force_mom2});
+        fns.push_back({"k_symm_few", &E.jit_symm_few});
+    } else {
+        fns.push_back({"k_symm_jit", &E.jit_symm});
+        fns.push_back({"k_force_jit", &E.jit_force});
+    }
+    for (auto &f : fns) {
+        cudaKernel_t k;
+        if (cudaLibraryGetKernel(&k, lib, f.first) != cudaSuccess) {
+            cudaGetLastError();
+            jit_release(E);
+            return "run-time kernels not found";
+        }
+        *f.second = (void *)k;
+        if (std::getenv("NNP_JIT_VERBOSE")) {    // registers and local memory of the compiled kernels
             cudaFuncAttributes a;
-            if (cudaFuncGetAttributes(&a, fns[q]) == cudaSuccess)
-                std::fprintf(stderr, "nnp jit: %s %d registers, %zu bytes local memory\n", names[q], a.numRegs,
+            if (cudaFuncGetAttributes(&a, (const void *)k) == cudaSuccess)
+                std::fprintf(stderr, "nnp jit: %s %d registers, %zu bytes local memory\n", f.first, a.numRegs,
                              a.localSizeBytes);
             else
                 cudaGetLastError();

@@ -1355,10 +1355,85 @@ std::string run_neighbors(Engine &E, int pbc)
     return cuda_msg("neighbour list");
 }
 
+// Moments of the batch: rows for all its centres when they fit NNP_MOM_BYTES
+// (and the device's free memory), else for as many as do; the force stage then
+// recomputes them part by part.
+#define NNP_MOM_BYTES ((size_t)8 << 30)
+static std::string mom_reserve(Engine &E)
+{
+    const size_t vals = mom_vals(E.dpot.ntypes, E.mom_ND, E.mom_L);
+    const int64_t most = (int64_t)(NNP_MOM_BYTES / (vals * sizeof(float2))) & ~(int64_t)3;
+    int64_t rows = std::min<int64_t>((E.n_centre + 3) & ~(int64_t)3, most);
+    cudaError_t e = E.mom.reserve((size_t)rows * vals);
+    while (e != cudaSuccess && rows > 4096) {
+        cudaGetLastError();
+        rows = (rows / 4) & ~(int64_t)3;
+        e = E.mom.reserve((size_t)rows * vals);
+    }
+    if (e == cudaSuccess) e = E.mom_cnt.reserve(8 * (size_t)rows);
+    if (e == cudaSuccess) e = E.mom_items.reserve((size_t)rows * (E.dpot.ntypes * (E.dpot.ntypes + 1) / 2));
+    E.mom_rows = rows;
+    return e == cudaSuccess ? "" : std::string("device allocation failed: ") + cudaGetErrorString(e);
+}
+
+#define NNP_MOM_THREAD_MIN 40000   // atoms from which a thread per atom is faster than a warp
+#define NNP_MOM_PAIR_MIN 20000     // atoms from which two atoms per warp are faster than one
+
+// Moments of atoms order[lo .. hi) and, unless G is NULL, symmetry functions.
+// first: the list of few-pair blocks is empty (cleared with the error record).
+static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, bool first)
+{
+    const int T = E.dpot.ntypes;
+    long long l = lo, h = hi;
+    int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
+    int *nitems = &E.err.p->few;
+    if (!first) cudaMemsetAsync(nitems, 0, sizeof(int), E.stream);
+    void *args[] = {&l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &E.order.p, &E.nbr.p, &E.nbr_cnt.p,
+                    &cap, &gs, &G, &E.mom.p, &E.mom_cnt.p, &E.mom_items.p, &nitems};
+    E.launches += 1;
+    if (!E.jit_symm_momt || hi - lo < NNP_MOM_THREAD_MIN) {
+        const size_t sm = (size_t)NNP_MOM_SYMM_WARPS * mom_symm_floats(T, E.mom_ND, E.mom_L, E.mom_NR, E.gstride) * sizeof(float);
+        return jit_launch(E.jit_symm_mom, grid_for(hi - lo, NNP_MOM_SYMM_WARPS, num_sms() * 64), NNP_MOM_SYMM_WARPS * 32, sm,
+                          E.stream, args);
+    }
+    std::string msg = jit_launch(E.jit_symm_momt, grid_for(hi - lo, NNP_MOM_THREADS, 1 << 30), NNP_MOM_THREADS,
+                                 mom_thread_floats(T, E.mom_ND, E.mom_L) * sizeof(float), E.stream, args);
+    if (!msg.empty() || !G) return msg;
+    void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &E.order.p, &E.nbr.p, &cap, &gs,
+                   &E.mom_cnt.p, &G};
+    E.launches += 1;
+    return jit_launch(E.jit_symm_few, num_sms() * 8, NNP_MOM_FEW_THREADS, 0, E.stream, few);
+}
+
+static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *vir)
+{
+    const int T = E.dpot.ntypes, na = (!vir && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
+    const size_t sm = (size_t)na * NNP_MOM_FORCE_WARPS * mom_force_floats(T, E.mom_ND, E.mom_L, E.gstride) * sizeof(float);
+    long long l = lo, h = hi;
+    int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
+    int nmain = grid_for(hi - lo, na * NNP_MOM_FORCE_WARPS, num_sms() * 32);
+    const int nfew = grid_for((hi - lo) * T * (T + 1) / 2, NNP_MOM_FORCE_WARPS * 2, num_sms() * 4);
+    const int *nitems = &E.err.p->few;
+    void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &E.order.p, &E.nbr.p, &E.nbr_cnt.p,
+                    &cap, &gs, &E.dEdG.p, &E.mom.p, &E.mom_cnt.p, &E.mom_items.p, &nitems, &E.force.p, &E.err.p,
+                    &E.atom_struct.p, &vir};
+    E.launches += 1;
+    return jit_launch(na == 2 ? E.jit_force_mom2 : E.jit_force_mom1, nmain + nfew, NNP_MOM_FORCE_WARPS * 32, sm, E.stream, args);
+}
+
 std::string run_symm(Engine &E)
 {
     const int64_t N = E.n_centre;      // centres: the first n_centre entries of `order`
+    E.mom_valid = false;
     if (N == 0) return "";
+    if (E.use_jit && E.jit_symm_mom && !E.acc64 && !E.symm64) {
+        std::string msg = mom_reserve(E);
+        for (int64_t lo = 0; lo < N && msg.empty(); lo += E.mom_rows)
+            msg = launch_symm_mom(E, lo, std::min(N, lo + E.mom_rows), E.G.p, lo == 0);
+        E.mom_valid = E.mom_rows >= N;
+        E.mark(2);
+        return msg;
+    }
     const size_t sm = view_bytes(E, false, false);
     const int grid = grid_for(N, WARPS, num_sms() * 16);
     E.launches += 1;
@@ -1421,6 +1496,22 @@ std::string run_force(Engine &E)
     cudaMemsetAsync(E.force.p, 0, 3 * (size_t)E.n_atoms * sizeof(double), E.stream);
     double *vir = E.want_virial ? E.vir.p : nullptr;
     if (vir) cudaMemsetAsync(vir, 0, 9 * (size_t)E.n_struct * sizeof(double), E.stream);
+    if (E.use_jit && E.jit_force_mom1) {
+        std::string msg;
+        if (E.mom_valid) {
+            msg = launch_force_mom(E, 0, N, vir);
+        } else if (N > 0) {
+            // moments not kept by the symmetry functions (FP64 ones, or more rows than memory): part by part
+            msg = mom_reserve(E);
+            for (int64_t lo = 0; lo < N && msg.empty(); lo += E.mom_rows) {
+                const int64_t hi = std::min(N, lo + E.mom_rows);
+                msg = launch_symm_mom(E, lo, hi, nullptr, false);
+                if (msg.empty()) msg = launch_force_mom(E, lo, hi, vir);
+            }
+        }
+        E.mark(4);
+        return msg;
+    }
     const size_t sm = view_bytes(E, true, E.use_jit && E.jit_force);
     const int grid = grid_for(N, WARPS, num_sms() * 16);
     E.launches += 1;

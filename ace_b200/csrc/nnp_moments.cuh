@@ -1,0 +1,1107 @@
+// nnp_moments.cuh -- symmetry functions and forces of GAUSS angular blocks
+// with integer zeta through moments of the neighbours' directions.
+//
+// A GAUSS angular function is (0.5 + lambda/2 cos)^zeta w_d(r_a) w_d(r_b)
+// summed over the pairs (a, b) of two neighbour elements, w_d(r) = fc(r)
+// exp(-a_d r^2) (BasisA::symmf, src/nnp/basis_angular.cpp:212-260).  For
+// integer zeta <= L the power is a polynomial in cos = u_a . u_b; expanded in
+// Legendre polynomials, sum_l c_l P_l(u_a . u_b), each P_l splits by the
+// addition theorem into products of one neighbour's functions, so the sum
+// over pairs becomes one over neighbours:
+//   A^J_{lm,d} = sum_{a in J} w_d(r_a) Y_lm(u_a)            (moments)
+//   S^{JK}_{l,d} = sum_m A^J_{lm,d} A^K_{lm,d}
+//   G_f = sum_l c_{f,l} S^{JK}_{l,d}                          (J != K)
+//   G_f = (sum_l c_{f,l} S^{JJ}_{l,d} - f_f(1) sum_a w_d^2) / 2   (J == K:
+//         the sum over ordered pairs without the pairs of a slot with itself)
+// and with e_f = dE/dG_f the derivative of the energy with respect to a
+// neighbour's displacement is that of sum_d w_d(r) sum_lm B^J_{lm,d} Y_lm(u),
+//   B^J_{lm,d} = sum_K (sum_f e_f c_{f,l} [1 + (J == K)]) A^K_{lm,d},
+// so neither pass visits pairs.  A pair term costs ~80 instructions in the
+// force pass and an atom of the batched workload has 1000 pairs; a neighbour
+// (45 per atom) costs ~500 there and ~400 in the symmetry functions.
+//
+// The moment form's rounding error is ~1e-7 of (sum w)^2, a pair sum's ~1e-7 of
+// the sum itself.  With few pairs the sum can be any fraction of (sum w)^2 (two
+// neighbours on opposite sides of the centre: ((1 + cos)/2)^8 ~ 0); above 15
+// pairs (six neighbours of one element) it is below 1/64 of it for under 10 %
+// of the blocks of the batched workloads and never below 1/1000.  So blocks of
+// at most NNP_MOM_FEW pairs are summed pair by pair (mom_few_symm,
+// mom_few_force_body), 16 lanes each, from a list that the symmetry functions
+// append to.
+//
+// Y_lm(u) = Q_lm(z) Re/Im (x + i y)^m with Q_lm the monic polynomial
+// proportional to d^m P_l / dz^m: Q_{l+1,m} = z Q_lm - beta_lm Q_{l-1,m},
+// beta_lm = (l^2 - m^2) / (4 l^2 - 1), and dQ_lm/dz = (l - m) Q_{l,m+1}.
+// The factors N_lm that make sum_m N_lm^2 Y_lm Y_lm = P_l multiply the sums.
+//
+// Plain CUDA C++ for NVRTC, like nnp_device.cuh.  The class M (written by
+// nnp_jit.cpp) gives the potential's sizes and its radial functions:
+//   T elements, L largest zeta, ND damping factors per centre element,
+//   NR radial and NA angular functions of the largest block, NCUT cutoffs,
+//   cut(c), rci_lo(c): cutoff c and the low part of its 1/rc,
+//   SAME: every centre element has the same damping factors, and then
+//   damp_a(d), damp_lo(d), damp_cut(d): exponent (high and low part) and cutoff,
+//   radial_row(II, t, r, fc, row): values of the radial functions of a
+//   neighbour of element t, radial_force(II, t, r, fc, fcd, eb, out): sum of
+//   eb_f dG_f/dr, few_symm(II, tt, cs, w, acc): acc_f += x_f^zeta w_d,
+//   few_force(II, tt, cs, e, wa, wda, wb, wdb, hc, ha, hb): dE/dcos, dE/dr_a and
+//   dE/dr_b of one pair.
+#pragma once
+
+#include "nnp_device.cuh"
+
+#define NNP_MOM_MAXL 8        // largest zeta taken (above, a moment set is larger than the pairs it replaces)
+#define NNP_MOM_MAXD 4        // damping factors of one centre element
+#define NNP_MOM_SYMM_WARPS 2  // warps per block, symmetry functions with a warp per atom (15 KB of shared memory each)
+#define NNP_MOM_THREADS 128   // threads per block, symmetry functions with a thread per atom
+#define NNP_MOM_THREAD_T 4    // most elements of that form (its sums of pairs of elements are unrolled)
+#define NNP_MOM_FORCE_WARPS 4 // warps per block, forces
+#define NNP_MOM_FEW 15        // blocks of at most this many pairs are summed pair by pair
+#define NNP_MOM_FEW_THREADS 128
+
+namespace nnp {
+
+// Components of one (element, damping pair): m = 0 first (l = 0..L, padded to
+// an even count), then for m = 1..L and l = m..L the cos and sin parts side by
+// side, so that one 16-byte load reads both parts for two damping factors.
+NNP_HD constexpr int mom_m0(int L) { return (L + 2) & ~1; }
+NNP_HD constexpr int mom_base(int L, int m)   // first component of m >= 1
+{
+    return mom_m0(L) + 2 * ((m - 1) * (L + 1) - (m * (m - 1)) / 2);
+}
+NNP_HD constexpr int mom_comps(int L) { return mom_base(L, L) + 2; }
+
+// Moments in memory: component k = ((element * pairs of damping factors) + pair)
+// * comps + component of row r (the r-th atom of the visiting order) is the
+// float2 at mom_at(r, k): four rows interleaved, so that a thread per row writes
+// whole 32-byte sectors and so does a warp that reads one row's components
+// next to its neighbours'.  mom_cnt holds 8 neighbour counts (by element) per
+// row, mom_items the (row, block) entries of few pairs (their number: DevErr::few).
+NNP_HD constexpr int mom_vals(int T, int ND, int L) { return T * ((ND + 1) / 2) * mom_comps(L); }
+NNP_HD inline i64 mom_at(i64 r, int k, int vals) { return ((r >> 2) * vals + k) * 4 + (r & 3); }
+
+// pairs of block (J, K) of an atom
+NNP_HD inline int mom_pairs(const unsigned short *cnt, int J, int K)
+{
+    return J == K ? cnt[J] * (cnt[J] - 1) / 2 : cnt[J] * cnt[K];
+}
+
+// Table of a potential (floats, nnp_api.cu):
+//   norm[comps] (factors of the monic Y_lm; 0 at the padding),
+//   fnorm[comps] (factors of d^m P_l / dz^m), deg[comps] (l, as int),
+//   per element: low parts of the damping exponents [NNP_MOM_MAXD],
+//   per element and angular function f, [L + 2][fmax]: coefficients c_0 .. c_L
+//   (halved for J == K), then f(1)/2 for J == K and 0 otherwise,
+//   per element and function, as int: tt | d << 8 | J << 16 | K << 24
+struct MomTab {
+    const float *norm, *fnorm;
+    const int *deg;
+    const float *a_lo;
+    const float *coef;
+    const int *fun;
+    int fmax;
+};
+
+NNP_HD inline int mom_tab_floats(int T, int L, int fmax)
+{
+    return 3 * mom_comps(L) + T * NNP_MOM_MAXD + T * fmax * (L + 3);
+}
+
+NNP_HD inline MomTab mom_tab(const float *p, int T, int L, int fmax)
+{
+    MomTab t;
+    t.norm = p; p += mom_comps(L);
+    t.fnorm = p; p += mom_comps(L);
+    t.deg = reinterpret_cast<const int *>(p); p += mom_comps(L);
+    t.a_lo = p; p += T * NNP_MOM_MAXD;
+    t.coef = p; p += T * fmax * (L + 2);
+    t.fun = reinterpret_cast<const int *>(p);
+    t.fmax = fmax;
+    return t;
+}
+
+// Shared memory of one warp.  Symmetry functions: 32 neighbour rows of
+// mom_stage floats (odd stride: lanes write their rows without bank
+// conflicts), damping factors per row, moments, sums of w_d^2, S, G row.
+NNP_HD constexpr int mom_stage(int L, int NR, int ND) { return (mom_comps(L) + NR + ND) | 1; }
+NNP_HD constexpr int mom_s_vals(int T, int ND, int L) { return T * (T + 1) / 2 * ((ND + 1) / 2) * (L + 1); }
+NNP_HD constexpr int mom_symm_floats(int T, int ND, int L, int NR, int gstride)
+{
+    return ((32 * mom_stage(L, NR, ND) + 3) & ~3) + 64 * ((ND + 1) / 2) + 2 * mom_vals(T, ND, L) + T * NNP_MOM_MAXD +
+           ((2 * mom_s_vals(T, ND, L) + 3) & ~3) + gstride + 4;
+}
+// One thread per atom: S and the sums of w_d^2 of its NNP_MOM_THREADS threads.
+NNP_HD constexpr int mom_thread_floats(int T, int ND, int L)
+{
+    return NNP_MOM_THREADS * 2 * (mom_s_vals(T, ND, L) + T * ((ND + 1) / 2));
+}
+// Forces, per atom of a warp's group: B, D, the self terms, the dE/dG row.
+NNP_HD constexpr int mom_force_floats(int T, int ND, int L, int gstride)
+{
+    return 2 * mom_vals(T, ND, L) + ((2 * mom_s_vals(T, ND, L) + 3) & ~3) + T * NNP_MOM_MAXD + gstride;
+}
+
+#if defined(__CUDACC__)
+
+// ---------------------------------------------------------------- packed FP32 pairs
+
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pk2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 dup2(float a) { return pk2(a, a); }
+__device__ __forceinline__ void up2(f32x2 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+NNP_HD constexpr float mom_beta(int l, int m) { return (float)((double)(l * l - m * m) / (double)(4 * l * l - 1)); }
+
+// ---------------------------------------------------------------- one neighbour
+
+// Distance, unit vector, cutoff values and damping factors of a neighbour.
+// The damping factors set the error of the moments, so what FP32 rounding of
+// their arguments would lose is put back to first order: r = r_hi + r_lo
+// from the residual of the square root, 1/rc and the exponents as hi + lo
+// (RMS error of w over a neighbour shell 1.2e-7 -> 0.65e-7).
+template <class M, bool DER>
+struct MomNbr {
+    float ux, uy, uz, r, ir;
+    float fc[M::NCUT], fd[M::NCUT];
+    float w[M::ND], wd[M::ND];
+
+    // Ty: centre element, a_lo: low parts of its damping exponents
+    __device__ __forceinline__ void set(const float4 e, const DevType &Ty, const float *a_lo)
+    {
+        const float r2 = fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z));
+        const float q = rsqrtf(r2);
+        r = r2 * q;
+        const float rlo = 0.5f * q * fmaf(-r, r, r2);
+        ir = fmaf(q * q, rlo, q);
+        ux = e.x * ir;
+        uy = e.y * ir;
+        uz = e.z * ir;
+#pragma unroll
+        for (int c = 0; c < M::NCUT; ++c) {
+            const DevCut C = M::cut(c);
+            cutoff_fg(C, r, fc[c], fd[c]);
+            const float x = r * C.rci;
+            // fc(r + rlo), its argument's rounding and the low part of 1/rc: f += f' rc dx
+            const float dx = fmaf(rlo, C.rci, fmaf(r, M::rci_lo(c), fmaf(r, C.rci, -x)));
+            fc[c] = fmaf(fd[c] * C.rc, dx, fc[c]);
+        }
+#pragma unroll
+        for (int d = 0; d < M::ND; ++d) {
+            w[d] = 0.f;
+            wd[d] = 0.f;
+            if (M::SAME || d < Ty.ndamp) {
+                const float a = M::SAME ? M::damp_a(d) : Ty.damp_a[d], t = -a * r2;
+                float ex = expf(t);
+                ex = fmaf(ex, fmaf(-a, r2, -t) - (M::SAME ? M::damp_lo(d) : a_lo[d]) * r2, ex);
+                const int dc = M::SAME ? M::damp_cut(d) : Ty.damp_cut[d];
+                float f = fc[0], g = fd[0];
+#pragma unroll
+                for (int c = 1; c < M::NCUT; ++c)
+                    if (dc == c) {
+                        f = fc[c];
+                        g = fd[c];
+                    }
+                w[d] = f * ex;
+                if (DER) wd[d] = (g - 2.f * a * r * f) * ex;
+            }
+        }
+    }
+};
+
+// Writes the L-moment functions Y_lm(u) of one neighbour to row (components
+// as mom_base; the padding is not written).
+template <int L>
+__device__ __forceinline__ void mom_harmonics(float x, float y, float z, float *row)
+{
+    float cm = 1.f, sm = 0.f;
+#pragma unroll
+    for (int m = 0; m <= L; ++m) {
+        float q0 = 1.f, q1 = 0.f;
+#pragma unroll
+        for (int l = m; l <= L; ++l) {
+            if (m == 0) {
+                row[l] = q0;
+            } else {
+                row[mom_base(L, m > 0 ? m : 1) + 2 * (l - m)] = q0 * cm;
+                row[mom_base(L, m > 0 ? m : 1) + 2 * (l - m) + 1] = q0 * sm;
+            }
+            const float t = (l == m) ? z * q0 : fmaf(z, q0, -mom_beta(l, m) * q1);
+            q1 = q0;
+            q0 = t;
+        }
+        const float c = cm * x - sm * y, s = sm * x + cm * y;
+        cm = c;
+        sm = s;
+    }
+}
+
+// d^m P_l / dz^m for l = m .. L (both halves equal):
+// (l + 1 - m) Q_{l+1} = (2l + 1) z Q_l - (l + m) Q_{l-1}, Q_mm = (2m - 1)!!.
+template <int L, int m>
+__device__ __forceinline__ void mom_polys(float z, f32x2 *q)
+{
+    float q0 = 1.f, q1 = 0.f;
+#pragma unroll
+    for (int k = 1; k < 2 * m; k += 2) q0 *= (float)k;
+#pragma unroll
+    for (int l = m; l <= L; ++l) {
+        q[l] = dup2(q0);
+        const float a = (float)(2 * l + 1) / (float)(l + 1 - m), b = (float)(l + m) / (float)(l + 1 - m);
+        const float t = (l == m) ? a * z * q0 : fmaf(a, z * q0, -b * q1);
+        q1 = q0;
+        q0 = t;
+    }
+}
+
+// Value V and gradient (X, Y, Z) of sum_lm B_lm Q_lm(z) Re/Im (x + i y)^m for
+// each damping factor: the terms of m and above, qa = Q_{l,m}, (cm, sm) = (x +
+// i y)^m, (cp, sp) = (x + i y)^(m - 1).
+template <int L, int NDP, int m>
+__device__ __forceinline__ void mom_gradient(const ulonglong2 *B, float x, float y, float z, const f32x2 *qa, float cm,
+                                             float sm, float cp, float sp, f32x2 *V, f32x2 *X, f32x2 *Y, f32x2 *Z)
+{
+    constexpr int NC = mom_comps(L);
+    f32x2 qb[L + 2];
+    if constexpr (m < L) mom_polys<L, m + 1>(z, qb);
+#pragma unroll
+    for (int p = 0; p < NDP; ++p) {
+        f32x2 C = 0ull, S = 0ull, Cz = 0ull, Sz = 0ull;
+        if constexpr (m == 0) {
+#pragma unroll
+            for (int l = 0; l <= L; l += 2) {
+                const ulonglong2 b = B[(p * NC + l) / 2];
+                C = fma2(b.x, qa[l], C);
+                if (l > 0) Cz = fma2(b.x, qb[l], Cz);
+                if (l + 1 <= L) {
+                    C = fma2(b.y, qa[l + 1], C);
+                    Cz = fma2(b.y, qb[l + 1], Cz);
+                }
+            }
+            V[p] = C;
+            X[p] = Y[p] = 0ull;
+            Z[p] = Cz;
+        } else {
+#pragma unroll
+            for (int l = m; l <= L; ++l) {
+                const ulonglong2 b = B[(p * NC + mom_base(L, m)) / 2 + (l - m)];
+                C = fma2(b.x, qa[l], C);
+                S = fma2(b.y, qa[l], S);
+                if (l > m) {
+                    Cz = fma2(b.x, qb[l], Cz);
+                    Sz = fma2(b.y, qb[l], Sz);
+                }
+            }
+            const f32x2 c2 = dup2(cm), s2 = dup2(sm), mc = dup2((float)m * cp), ms = dup2((float)m * sp),
+                        nms = dup2(-(float)m * sp);
+            V[p] = fma2(C, c2, fma2(S, s2, V[p]));
+            X[p] = fma2(C, mc, fma2(S, ms, X[p]));
+            Y[p] = fma2(C, nms, fma2(S, mc, Y[p]));
+            if (m < L) Z[p] = fma2(Cz, c2, fma2(Sz, s2, Z[p]));
+        }
+    }
+    if constexpr (m < L)
+        mom_gradient<L, NDP, m + 1>(B, x, y, z, qb, cm * x - sm * y, sm * x + cm * y, cm, sm, V, X, Y, Z);
+}
+
+// ---------------------------------------------------------------- blocks of few pairs
+
+// Block (J, K) of few pairs as 16 lanes see it: lane h < no owns neighbour slot
+// so + h of the larger element (J == K: of the element), every owner meets the
+// np <= 5 slots sp .. of the other (J == K: the others).
+struct MomFew {
+    int J, K, so, no, sp, np;
+};
+
+__device__ __forceinline__ MomFew mom_few(const unsigned short *cnt, int T, int tt)
+{
+    MomFew b;
+    b.K = 0;
+    for (int k = 1; k < T; ++k) b.K += tt >= k * (k + 1) / 2;
+    b.J = tt - b.K * (b.K + 1) / 2;
+    const int big = cnt[b.J] >= cnt[b.K] ? b.J : b.K, other = b.J + b.K - big;
+    b.so = b.sp = 0;
+    for (int k = 0; k < big; ++k) b.so += cnt[k];
+    for (int k = 0; k < other; ++k) b.sp += cnt[k];
+    b.no = cnt[big];
+    b.np = cnt[other];
+    return b;
+}
+
+// Symmetry functions of block tt by the 16 lanes `mask` (h: lane among them),
+// to Gb (the block's functions).  src: the atom's records.
+template <class M>
+__device__ __forceinline__ void mom_few_symm(unsigned mask, int h, const float4 *__restrict__ src,
+                                             const unsigned short *cnt, const DevType &Ty, int II, int tt,
+                                             const float *a_lo, float *Gb)
+{
+    const MomFew b = mom_few(cnt, M::T, tt);
+    MomNbr<M, false> v, o;
+    v.set(src[b.so + min(h, b.no - 1)], Ty, a_lo);
+    if (b.J != b.K) o.set(src[b.sp + min(h, b.np - 1)], Ty, a_lo);
+    else o = v;
+    float acc[M::NA];
+#pragma unroll
+    for (int f = 0; f < M::NA; ++f) acc[f] = 0.f;
+#pragma unroll 1
+    for (int k = 0; k < b.np; ++k) {
+        const float cs = v.ux * __shfl_sync(mask, o.ux, k, 16) + v.uy * __shfl_sync(mask, o.uy, k, 16) +
+                         v.uz * __shfl_sync(mask, o.uz, k, 16);
+        float w[M::ND];
+#pragma unroll
+        for (int d = 0; d < M::ND; ++d) w[d] = v.w[d] * __shfl_sync(mask, o.w[d], k, 16);
+        if (h < b.no && (b.J != b.K || k > h)) M::few_symm(II, tt, cs, w, acc);
+    }
+    const int n = Ty.ba[tt].n;
+#pragma unroll
+    for (int f = 0; f < M::NA; ++f) {
+        float s = acc[f];
+#pragma unroll
+        for (int q = 8; q; q >>= 1) s += __shfl_xor_sync(mask, s, q, 16);
+        if (h == 0 && f < n) Gb[f] = s;
+    }
+}
+
+// Symmetry functions of the listed blocks (thread-per-atom form), 16 lanes each.
+template <class M>
+__device__ void mom_few_symm_body(const int2 *__restrict__ items, const int *__restrict__ nitems, i64 lo,
+                                  const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+                                  const int *__restrict__ type, const int *__restrict__ order,
+                                  const float4 *__restrict__ nbr, int cap, int gstride,
+                                  const unsigned short *__restrict__ mom_cnt, float *__restrict__ G)
+{
+    const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
+    const int n = *nitems, h = threadIdx.x & 15;
+    const unsigned mask = 0xffffu << (threadIdx.x & 16);
+    for (int q = (blockIdx.x * NNP_MOM_FEW_THREADS + threadIdx.x) >> 4; q < n; q += gridDim.x * (NNP_MOM_FEW_THREADS / 16)) {
+        const int2 it = items[q];
+        const i64 i = order[lo + it.x];
+        const int II = type[i];
+        const DevType &Ty = pot->t[II];
+        mom_few_symm<M>(mask, h, nbr + i * cap, mom_cnt + 8 * (i64)it.x, Ty, II, it.y, tb.a_lo + II * NNP_MOM_MAXD,
+                        G + i * gstride + Ty.ba[it.y].off_g);
+    }
+}
+
+// Forces of the listed blocks, 16 lanes each: an owner evaluates its pairs; for
+// J != K the partner's gradient is summed over the owners, for J == K every
+// pair is evaluated from both sides.
+template <class M>
+__device__ void mom_few_force_body(int block, int nblock, int threads, const int2 *__restrict__ items,
+                                   const int *__restrict__ nitems, i64 lo, const DevPot *__restrict__ pot,
+                                   const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+                                   const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+                                   const unsigned short *__restrict__ mom_cnt, const float *__restrict__ dEdG,
+                                   double *__restrict__ F, DevErr *err, const int *__restrict__ atom_struct,
+                                   double *__restrict__ vir)
+{
+    const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
+    const int n = *nitems, h = threadIdx.x & 15;
+    const unsigned mask = 0xffffu << (threadIdx.x & 16);
+    for (int q = (block * threads + (int)threadIdx.x) >> 4; q < n; q += nblock * (threads / 16)) {
+        const int2 it = items[q];
+        const i64 i = order[lo + it.x];
+        const int II = type[i], tt = it.y;
+        const DevType &Ty = pot->t[II];
+        const MomFew b = mom_few(mom_cnt + 8 * (i64)it.x, M::T, tt);
+        const float4 *src = nbr + i * cap;
+        const float *a_lo = tb.a_lo + II * NNP_MOM_MAXD, *e = dEdG + i * gstride + Ty.ba[tt].off_g;
+        MomNbr<M, true> v, o;
+        const float4 rv = src[b.so + min(h, b.no - 1)], ro = src[b.sp + min(h, b.np - 1)];
+        v.set(rv, Ty, a_lo);
+        if (b.J != b.K) o.set(ro, Ty, a_lo);
+        else o = v;
+        float g[3] = {0.f, 0.f, 0.f}, p[3] = {0.f, 0.f, 0.f};   // gradient at the lane's owner, at partner h
+#pragma unroll 1
+        for (int k = 0; k < b.np; ++k) {
+            const float px = __shfl_sync(mask, o.ux, k, 16), py = __shfl_sync(mask, o.uy, k, 16),
+                        pz = __shfl_sync(mask, o.uz, k, 16), pir = __shfl_sync(mask, o.ir, k, 16);
+            float w[M::ND], wd[M::ND];
+#pragma unroll
+            for (int d = 0; d < M::ND; ++d) {
+                w[d] = __shfl_sync(mask, o.w[d], k, 16);
+                wd[d] = __shfl_sync(mask, o.wd[d], k, 16);
+            }
+            const float cs = v.ux * px + v.uy * py + v.uz * pz;
+            float hc = 0.f, ha = 0.f, hb = 0.f;                  // dE/dcos, dE/dr of owner and partner
+            if (h < b.no && (b.J != b.K || k != h)) M::few_force(II, tt, cs, e, v.w, v.wd, w, wd, hc, ha, hb);
+            const float t = hc * v.ir, s = ha - t * cs;          // dcos/dd_a = (u_b - cos u_a) / r_a
+            g[0] = fmaf(s, v.ux, fmaf(t, px, g[0]));
+            g[1] = fmaf(s, v.uy, fmaf(t, py, g[1]));
+            g[2] = fmaf(s, v.uz, fmaf(t, pz, g[2]));
+            if (b.J != b.K) {
+                const float tp = hc * pir, sp = hb - tp * cs;
+                float c[3] = {fmaf(sp, px, tp * v.ux), fmaf(sp, py, tp * v.uy), fmaf(sp, pz, tp * v.uz)};
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+#pragma unroll
+                    for (int r = 8; r; r >>= 1) c[x] += __shfl_xor_sync(mask, c[x], r, 16);
+                    if (h == k) p[x] = c[x];
+                }
+            }
+        }
+        const bool own = h < b.no, par = b.J != b.K && h < b.np;
+        const i64 ja = __float_as_int(rv.w) & 0x0fffffff, jb = __float_as_int(ro.w) & 0x0fffffff;
+        bool bad = false;
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            bad |= (own && !(fabsf(g[x]) <= 3.402823466e38f)) || (par && !(fabsf(p[x]) <= 3.402823466e38f));
+            if (own) atomicAdd(&F[3 * ja + x], (double)g[x]);
+            if (par) atomicAdd(&F[3 * jb + x], (double)p[x]);
+            double f = (own ? (double)g[x] : 0.0) + (par ? (double)p[x] : 0.0);
+#pragma unroll
+            for (int r = 8; r; r >>= 1) f += __shfl_xor_sync(mask, f, r, 16);
+            if (h == x) atomicAdd(&F[3 * i + x], -f);
+        }
+        if (vir) {
+            double *ws = vir + 9 * (i64)atom_struct[i];
+            const double da[3] = {rv.x, rv.y, rv.z}, db[3] = {ro.x, ro.y, ro.z};
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+#pragma unroll
+                for (int y = 0; y < 3; ++y) {
+                    double w = -((own ? (double)g[x] * da[y] : 0.0) + (par ? (double)p[x] * db[y] : 0.0));
+#pragma unroll
+                    for (int r = 8; r; r >>= 1) w += __shfl_xor_sync(mask, w, r, 16);
+                    if (h == 0) atomicAdd(ws + 3 * x + y, w);
+                }
+        }
+        if (bad) atomicMax(&err->nonfinite, 1);
+    }
+}
+
+// ---------------------------------------------------------------- symmetry functions
+
+// G_f of one angular function from S (float2 [tt][pair][l], stride ss between
+// entries) and the sum of w_d^2; a block of few pairs is 0 here.
+template <int L, int NDP>
+__device__ __forceinline__ float mom_function(const MomTab &tb, int fu, const float *cf, const float2 *S, int ss,
+                                             const float *w2, const unsigned short *cnt)
+{
+    const int tt = fu & 0xff, d = (fu >> 8) & 0xff;
+    if (mom_pairs(cnt, (fu >> 16) & 0xff, (fu >> 24) & 0xff) <= NNP_MOM_FEW) return 0.f;
+    const float2 *s = S + (i64)((tt * NDP + (d >> 1)) * (L + 1)) * ss;
+    float g = 0.f;
+#pragma unroll
+    for (int l = L; l >= 0; --l) g = fmaf(cf[l * tb.fmax], (d & 1) ? s[l * ss].y : s[l * ss].x, g);
+    return fmaf(-cf[(L + 1) * tb.fmax], *w2, g);
+}
+
+// appends block tt of row r to the list when it has few pairs
+template <int T>
+__device__ __forceinline__ void mom_push(int2 *items, int *nitems, i64 r, int tt, const unsigned short *cnt)
+{
+    int K = 0;
+#pragma unroll
+    for (int k = 1; k < T; ++k) K += tt >= k * (k + 1) / 2;
+    const int np = mom_pairs(cnt, tt - K * (K + 1) / 2, K);
+    if (np > 0 && np <= NNP_MOM_FEW) items[atomicAdd(nitems, 1)] = make_int2((int)r, tt);
+}
+
+// Symmetry functions of atoms order[lo .. hi) and their moments (row idx - lo),
+// one warp per atom (NNP::compute_symm, src/nnp/nnp.cpp:350-392): for batches
+// too small to fill the GPU with a thread per atom.
+// Lane = neighbour for the geometry, the radial functions, the damping factors
+// and the Y_lm, which it leaves as a row in shared memory; then lane =
+// component for the sums over the rows of each neighbour element (the rows are
+// grouped by element), radial functions and w_d as further components.  Sums
+// run in two chains per 32-row chunk; that of Y_00, whose terms all have one
+// sign and whose rounding sets the error of G, is a shuffle tree.  G may be
+// NULL (moments only).
+// Bound: shared-memory wavefronts of the rows and instruction issue.
+template <class M>
+__device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+                              const int *__restrict__ type, const int *__restrict__ order,
+                              const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride,
+                              float *__restrict__ G, float2 *__restrict__ mom, unsigned short *__restrict__ mom_cnt,
+                              int2 *__restrict__ items, int *__restrict__ nitems, float *smem)
+{
+    constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
+                  NR = M::NR, ROW = mom_stage(L, NR, ND), NQ = (NC + NR + ND + 31) / 32,
+                  NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float *rows = smem + (size_t)warp * mom_symm_floats(T, ND, L, NR, gstride);
+    float *W = rows + ((32 * ROW + 3) & ~3);                     // [32][2 NDP]
+    float *A = W + 64 * NDP;                                     // [T][NDP][NC] float2
+    float *W2 = A + 2 * NV;                                      // [T][NNP_MOM_MAXD]
+    float *S = W2 + T * NNP_MOM_MAXD;
+    float *Gs = S + ((NS * 2 + 3) & ~3);
+    unsigned short *cnt = reinterpret_cast<unsigned short *>(Gs + gstride);   // [8]
+    const DevPot &P = *pot;
+    const MomTab tb = mom_tab(tab, T, L, fmax);
+    float nl[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) nl[q] = (lane + 32 * q < NC) ? tb.norm[lane + 32 * q] : 0.f;
+    // the padding component and unused radial slots of the rows stay 0
+    for (int k = lane; k < 32 * ROW; k += 32) rows[k] = 0.f;
+    __syncwarp();
+    for (i64 idx = lo + blockIdx.x * (i64)NNP_MOM_SYMM_WARPS + warp; idx < hi; idx += (i64)gridDim.x * NNP_MOM_SYMM_WARPS) {
+        const i64 i = order[idx];
+        const int II = type[i], n = nbr_cnt[i];
+        if ((unsigned)II >= (unsigned)T) continue;               // type out of range (reported by the call)
+        const DevType &Ty = P.t[II];
+        const float4 *src = nbr + i * cap;
+        for (int k = lane; 4 * k < 2 * NV + T * NNP_MOM_MAXD; k += 32)
+            reinterpret_cast<float4 *>(A)[k] = make_float4(0.f, 0.f, 0.f, 0.f);   // A, W2
+        for (int k = lane; 4 * k < gstride + 4; k += 32)          // G row, counts
+            reinterpret_cast<float4 *>(Gs)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+        for (int kb = 0; kb < n; kb += 32) {
+            int t = T;
+            float w[2 * NDP];
+#pragma unroll
+            for (int d = 0; d < 2 * NDP; ++d) w[d] = 0.f;
+            if (kb + lane < n) {
+                const float4 e = src[kb + lane];
+                t = (int)((unsigned)__float_as_int(e.w) >> 28);
+                MomNbr<M, false> v;
+                v.set(e, Ty, tb.a_lo + II * NNP_MOM_MAXD);
+                float *row = rows + lane * ROW;
+                mom_harmonics<L>(v.ux, v.uy, v.uz, row);
+                M::radial_row(II, t, v.r, v.fc, row + NC);
+#pragma unroll
+                for (int d = 0; d < 2 * NDP; ++d) {
+                    if (d < ND) row[NC + NR + d] = w[d] = v.w[d < ND ? d : 0];
+                    W[lane * 2 * NDP + d] = w[d];
+                }
+            }
+            __syncwarp();
+            int k0 = 0;
+#pragma unroll 1
+            for (int J = 0; J < T; ++J) {
+                const int nj = __popc(__ballot_sync(NNP_FULL, t == J));
+                if (nj == 0) continue;
+                if (lane == 0) cnt[J] += nj;
+                f32x2 acc[2][NQ][NDP];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                        for (int p = 0; p < NDP; ++p) acc[h][q][p] = 0ull;
+                auto add = [&](int h, int k) {
+                    const float *row = rows + k * ROW + lane;
+                    f32x2 f[NDP];
+#pragma unroll
+                    for (int p = 0; p < NDP; ++p) f[p] = reinterpret_cast<const f32x2 *>(W)[k * NDP + p];
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        // (the last group's lanes past the row read the next row or W; their sums are not used)
+                        const f32x2 y = dup2(row[32 * q]);
+                        const bool any_rad = 32 * q + 31 >= NC && 32 * q < NC + NR;
+                        const bool rad = any_rad && lane + 32 * q >= NC && lane + 32 * q < NC + NR;
+#pragma unroll
+                        for (int p = 0; p < NDP; ++p) {
+                            const f32x2 g = rad ? 0x3f8000003f800000ull : f[p];
+                            acc[h][q][p] = fma2(y, g, acc[h][q][p]);
+                        }
+                    }
+                };
+                int k = k0;
+#pragma unroll 2
+                for (; k + 1 < k0 + nj; k += 2) {
+                    add(0, k);
+                    add(1, k + 1);
+                }
+                if (k < k0 + nj) add(0, k);
+                k0 += nj;
+                const DevBlockR B = Ty.br[J];
+#pragma unroll
+                for (int p = 0; p < NDP; ++p) {
+                    const float t0 = warp_sum(t == J ? w[2 * p] : 0.f), t1 = warp_sum(t == J ? w[2 * p + 1] : 0.f);
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        const int c = lane + 32 * q;
+                        float a0, a1, b0, b1;
+                        up2(acc[0][q][p], a0, a1);
+                        up2(acc[1][q][p], b0, b1);
+                        a0 += b0;
+                        a1 += b1;
+                        if (c == 0) {                            // Y_00 = 1
+                            a0 = t0;
+                            a1 = t1;
+                        }
+                        if (c < NC) {
+                            float2 *dst = reinterpret_cast<float2 *>(A) + (J * NDP + p) * NC + c;
+                            *dst = make_float2(fmaf(a0, nl[q], dst->x), fmaf(a1, nl[q], dst->y));
+                        } else if (c < NC + NR) {
+                            if (p == 0 && c - NC < B.n) Gs[B.off_g + c - NC] += a0;
+                        } else if (c < NC + NR + ND) {
+                            const int d = c - NC - NR;
+                            if ((d >> 1) == p) W2[J * NNP_MOM_MAXD + d] += (d & 1) ? a1 : a0;
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+        if (G) {
+            // S^{JK}_{l,d}: lane = (l, pair of damping factors, element pair), largest l first
+            for (int s = lane; s < NS; s += 32) {
+                const int l = L - s / (TT * NDP), rem = s % (TT * NDP), p = rem / TT, tt = rem % TT;
+                int K = 0;
+#pragma unroll
+                for (int k = 1; k < T; ++k) K += tt >= k * (k + 1) / 2;
+                const int J = tt - K * (K + 1) / 2;
+                const f32x2 *a = reinterpret_cast<const f32x2 *>(A) + (J * NDP + p) * NC;
+                const f32x2 *b = reinterpret_cast<const f32x2 *>(A) + (K * NDP + p) * NC;
+                f32x2 s0 = mul2(a[l], b[l]), s1 = 0ull;
+#pragma unroll
+                for (int m = 1; m <= L; ++m) {
+                    if (m <= l) {
+                        const int c = mom_base(L, m) + 2 * (l - m);
+                        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(a + c);
+                        const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(b + c);
+                        s0 = fma2(x.x, y.x, s0);
+                        s1 = fma2(x.y, y.y, s1);
+                    }
+                }
+                reinterpret_cast<f32x2 *>(S)[(tt * NDP + p) * (L + 1) + l] = add2(s0, s1);
+            }
+            __syncwarp();
+            // G: lane = angular function
+            const int na = Ty.n_input - Ty.n_input_r;
+            for (int f = lane; f < na; f += 32) {
+                const int fu = tb.fun[II * fmax + f];
+                Gs[Ty.n_input_r + f] = mom_function<L, NDP>(tb, fu, tb.coef + (i64)II * (L + 2) * fmax + f,
+                                                             reinterpret_cast<const float2 *>(S), 1,
+                                                             W2 + ((fu >> 16) & 0xff) * NNP_MOM_MAXD + ((fu >> 8) & 0xff), cnt);
+            }
+            __syncwarp();
+            // blocks of few pairs, one per half warp
+            unsigned long long few = 0;
+            for (int K = 0, tt = 0; K < T; ++K)
+                for (int J = 0; J <= K; ++J, ++tt) {
+                    const int np = mom_pairs(cnt, J, K);
+                    if (np > 0 && np <= NNP_MOM_FEW && Ty.ba[tt].n > 0) few |= 1ull << tt;
+                }
+            while (few) {
+                const int t0 = __ffsll(few) - 1;
+                few &= few - 1;
+                const int t1 = few ? __ffsll(few) - 1 : -1, tt = lane < 16 ? t0 : t1;
+                few &= few - 1;
+                if (tt >= 0)
+                    mom_few_symm<M>(0xffffu << (lane & 16), lane & 15, src, cnt, Ty, II, tt, tb.a_lo + II * NNP_MOM_MAXD,
+                                    Gs + Ty.ba[tt].off_g);
+            }
+            __syncwarp();
+            for (int k = lane; 4 * k < gstride; k += 32)
+                reinterpret_cast<float4 *>(G + i * gstride)[k] = reinterpret_cast<const float4 *>(Gs)[k];
+        }
+        {
+            const i64 r = idx - lo;
+            for (int k = lane; k < NV; k += 32) mom[mom_at(r, k, NV)] = reinterpret_cast<const float2 *>(A)[k];
+            if (lane < 8) mom_cnt[8 * r + lane] = cnt[lane];
+            for (int tt = lane; tt < TT; tt += 32) mom_push<T>(items, nitems, r, tt, cnt);
+        }
+        __syncwarp();
+    }
+}
+
+// The same with one thread per atom: the moments of one neighbour element and
+// damping pair are the thread's registers (81 packed pairs for L = 8) while it
+// walks that element's segment of its list, so nothing is staged, exchanged or
+// reduced; the finished moments go to mom, from which the thread forms S
+// (through shared memory, entry-major) and G.  Lanes differ in the length of a
+// segment, which costs ~1.4x on the batched workload, against the staging,
+// flushes and partly filled 32-row chunks of the warp form.
+// Y_00's sum keeps its rounding errors in a second register (see above).
+// Bound: FP32 issue at 8 warps per SM (registers).
+template <class M>
+__device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab,
+                                     int fmax, const int *__restrict__ type, const int *__restrict__ order,
+                                     const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap,
+                                     int gstride, float *__restrict__ G, float2 *mom,
+                                     unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems, float *smem)
+{
+    constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
+                  NR = M::NR, NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), BT = NNP_MOM_THREADS;
+    f32x2 *S = reinterpret_cast<f32x2 *>(smem) + threadIdx.x;    // [NS][BT]
+    f32x2 *W2 = S + NS * BT;                                     // [T][NDP][BT]
+    const DevPot &P = *pot;
+    const MomTab tb = mom_tab(tab, T, L, fmax);
+    for (i64 idx = lo + blockIdx.x * (i64)BT + threadIdx.x; idx < hi; idx += (i64)gridDim.x * BT) {
+        const i64 i = order[idx], r = idx - lo;
+        const int II = type[i];
+        if ((unsigned)II >= (unsigned)T) continue;               // type out of range (reported by the call)
+        const int n = nbr_cnt[i];
+        const DevType &Ty = P.t[II];
+        const float4 *src = nbr + i * cap;
+        float *Gi = G ? G + i * gstride : nullptr;
+        unsigned short *cnt = mom_cnt + 8 * r;
+#pragma unroll 1
+        for (int p = 0; p < NDP; ++p) {
+            int k = 0;
+            float4 e = n > 0 ? src[0] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+#pragma unroll 1
+            for (int J = 0; J < T; ++J) {
+                const int k0 = k;
+                f32x2 acc[NC], c00 = 0ull, ww = 0ull;
+                float rad[NR];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) acc[c] = 0ull;
+#pragma unroll
+                for (int f = 0; f < NR; ++f) rad[f] = 0.f;
+#pragma unroll 1
+                while ((int)((unsigned)__float_as_int(e.w) >> 28) == J) {
+                    MomNbr<M, false> v;
+                    v.set(e, Ty, tb.a_lo + II * NNP_MOM_MAXD);
+                    ++k;
+                    e = k < n ? src[k] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+                    f32x2 cw = pk2(v.w[0], ND > 1 ? v.w[ND > 1 ? 1 : 0] : 0.f);
+                    if (NDP > 1 && p > 0) cw = pk2(v.w[ND > 2 ? 2 : 0], ND > 3 ? v.w[ND > 3 ? 3 : 0] : 0.f);
+                    ww = fma2(cw, cw, ww);
+                    {                                            // two-sum of acc[0] and w
+                        const f32x2 neg = dup2(-1.f);
+                        const f32x2 s = add2(acc[0], cw), bb = fma2(neg, acc[0], s);
+                        c00 = add2(c00, add2(fma2(neg, fma2(neg, bb, s), acc[0]), fma2(neg, bb, cw)));
+                        acc[0] = s;
+                    }
+                    const f32x2 x2 = dup2(v.ux), y2 = dup2(v.uy), ny2 = dup2(-v.uy);
+                    f32x2 sw = 0ull;
+#pragma unroll
+                    for (int m = 0; m <= L; ++m) {               // (cw, sw) = w Re/Im (x + i y)^m
+                        float q0 = 1.f, q1 = 0.f;
+#pragma unroll
+                        for (int l = m; l <= L; ++l) {
+                            const f32x2 q2 = dup2(q0);
+                            if (m == 0) {
+                                if (l > 0) acc[l] = fma2(q2, cw, acc[l]);
+                            } else {
+                                const int c = mom_base(L, m > 0 ? m : 1) + 2 * (l - m);
+                                acc[c] = fma2(q2, cw, acc[c]);
+                                acc[c + 1] = fma2(q2, sw, acc[c + 1]);
+                            }
+                            const float t = (l == m) ? v.uz * q0 : fmaf(v.uz, q0, -mom_beta(l, m) * q1);
+                            q1 = q0;
+                            q0 = t;
+                        }
+                        const f32x2 c = cw;
+                        cw = m == 0 ? mul2(c, x2) : fma2(sw, ny2, mul2(c, x2));
+                        sw = m == 0 ? mul2(c, y2) : fma2(sw, x2, mul2(c, y2));
+                    }
+                    if (NDP == 1 || p == 0) {
+                        float rv[NR];
+#pragma unroll
+                        for (int f = 0; f < NR; ++f) rv[f] = 0.f;
+                        M::radial_row(II, J, v.r, v.fc, rv);
+#pragma unroll
+                        for (int f = 0; f < NR; ++f) rad[f] += rv[f];
+                    }
+                }
+                cnt[J] = (unsigned short)(k - k0);
+                acc[0] = add2(acc[0], c00);
+                f32x2 *dst = reinterpret_cast<f32x2 *>(mom) + mom_at(r, (J * NDP + p) * NC, NV);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) dst[4 * c] = mul2(acc[c], dup2(tb.norm[c]));
+                W2[(J * NDP + p) * BT] = ww;
+                if (G && p == 0) {
+                    const DevBlockR B = Ty.br[J];
+#pragma unroll
+                    for (int f = 0; f < NR; ++f)
+                        if (f < B.n) Gi[B.off_g + f] = rad[f];
+                }
+            }
+        }
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) mom_push<T>(items, nitems, r, tt, cnt);
+        if (!G) continue;
+        const f32x2 *a = reinterpret_cast<const f32x2 *>(mom) + mom_at(r, 0, NV);
+#pragma unroll 1
+        for (int p = 0; p < NDP; ++p)
+#pragma unroll
+            for (int l = 0; l <= L; ++l) {
+                f32x2 s[TT];
+#pragma unroll
+                for (int m = 0; m <= l; ++m)
+#pragma unroll
+                    for (int h = 0; h < (m ? 2 : 1); ++h) {
+                        const int c = m == 0 ? l : mom_base(L, m > 0 ? m : 1) + 2 * (l - m) + h;
+                        f32x2 v[T];
+#pragma unroll
+                        for (int J = 0; J < T; ++J) v[J] = a[4 * ((J * NDP + p) * NC + c)];
+#pragma unroll
+                        for (int K = 0; K < T; ++K)
+#pragma unroll
+                            for (int J = 0; J <= K; ++J) {
+                                const int tt = K * (K + 1) / 2 + J;
+                                s[tt] = m == 0 ? mul2(v[J], v[K]) : fma2(v[J], v[K], s[tt]);
+                            }
+                    }
+#pragma unroll
+                for (int tt = 0; tt < TT; ++tt) S[((tt * NDP + p) * (L + 1) + l) * BT] = s[tt];
+            }
+        const int na = Ty.n_input - Ty.n_input_r;
+#pragma unroll 1
+        for (int f = 0; f < na; ++f) {
+            const int fu = tb.fun[II * fmax + f], d = (fu >> 8) & 0xff;
+            const float *w2 = reinterpret_cast<const float *>(W2 + ((((fu >> 16) & 0xff) * NDP + (d >> 1)) * BT)) + (d & 1);
+            Gi[Ty.n_input_r + f] = mom_function<L, NDP>(tb, fu, tb.coef + (i64)II * (L + 2) * fmax + f,
+                                                         reinterpret_cast<const float2 *>(S), BT, w2, cnt);
+        }
+        for (int f = Ty.n_input; f < gstride; ++f) Gi[f] = 0.f;
+    }
+}
+
+// ---------------------------------------------------------------- forces
+
+// Forces from the moments (NNP::compute_force, src/nnp/nnp.cpp:412-476): a
+// warp takes NA atoms (2 when there are enough atoms: 45 neighbours leave the
+// second of two 32-lane passes half empty, the 90 of two atoms fill three;
+// the virial takes NA = 1).
+// It forms B of each atom from its moments and dE/dG, then lane = neighbour
+// evaluates sum_d w_d sum_lm B Y_lm and its gradient with the broadcast B (two
+// damping factors per 8-byte half, cos and sin parts per 16-byte load, packed
+// FP32 arithmetic), adds the radial terms and scatters dE_i/dd_j in FP64 as
+// force_body does.  Here Q_lm = d^m P_l / dz^m, so that dQ_lm/dz = Q_{l,m+1}
+// needs no factor.  Blocks of the launch from nblock on take the blocks of few pairs.
+// Bound: instruction issue (FP32 pipe).
+template <class M, int NA>
+__device__ void mom_force_body(int nblock, i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+                               const float2 *__restrict__ rpar, const int *__restrict__ type,
+                               const int *__restrict__ order, const float4 *__restrict__ nbr,
+                               const int *__restrict__ nbr_cnt, int cap, int gstride, const float *__restrict__ dEdG,
+                               const float2 *__restrict__ mom, const unsigned short *__restrict__ mom_cnt,
+                               double *__restrict__ F, DevErr *err, const int *__restrict__ atom_struct,
+                               double *__restrict__ vir, float *smem)
+{
+    constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
+                  NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), LA = NA == 1 ? 0 : 1;
+    static_assert(NA == 1 || NA == 2, "atoms per warp");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = mom_force_floats(T, ND, L, gstride);         // floats per atom
+    float *base = smem + (size_t)warp * NA * per;
+    const int oD = 2 * NV, oD1 = oD + ((2 * NS + 3) & ~3), oE = oD1 + T * NNP_MOM_MAXD;
+    const DevPot &P = *pot;
+    const MomTab tb = mom_tab(tab, T, L, fmax);
+    const i64 step = (i64)nblock * NNP_MOM_FORCE_WARPS * NA;
+    for (i64 idx = lo + (blockIdx.x * (i64)NNP_MOM_FORCE_WARPS + warp) * NA; idx < hi; idx += step) {
+        // atom lane & (NA - 1) of the group (II = T: none)
+        const int al = lane & (NA - 1);
+        i64 i_l = 0;
+        int II_l = T, n_l = 0;
+        if (idx + al < hi) {
+            i_l = order[idx + al];
+            const int t = type[i_l];
+            if ((unsigned)t < (unsigned)T) {                     // else out of range (reported by the call)
+                II_l = t;
+                n_l = nbr_cnt[i_l];
+            }
+        }
+        const int n0 = __shfl_sync(NNP_FULL, n_l, 0), n1 = NA == 2 ? __shfl_sync(NNP_FULL, n_l, NA - 1) : 0;
+        const i64 i0 = __shfl_sync(NNP_FULL, i_l, 0), i1 = __shfl_sync(NNP_FULL, i_l, NA - 1);
+        const int II0 = __shfl_sync(NNP_FULL, II_l, 0), II1 = __shfl_sync(NNP_FULL, II_l, NA - 1);
+        const i64 row = idx - lo;
+        for (int k = lane; k < gstride; k += 32) {
+            base[oE + k] = dEdG[i0 * gstride + k];
+            if (NA == 2) base[per + oE + k] = dEdG[i1 * gstride + k];   // (no second atom: atom 0's row, not used)
+        }
+        __syncwarp();
+        // D^{JK}_{l,d} = sum_f e_f c_{f,l} [1 + (J == K)], and the self terms
+        if (II_l < T) {
+            float *mine = base + al * per;
+            const float *e = mine + oE;
+            const DevType &Ty = P.t[II_l];
+            const unsigned short *cnt = mom_cnt + 8 * (row + al);
+            for (int s = lane >> LA; s < TT * NDP * (L + 2); s += 32 / NA) {
+                const int l = s % (L + 2), rem = s / (L + 2), p = rem % NDP, tt = rem / NDP;
+                int K = 0;
+#pragma unroll
+                for (int k = 1; k < T; ++k) K += tt >= k * (k + 1) / 2;
+                const int J = tt - K * (K + 1) / 2;
+                const int bn = Ty.ba[tt].n, off = Ty.ba[tt].off_g, f0 = off - Ty.n_input_r;
+                float s0 = 0.f, s1 = 0.f;
+                if (mom_pairs(cnt, J, K) > NNP_MOM_FEW) {
+                    const float *cf = tb.coef + ((i64)II_l * (L + 2) + l) * fmax + f0;
+                    const int *fu = tb.fun + II_l * fmax + f0;
+#pragma unroll 2
+                    for (int f = 0; f < bn; ++f) {
+                        const int d = (fu[f] >> 8) & 0xff;
+                        const float v = (NDP == 1 || (d >> 1) == p) ? cf[f] * e[off + f] : 0.f;
+                        s0 += (d & 1) ? 0.f : v;
+                        s1 += (d & 1) ? v : 0.f;
+                    }
+                }
+                if (J == K) {
+                    s0 *= 2.f;
+                    s1 *= 2.f;
+                }
+                if (l <= L) {
+                    reinterpret_cast<float2 *>(mine + oD)[(tt * NDP + p) * (L + 1) + l] = make_float2(s0, s1);
+                } else if (J == K) {
+                    mine[oD1 + J * NNP_MOM_MAXD + 2 * p] = s0;
+                    mine[oD1 + J * NNP_MOM_MAXD + 2 * p + 1] = s1;
+                }
+            }
+        }
+        __syncwarp();
+        if (II_l < T) {
+            float *mine = base + al * per;
+            const f32x2 *src = reinterpret_cast<const f32x2 *>(mom) + mom_at(row + al, 0, NV);
+#pragma unroll 2
+            for (int c = lane >> LA; c < NC; c += 32 / NA) {
+                const int l = tb.deg[c];
+                const f32x2 nn = dup2(tb.fnorm[c]);
+#pragma unroll
+                for (int p = 0; p < NDP; ++p) {
+                    f32x2 a[T];
+#pragma unroll
+                    for (int K = 0; K < T; ++K) a[K] = __ldg(src + 4 * ((K * NDP + p) * NC + c));
+#pragma unroll
+                    for (int J = 0; J < T; ++J) {
+                        f32x2 b = 0ull;
+#pragma unroll
+                        for (int K = 0; K < T; ++K) {
+                            const int tt = J > K ? J * (J + 1) / 2 + K : K * (K + 1) / 2 + J;
+                            b = fma2(reinterpret_cast<const f32x2 *>(mine + oD)[(tt * NDP + p) * (L + 1) + l], a[K], b);
+                        }
+                        reinterpret_cast<f32x2 *>(mine)[(J * NDP + p) * NC + c] = mul2(b, nn);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        double f0[3] = {0, 0, 0}, f1[3] = {0, 0, 0};
+        double wv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        bool bad = false;
+        for (int q = lane; q < n0 + n1; q += 32) {
+            const bool sec = NA == 2 && q >= n0;                 // neighbour of the second atom
+            const i64 i = sec ? i1 : i0;
+            const int II = sec ? II1 : II0;
+            const float *mine = base + (sec ? per : 0);
+            const float4 rec = nbr[i * cap + (sec ? q - n0 : q)];
+            const int jt = __float_as_int(rec.w);
+            const int t = (int)((unsigned)jt >> 28);
+            const DevType &Ty = P.t[II];
+            MomNbr<M, true> v;
+            v.set(rec, Ty, tb.a_lo + II * NNP_MOM_MAXD);
+            f32x2 V[NDP], X[NDP], Y[NDP], Z[NDP];
+            f32x2 q0[L + 2];
+            mom_polys<L, 0>(v.uz, q0);
+            mom_gradient<L, NDP, 0>(reinterpret_cast<const ulonglong2 *>(mine + t * (NDP * NC * 2)), v.ux, v.uy, v.uz, q0,
+                                    1.f, 0.f, 0.f, 0.f, V, X, Y, Z);
+            // radial terms
+            const DevBlockR Br = Ty.br[t];
+            const float *e = mine + oE;
+            float fc = v.fc[0], fd = v.fd[0];
+#pragma unroll
+            for (int c = 1; c < M::NCUT; ++c)
+                if (Br.cut == c) {
+                    fc = v.fc[c];
+                    fd = v.fd[c];
+                }
+            float gr = 0.f;
+            if (!M::radial_force(II, t, v.r, fc, fd, e + Br.off_g, gr)) {
+                for (int f = 0; f < Br.n; ++f) {
+                    const float2 q2 = rpar[Br.par + f];
+                    float val, der;
+                    radial_fd(Br.form, v.r, q2.x, q2.y, fc, fd, val, der);
+                    gr = fmaf(e[Br.off_g + f], der, gr);
+                }
+            }
+            float gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+            for (int p = 0; p < NDP; ++p) {
+                float v0, v1, x0, x1, y0, y1, z0, z1;
+                up2(V[p], v0, v1);
+                up2(X[p], x0, x1);
+                up2(Y[p], y0, y1);
+                up2(Z[p], z0, z1);
+                {
+                    const float w = v.w[2 * p], dw = v.wd[2 * p];
+                    gr = fmaf(fmaf(-mine[oD1 + t * NNP_MOM_MAXD + 2 * p], w, v0), dw, gr);
+                    gx = fmaf(w, x0, gx);
+                    gy = fmaf(w, y0, gy);
+                    gz = fmaf(w, z0, gz);
+                }
+                if (2 * p + 1 < ND) {
+                    const float w = v.w[2 * p + 1 < ND ? 2 * p + 1 : 0], dw = v.wd[2 * p + 1 < ND ? 2 * p + 1 : 0];
+                    gr = fmaf(fmaf(-mine[oD1 + t * NNP_MOM_MAXD + 2 * p + 1], w, v1), dw, gr);
+                    gx = fmaf(w, x1, gx);
+                    gy = fmaf(w, y1, gy);
+                    gz = fmaf(w, z1, gz);
+                }
+            }
+            // dE/dd = u dE/dr + (I - u u^T) dE/du / r
+            const float pr = gr - v.ir * (gx * v.ux + gy * v.uy + gz * v.uz);
+            const float h[3] = {fmaf(gx, v.ir, pr * v.ux), fmaf(gy, v.ir, pr * v.uy), fmaf(gz, v.ir, pr * v.uz)};
+            const i64 j = jt & 0x0fffffff;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                bad |= !(fabsf(h[x]) <= 3.402823466e38f);
+                atomicAdd(&F[3 * j + x], (double)h[x]);
+                f0[x] += (double)(sec ? 0.f : h[x]);
+                if (NA == 2) f1[x] += (double)(sec ? h[x] : 0.f);
+            }
+            if (NA == 1 && vir) {
+                // virial W_ab = -sum_k g_a d_b (see force_body)
+                const double d3[3] = {rec.x, rec.y, rec.z};
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+#pragma unroll
+                    for (int y = 0; y < 3; ++y) wv[3 * x + y] -= (double)h[x] * d3[y];
+            }
+        }
+        __syncwarp();
+        if (NA == 1) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) f0[x] = warp_sum(f0[x]);
+            if (lane < 3 && II0 < T) atomicAdd(&F[3 * i0 + lane], lane == 0 ? -f0[0] : lane == 1 ? -f0[1] : -f0[2]);
+        } else {
+            // lanes below 16 keep the first atom's sums, the others the second's
+            const bool up = lane >= 16;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                double s = (up ? f1[x] : f0[x]) + __shfl_xor_sync(NNP_FULL, up ? f0[x] : f1[x], 16);
+#pragma unroll
+                for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(NNP_FULL, s, o);
+                f0[x] = s;
+            }
+            const int x = lane & 15;
+            if (x < 3 && (up ? II1 : II0) < T)
+                atomicAdd(&F[3 * (up ? i1 : i0) + x], x == 0 ? -f0[0] : x == 1 ? -f0[1] : -f0[2]);
+        }
+        if (vir && NA == 1) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) wv[q] = warp_sum(wv[q]);
+            if (lane == 0 && II0 < T) {
+                double *ws = vir + 9 * (i64)atom_struct[i0];
+#pragma unroll
+                for (int q = 0; q < 9; ++q) atomicAdd(ws + q, wv[q]);
+            }
+        }
+        if (__any_sync(NNP_FULL, bad) && lane == 0) atomicMax(&err->nonfinite, 1);
+        __syncwarp();
+    }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace nnp

@@ -51,15 +51,18 @@ constexpr int kReps = 3;        // timed repetitions per candidate (median)
 template <class T, size_t N>
 const T &pick(const T (&a)[N], int k) { return a[std::min<size_t>((size_t)k, N - 1)]; }
 
-TuneParams candidate(int k)
+// The moment form of the angular functions has no such choices: there only
+// the network option varies.
+TuneParams candidate(const Engine &E, int k)
 {
     TuneParams p;
+    p.tc_per_sm = pick(kTcPerSm, k);
+    if (E.mom_ok) return p;
     p.symm_minb = pick(kSymmMinb, k);
     const ForceOpt &f = pick(kForce, k);
     p.force_minb = f.minb;
     p.force_unroll = f.unroll;
     p.force_chunk = f.chunk;
-    p.tc_per_sm = pick(kTcPerSm, k);
     return p;
 }
 
@@ -238,8 +241,9 @@ std::string autotune(Engine &E, int cap, const std::function<std::string()> &run
     }
     // compile every candidate (NVRTC; in parallel, results land in the caches)
     std::vector<TuneParams> cand;
-    for (int k = 0; k < kCandidates; ++k) cand.push_back(candidate(k));
-    {
+    const int ncand = E.mom_ok ? (int)(sizeof kTcPerSm / sizeof kTcPerSm[0]) : kCandidates;
+    for (int k = 0; k < ncand; ++k) cand.push_back(candidate(E, k));
+    if (!E.mom_ok) {
         std::vector<std::thread> th;
         std::vector<std::string> errs(cand.size());
         for (size_t k = 0; k < cand.size(); ++k)
