@@ -1297,6 +1297,7 @@ int nnp_compute_energy_symm(nnp_handle *h, int32_t n_struct, const int64_t *atom
     }
     cudaError_t ce = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (x != cudaSuccess && ce == cudaSuccess) ce = x; };
+    E.n_ghost = 0;
     std::string msg = nnp::run_prepare(E, N, n_struct, 0);
     if (!msg.empty()) return fail(h, NNP_ERR_CUDA, msg);
     chk(E.atom_off.reserve(n_struct + 1));

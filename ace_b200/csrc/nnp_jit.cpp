@@ -743,9 +743,9 @@ std::string jit_compile_params(const Engine &E, const TuneParams &tp, std::strin
     const char *hdr_name[2] = {"nnp_device.cuh", "nnp_moments.cuh"};
     if (nvrtcCreateProgram(&prog, source.c_str(), "nnp_jit.cu", 2, hdr_src, hdr_name) != NVRTC_SUCCESS)
         return "nvrtcCreateProgram failed";
-    const char *opts[] = {"--gpu-architecture=sm_100a", "-std=c++17", "-lineinfo", "--fmad=true",
+    const char *opts[] = {"--gpu-architecture=sm_100a", "-std=c++17", "--fmad=true",
                           "--ptxas-options=-v"};
-    const nvrtcResult rc = nvrtcCompileProgram(prog, 5, opts);
+    const nvrtcResult rc = nvrtcCompileProgram(prog, 4, opts);
     size_t logn = 0;
     nvrtcGetProgramLogSize(prog, &logn);
     std::string log(logn, '\0');

@@ -1151,6 +1151,280 @@ __global__ void __launch_bounds__(WARPS * 32) k_nn_fp32(int64_t N, const DevPot 
     }
 }
 
+// ------------------------------------------------------------------ networks (FP32), tiles of atoms
+//
+// Forward pass, atomic energy and input gradient dE/dG (ANN::fpbp + DODZ::grad,
+// ml/nn.cpp:1402-1420, 1836-1859) for tiles of 32 atoms of one element: a
+// layer is a small product of the element's weights with the tile's
+// activations, both in shared memory, a thread holding 4 atoms x 2 or 4
+// neurons, so that one or two 16-byte loads of each side feed 8 or 16
+// multiply-adds (a warp per atom, one load of a weight and one of an
+// activation per multiply-add, is bound by those loads; it stays below for
+// networks that do not fit).  Sums run in the order of the inputs, as there.
+// Activations are [neuron][NNT_ROW] with the atom fastest; the stride keeps the
+// transposing loads and stores of the G and dE/dG rows free of bank conflicts.
+// Weights of hidden layers are kept in both orders, read by rows in either
+// direction.  NT threads: 128, or 256 when there are fewer tiles than SMs (a
+// tile alone on its SM is a latency chain that more warps shorten).  The tiles run over the atoms sorted by element (`order`).
+#define NNT_ATOMS 32
+#define NNT_ROW 36
+
+struct NntPlan {
+    int wf[NNP_MAX_LAYERS], wb[NNP_MAX_LAYERS];   // weights of hidden layer h: [in][sf], [out][sb]
+    int bias[NNP_MAX_LAYERS], dd[NNP_MAX_LAYERS]; // biases, f'(z) rows
+    int inpw, inpb, wout, xa, xb;                 // input scaling, output weights, activations (ping, pong)
+    int total;                                    // floats
+};
+
+// row stride of a weight matrix of n columns: a multiple of 4 (16-byte loads),
+// an odd one so that transposed stores spread over the banks
+__host__ __device__ inline int nnt_stride(int n)
+{
+    const int s = (n + 3) & ~3;
+    return ((s >> 2) & 1) ? s : s + 4;
+}
+
+__host__ __device__ __forceinline__ void nnt_plan(int L, const int *nodes, NntPlan &p)
+{
+    int o = 0, wide = nodes[0];
+#pragma unroll
+    for (int h = 0; h + 1 < L; ++h) {
+        p.wf[h] = o; o += nodes[h] * nnt_stride(nodes[h + 1]);
+        p.wb[h] = o; o += nodes[h + 1] * nnt_stride(nodes[h]);
+        p.dd[h] = o; o += nodes[h + 1] * NNT_ROW;
+        wide = wide > nodes[h + 1] ? wide : nodes[h + 1];
+    }
+    p.xa = o; o += wide * NNT_ROW;
+    p.xb = o; o += wide * NNT_ROW;
+    p.inpw = o; o += nodes[0];
+    p.inpb = o; o += nodes[0];
+    p.wout = o; o += nodes[L - 1];
+#pragma unroll
+    for (int h = 0; h + 1 < L; ++h) { p.bias[h] = o; o += nodes[h + 1]; }
+    p.total = (o + 3) & ~3;
+}
+
+// tanh inline, the other activations through one copy of the switch
+__device__ __noinline__ void nnt_activation_call(int neuron, float c, float z, float &a, float &d)
+{
+    float d2;
+    activation(neuron, c, z, a, d, d2);
+}
+
+// out(n, acc): for neurons n < no, acc[4] = init(n) + sum_k W[k][n] X[k][4 ag ..]
+template <int NT, int NPT, class Init, class Out>
+__device__ __forceinline__ void nnt_layer(const float *X, const float *W, int ws, int K, int no, Init init, Out out)
+{
+    const int ag = threadIdx.x & 7, ng = threadIdx.x >> 3;
+    for (int n0 = ng * NPT; n0 < no; n0 += NT / 8 * NPT) {
+        float acc[NPT][4];
+#pragma unroll
+        for (int u = 0; u < NPT; ++u) {
+            const float b = n0 + u < no ? init(n0 + u) : 0.f;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) acc[u][a] = b;
+        }
+        const float *x = X + 4 * ag, *w = W + n0;
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const float4 xv = *reinterpret_cast<const float4 *>(x + k * NNT_ROW);
+            float wv[NPT];
+            if (NPT == 4) {
+                const float4 q = *reinterpret_cast<const float4 *>(w + k * ws);
+                wv[0] = q.x; wv[1] = q.y; wv[NPT - 2] = q.z; wv[NPT - 1] = q.w;
+            } else {
+                const float2 q = *reinterpret_cast<const float2 *>(w + k * ws);
+                wv[0] = q.x; wv[1] = q.y;
+            }
+#pragma unroll
+            for (int u = 0; u < NPT; ++u) {
+                acc[u][0] = fmaf(wv[u], xv.x, acc[u][0]);
+                acc[u][1] = fmaf(wv[u], xv.y, acc[u][1]);
+                acc[u][2] = fmaf(wv[u], xv.z, acc[u][2]);
+                acc[u][3] = fmaf(wv[u], xv.w, acc[u][3]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < NPT; ++u)
+            if (n0 + u < no) out(n0 + u, acc[u]);
+    }
+}
+
+template <int NT, class Init, class Out>
+__device__ __forceinline__ void nnt_product(const float *X, const float *W, int ws, int K, int no, Init init, Out out)
+{
+    if (no > 2 * (NT / 8)) nnt_layer<NT, 4>(X, W, ws, K, no, init, out);
+    else nnt_layer<NT, 2>(X, W, ws, K, no, init, out);
+    __syncthreads();
+}
+
+// LT: number of layers when every element has that many (the plan and the
+// widths are then registers; 0: any)
+template <int NT, int LT>
+__global__ void __launch_bounds__(NT) k_nn_tile(const DevPot *__restrict__ pot, const float *__restrict__ wpar,
+                                                         const int *__restrict__ type_count,
+                                                         const int *__restrict__ order, const float *__restrict__ G,
+                                                         int gstride, float *__restrict__ e_atom,
+                                                         float *__restrict__ dEdG)
+{
+    extern __shared__ float smem[];
+    const DevPot &P = *pot;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, ag = t & 7;
+    int staged = -1, T = 0, first = 0, base = 0;                 // element, its first tile and atom
+    for (int g = blockIdx.x;; g += gridDim.x) {
+        while (T < P.ntypes && g >= first + (type_count[T] + NNT_ATOMS - 1) / NNT_ATOMS) {
+            first += (type_count[T] + NNT_ATOMS - 1) / NNT_ATOMS;
+            base += type_count[T];
+            ++T;
+        }
+        if (T == P.ntypes) break;                                // uniform over the block
+        const DevType &DT = P.t[T];
+        const int L = LT ? LT : DT.nlayer;
+        int nd[LT ? LT + 1 : NNP_MAX_LAYERS + 1];
+#pragma unroll
+        for (int l = 0; l <= (LT ? LT : L); ++l) nd[l] = DT.nodes[l];
+        NntPlan p;
+        nnt_plan(L, nd, p);
+        const int nin = nd[0];
+        const float *net = wpar + DT.woff;
+        const float *inpw = smem + p.inpw, *wout = smem + p.wout;
+        float *xa = smem + p.xa, *xb = smem + p.xb;
+        const int a0 = (g - first) * NNT_ATOMS, live = min(NNT_ATOMS, type_count[T] - a0);
+        const int *ord = order + base + a0;
+        if (staged != T) {                                       // (the previous tile ended with a barrier)
+            staged = T;
+            for (int k = t; k < nin; k += NT) {
+                smem[p.inpw + k] = net[k];
+                smem[p.inpb + k] = net[nin + k];
+            }
+            const float *q = net + 2 * nin + 2 * nd[L];
+#pragma unroll
+            for (int h = 0; h + 1 < L; ++h) {
+                const int ni = nd[h], no = nd[h + 1], ws = wt_stride(no), sf = nnt_stride(no), sb = nnt_stride(ni);
+                for (int n = t; n < no; n += NT) smem[p.bias[h] + n] = q[n];
+                q += no;
+                float *f = smem + p.wf[h], *b = smem + p.wb[h];
+                // 16 loads in flight per thread: the load latency, not the bytes, is what staging costs
+                for (int n = lane; n < no; n += 32)
+                    for (int m0 = warp; m0 < ni; m0 += 16 * (NT / 32)) {
+                        float w[16];
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) {
+                            const int m = m0 + u * (NT / 32);
+                            w[u] = m < ni ? q[m * ws + n] : 0.f;
+                        }
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) {
+                            const int m = m0 + u * (NT / 32);
+                            if (m < ni) {
+                                f[m * sf + n] = w[u];
+                                b[n * sb + m] = w[u];
+                            }
+                        }
+                    }
+                q += (i64)ni * ws;
+            }
+            q += 1;                                              // the output bias
+            for (int m = t; m < nd[L - 1]; m += NT) smem[p.wout + m] = q[m * wt_stride(1)];
+            __syncthreads();
+        }
+        const float outw = net[2 * nin], outb = net[2 * nin + 1];
+        int obias = 2 * nin + 2;
+#pragma unroll
+        for (int h = 0; h + 1 < L; ++h) obias += nd[h + 1] + nd[h] * wt_stride(nd[h + 1]);
+        const float bout = net[obias];
+        // A_0 = inpw (G + inpb): 4 atoms x 8 inputs (a 32-byte sector) per warp load
+        for (int a = 4 * warp + (lane >> 3); a < NNT_ATOMS; a += NT / 8) {
+            const float *Gi = G + (i64)ord[a < live ? a : 0] * gstride;
+            for (int k0 = lane & 7; k0 < nin; k0 += 64) {
+                float v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = k0 + 8 * u < nin ? Gi[k0 + 8 * u] : 0.f;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int k = k0 + 8 * u;
+                    if (k < nin) xa[k * NNT_ROW + a] = a < live ? inpw[k] * (v[u] + smem[p.inpb + k]) : 0.f;
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h + 1 < L; ++h) {
+            const float *bias = smem + p.bias[h];
+            float *dd = smem + p.dd[h];
+            const int neuron = DT.neuron;
+            const float c = DT.c;
+            nnt_product<NT>(xa, smem + p.wf[h], nnt_stride(nd[h + 1]), nd[h], nd[h + 1],
+                        [&](int n) { return bias[n]; },
+                        [&](int n, const float *z) {
+                            float a[4], d[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                if (neuron == NEU_TANH) {
+                                    a[k] = tanhf(c * z[k]);
+                                    d[k] = c * (1.f - a[k] * a[k]);
+                                } else {
+                                    nnt_activation_call(neuron, c, z[k], a[k], d[k]);
+                                }
+                            }
+                            *reinterpret_cast<float4 *>(xb + n * NNT_ROW + 4 * ag) = make_float4(a[0], a[1], a[2], a[3]);
+                            *reinterpret_cast<float4 *>(dd + n * NNT_ROW + 4 * ag) = make_float4(d[0], d[1], d[2], d[3]);
+                        });
+            float *x = xa; xa = xb; xb = x;
+        }
+        // output neuron (linear) and the first delta, outw W_out f'(z)
+        const int nl = nd[L - 1];
+        if (t < live) {
+            float z = bout;
+#pragma unroll 8
+            for (int m = 0; m < nl; ++m) z = fmaf(wout[m], xa[m * NNT_ROW + t], z);
+            e_atom[ord[t]] = outb + z * outw;
+        }
+        for (int q = t; q < nl * NNT_ATOMS; q += NT) {
+            const int m = q / NNT_ATOMS, a = q % NNT_ATOMS;
+            const float w = wout[m] * outw;
+            xb[m * NNT_ROW + a] = L > 1 ? w * smem[p.dd[L > 1 ? L - 2 : 0] + m * NNT_ROW + a] : w * inpw[m];
+        }
+        __syncthreads();
+        float *dl = xb, *dn = xa;
+#pragma unroll
+        for (int h = L - 2; h >= 0; --h) {
+            const float *scale = h > 0 ? smem + p.dd[h - 1] : nullptr;
+            nnt_product<NT>(dl, smem + p.wb[h], nnt_stride(nd[h]), nd[h + 1], nd[h],
+                        [&](int) { return 0.f; },
+                        [&](int m, const float *v) {
+                            float4 s;
+                            if (scale) {
+                                s = *reinterpret_cast<const float4 *>(scale + m * NNT_ROW + 4 * ag);
+                            } else {
+                                s.x = s.y = s.z = s.w = inpw[m];
+                            }
+                            *reinterpret_cast<float4 *>(dn + m * NNT_ROW + 4 * ag) =
+                                make_float4(v[0] * s.x, v[1] * s.y, v[2] * s.z, v[3] * s.w);
+                        });
+            float *x = dl; dl = dn; dn = x;
+        }
+        for (int a = 4 * warp + (lane >> 3); a < live; a += NT / 8) {
+            float *out = dEdG + (i64)ord[a] * gstride;
+            for (int k = lane & 7; k < nin; k += 8) out[k] = dl[k * NNT_ROW + a];
+        }
+        __syncthreads();
+    }
+}
+
+// shared-memory bytes of the largest element's tile, or 0 when one does not fit
+static size_t nnt_bytes(const Engine &E)
+{
+    int big = 0;
+    for (int T = 0; T < E.dpot.ntypes; ++T) {
+        if (E.dpot.t[T].nodes[E.dpot.t[T].nlayer] != 1) return 0;
+        NntPlan p;
+        nnt_plan(E.dpot.t[T].nlayer, E.dpot.t[T].nodes, p);
+        big = std::max(big, p.total);
+    }
+    return big * sizeof(float) <= 227 * 1024 ? big * sizeof(float) : 0;
+}
+
 // ------------------------------------------------------------------ forces
 
 __global__ void __launch_bounds__(WARPS * 32, 1) k_force(int64_t N, const DevPot *__restrict__ pot,
@@ -1172,10 +1446,11 @@ __global__ void k_energy(const int64_t *__restrict__ off, int64_t n_centre, cons
                          const int *__restrict__ type, const DevPot *__restrict__ pot, int vacuum,
                          const double *__restrict__ vac, double *__restrict__ e_struct, DevErr *err)
 {
-    __shared__ double part[256];
+    __shared__ double part[1024];
     const int s = blockIdx.x;
     double sum = 0.0;
     const int64_t a1 = off[s + 1] < n_centre ? off[s + 1] : n_centre;     // ghosts carry no energy
+#pragma unroll 8
     for (int64_t a = off[s] + threadIdx.x; a < a1; a += blockDim.x) {
         sum += (double)e_atom[a];
         if (vacuum) {
@@ -1299,6 +1574,16 @@ std::string run_prepare(Engine &E, int64_t n_atoms, int n_struct, int pbc)
     return cuda_msg("prepare");
 }
 
+// atoms grouped by element: counts in type_fill, the visiting order
+static void run_type_order(Engine &E)
+{
+    const int64_t N = E.n_atoms;
+    cudaMemsetAsync(E.type_fill.p, 0, (NEIGH_ITEM_COUNTER + 1) * sizeof(int), E.stream);
+    k_type_count<<<grid_for(N, 256, 1 << 30), 256, 0, E.stream>>>(N, E.n_centre, E.type.p, E.dpot.ntypes, E.type_fill.p);
+    k_type_scatter<<<grid_for(N, 256, 1 << 30), 256, 0, E.stream>>>(N, E.n_centre, E.type.p, E.dpot.ntypes, E.type_fill.p,
+                                                                    E.type_fill.p + NNP_MAX_TYPES + 1, E.order.p);
+}
+
 std::string run_neighbors(Engine &E, int pbc)
 {
     const int64_t N = E.n_atoms;
@@ -1325,10 +1610,7 @@ std::string run_neighbors(Engine &E, int pbc)
             E.neigh_items.p, E.err.p);
     } else {
         E.launches += 11;
-        cudaMemsetAsync(E.type_fill.p, 0, (NEIGH_ITEM_COUNTER + 1) * sizeof(int), st);
-        k_type_count<<<grid_for(N, 256, 1 << 30), 256, 0, st>>>(N, E.n_centre, E.type.p, E.dpot.ntypes, E.type_fill.p);
-        k_type_scatter<<<grid_for(N, 256, 1 << 30), 256, 0, st>>>(N, E.n_centre, E.type.p, E.dpot.ntypes, E.type_fill.p,
-                                                                   E.type_fill.p + NNP_MAX_TYPES + 1, E.order.p);
+        run_type_order(E);
         k_atom_struct<<<grid_for(N, 256, 1 << 30), 256, 0, st>>>(E.atom_off.p, S, N, E.atom_struct.p, E.type.p,
                                                                  E.dpot.ntypes, E.err.p);
         if (!pbc) k_struct_bbox<<<S, 256, 0, st>>>(E.pos.p, E.atom_off.p, E.bbox.p);
@@ -1478,6 +1760,21 @@ std::string run_nn(Engine &E)
     // BF16 / split-BF16 tensor-core layers when every network fits them
     if (E.precision != NNP_PREC_FP32 && tc_smem_bytes(E, E.precision == NNP_PREC_BF16X3) > 0)
         return run_nn_tc(E, E.precision == NNP_PREC_BF16X3);
+    if (const size_t smt = nnt_bytes(E)) {
+        int L = E.dpot.t[0].nlayer;
+        for (int T = 1; T < E.dpot.ntypes; ++T) L = E.dpot.t[T].nlayer == L ? L : 0;
+        const int64_t tiles = (E.n_centre + NNT_ATOMS - 1) / NNT_ATOMS + E.dpot.ntypes;
+        const int nt = tiles <= num_sms() + E.dpot.ntypes ? 256 : 128;
+        auto kern = nt == 256 ? (L == 2 ? k_nn_tile<256, 2> : L == 3 ? k_nn_tile<256, 3> : k_nn_tile<256, 0>)
+                              : (L == 2 ? k_nn_tile<128, 2> : L == 3 ? k_nn_tile<128, 3> : k_nn_tile<128, 0>);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
+        const int per_sm = (int)std::min<size_t>(8, std::max<size_t>(1, (228 * 1024) / (smt + 1024)));
+        kern<<<grid_for(tiles, 1, num_sms() * per_sm), nt, smt, E.stream>>>(
+            E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride, E.e_atom.p, E.dEdG.p);
+        E.launches += 1;
+        E.mark(3);
+        return cuda_msg("networks");
+    }
     const int maxn = max_nodes(E);
     const size_t sm = (size_t)(((E.wfloats + 3) & ~3) + WARPS * (NNP_MAX_LAYERS + 2) * maxn) * sizeof(float);
     if (sm > 220 * 1024) return "networks too large for the shared-memory FP32 path";
@@ -1535,7 +1832,10 @@ std::string run_force(Engine &E)
 std::string run_energy(Engine &E, bool vacuum)
 {
     if (E.n_struct == 0) return "";
-    k_energy<<<E.n_struct, 256, 0, E.stream>>>(E.atom_off.p, E.n_centre, E.e_atom.p, E.type.p, E.d_pot, vacuum ? 1 : 0,
+    // a block per structure: 1024 threads when structures are large (one of
+    // 131072 atoms: 76 us with 256 threads, 13 with 1024 and 8 loads in flight)
+    const int threads = E.n_atoms >= (int64_t)E.n_struct * 4096 ? 1024 : 256;
+    k_energy<<<E.n_struct, threads, 0, E.stream>>>(E.atom_off.p, E.n_centre, E.e_atom.p, E.type.p, E.d_pot, vacuum ? 1 : 0,
                                                E.vac.p, E.e_struct.p, E.err.p);
     E.launches += 1;
     E.mark(5);
@@ -1577,6 +1877,7 @@ std::string run_nn_from_symm(Engine &E, const double *symm_d, int gstride_in)
     const int64_t n = E.n_atoms * E.gstride;
     if (n == 0) return "";
     k_d2f<<<grid_for(n, 256, 1 << 30), 256, 0, E.stream>>>(n, symm_d, E.G.p);
+    run_type_order(E);           // the networks walk the atoms by element
     return run_nn(E);
 }
 
