@@ -579,12 +579,13 @@ name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot,
      const int *__restrict__ atom_struct, double *__restrict__ vir) \
 { \
     extern __shared__ float4 smem4[]; \
-    if ((int)blockIdx.x >= nmain) \
-        nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x - nmain, (int)gridDim.x - nmain, \
+    const int nfew = (int)gridDim.x - nmain; \
+    if ((int)blockIdx.x < nfew) \
+        nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x, nfew, \
             NNP_MOM_FORCE_WARPS * 32, items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, \
             err, atom_struct, vir); \
     else \
-        nnp::mom_force_body<nnp::JitMoments, na>(nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr, nbr_cnt, cap, \
+        nnp::mom_force_body<nnp::JitMoments, na>((int)blockIdx.x - nfew, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr, nbr_cnt, cap, \
             gstride, dEdG, mom, mom_cnt, F, err, atom_struct, vir, reinterpret_cast<float *>(smem4)); \
 }
 NNP_FORCE_KERNEL(k_force_jit, 1)

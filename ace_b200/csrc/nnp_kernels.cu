@@ -8,8 +8,8 @@
 //   k_cell_start   per-structure scan of the cell counts
 //   k_fill, k_sort_cells   cell member lists, sorted by type and atom index;
 //                  the neighbour search's work items (a cell or a part of it)
-//   k_prologue_small  the steps above in one thread block, for a periodic
-//                  batch of at most 2048 atoms and 32 structures
+//   k_prologue_small  the steps above in one thread block, for a batch of at
+//                  most 2048 atoms and 32 structures
 //   k_neigh        one block per cell or part of a cell: candidates from the
 //                  (2m+1)^3 cells gathered in shared memory, one warp per atom,
 //                  exact FP64 displacement test, neighbours grouped by type
@@ -149,8 +149,9 @@ __global__ void k_struct_bbox(const double *__restrict__ pos, const int64_t *__r
 
 // A free structure of more than this many atoms is searched through a cell
 // grid over its bounding box (smaller ones are one cell, every atom a
-// candidate of every other).
-#define NNP_FREE_ONE_CELL 2048
+// candidate of every other; 27 cells hold some 300 candidates).  A domain of
+// 256 atoms with 1244 ghosts: 433 us as one cell, 55 us through the grid.
+#define NNP_FREE_ONE_CELL 512
 
 __device__ void struct_setup_one(int s, const double *__restrict__ cell, const int64_t *__restrict__ off, int pbc,
                                  double rc, const double *__restrict__ bbox, StructGrid *__restrict__ grid,
@@ -468,8 +469,7 @@ __global__ void k_cell_pos(int64_t N, const int *__restrict__ cell_atoms, const 
     if (s < N) cell_pos_one(s, cell_atoms, xw, type, ntypes, cell_pos);
 }
 
-// The neighbour-search prologue of a small periodic batch (one MD-style cell
-// or a few) in one thread block: the steps of the launch sequence k_type_count
+// The neighbour-search prologue of a small batch (one MD-style cell or a few) in one thread block: the steps of the launch sequence k_type_count
 // ... k_cell_pos with block barriers between them instead of launches, on the
 // same device functions.  Element counts and fill cursors land in type_fill
 // as k_type_count / k_type_scatter leave them; `order` lists each element's
@@ -482,7 +482,7 @@ __global__ void k_cell_pos(int64_t N, const int *__restrict__ cell_atoms, const 
 __global__ void __launch_bounds__(PRO_THREADS)
 k_prologue_small(int64_t N, int64_t n_centre, int S, int cell_bound, const int64_t *__restrict__ off,
                  const double *__restrict__ pos, const double *__restrict__ cell, const int *__restrict__ type,
-                 int ntypes, double rc, int budget, StructGrid *__restrict__ grid, int *__restrict__ ncells,
+                 int ntypes, double rc, int budget, int pbc, double *__restrict__ bbox, StructGrid *__restrict__ grid, int *__restrict__ ncells,
                  int *__restrict__ atom_struct, double *__restrict__ xw, int *__restrict__ atom_cell,
                  int *__restrict__ cell_cnt, int *__restrict__ cell_start, int *__restrict__ cell_fill,
                  int *__restrict__ cell_atoms, int *__restrict__ cell_tcnt, double4 *__restrict__ cell_pos,
@@ -497,6 +497,27 @@ k_prologue_small(int64_t N, int64_t n_centre, int S, int cell_bound, const int64
         cur[t] = 0;
     }
     if (t == 0) *items_n = 0;
+    if (!pbc) {                                                  // bounding boxes of free structures, a warp each
+        for (int s = warp; s < S; s += PRO_THREADS / 32) {
+            double l[3] = {1e300, 1e300, 1e300}, h[3] = {-1e300, -1e300, -1e300};
+            for (int64_t a = off[s] + lane; a < off[s + 1]; a += 32)
+                for (int d = 0; d < 3; ++d) {
+                    l[d] = fmin(l[d], pos[3 * a + d]);
+                    h[d] = fmax(h[d], pos[3 * a + d]);
+                }
+            for (int d = 0; d < 3; ++d) {
+                for (int q = 16; q; q >>= 1) {
+                    l[d] = fmin(l[d], __shfl_xor_sync(0xffffffffu, l[d], q));
+                    h[d] = fmax(h[d], __shfl_xor_sync(0xffffffffu, h[d], q));
+                }
+                if (lane == 0) {
+                    bbox[6 * s + d] = l[d];
+                    bbox[6 * s + 3 + d] = h[d];
+                }
+            }
+        }
+        __syncthreads();
+    }
     for (int c = t; c < cell_bound; c += PRO_THREADS) cell_cnt[c] = 0;
     __syncthreads();
     // atom -> structure, element counts (ghosts and bad types in slot ntypes), structure grids
@@ -505,7 +526,7 @@ k_prologue_small(int64_t N, int64_t n_centre, int S, int cell_bound, const int64
         const int ty = type[i];
         atomicAdd(&cnt[(ty >= 0 && ty < ntypes && i < n_centre) ? ty : ntypes], 1);
     }
-    for (int s = t; s < S; s += PRO_THREADS) struct_setup_one(s, cell, off, 1, rc, nullptr, grid, ncells, err);
+    for (int s = t; s < S; s += PRO_THREADS) struct_setup_one(s, cell, off, pbc, rc, bbox, grid, ncells, err);
     __syncthreads();
     if (t <= NNP_MAX_TYPES) {
         int b = 0;
@@ -586,6 +607,8 @@ struct NeighShared {
         } c;
         float4 lst[NEIGH_WARPS][NNP_MAX_NBR]; // global-memory search: accepted, j | type << 28 in .w
     };
+    float box[NEIGH_WARPS][6];                // bounds of the warps' atoms (low, high)
+    int kept[NEIGH_WARPS];                    // candidates in each warp's part of c (a multiple of 32)
     int count[NEIGH_ATOMS];                   // running neighbour counts (chunked lists)
     int pre[NEIGH_ENT + 1];                   // exclusive scan of the segment lengths
     int start[NEIGH_ENT];                     // first member slot of each segment
@@ -612,71 +635,130 @@ __device__ __forceinline__ int cell_offset(const StructGrid &g, int c0, int c1, 
     return g.cell_base + ((t0 - q0 * g.nc[0]) * g.nc[1] + (t1 - q1 * g.nc[1])) * g.nc[2] + (t2 - q2 * g.nc[2]);
 }
 
-// Candidates [k0, k1) of the cell's list into shared memory slots [0, k1-k0),
-// slots up to kp filled with NaN positions (never accepted).
-__device__ __forceinline__ void load_candidates(NeighShared &sh, int k0, int k1, int kp, int NE, const StructGrid &g,
-                                                const double4 *__restrict__ cell_pos,
-                                                const int *__restrict__ cell_atoms, int tid)
+// Bounds of the item's atoms.
+__device__ __forceinline__ void atoms_box(NeighShared &sh, int cs, int a_lo, int a_hi, const double4 *__restrict__ cell_pos, int warp, int lane, float *lo, float *hi)
 {
-    const double R0 = g.R[0], R1 = g.R[1], R2 = g.R[2], R3 = g.R[3], R4 = g.R[4], R5 = g.R[5], R6 = g.R[6],
-                 R7 = g.R[7], R8 = g.R[8];
-    for (int s = tid; s < kp; s += NEIGH_THREADS) {
-        const int k = k0 + s;
-        if (k >= k1) {
-            const double nan = __longlong_as_double(0x7ff8000000000000ll);
-            sh.c.x[s] = sh.c.y[s] = sh.c.z[s] = nan;
-            sh.c.jt[s] = 0;
-            continue;
+    float l[3] = {3e38f, 3e38f, 3e38f}, h[3] = {-3e38f, -3e38f, -3e38f};
+    for (int a = a_lo + warp * 32 + lane; a < a_hi; a += NEIGH_THREADS) {
+        const double4 x = cell_pos[cs + a];
+        const float v[3] = {(float)x.x, (float)x.y, (float)x.z};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            l[d] = fminf(l[d], v[d]);
+            h[d] = fmaxf(h[d], v[d]);
         }
-        int lo = 0, hi = NE;                                     // last segment with pre <= k
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (sh.pre[mid] <= k) lo = mid; else hi = mid;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            l[d] = fminf(l[d], __shfl_xor_sync(FULL, l[d], o));
+            h[d] = fmaxf(h[d], __shfl_xor_sync(FULL, h[d], o));
         }
-        const int slot = sh.start[lo] + k - sh.pre[lo];
-        const double4 xj = cell_pos[slot];
-        const int j = cell_atoms[slot];
-        if (xj.w < 0.0) {                                        // type out of range: never a neighbour
-            const double nan = __longlong_as_double(0x7ff8000000000000ll);
-            sh.c.x[s] = sh.c.y[s] = sh.c.z[s] = nan;
-            sh.c.jt[s] = 0;
-            continue;
+    if (lane == 0)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            sh.box[warp][d] = l[d];
+            sh.box[warp][3 + d] = h[d];
         }
-        const int qp = sh.q[lo];
-        const double Q0 = (qp & 255) - 128, Q1 = ((qp >> 8) & 255) - 128, Q2 = ((qp >> 16) & 255) - 128;
-        sh.c.x[s] = xj.x + (R0 * Q0 + R3 * Q1 + R6 * Q2);
-        sh.c.y[s] = xj.y + (R1 * Q0 + R4 * Q1 + R7 * Q2);
-        sh.c.z[s] = xj.z + (R2 * Q0 + R5 * Q1 + R8 * Q2);
-        sh.c.jt[s] = j | ((int)xj.w << 28);
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = sh.box[0][d];
+        hi[d] = sh.box[0][3 + d];
+#pragma unroll
+        for (int w = 1; w < NEIGH_WARPS; ++w) {
+            lo[d] = fminf(lo[d], sh.box[w][d]);
+            hi[d] = fmaxf(hi[d], sh.box[w][3 + d]);
+        }
     }
 }
 
-// Tests atom i against shared slots [0, kp) (kp a multiple of 64, two batches
-// of 32 in flight), appending accepted candidates to out[count..cap) in slot
-// order; returns the new count.
-__device__ __forceinline__ int test_candidates(const NeighShared &sh, int kp, int lane, int i, double xi0, double xi1,
+// Candidates [k0, k1) of the cell's list (at most NEIGH_CAND) into shared
+// memory.  Each warp takes a quarter of the range, in order, and keeps in its
+// quarter of the buffer those within rc of the box of the item's atoms
+// (distance^2 to the box <= rc2m, FP32 with a margin): of the 27 images of a
+// structure of one cell two in five, of cells between rc and 2 rc wide half.
+// The kept ones are padded to a multiple of 32 with NaN positions (never
+// accepted).
+__device__ __forceinline__ void load_candidates(NeighShared &sh, int k0, int k1, int NE, const StructGrid &g,
+                                                const double4 *__restrict__ cell_pos,
+                                                const int *__restrict__ cell_atoms, const float *lo3, const float *hi3,
+                                                float rc2m, int warp, int lane)
+{
+    const double R0 = g.R[0], R1 = g.R[1], R2 = g.R[2], R3 = g.R[3], R4 = g.R[4], R5 = g.R[5], R6 = g.R[6],
+                 R7 = g.R[7], R8 = g.R[8];
+    const unsigned lt = (1u << lane) - 1u;
+    const int base = warp * (NEIGH_CAND / NEIGH_WARPS);
+    const int per = ((k1 - k0 + 32 * NEIGH_WARPS - 1) / (32 * NEIGH_WARPS)) * 32;
+    const int kb = k0 + warp * per, ke = min(k1, kb + per);
+    int kept = 0;
+    for (int k1w = kb; k1w < ke; k1w += 32) {
+        const int k = k1w + lane;
+        bool in = false;
+        double x = 0.0, y = 0.0, z = 0.0;
+        int jt = 0;
+        if (k < ke) {
+            int lo = 0, hi = NE;                                 // last segment with pre <= k
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (sh.pre[mid] <= k) lo = mid; else hi = mid;
+            }
+            const int slot = sh.start[lo] + k - sh.pre[lo];
+            const double4 xj = cell_pos[slot];
+            const int qp = sh.q[lo];
+            const double Q0 = (qp & 255) - 128, Q1 = ((qp >> 8) & 255) - 128, Q2 = ((qp >> 16) & 255) - 128;
+            x = xj.x + (R0 * Q0 + R3 * Q1 + R6 * Q2);
+            y = xj.y + (R1 * Q0 + R4 * Q1 + R7 * Q2);
+            z = xj.z + (R2 * Q0 + R5 * Q1 + R8 * Q2);
+            const float fx = (float)x, fy = (float)y, fz = (float)z;
+            const float dx = fmaxf(fmaxf(lo3[0] - fx, fx - hi3[0]), 0.f), dy = fmaxf(fmaxf(lo3[1] - fy, fy - hi3[1]), 0.f),
+                        dz = fmaxf(fmaxf(lo3[2] - fz, fz - hi3[2]), 0.f);
+            in = xj.w >= 0.0 && !(dx * dx + dy * dy + dz * dz > rc2m);   // (type out of range: never a neighbour)
+            jt = in ? cell_atoms[slot] | ((int)xj.w << 28) : 0;
+        }
+        const unsigned b = __ballot_sync(FULL, in);
+        if (in) {
+            const int s = base + kept + __popc(b & lt);
+            sh.c.x[s] = x;
+            sh.c.y[s] = y;
+            sh.c.z[s] = z;
+            sh.c.jt[s] = jt;
+        }
+        kept += __popc(b);
+    }
+    const int pad = (kept + 31) & ~31;
+    if (kept + lane < pad) {
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        sh.c.x[base + kept + lane] = sh.c.y[base + kept + lane] = sh.c.z[base + kept + lane] = nan;
+        sh.c.jt[base + kept + lane] = 0;
+    }
+    if (lane == 0) sh.kept[warp] = pad;
+}
+
+// Tests atom i against the kept candidates (one warp), appending accepted ones
+// to out[count..cap) in list order; returns the new count.
+__device__ __forceinline__ int test_candidates(const NeighShared &sh, int lane, int i, double xi0, double xi1,
                                                double xi2, double rc2, int count, int cap, float4 *__restrict__ out)
 {
     const unsigned lt = (1u << lane) - 1u;
-    for (int kb = 0; kb < kp; kb += 64) {
-        const int ka = kb + lane, kc = ka + 32;
-        const double ax = xi0 - sh.c.x[ka], ay = xi1 - sh.c.y[ka], az = xi2 - sh.c.z[ka];
-        const double cx = xi0 - sh.c.x[kc], cy = xi1 - sh.c.y[kc], cz = xi2 - sh.c.z[kc];
-        const double ra = ax * ax + ay * ay + az * az, rb = cx * cx + cy * cy + cz * cz;
-        bool acca = ra < rc2, accb = rb < rc2;
-        if (acca && !(ra > 1e-12)) acca = (sh.c.jt[ka] & 0x0fffffff) != i;
-        if (accb && !(rb > 1e-12)) accb = (sh.c.jt[kc] & 0x0fffffff) != i;
-        const unsigned ba = __ballot_sync(FULL, acca), bb = __ballot_sync(FULL, accb);
-        if (acca) {
-            const int p = count + __popc(ba & lt);
-            if (p < cap) out[p] = make_float4((float)ax, (float)ay, (float)az, __int_as_float(sh.c.jt[ka]));
+#pragma unroll 1
+    for (int w = 0; w < NEIGH_WARPS; ++w) {
+        const int b0 = w * (NEIGH_CAND / NEIGH_WARPS), b1 = b0 + sh.kept[w];
+#pragma unroll 2
+        for (int k0 = b0; k0 < b1; k0 += 32) {
+            const int k = k0 + lane;
+            const double ax = xi0 - sh.c.x[k], ay = xi1 - sh.c.y[k], az = xi2 - sh.c.z[k];
+            const double ra = ax * ax + ay * ay + az * az;
+            bool acc = ra < rc2;
+            if (acc && !(ra > 1e-12)) acc = (sh.c.jt[k] & 0x0fffffff) != i;
+            const unsigned b = __ballot_sync(FULL, acc);
+            if (acc) {
+                const int p = count + __popc(b & lt);
+                if (p < cap) out[p] = make_float4((float)ax, (float)ay, (float)az, __int_as_float(sh.c.jt[k]));
+            }
+            count += __popc(b);
         }
-        count += __popc(ba);
-        if (accb) {
-            const int p = count + __popc(bb & lt);
-            if (p < cap) out[p] = make_float4((float)cx, (float)cy, (float)cz, __int_as_float(sh.c.jt[kc]));
-        }
-        count += __popc(bb);
     }
     return count;
 }
@@ -834,14 +916,20 @@ __global__ void __launch_bounds__(NEIGH_THREADS, NEIGH_BLOCKS) k_neigh(const int
         }
         __syncthreads();
         const int T = sh.pre[NE];
+        float lo3[3], hi3[3];
+        atoms_box(sh, cs, a_lo, a_hi, cell_pos, warp, lane, lo3, hi3);
+        // FP32 rounding of the coordinates: 2^-24 of the largest in either, over two of them
+        float big = 0.f;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) big = fmaxf(big, fmaxf(fabsf(lo3[d]), fabsf(hi3[d])));
+        const float rcm = (float)sqrt(rc2) * 1.00001f + 1e-6f * big, rc2m = rcm * rcm;
         if (T <= NEIGH_CAND) {
-            const int kp = (T + 63) & ~63;
-            load_candidates(sh, 0, T, kp, NE, g, cell_pos, cell_atoms, tid);
+            load_candidates(sh, 0, T, NE, g, cell_pos, cell_atoms, lo3, hi3, rc2m, warp, lane);
             __syncthreads();
             for (int a = a_lo + warp; a < a_hi; a += NEIGH_WARPS) {
                 const int i = cell_atoms[cs + a];
                 const double4 xi = cell_pos[cs + a];
-                const int count = test_candidates(sh, kp, lane, i, xi.x, xi.y, xi.z, rc2, 0, cap, nbr + (int64_t)i * cap);
+                const int count = test_candidates(sh, lane, i, xi.x, xi.y, xi.z, rc2, 0, cap, nbr + (int64_t)i * cap);
                 if (lane == 0) finish_atom(i, count, cap, nbr_cnt, err);
             }
         } else {
@@ -849,15 +937,15 @@ __global__ void __launch_bounds__(NEIGH_THREADS, NEIGH_BLOCKS) k_neigh(const int
                 const int a1 = min(a_hi, a0 + NEIGH_ATOMS);
                 for (int a = a0 + tid; a < a1; a += NEIGH_THREADS) sh.count[a - a0] = 0;
                 for (int k0 = 0; k0 < T; k0 += NEIGH_CAND) {
-                    const int k1 = min(T, k0 + NEIGH_CAND), kp = (k1 - k0 + 63) & ~63;
+                    const int k1 = min(T, k0 + NEIGH_CAND);
                     __syncthreads();                             // the previous chunk is tested
-                    load_candidates(sh, k0, k1, kp, NE, g, cell_pos, cell_atoms, tid);
+                    load_candidates(sh, k0, k1, NE, g, cell_pos, cell_atoms, lo3, hi3, rc2m, warp, lane);
                     __syncthreads();
                     for (int a = a0 + warp; a < a1; a += NEIGH_WARPS) {
                         const int i = cell_atoms[cs + a];
                         const double4 xi = cell_pos[cs + a];
-                        const int count = test_candidates(sh, kp, lane, i, xi.x, xi.y, xi.z, rc2, sh.count[a - a0],
-                                                          cap, nbr + (int64_t)i * cap);
+                        const int count = test_candidates(sh, lane, i, xi.x, xi.y, xi.z, rc2, sh.count[a - a0], cap,
+                                                          nbr + (int64_t)i * cap);
                         __syncwarp();
                         if (lane == 0) sh.count[a - a0] = count;
                     }
@@ -1600,12 +1688,12 @@ std::string run_neighbors(Engine &E, int pbc)
     const double rc2 = E.dpot.rc_d * E.dpot.rc_d;
     const int nsm = sizeof(NeighShared);
     cudaFuncSetAttribute(k_neigh, cudaFuncAttributeMaxDynamicSharedMemorySize, nsm);
-    if (pbc && N <= PRO_MAX_ATOMS && S <= PRO_MAX_STRUCT) {
-        // a small periodic batch: the whole prologue in one block
+    if (N <= PRO_MAX_ATOMS && S <= PRO_MAX_STRUCT) {
+        // a small batch: the whole prologue in one block
         E.launches += 2;
         k_prologue_small<<<1, PRO_THREADS, 0, st>>>(
             N, E.n_centre, S, (int)cell_bound, E.atom_off.p, E.pos.p, E.cell.p, E.type.p, E.dpot.ntypes,
-            E.dpot.rc_d, budget, E.grid.p, E.scan_tmp.p, E.atom_struct.p, E.xw.p, E.atom_cell.p, E.cell_cnt.p,
+            E.dpot.rc_d, budget, pbc, E.bbox.p, E.grid.p, E.scan_tmp.p, E.atom_struct.p, E.xw.p, E.atom_cell.p, E.cell_cnt.p,
             E.cell_start.p, E.cell_fill.p, E.cell_atoms.p, E.cell_tcnt.p, E.cell_pos.p, E.type_fill.p, E.order.p,
             E.neigh_items.p, E.err.p);
     } else {

@@ -881,10 +881,11 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
 // damping factors per 8-byte half, cos and sin parts per 16-byte load, packed
 // FP32 arithmetic), adds the radial terms and scatters dE_i/dd_j in FP64 as
 // force_body does.  Here Q_lm = d^m P_l / dz^m, so that dQ_lm/dz = Q_{l,m+1}
-// needs no factor.  Blocks of the launch from nblock on take the blocks of few pairs.
+// needs no factor.  The launch's first blocks take the blocks of few pairs
+// (behind the others they were a tail of 0.10 of 3.39 ms).
 // Bound: instruction issue (FP32 pipe).
 template <class M, int NA>
-__device__ void mom_force_body(int nblock, i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+__device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
                                const float2 *__restrict__ rpar, const int *__restrict__ type,
                                const int *__restrict__ order, const float4 *__restrict__ nbr,
                                const int *__restrict__ nbr_cnt, int cap, int gstride, const float *__restrict__ dEdG,
@@ -902,7 +903,7 @@ __device__ void mom_force_body(int nblock, i64 lo, i64 hi, const DevPot *__restr
     const DevPot &P = *pot;
     const MomTab tb = mom_tab(tab, T, L, fmax);
     const i64 step = (i64)nblock * NNP_MOM_FORCE_WARPS * NA;
-    for (i64 idx = lo + (blockIdx.x * (i64)NNP_MOM_FORCE_WARPS + warp) * NA; idx < hi; idx += step) {
+    for (i64 idx = lo + (block * (i64)NNP_MOM_FORCE_WARPS + warp) * NA; idx < hi; idx += step) {
         // atom lane & (NA - 1) of the group (II = T: none)
         const int al = lane & (NA - 1);
         i64 i_l = 0;

@@ -89,3 +89,51 @@ def test_empty_cells_have_no_candidates(tmp_path, n, free):
     got = nn.neighbor_counts(b.n_atoms)
     nn.close()
     assert np.array_equal(got, oracle_counts(pot.rc, b, 3))
+
+
+@pytest.mark.parametrize("n, shift", [(512, 0.0), (513, 0.0), (300, 5000.0), (700, -3000.0)])
+def test_free_structures_around_the_grid_limit(tmp_path, n, shift):
+    """Free structures up to 512 atoms are one cell, larger ones searched
+    through a grid; far from the origin the candidates' FP32 box test has its
+    coordinates rounded to 2^-12 A."""
+    pot = synth.potential_config(2)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    b = synth.batch_random(17, [n, 5], 3)
+    b = synth.Batch(b.atom_off, b.pos + shift, b.type, b.cell, pbc=False)
+    nn = NNP.read(path)
+    nn.compute_batch(b.atom_off, b.pos, b.type, None, pbc=False)
+    got = nn.neighbor_counts(b.n_atoms)
+    nn.close()
+    assert np.array_equal(got, oracle_counts(pot.rc, b, 3))
+
+
+def brute_counts(rc, pos, typ, cell, ntypes, images):
+    """Counts over wrapped positions and all images up to `images` (the oracle
+    takes its range from the edges' lengths, too few for a strong shear)."""
+    frac = pos @ np.linalg.inv(cell)
+    q = (frac - np.floor(frac)) @ cell
+    sh = np.array(list(np.ndindex(*[2 * m + 1 for m in images]))) - np.array(images)
+    out = np.zeros((len(pos), ntypes), np.int32)
+    for i in range(len(pos)):
+        r2 = ((q[i] - (q[None] + (sh @ cell)[:, None])) ** 2).sum(-1)
+        np.add.at(out[i], typ[np.nonzero((r2 < rc * rc) & (r2 > 1e-12))[1]], 1)
+    return out
+
+
+def test_thin_and_skewed_cells(tmp_path):
+    """A cell thinner than the cutoff (many images) and a strongly sheared one."""
+    pot = synth.potential_config(2)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    rng = np.random.default_rng(3)
+    cells = np.array([np.diag([2.2, 14.0, 30.0]), [[15.0, 0, 0], [9.0, 13.0, 0], [-8.0, 7.0, 14.0]]])
+    off = np.array([0, 40, 170])
+    pos = np.concatenate([rng.uniform(0, 1, (40, 3)) @ cells[0], rng.uniform(-1, 2, (130, 3)) @ cells[1]])
+    b = synth.Batch(off, pos, rng.integers(0, 3, 170).astype(np.int32), cells, True)
+    nn = NNP.read(path)
+    nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    got = nn.neighbor_counts(b.n_atoms)
+    nn.close()
+    want = np.concatenate([brute_counts(pot.rc, *b.structure(s), 3, m) for s, m in ((0, (4, 2, 2)), (1, (3, 3, 3)))])
+    assert np.array_equal(got, want)
