@@ -3,13 +3,12 @@
 //
 // The prebuilt kernels read every angular function's (lambda, zeta, eta) from
 // memory and branch on them per pair.  Here the host writes CUDA source in
-// which each GAUSS angular block of the potential is straight-line code: the
-// bases 0.5 +- 0.5 cos, their powers as a shared multiply ladder, the damping
-// products once per group, and every parameter a literal.  NVRTC compiles it
+// which each angular block of the potential is straight-line code: the
+// bases 0.5 +- 0.5 cos, their powers as a shared multiply ladder, the radial
+// factors once per width, and every parameter a literal.  NVRTC compiles it
 // for sm_100a when the handle is created; the kernels reuse the per-atom
 // skeleton of nnp_device.cuh (symm_body / force_body) through a Blocks policy,
-// so only the block arithmetic differs from the prebuilt path.  Blocks of
-// other forms fall through to the generic code inside the same kernels.
+// so only the block arithmetic differs from the prebuilt path.
 #include <cuda_runtime.h>
 #include <nvrtc.h>
 
@@ -104,6 +103,16 @@ std::vector<Fn> block_fns(const Engine &E, const DevBlockA &B)
         std::memcpy(&pk, &q.w, sizeof pk);
         fs.push_back({q.x, q.y, q.z, pk & 0xff, (pk >> 8) - 1});
     }
+    // radial groups: GAUSS has its damping factors, the other forms one per width
+    if (B.form != ANG_GAUSS) {
+        std::vector<float> widths;
+        for (Fn &f : fs) {
+            size_t g = 0;
+            while (g < widths.size() && widths[g] != f.ieta2) ++g;
+            if (g == widths.size()) widths.push_back(f.ieta2);
+            f.damp = (int)g;
+        }
+    }
     return fs;
 }
 
@@ -119,34 +128,69 @@ void gen_bases(std::ostringstream &os, const std::vector<Fn> &fs, std::vector<fl
         os << "            const float x" << b << " = fabsf(fmaf(" << flit(bases[b]) << ", cs, 0.5f));\n";
 }
 
-// common per-pair prologue: geometry, bases, damping factors of the used groups
-void pair_prologue(std::ostringstream &os, const std::vector<Fn> &fs, std::vector<float> &bases,
-                   std::set<int> &damps, bool force)
+// Common per-pair prologue: geometry, bases, and for each radial group g of
+// the block its value P_g (for GAUSS the product of the two neighbours' staged
+// damping factors, for the other forms the radial factor times both cutoffs,
+// angular_generic's formulas with the width as a literal, once for all
+// functions that share it) and, with der, its derivatives A_g, B_g with respect
+// to the two distances.
+void pair_prologue(std::ostringstream &os, const DevBlockA &B, const std::vector<Fn> &fs, std::vector<float> &bases,
+                   std::set<int> &groups, bool der)
 {
     os << "            int a, b;\n"
           "            pit_slots(k, it, a, b);\n"
           "            const float4 ua = v.u[a], ub = v.u[b];\n"
           "            const float cs = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;\n";
     gen_bases(os, fs, bases);
-    for (const Fn &f : fs) damps.insert(f.damp);
+    for (const Fn &f : fs) groups.insert(f.damp);
+    if (B.form != ANG_GAUSS) {
+        const std::string c = std::to_string(B.cut);
+        os << "            const float ra = v.r[a], rb = v.r[b], ca = v.fc[" << c << " * cap + a], cb = v.fc[" << c
+           << " * cap + b], r2 = fmaf(ra, ra, rb * rb), cc = ca * cb;\n";
+        if (der)
+            os << "            const float ga = v.fd[" << c << " * cap + a], gb = v.fd[" << c << " * cap + b];\n";
+        for (int g : groups) {
+            float w = 0.f;
+            for (const Fn &f : fs)
+                if (f.damp == g) w = f.ieta2;
+            const std::string G = std::to_string(g);
+            const float pw = 0.5f * 3.14159265358979f * w;
+            std::string df;                                       // d(rad)/dr = -2 r df rad
+            if (B.form == ANG_GAUSS2 || B.form == ANG_SECH) {
+                const bool sech = B.form == ANG_SECH;
+                os << "            const float f" << G << " = expf(" << flit(-pw) << " * r2), n" << G << " = 1.f / (1.f + f" << G
+                   << (sech ? " * f" + G : std::string()) << "), h" << G << " = 2.f * f" << G << " * n" << G << ";\n";
+                df = flit(pw) + " * n" + G + (sech ? " * (1.f - f" + G + " * f" + G + ")" : "");
+            } else {
+                const int e = 4 + (B.form - ANG_STUDENT3);
+                os << "            const float n" << G << " = rsqrtf(fmaf(" << flit(w) << ", r2, 1.f)), h" << G << " = ipow(n" << G
+                   << ", " << e << ");\n";
+                df = flit(0.5f * (float)e * w) + " * n" + G + " * n" + G;
+            }
+            os << "            const float P" << G << " = h" << G << " * cc;\n";
+            if (der)
+                os << "            const float d" << G << " = -2.f * " << df << ", A" << G << " = h" << G << " * cb * fmaf(ra * ca, d"
+                   << G << ", ga), B" << G << " = h" << G << " * ca * fmaf(rb * cb, d" << G << ", gb);\n";
+        }
+        return;
+    }
     // damping factors: groups 2m and 2m+1 of a neighbour are one float2 (wix)
     std::set<int> pairs;
-    for (int d : damps) pairs.insert(d >> 1);
+    for (int d : groups) pairs.insert(d >> 1);
     for (int m : pairs) {
         const std::string M = std::to_string(m);
         os << "            const float2 wpa" << M << " = reinterpret_cast<const float2 *>(v.w)[" << M
            << " * cap + a], wpb" << M << " = reinterpret_cast<const float2 *>(v.w)[" << M << " * cap + b];\n";
-        if (force)
+        if (der)
             os << "            const float2 dpa" << M << " = reinterpret_cast<const float2 *>(v.wd)[" << M
                << " * cap + a], dpb" << M << " = reinterpret_cast<const float2 *>(v.wd)[" << M << " * cap + b];\n";
     }
-    for (int d : damps) {
-        const std::string M = std::to_string(d >> 1), c = (d & 1) ? ".y" : ".x";
-        os << "            const float wa" << d << " = wpa" << M << c << ", wb" << d << " = wpb" << M << c << ";\n";
-        if (force)
-            os << "            const float da" << d << " = dpa" << M << c << ", db" << d << " = dpb" << M << c << ";\n";
-        else
-            os << "            const float w" << d << " = wa" << d << " * wb" << d << ";\n";
+    for (int d : groups) {
+        const std::string M = std::to_string(d >> 1), c = (d & 1) ? ".y" : ".x", D = std::to_string(d);
+        os << "            const float P" << D << " = wpa" << M << c << " * wpb" << M << c << ";\n";
+        if (der)
+            os << "            const float A" << D << " = dpa" << M << c << " * wpb" << M << c << ", B" << D << " = wpa" << M << c
+               << " * dpb" << M << c << ";\n";
     }
 }
 
@@ -197,7 +241,7 @@ std::string gen_reduce_store(size_t nf, const std::string &acc, const std::strin
     return os.str();
 }
 
-// Body of one GAUSS block's symmetry functions; written relative to the
+// Body of one block's symmetry functions; written relative to the
 // block's first function (Gb), so blocks with equal parameters share it.
 std::string gen_symm_body(const Engine &E, const DevBlockA &B)
 {
@@ -211,11 +255,11 @@ std::string gen_symm_body(const Engine &E, const DevBlockA &B)
     std::ostringstream body;
     std::vector<float> bases;
     std::set<int> damps;
-    pair_prologue(body, fs, bases, damps, false);
+    pair_prologue(body, B, fs, bases, damps, false);
     Powers P(body);
     for (size_t f = 0; f < fs.size(); ++f) {
         const std::string x = P.power(base_of(bases, fs[f].lf), fs[f].zeta, fs[f].iz);
-        body << "            acc_add(s" << f << ", " << x << ", w" << fs[f].damp << ");\n";
+        body << "            acc_add(s" << f << ", " << x << ", P" << fs[f].damp << ");\n";
     }
     os << body.str() << "            }\n";
     os << gen_reduce_store(fs.size(), "Acc", "Gb", true);
@@ -223,7 +267,7 @@ std::string gen_symm_body(const Engine &E, const DevBlockA &B)
     return os.str();
 }
 
-// Pair pass of one GAUSS block (see force_pairs_generic), relative to the
+// Pair pass of one block (see force_pairs_generic), relative to the
 // block's first dE/dG (eb); coefficients of pair (g, f) at g s + f - qoff
 // (qoff: no generated local may take a parameter's name).
 std::string gen_force_body(const Engine &E, const DevBlockA &B)
@@ -242,7 +286,7 @@ std::string gen_force_body(const Engine &E, const DevBlockA &B)
     std::ostringstream body;
     std::vector<float> bases;
     std::set<int> damps;
-    pair_prologue(body, fs, bases, damps, true);
+    pair_prologue(body, B, fs, bases, damps, true);
     Powers P(body);
     std::map<int, std::string> sc, sp;   // per damping group
     for (size_t f = 0; f < fs.size(); ++f) {
@@ -265,25 +309,29 @@ std::string gen_force_body(const Engine &E, const DevBlockA &B)
         const std::string s = sp[d].empty() ? "0.f" : sp[d];
         body << "            { const float gsc = " << c << ";\n";
         body << "              const float gsp = " << s << ";\n";
-        body << "              hc = fmaf(gsc, wa" << d << " * wb" << d << ", hc);\n";
-        body << "              hra = fmaf(gsp, da" << d << " * wb" << d << ", hra);\n";
-        body << "              hrb = fmaf(gsp, wa" << d << " * db" << d << ", hrb); }\n";
+        body << "              hc = fmaf(gsc, P" << d << ", hc);\n";
+        body << "              hra = fmaf(gsp, A" << d << ", hra);\n";
+        body << "              hrb = fmaf(gsp, B" << d << ", hrb); }\n";
     }
     body << "            pair_coeffs(v.pc, v.pcs, it.g * k.s + it.f - qoff, hc, hra, hrb, cs, ua.w, ub.w);\n";
     os << body.str() << "            }\n            return true;\n        }\n";
     return os.str();
 }
 
-// Radial term of one neighbour in the force kernel for a GAUSSIAN block:
-// amp = sum_f e_f dG_f/dr with dG_f/dr = exp(-g^2) (-2 eta g fc + fc'),
-// g = eta (r - rs), (rs, eta) as literals; relative to the block's first
-// dE/dG (eb).
+// Radial term of one neighbour in the force kernel: amp = sum_f e_f dG_f/dr,
+// (rs, eta) and the form as literals, for GAUSSIAN dG_f/dr = exp(-g^2) (-2 eta
+// g fc + fc'), g = eta (r - rs); relative to the block's first dE/dG (eb).
 std::string gen_radial_force_body(const Engine &E, const DevBlockR &B)
 {
     std::ostringstream os;
     os << "        {\n            float amp = 0.f;\n";
     for (int f = 0; f < B.n; ++f) {
         const float2 q = E.rpar_host[B.par + f];
+        if (B.form != RAD_GAUSSIAN) {
+            os << "            { float val, der; radial_fd(" << B.form << ", r, " << flit(q.x) << ", " << flit(q.y)
+               << ", fc, fcd, val, der); amp = fmaf(eb[" << f << "], der, amp); }\n";
+            continue;
+        }
         os << "            { const float g = " << flit(q.y) << " * (r - " << flit(q.x) << ");\n"
            << "              amp = fmaf(eb[" << f << "], expf(-g * g) * fmaf(" << flit(-2.f * q.y)
            << " * g, fc, fcd), amp); }\n";
@@ -389,9 +437,9 @@ std::string gen_radial_row_body(const Engine &E, const DevBlockR &B)
     return os.str();
 }
 
-// Tangent of one GAUSS block's symmetry functions along the displacement
-// field (see tangent_body): per pair dG_f = zeta lf x^(zeta-1) w_a w_b dcos
-// + x^zeta (w'_a w_b rr_a + w_a w'_b rr_b), relative to the block's first
+// Tangent of one block's symmetry functions along the displacement field
+// (see tangent_body): per pair dG_f = zeta lf x^(zeta-1) P dcos
+// + x^zeta (A rr_a + B rr_b), relative to the block's first
 // entry of the tangent row (Cb).
 std::string gen_tangent_body(const Engine &E, const DevBlockA &B)
 {
@@ -405,15 +453,14 @@ std::string gen_tangent_body(const Engine &E, const DevBlockA &B)
     std::ostringstream body;
     std::vector<float> bases;
     std::set<int> damps;
-    pair_prologue(body, fs, bases, damps, true);
+    pair_prologue(body, B, fs, bases, damps, true);
     body << "            const float rra = v.pc[a], rrb = v.pc[b];\n"
             "            const float uba = ub.x * v.gx[a] + ub.y * v.gy[a] + ub.z * v.gz[a];\n"
             "            const float uab = ua.x * v.gx[b] + ua.y * v.gy[b] + ua.z * v.gz[b];\n"
             "            const float dcos = (uba - cs * rra) * ua.w + (uab - cs * rrb) * ub.w;\n";
     for (int d : damps) {
-        body << "            const float W" << d << " = wa" << d << " * wb" << d << " * dcos;\n";
-        body << "            const float R" << d << " = fmaf(da" << d << " * wb" << d << ", rra, wa" << d << " * db" << d
-             << " * rrb);\n";
+        body << "            const float W" << d << " = P" << d << " * dcos;\n";
+        body << "            const float R" << d << " = fmaf(A" << d << ", rra, B" << d << " * rrb);\n";
     }
     Powers P(body);
     for (size_t f = 0; f < fs.size(); ++f) {
@@ -484,13 +531,13 @@ std::string make_source(const Engine &E, const TuneParams &tp)
     for (int II = 0; II < T; ++II)
         for (int J = 0; J < T; ++J) {
             const DevBlockR &B = E.dpot.t[II].br[J];
-            if (B.n > 0 && B.form == RAD_GAUSSIAN) ra.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_force_body(E, B));
+            if (B.n > 0) ra.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_force_body(E, B));
             if (B.n > 0 && E.mom_ok) rr.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_row_body(E, B));
         }
     for (int II = 0; II < T; ++II)
         for (int tt = 0; tt < TT; ++tt) {
             const DevBlockA &B = E.dpot.t[II].ba[tt];
-            if (B.n == 0 || B.form != ANG_GAUSS) continue;
+            if (B.n == 0) continue;
             na = std::max(na, B.n);
             if (E.mom_ok) {
                 fy.emplace_back(II * NNP_MAX_TT + tt, gen_few_symm_body(E, B));
