@@ -26,6 +26,9 @@ namespace {
 
 thread_local std::string g_create_error;
 
+constexpr size_t H_COUNT_OFF = 64;    // of the atom count behind the pinned error record
+static_assert(sizeof(nnp::DevErr) <= H_COUNT_OFF, "error record");
+
 int fail(nnp_handle *h, int code, const std::string &msg)
 {
     if (h) h->E.last_error = msg;
@@ -142,6 +145,9 @@ void Engine::free_all()
     if (h_stage) cudaFreeHost(h_stage);
     h_stage = nullptr;
     h_stage_bytes = 0;
+    if (h_out) cudaFreeHost(h_out);
+    h_out = nullptr;
+    h_out_bytes = 0;
     if (own_stream && stream) cudaStreamDestroy(stream);
     stream = nullptr;
     own_stream = false;
@@ -442,7 +448,7 @@ int finish_create(nnp_handle *h, nnp_handle **out)
         return fail(nullptr, NNP_ERR_CUDA, "cudaStreamCreate failed");
     }
     E.own_stream = true;
-    if (cudaMallocHost((void **)&E.h_err, sizeof(nnp::DevErr)) != cudaSuccess) {
+    if (cudaMallocHost((void **)&E.h_err, H_COUNT_OFF + sizeof(int64_t)) != cudaSuccess) {
         E.free_all();
         delete h;
         return fail(nullptr, NNP_ERR_CUDA, "cudaMallocHost failed");
@@ -493,6 +499,62 @@ cudaError_t h2d(nnp::Engine &E, void *dst, const void *src, size_t bytes, size_t
     stage_off += (bytes + 255) & ~(size_t)255;
     return cudaMemcpyAsync(dst, st, bytes, cudaMemcpyHostToDevice, E.stream);
 }
+
+// Results of a host-pointer call.  Small ones are copied to pinned memory
+// behind the step, so that the call waits once for results and error record
+// together and the caller's arrays are written only when it succeeds; a copy
+// to pageable memory waits for the device by itself, ~10 us each.  Larger ones,
+// and those whose arrays are pinned, are copied after the check.
+struct OutCopies {
+    struct Copy { void *dst; const void *src; size_t bytes; };
+    std::vector<Copy> list;
+    size_t bytes = 0;
+    bool staged = false;
+    void add(void *dst, const void *src, size_t n)
+    {
+        if (!dst || !n) return;
+        list.push_back({dst, src, n});
+        bytes += (n + 255) & ~(size_t)255;
+    }
+    // stage them if that pays; false: a CUDA error
+    cudaError_t enqueue(nnp::Engine &E)
+    {
+        constexpr size_t most = (size_t)8 << 20;
+        staged = !list.empty() && bytes <= most;
+        if (!staged) return cudaSuccess;
+        if (bytes > E.h_out_bytes) {
+            if (E.h_out) cudaFreeHost(E.h_out);
+            E.h_out = nullptr;
+            E.h_out_bytes = 0;
+            const size_t want = std::min(most, 2 * bytes + 4096);
+            const cudaError_t e = cudaMallocHost(&E.h_out, want);
+            if (e != cudaSuccess) return e;
+            E.h_out_bytes = want;
+        }
+        size_t o = 0;
+        for (const Copy &c : list) {
+            const cudaError_t e = cudaMemcpyAsync((char *)E.h_out + o, c.src, c.bytes, cudaMemcpyDeviceToHost, E.stream);
+            if (e != cudaSuccess) return e;
+            o += (c.bytes + 255) & ~(size_t)255;
+        }
+        return cudaSuccess;
+    }
+    // after the stream has been waited for and the step checked
+    cudaError_t finish(nnp::Engine &E)
+    {
+        size_t o = 0;
+        for (const Copy &c : list) {
+            if (staged) {
+                std::memcpy(c.dst, (char *)E.h_out + o, c.bytes);
+                o += (c.bytes + 255) & ~(size_t)255;
+            } else {
+                const cudaError_t e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, E.stream);
+                if (e != cudaSuccess) return e;
+            }
+        }
+        return staged || list.empty() ? cudaSuccess : cudaStreamSynchronize(E.stream);
+    }
+};
 
 int estimate_cap(const nnp_batch *b, double rc, int64_t n_ghost)
 {
@@ -879,11 +941,11 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
         if (b->pbc) chk(h2d(E, E.cell.p, b->cell, bc, so));
         if (ce != cudaSuccess) return fail(h, NNP_ERR_CUDA, std::string("input copy failed: ") + cudaGetErrorString(ce));
     } else {
-        int64_t n = 0;
-        chk(cudaMemcpyAsync(&n, b->atom_off + S, sizeof n, cudaMemcpyDeviceToHost, E.stream));
+        int64_t *n = reinterpret_cast<int64_t *>(reinterpret_cast<char *>(E.h_err) + H_COUNT_OFF);
+        chk(cudaMemcpyAsync(n, b->atom_off + S, sizeof *n, cudaMemcpyDeviceToHost, E.stream));
         chk(cudaStreamSynchronize(E.stream));
         if (ce != cudaSuccess) return fail(h, NNP_ERR_CUDA, std::string("reading atom count failed: ") + cudaGetErrorString(ce));
-        N = n;
+        N = *n;
         if (N < 0 || N >= (int64_t)1 << 28) return fail(h, NNP_ERR_ARG, "bad atom count in atom_off");
         if (E.cap < 128) E.cap = 128;
         // run on the caller's arrays in place
@@ -971,6 +1033,26 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
             msg = step();
         }
         if (!msg.empty()) { rc = fail(h, NNP_ERR_CUDA, msg); break; }
+        // results: behind the step where their arrays stay untouched if it failed
+        OutCopies out;
+        const bool plain = devp && !(flags & NNP_SYMM) && !atom_energy && !virial;
+        if (!devp) {
+            if (flags & NNP_ENERGY) out.add(energy, E.e_struct.p, sizeof(double) * S);
+            if (flags & NNP_FORCES) out.add(forces, E.force.p, sizeof(double) * 3 * N);
+            if (flags & NNP_SYMM) {
+                chk(E.symm_d.reserve((size_t)N * E.gstride + 1));
+                if (ce == cudaSuccess) nnp::run_symm_to_double(E, E.symm_d.p);
+                out.add(symm_out, E.symm_d.p, sizeof(double) * N * E.gstride);
+            }
+            if (atom_energy) {
+                nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, E.eatom_d.p);
+                out.add(atom_energy, E.eatom_d.p, sizeof(double) * (N - n_ghost));
+            }
+            if (virial) out.add(virial, E.vir.p, sizeof(double) * 9 * S);
+            if (ce == cudaSuccess) chk(out.enqueue(E));
+        } else if (plain && (energy || forces)) {
+            nnp::run_outputs(E, (flags & NNP_ENERGY) ? energy : nullptr, (flags & NNP_FORCES) ? forces : nullptr);
+        }
         chk(cudaMemcpyAsync(E.h_err, E.err.p, sizeof(nnp::DevErr), cudaMemcpyDeviceToHost, E.stream));
         chk(cudaStreamSynchronize(E.stream));
         if (ce != cudaSuccess) { rc = fail(h, NNP_ERR_CUDA, std::string("kernel failure: ") + cudaGetErrorString(ce)); break; }
@@ -1006,30 +1088,16 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
             if (!tm.empty()) { rc = fail(h, NNP_ERR_CUDA, tm); break; }
             continue;
         }
-        // outputs
         if (!devp) {
-            const size_t be = sizeof(double) * S, bf = sizeof(double) * 3 * N;
-            if ((flags & NNP_ENERGY) && energy) chk(cudaMemcpyAsync(energy, E.e_struct.p, be, cudaMemcpyDeviceToHost, E.stream));
-            if ((flags & NNP_FORCES) && forces) chk(cudaMemcpyAsync(forces, E.force.p, bf, cudaMemcpyDeviceToHost, E.stream));
-            if (flags & NNP_SYMM) {
-                chk(E.symm_d.reserve((size_t)N * E.gstride + 1));
-                nnp::run_symm_to_double(E, E.symm_d.p);
-                chk(cudaMemcpyAsync(symm_out, E.symm_d.p, sizeof(double) * N * E.gstride, cudaMemcpyDeviceToHost, E.stream));
-            }
-            if (atom_energy) {
-                nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, E.eatom_d.p);
-                chk(cudaMemcpyAsync(atom_energy, E.eatom_d.p, sizeof(double) * (N - n_ghost), cudaMemcpyDeviceToHost,
-                                    E.stream));
-            }
-            if (virial) chk(cudaMemcpyAsync(virial, E.vir.p, sizeof(double) * 9 * S, cudaMemcpyDeviceToHost, E.stream));
-        } else {
+            chk(out.finish(E));
+        } else if (!plain) {
             if ((flags & NNP_ENERGY) && energy) chk(cudaMemcpyAsync(energy, E.e_struct.p, sizeof(double) * S, cudaMemcpyDeviceToDevice, E.stream));
             if ((flags & NNP_FORCES) && forces) chk(cudaMemcpyAsync(forces, E.force.p, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, E.stream));
             if (flags & NNP_SYMM) nnp::run_symm_to_double(E, symm_out);
             if (atom_energy) nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, atom_energy);
             if (virial) chk(cudaMemcpyAsync(virial, E.vir.p, sizeof(double) * 9 * S, cudaMemcpyDeviceToDevice, E.stream));
+            chk(cudaStreamSynchronize(E.stream));
         }
-        chk(cudaStreamSynchronize(E.stream));
         if (ce != cudaSuccess) rc = fail(h, NNP_ERR_CUDA, std::string("output copy failed: ") + cudaGetErrorString(ce));
         break;
     }
@@ -1639,11 +1707,14 @@ int nnp_train_grad(nnp_handle *h, const nnp_batch *batch, const double *e_ref, c
     }
     msg = nnp::run_gather_grad(E, E.pack_idx.p, E.pack_n, E.grad_pack.p);
     if (!msg.empty()) return fail(h, NNP_ERR_CUDA, msg);
-    chk(cudaMemcpyAsync(loss, E.loss_part.p + S, sizeof(double), cudaMemcpyDeviceToHost, E.stream));
-    chk(cudaMemcpyAsync(grad, E.grad_pack.p, sizeof(double) * E.pack_n, cudaMemcpyDeviceToHost, E.stream));
-    if (e_out) chk(cudaMemcpyAsync(e_out, E.e_struct.p, sizeof(double) * S, cudaMemcpyDeviceToHost, E.stream));
-    if (f_out) chk(cudaMemcpyAsync(f_out, E.force.p, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, E.stream));
+    OutCopies out;
+    out.add(loss, E.loss_part.p + S, sizeof(double));
+    out.add(grad, E.grad_pack.p, sizeof(double) * E.pack_n);
+    out.add(e_out, E.e_struct.p, sizeof(double) * S);
+    out.add(f_out, E.force.p, sizeof(double) * 3 * N);
+    chk(out.enqueue(E));
     chk(cudaStreamSynchronize(E.stream));
+    if (ce == cudaSuccess) chk(out.finish(E));
     if (ce != cudaSuccess) return fail(h, NNP_ERR_CUDA, std::string("gradient failed: ") + cudaGetErrorString(ce));
     return NNP_OK;
 }

@@ -169,10 +169,12 @@ struct Engine {
     int loss_kind = 1;            // energy-loss kind of nnp_train_grad (NNP_LOSS_*)
     double loss_delta = 1.0;      // its width (HUBER, ASINH)
     float *noalloc_e_atom = nullptr;  // device address of the allocation-free call's scratch (looked up once)
-    DevErr *h_err = nullptr;      // pinned
+    DevErr *h_err = nullptr;      // pinned: the error record, then the atom count of device-pointer calls (H_COUNT_OFF)
     // pinned staging for host-pointer calls
     void *h_stage = nullptr;
     size_t h_stage_bytes = 0;
+    void *h_out = nullptr;          // the same for their results (OutCopies)
+    size_t h_out_bytes = 0;
 
     std::string last_error;
 
@@ -216,6 +218,7 @@ std::string run_force(Engine &E);
 std::string run_energy(Engine &E, bool vacuum);
 std::string run_symm_to_double(Engine &E, double *out);
 std::string run_atom_energy(Engine &E, bool vacuum, double *out);
+std::string run_outputs(Engine &E, double *energy, double *forces);
 std::string run_nn_from_symm(Engine &E, const double *symm_d, int gstride_in);
 std::string run_neighbor_counts(Engine &E, int *d_counts);
 std::string run_train_grad(Engine &E, bool with_force);

@@ -1951,6 +1951,27 @@ std::string run_atom_energy(Engine &E, bool vacuum, double *out)
     return cuda_msg("per-atom energies");
 }
 
+// Energies and forces to the caller's device arrays, unless the step failed in
+// a way that returns without results (the cases of compute_impl's checks).
+__global__ void k_outputs(const DevErr *__restrict__ err, int cap, int64_t ne, const double *__restrict__ es,
+                          double *__restrict__ energy, int64_t nf, const double *__restrict__ fs,
+                          double *__restrict__ forces)
+{
+    if (err->bad_type || err->bad_cell || err->need_cap > cap || err->nonfinite == 2) return;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = t; i < nf; i += step) forces[i] = fs[i];
+    for (int64_t i = t; i < ne; i += step) energy[i] = es[i];
+}
+
+std::string run_outputs(Engine &E, double *energy, double *forces)
+{
+    const int64_t ne = energy ? E.n_struct : 0, nf = forces ? 3 * E.n_atoms : 0;
+    k_outputs<<<grid_for(std::max(ne, nf), 512, num_sms() * 8), 256, 0, E.stream>>>(E.err.p, E.cap, ne, E.e_struct.p, energy,
+                                                                                 nf, E.force.p, forces);
+    E.launches += 1;
+    return cuda_msg("outputs");
+}
+
 std::string run_symm_to_double(Engine &E, double *out)
 {
     const int64_t n = E.n_atoms * E.gstride;
