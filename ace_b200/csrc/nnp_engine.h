@@ -56,7 +56,7 @@ struct TuneParams {
     int force_minb = 1;         // the same for the specialised force kernel (1..4)
     int force_unroll = 1;       // unroll factor of the specialised force kernel's pair loop (1..4)
     int force_chunk = NNP_PCH;  // pair coefficients per chunk of the force kernel (8..NNP_PCH); sets its shared memory
-    int tc_per_sm = 0;          // CTAs per SM of the tensor-core network kernel (0: as many as fit, at most 4)
+    int tc_per_sm = 0;          // tiles in flight per SM of the tensor-core network kernel (0: as many as fit, at most 4)
     bool operator==(const TuneParams &o) const
     {
         return symm_minb == o.symm_minb && force_minb == o.force_minb && force_unroll == o.force_unroll &&
@@ -231,7 +231,7 @@ std::string taylor_expand(int S, const int64_t *atom_off, const double *pos, con
                           const double *forces, int nadd, int dist, double rdelta, uint64_t seed,
                           std::vector<int64_t> &out_off, std::vector<int> &out_src, std::vector<double> &out_pos,
                           std::vector<double> &out_energy);
-int tc_smem_bytes(const Engine &E, bool split);     // 0: networks do not fit the tensor-core path
+int tc_fits(const Engine &E, bool split);           // 0: networks do not fit the tensor-core path
 std::string run_nn_tc(Engine &E, bool split);
 std::string run_energy_symm_noalloc(Engine &E, int S, int64_t N, const int64_t *off, const int *type,
                                     const float *G, int gstride, bool vacuum, double *energy);

@@ -1846,7 +1846,7 @@ std::string run_nn(Engine &E)
     const int64_t N = E.n_atoms;
     if (N == 0) return "";
     // BF16 / split-BF16 tensor-core layers when every network fits them
-    if (E.precision != NNP_PREC_FP32 && tc_smem_bytes(E, E.precision == NNP_PREC_BF16X3) > 0)
+    if (E.precision != NNP_PREC_FP32 && tc_fits(E, E.precision == NNP_PREC_BF16X3))
         return run_nn_tc(E, E.precision == NNP_PREC_BF16X3);
     if (const size_t smt = nnt_bytes(E)) {
         int L = E.dpot.t[0].nlayer;

@@ -13,9 +13,21 @@
 // BF16X3 every operand is split into hi + lo BF16 parts and each product is
 // hi*hi + hi*lo + lo*hi (FP32 accumulation), which keeps ~16 significant bits.
 //
-// One CTA = 4 warps; thread r owns row r of the tile (TMEM lane r).  Tiles are
-// enumerated element by element over the element-sorted atom order, and a CTA
-// restages its weights only when the element changes.
+// A tile is a chain of dependent MMAs and epilogues, so what matters is how many
+// tiles an SM has in flight.  A CTA (one per SM) has up to four warpgroups, each
+// with its own tile, sharing the element's weights; a tile keeps one operand
+// region in shared memory (an epilogue overwrites the operand its MMA has
+// consumed) and its f'(z) in TMEM columns behind the accumulator.  With weights
+// and f'(z) in every tile's shared memory 2 (56-32-32-1), 1 (64-48-48-1) and 1
+// (80-64-64-1) tiles fitted an SM, now 4, 3 and 2.  With the layer count as a
+// template parameter (plan and widths in registers) and TMEM read 16 columns at
+// a time: 1,088,749 atoms of three elements (56-32-32-1) 768 -> 433 us, 353,589
+// of four (64-48-48-1) 562 -> 251 us, 131,072 of two (80-64-64-1) 301 -> 175 us.
+// Bound: the serial chain of MMAs and epilogues of a tile.
+// Thread r of a warpgroup owns row r of its tile (TMEM lane r).  Tiles are taken
+// in groups of one per warpgroup, all of one element, element by element over
+// the element-sorted atom order; the CTA meets only to restage the weights when
+// the element changes.
 #include <cuda_bf16.h>
 
 #include "nnp_device.cuh"
@@ -27,70 +39,72 @@ namespace nnp {
 namespace {
 
 constexpr int TILE = 128;
-constexpr uint32_t TMEM_COLS = 128;          // widest padded layer (NNP_MAX_NODES)
+constexpr uint32_t TMEM_COLS = 512;           // allocated: all of the SM's
+constexpr int MAX_GROUPS = 4;                 // tiles in flight per CTA
 constexpr uint32_t WAIT_POLLS = 1u << 26;     // default bound of one MMA-chain wait (~0.1-1 s); the final drain always uses it
-constexpr int HEADER = 128;                   // mbarrier (8 B) and TMEM address slot (4 B); operands follow
+constexpr int HEADER = 128;                   // mbarriers (8 B each) and TMEM address slot (4 B); operands follow
 
 __host__ __device__ inline int pad16(int n) { return (n + 15) & ~15; }
+__host__ __device__ inline int pad8(int n) { return (n + 7) & ~7; }
 
-// Shared-memory plan of one network shape (identical on host and device).
+// Shared-memory and TMEM plan of one network shape (identical on host and device).
 struct TcPlan {
-    int L;                       // layers (hidden layers = L - 1)
     int P[NNP_MAX_LAYERS + 1];   // padded widths of every layer's input
     int wf[NNP_MAX_LAYERS];      // bf16 offset of W_h   [P_{h+1} x P_h]  (forward B operand)
     int wb[NNP_MAX_LAYERS];      // bf16 offset of W_h^T [P_h x P_{h+1}]  (backward B operand)
+    int dcol[NNP_MAX_LAYERS];    // TMEM column of f'(z_h), behind the accumulator
     int wbytes;                  // bytes of one copy (hi or lo) of all weight operands
-    int tile[NNP_MAX_LAYERS];    // bf16 offset of region h: A_h [128 x P_h] forward, D_h [128 x P_{h+1}] backward
-    int tbytes;                  // bytes of one copy of all activation regions
-    int dfloats;                 // f'(z_h) of every hidden layer, [n][128] FP32
-    int vfloats;                 // inpw, inpb, hidden biases, output-layer weights (FP32, after d)
-    int total;                   // bytes of the whole plan incl. the header
+    int tbytes;                  // bytes of one copy of a tile's operand region
+    int cols;                    // TMEM columns of one tile
+    int vfloats;                 // inpw, inpb, hidden biases, output-layer weights (FP32)
+    int copies;
+    __host__ __device__ int total(int groups) const { return HEADER + copies * (wbytes + groups * tbytes) + 4 * vfloats; }
 };
 
-__host__ __device__ inline void make_plan(const DevType &T, bool split, TcPlan &p)
+__host__ __device__ __forceinline__ void make_plan(int L, const int *nodes, bool split, TcPlan &p)
 {
-    p.L = T.nlayer;
-    for (int l = 0; l < T.nlayer; ++l) p.P[l] = pad16(T.nodes[l]);
-    int w = 0, t = 0, d = 0;
-    for (int h = 0; h + 1 < p.L; ++h) {
+    int w = 0, wide = 0;
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        p.P[l] = pad16(nodes[l]);
+        wide = wide > p.P[l] ? wide : p.P[l];
+    }
+    int col = (wide + 31) & ~31;
+#pragma unroll
+    for (int h = 0; h + 1 < L; ++h) {
         p.wf[h] = w;
         w += p.P[h + 1] * p.P[h];
         p.wb[h] = w;
         w += p.P[h] * p.P[h + 1];
-        p.tile[h] = t;
-        t += TILE * (p.P[h] > p.P[h + 1] ? p.P[h] : p.P[h + 1]);
-        d += TILE * T.nodes[h + 1];
+        p.dcol[h] = col;
+        col += pad8(nodes[h + 1]);
     }
     p.wbytes = w * 2;
-    p.tbytes = t * 2;
-    p.dfloats = d;
-    int v = 2 * T.nodes[0] + T.nodes[p.L - 1];
-    for (int h = 0; h + 1 < p.L; ++h) v += T.nodes[h + 1];
-    p.vfloats = v;
-    const int copies = split ? 2 : 1;
-    p.total = HEADER + copies * (p.wbytes + p.tbytes) + 4 * (d + v);
+    p.tbytes = TILE * wide * 2;
+    p.cols = (col + 31) & ~31;
+    int v = 2 * nodes[0] + nodes[L - 1];
+#pragma unroll
+    for (int h = 0; h + 1 < L; ++h) v += nodes[h + 1];
+    p.vfloats = (v + 3) & ~3;
+    p.copies = split ? 2 : 1;
 }
 
 struct Smem {
     __nv_bfloat16 *w_hi, *w_lo, *t_hi, *t_lo;
-    float *d;
     float *vec;        // [inpw | inpb | bias of hidden layer 0, 1, ... | W_out[0][n]]
-    uint64_t *bar;
-    uint32_t *slot;
+    uint64_t *bar;     // this warpgroup's
 };
 
-__device__ inline Smem carve(unsigned char *base, const TcPlan &p, bool split)
+__device__ inline Smem carve(unsigned char *base, const TcPlan &p, bool split, int group, int groups)
 {
     Smem s;
-    s.bar = reinterpret_cast<uint64_t *>(base);
-    s.slot = reinterpret_cast<uint32_t *>(base + 8);
+    s.bar = reinterpret_cast<uint64_t *>(base) + group;
     unsigned char *q = base + HEADER;
     s.w_hi = reinterpret_cast<__nv_bfloat16 *>(q); q += p.wbytes;
     s.w_lo = split ? reinterpret_cast<__nv_bfloat16 *>(q) : nullptr; q += split ? p.wbytes : 0;
-    s.t_hi = reinterpret_cast<__nv_bfloat16 *>(q); q += p.tbytes;
-    s.t_lo = split ? reinterpret_cast<__nv_bfloat16 *>(q) : nullptr; q += split ? p.tbytes : 0;
-    s.d = reinterpret_cast<float *>(q);
-    s.vec = s.d + p.dfloats;
+    s.t_hi = reinterpret_cast<__nv_bfloat16 *>(q + (size_t)group * p.copies * p.tbytes);
+    s.t_lo = split ? reinterpret_cast<__nv_bfloat16 *>(q + (size_t)group * p.copies * p.tbytes + p.tbytes) : nullptr;
+    s.vec = reinterpret_cast<float *>(q + (size_t)groups * p.copies * p.tbytes);
     return s;
 }
 
@@ -140,23 +154,24 @@ __device__ __forceinline__ void tc_activation(int neuron, float c, float z, floa
     }
 }
 
-// One MMA chain D[128 x N] = A[128 x K] * B[N x K]^T issued by thread 0 and
-// waited for by every thread, at most `polls` tests of the barrier each.
-// The result is the same in every thread of the block (a wait that gave up
-// in any thread fails it for all), so the block leaves its tile loop as one
-// and no thread is left at a barrier the others skip.  On failure the phase
-// is not advanced: the drain before the TMEM release waits for that chain.
-__device__ bool gemm(const Smem &s, int a_off, int b_off, int K, int N, bool split, uint32_t tmem, uint32_t &phase,
+// One MMA chain D[128 x N] = A[128 x K] * B[N x K]^T issued by the warpgroup's
+// first thread and waited for by every one of its threads, at most `polls`
+// tests of the barrier each.  The result is the same in every thread of the
+// group (a wait that gave up in any thread fails it for all), so the group
+// leaves its tile as one and no thread is left at a barrier the others skip.
+// On failure the phase is not advanced: the drain before the TMEM release
+// waits for that chain.
+__device__ bool gemm(const Smem &s, int group, int b_off, int K, int N, bool split, uint32_t tmem, uint32_t &phase,
                      uint32_t polls)
 {
     tc::fence_async_smem();
     tc::fence_before_sync();
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    tc::group_sync(group + 1);
+    if ((threadIdx.x & (TILE - 1)) == 0) {
         tc::fence_after_sync();
         const uint32_t id = tc::idesc_bf16(TILE, N);
         const uint32_t sbo = (K / 8) * 128;
-        const uint32_t a_hi = tc::smem_u32(s.t_hi + a_off), b_hi = tc::smem_u32(s.w_hi + b_off);
+        const uint32_t a_hi = tc::smem_u32(s.t_hi), b_hi = tc::smem_u32(s.w_hi + b_off);
         uint32_t acc = 0;
         for (int kk = 0; kk < K / 16; ++kk) {
             const uint64_t ad = tc::sdesc(a_hi + kk * 256, 128, sbo);
@@ -164,14 +179,14 @@ __device__ bool gemm(const Smem &s, int a_off, int b_off, int K, int N, bool spl
             tc::mma_bf16(tmem, ad, bd, id, acc);
             acc = 1;
             if (split) {
-                const uint32_t a_lo = tc::smem_u32(s.t_lo + a_off), b_lo = tc::smem_u32(s.w_lo + b_off);
+                const uint32_t a_lo = tc::smem_u32(s.t_lo), b_lo = tc::smem_u32(s.w_lo + b_off);
                 tc::mma_bf16(tmem, ad, tc::sdesc(b_lo + kk * 256, 128, sbo), id, 1);
                 tc::mma_bf16(tmem, tc::sdesc(a_lo + kk * 256, 128, sbo), bd, id, 1);
             }
         }
         tc::mma_commit(s.bar);
     }
-    const bool ok = __syncthreads_and(tc::mbar_wait(s.bar, phase, polls)) != 0;
+    const bool ok = tc::group_sync_and(group + 1, tc::mbar_wait(s.bar, phase, polls));
     if (ok) phase ^= 1u;
     tc::fence_after_sync();
     return ok;
@@ -179,80 +194,71 @@ __device__ bool gemm(const Smem &s, int a_off, int b_off, int K, int N, bool spl
 
 }  // namespace
 
-template <bool SPLIT>
-__global__ void __launch_bounds__(TILE) k_nn_tc(const DevPot *__restrict__ pot, const float *__restrict__ wpar,
-                                                const int *__restrict__ type_count, const int *__restrict__ order,
-                                                const float *__restrict__ G, int gstride, float *__restrict__ e_atom,
-                                                float *__restrict__ dEdG, DevErr *err, uint32_t polls)
+// LT: number of layers when every element has that many (plan and widths are then
+// registers; 0: any)
+template <bool SPLIT, int LT>
+__global__ void __launch_bounds__(MAX_GROUPS * TILE) k_nn_tc(const DevPot *__restrict__ pot,
+                                                             const float *__restrict__ wpar,
+                                                             const int *__restrict__ type_count,
+                                                             const int *__restrict__ order, const float *__restrict__ G,
+                                                             int gstride, float *__restrict__ e_atom,
+                                                             float *__restrict__ dEdG, DevErr *err, uint32_t polls)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const DevPot &P = *pot;
-    const int t = threadIdx.x, warp = t >> 5;
-    // tiles per element and the first one of each
-    int first[NNP_MAX_TYPES + 1], base[NNP_MAX_TYPES + 1];
-    first[0] = 0;
-    base[0] = 0;
-    for (int T = 0; T < P.ntypes; ++T) {
-        const int c = type_count[T];
-        first[T + 1] = first[T] + (c + TILE - 1) / TILE;
-        base[T + 1] = base[T] + c;
-    }
-    const int ntiles = first[P.ntypes];
-    Smem s0;
-    s0.bar = reinterpret_cast<uint64_t *>(smem_raw);
-    s0.slot = reinterpret_cast<uint32_t *>(smem_raw + 8);
-    if (t == 0) {
-        tc::mbar_init(s0.bar, 1);
+    const int group = threadIdx.x / TILE, groups = blockDim.x / TILE, t = threadIdx.x & (TILE - 1);
+    const int warp = threadIdx.x >> 5;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(smem_raw + 8 * MAX_GROUPS);
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < groups; ++q) tc::mbar_init(bars + q, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tc::tmem_alloc(s0.slot, TMEM_COLS);
+    if (warp == 0) tc::tmem_alloc(slot, TMEM_COLS);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = *s0.slot;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    const uint32_t tmem_base = *slot;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t phase = 0;
-    int staged = -1;
+    int staged = -1, T = 0, first = 0, base = 0;   // element, its first tile group and atom
     bool ok = true;
-    // The first 64 values of this thread's G row of the next tile are loaded
-    // into registers while the current tile computes.
-    float4 row[16];
-    auto fetch_row = [&](int gg) {
-        if (gg >= ntiles) return;
-        int Tn = 0;
-        while (gg >= first[Tn + 1]) ++Tn;
-        const int jn = (gg - first[Tn]) * TILE + t;
-        const bool ln = jn < type_count[Tn];
-        const float *Gn = G + (ln ? order[base[Tn] + jn] : 0) * (i64)gstride;
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-            row[q] = (ln && 4 * q + 4 <= gstride) ? *reinterpret_cast<const float4 *>(Gn + 4 * q)
-                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    fetch_row(blockIdx.x);
-    for (int g = blockIdx.x; g < ntiles && ok; g += gridDim.x) {
-        int T = 0;
-        while (g >= first[T + 1]) ++T;
+    for (int g = blockIdx.x;; g += gridDim.x) {
+        while (T < P.ntypes) {
+            const int n = (type_count[T] + groups * TILE - 1) / (groups * TILE);
+            if (g < first + n) break;
+            first += n;
+            base += type_count[T];
+            ++T;
+        }
+        if (T == P.ntypes) break;                  // uniform over the CTA
         const DevType &DT = P.t[T];
+        const int L = LT ? LT : DT.nlayer;
+        int nd[LT ? LT + 1 : NNP_MAX_LAYERS + 1];
+#pragma unroll
+        for (int l = 0; l <= (LT ? LT : L); ++l) nd[l] = DT.nodes[l];
         TcPlan p;
-        make_plan(DT, SPLIT, p);
-        const Smem s = carve(smem_raw, p, SPLIT);
+        make_plan(L, nd, SPLIT, p);
+        const Smem s = carve(smem_raw, p, SPLIT, group, groups);
+        const uint32_t tmem = tmem_base + group * p.cols;
         const float *net = wpar + DT.woff;
-        const int L = DT.nlayer, nin = DT.nodes[0], nout = DT.nodes[L];
+        const int nin = nd[0], nout = nd[L];
         const float *inpw = net, *inpb = net + nin, *outw = net + 2 * nin, *outb = outw + nout;
         const float *b_out, *w_out;
         int ws_out;
         layer_ptrs(net, DT, L - 1, b_out, w_out, ws_out);
         // ---- weights of this element in the operand layouts (zero padded)
         if (staged != T) {
-            __syncthreads();
+            __syncthreads();                       // every group is done with the previous element
+#pragma unroll
             for (int h = 0; h + 1 < L; ++h) {
-                const int ni = DT.nodes[h], no = DT.nodes[h + 1], Pi = p.P[h], Po = p.P[h + 1];
+                const int ni = nd[h], no = nd[h + 1], Pi = p.P[h], Po = p.P[h + 1];
                 const float *bh, *wth;
                 int ws;
                 layer_ptrs(net, DT, h, bh, wth, ws);
-                for (int q = t; q < Po * Pi; q += TILE) {
-                    const int n = q / Pi, m = q - n * Pi;       // W[n][m], n < Po (out), m < Pi (in)
+#pragma unroll 4
+                for (int q = threadIdx.x; q < Po * Pi; q += blockDim.x) {
+                    const int m = q / Po, n = q - m * Po;       // W[n][m], n < Po (out), m < Pi (in)
                     const float w = (n < no && m < ni) ? wth[m * ws + n] : 0.f;
                     const __nv_bfloat16 hi = __float2bfloat16_rn(w);
                     s.w_hi[p.wf[h] + tc::kmaj(n, m, Pi)] = hi;
@@ -267,7 +273,7 @@ __global__ void __launch_bounds__(TILE) k_nn_tc(const DevPot *__restrict__ pot, 
             // per-element vectors, read by every thread in the epilogues
             {
                 float *vb = s.vec + 2 * nin;
-                for (int q = t; q < nin; q += TILE) {
+                for (int q = threadIdx.x; q < nin; q += blockDim.x) {
                     s.vec[q] = inpw[q];
                     s.vec[nin + q] = inpb[q];
                 }
@@ -275,168 +281,137 @@ __global__ void __launch_bounds__(TILE) k_nn_tc(const DevPot *__restrict__ pot, 
                     const float *bh, *wth;
                     int ws;
                     layer_ptrs(net, DT, h, bh, wth, ws);
-                    for (int q = t; q < DT.nodes[h + 1]; q += TILE) vb[q] = bh[q];
-                    vb += DT.nodes[h + 1];
+                    for (int q = threadIdx.x; q < nd[h + 1]; q += blockDim.x) vb[q] = bh[q];
+                    vb += nd[h + 1];
                 }
-                for (int q = t; q < DT.nodes[L - 1]; q += TILE) vb[q] = w_out[q * ws_out];
+                for (int q = threadIdx.x; q < nd[L - 1]; q += blockDim.x) vb[q] = w_out[q * ws_out];
             }
             staged = T;
-            __syncthreads();        // the vectors are read below by every thread (A_0 conversion)
+            tc::fence_async_smem();
+            __syncthreads();
         }
+        const int a0 = ((g - first) * groups + group) * TILE;    // this group's tile of the element
+        if (!ok || a0 >= type_count[T]) continue;                // (uniform over the group)
         const int neuron = DT.neuron;
         const float cn = DT.c, outw0 = outw[0], eoff = outb[0] + b_out[0] * outw[0];
-        const float *v_inpw = s.vec, *v_inpb = s.vec + nin, *v_wout = s.vec + p.vfloats - DT.nodes[L - 1];
+        const float *v_inpw = s.vec, *v_inpb = s.vec + nin, *v_bias = s.vec + 2 * nin;
+        const float *v_wout = v_bias;
+#pragma unroll
+        for (int h = 0; h + 1 < L; ++h) v_wout += nd[h + 1];
         // ---- this thread's atom
-        const int j = (g - first[T]) * TILE + t;
-        const bool live = j < type_count[T];
-        const i64 i = live ? order[base[T] + j] : 0;
+        const bool live = a0 + t < type_count[T];
+        const i64 i = live ? order[base + a0 + t] : 0;
         // A_0 = inpw * (G + inpb), zero padded; the row is read as float4
-        // (gstride is a multiple of 4 and rows start 16-byte aligned): the
-        // first 64 values prefetched during the previous tile, the rest here
+        // (gstride is a multiple of 4 and rows start 16-byte aligned)
         {
-#pragma unroll
-            for (int k0 = 0; k0 < 64; k0 += 8) {            // from the prefetched registers
-                if (k0 < p.P[0]) {
-                    const float4 lo4 = row[k0 / 4], hi4 = row[k0 / 4 + 1];
-                    const float g8[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
-                    float v[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const int k = k0 + q;
-                        v[q] = (live && k < nin) ? v_inpw[k] * (g8[q] + v_inpb[k]) : 0.f;
-                    }
-                    store8(s.t_hi, SPLIT ? s.t_lo : nullptr, p.tile[0] + tc::kmaj(t, k0, p.P[0]), v);
-                }
-            }
             const float *Gi = G + i * gstride;
 #pragma unroll 4
-            for (int k0 = 64; k0 < p.P[0]; k0 += 8) {
+            for (int k0 = 0; k0 < p.P[0]; k0 += 8) {
                 float4 lo4 = make_float4(0.f, 0.f, 0.f, 0.f), hi4 = lo4;
                 if (live && k0 + 4 <= gstride) lo4 = *reinterpret_cast<const float4 *>(Gi + k0);
                 if (live && k0 + 8 <= gstride) hi4 = *reinterpret_cast<const float4 *>(Gi + k0 + 4);
-                const float g[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+                const float g8[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
                 float v[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const int k = k0 + q;
-                    v[q] = (live && k < nin) ? v_inpw[k] * (g[q] + v_inpb[k]) : 0.f;
+                    v[q] = (live && k < nin) ? v_inpw[k] * (g8[q] + v_inpb[k]) : 0.f;
                 }
-                store8(s.t_hi, SPLIT ? s.t_lo : nullptr, p.tile[0] + tc::kmaj(t, k0, p.P[0]), v);
+                store8(s.t_hi, SPLIT ? s.t_lo : nullptr, tc::kmaj(t, k0, p.P[0]), v);
             }
         }
-        fetch_row(g + gridDim.x);
         // ---- forward through the hidden layers
         float e = 0.f;
-        for (int h = 0; h + 1 < L && ok; ++h) {
-            const int no = DT.nodes[h + 1], Po = p.P[h + 1];
-            ok = gemm(s, p.tile[h], p.wf[h], p.P[h], Po, SPLIT, tmem, phase, polls);
+        const float *bh = v_bias;
+#pragma unroll
+        for (int h = 0; h + 1 < L; ++h) {
+            if (!ok) break;
+            const int no = nd[h + 1], Po = p.P[h + 1];
+            ok = gemm(s, group, p.wf[h], p.P[h], Po, SPLIT, tmem, phase, polls);
             if (!ok) break;
             const bool last = (h + 2 == L);
-            int doff = 0, boff = 2 * nin;
-            for (int q = 0; q < h; ++q) {
-                doff += TILE * DT.nodes[q + 1];
-                boff += DT.nodes[q + 1];
-            }
-            float *dh = s.d + doff;
-            const float *bh = s.vec + boff;
-            for (int c0 = 0; c0 < Po; c0 += 32) {
-                uint32_t r[4][8];                        // up to 32 columns in flight
+#pragma unroll 1
+            for (int c0 = 0; c0 < Po; c0 += 16) {
+                uint32_t r[2][8];
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < 2; ++u)
                     if (c0 + 8 * u < Po) tc::tmem_ld8_raw(tmem + lane_base + c0 + 8 * u, r[u]);
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < 2; ++u)
                     if (c0 + 8 * u < Po) tc::tmem_wait_tie(r[u]);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < 2; ++u) {
                     const int cb = c0 + 8 * u;
                     if (cb >= Po) break;
-                    float out[8];
+                    float out[8], d8[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int n = cb + q;
                         out[q] = 0.f;
+                        d8[q] = 0.f;
                         if (n < no) {
-                            float a, d;
-                            tc_activation(neuron, cn, __uint_as_float(r[u][q]) + bh[n], a, d);
-                            dh[n * TILE + t] = d;
+                            float a;
+                            tc_activation(neuron, cn, __uint_as_float(r[u][q]) + bh[n], a, d8[q]);
                             if (last) {
                                 // output layer: e = b + sum_n W[0][n] a_n; D = outw W[0][n] f'(z_n)
                                 const float wo = v_wout[n];
                                 e = fmaf(wo, a, e);
-                                out[q] = outw0 * wo * d;
+                                out[q] = outw0 * wo * d8[q];
                             } else {
                                 out[q] = a;
                             }
                         }
                     }
+                    if (!last && cb < pad8(no)) tc::tmem_st8(tmem + lane_base + p.dcol[h] + cb, d8);
                     // next layer's input A_{h+1}, or (last hidden layer) the first
-                    // backward operand D_h in region h; both have K = P_{h+1}
-                    store8(s.t_hi, SPLIT ? s.t_lo : nullptr, p.tile[last ? h : h + 1] + tc::kmaj(t, cb, Po), out);
+                    // backward operand D_h; both have K = P_{h+1}
+                    store8(s.t_hi, SPLIT ? s.t_lo : nullptr, tc::kmaj(t, cb, Po), out);
                 }
             }
+            if (!last) tc::tmem_wait_st();
+            bh += no;
             if (last && live) e_atom[i] = eoff + e * outw0;
         }
-        if (!ok) break;
-        // ---- backward: D_{h-1} = (D_h W_h) * f'(z_{h-1}), dE/dG = (D_0 W_0) * inpw;
-        // D_h sits in region h with K = P_{h+1}
-        for (int h = L - 2; h >= 0 && ok; --h) {
-            const int Pi = p.P[h], Po = p.P[h + 1];
-            ok = gemm(s, p.tile[h], p.wb[h], Po, Pi, SPLIT, tmem, phase, polls);
+        // ---- backward: D_{h-1} = (D_h W_h) * f'(z_{h-1}), dE/dG = (D_0 W_0) * inpw
+#pragma unroll
+        for (int h = L - 2; h >= 0; --h) {
             if (!ok) break;
-            if (h > 0) {
-                int doff = 0;
-                for (int q = 0; q < h - 1; ++q) doff += TILE * DT.nodes[q + 1];
-                const float *dprev = s.d + doff;
-                const int ni = DT.nodes[h];
-                for (int c0 = 0; c0 < Pi; c0 += 32) {
-                    uint32_t r[4][8];
+            const int Pi = p.P[h], Po = p.P[h + 1];
+            ok = gemm(s, group, p.wb[h], Po, Pi, SPLIT, tmem, phase, polls);
+            if (!ok) break;
+            const int ni = nd[h];
+            float *o = dEdG + i * gstride;
+#pragma unroll 1
+            for (int c0 = 0; c0 < Pi; c0 += 16) {
+                uint32_t r[2][8], f[2][8];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (c0 + 8 * u < Pi) tc::tmem_ld8_raw(tmem + lane_base + c0 + 8 * u, r[u]);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (c0 + 8 * u < Pi) tc::tmem_wait_tie(r[u]);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int cb = c0 + 8 * u;
-                        if (cb >= Pi) break;
-                        float out[8];
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const int n = cb + q;
-                            out[q] = (n < ni) ? __uint_as_float(r[u][q]) * dprev[n * TILE + t] : 0.f;
-                        }
-                        store8(s.t_hi, SPLIT ? s.t_lo : nullptr, p.tile[h - 1] + tc::kmaj(t, cb, Pi), out);
+                for (int u = 0; u < 2; ++u)
+                    if (c0 + 8 * u < Pi) {
+                        tc::tmem_ld8_raw(tmem + lane_base + c0 + 8 * u, r[u]);
+                        if (h > 0 && c0 + 8 * u < pad8(ni)) tc::tmem_ld8_raw(tmem + lane_base + p.dcol[h > 0 ? h - 1 : 0] + c0 + 8 * u, f[u]);
                     }
-                }
-            } else {
-                // dE/dG row, written as float4 (gstride is a multiple of 4)
-                float *o = dEdG + i * gstride;
-                for (int c0 = 0; c0 < Pi; c0 += 32) {
-                    uint32_t r[4][8];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (c0 + 8 * u < Pi) tc::tmem_ld8_raw(tmem + lane_base + c0 + 8 * u, r[u]);
+                for (int u = 0; u < 2; ++u)
+                    if (c0 + 8 * u < Pi) {
+                        tc::tmem_wait_tie(r[u]);
+                        if (h > 0 && c0 + 8 * u < pad8(ni)) tc::tmem_wait_tie(f[u]);
+                    }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (c0 + 8 * u < Pi) tc::tmem_wait_tie(r[u]);
-                    if (live) {
+                for (int u = 0; u < 2; ++u) {
+                    const int cb = c0 + 8 * u;
+                    if (cb >= Pi) break;
+                    float w[8];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int cb = c0 + 8 * u;
-                            if (cb >= Pi) break;
-                            float w[8];
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) {
-                                const int n = cb + q;
-                                w[q] = (n < nin) ? __uint_as_float(r[u][q]) * v_inpw[n] : 0.f;
-                            }
-                            if (cb + 4 <= gstride)
-                                *reinterpret_cast<float4 *>(o + cb) = make_float4(w[0], w[1], w[2], w[3]);
-                            if (cb + 8 <= gstride)
-                                *reinterpret_cast<float4 *>(o + cb + 4) = make_float4(w[4], w[5], w[6], w[7]);
-                        }
+                    for (int q = 0; q < 8; ++q) {
+                        const int n = cb + q;
+                        w[q] = (n < ni) ? __uint_as_float(r[u][q]) * (h > 0 ? __uint_as_float(f[u][q]) : v_inpw[n]) : 0.f;
+                    }
+                    if (h > 0) {
+                        store8(s.t_hi, SPLIT ? s.t_lo : nullptr, tc::kmaj(t, cb, Pi), w);
+                    } else if (live) {
+                        // dE/dG row, written as float4 (gstride is a multiple of 4)
+                        if (cb + 4 <= gstride) *reinterpret_cast<float4 *>(o + cb) = make_float4(w[0], w[1], w[2], w[3]);
+                        if (cb + 8 <= gstride) *reinterpret_cast<float4 *>(o + cb + 4) = make_float4(w[4], w[5], w[6], w[7]);
                     }
                 }
             }
@@ -444,56 +419,78 @@ __global__ void __launch_bounds__(TILE) k_nn_tc(const DevPot *__restrict__ pot, 
     }
     if (!ok && t == 0) atomicMax(&err->nonfinite, 2);
     // every issued MMA chain was waited for unless a wait gave up (in every
-    // thread alike); then the chain still in flight is waited for once more,
-    // with the full default bound, before the TMEM is released
-    if (!ok) tc::mbar_wait(s0.bar, phase, WAIT_POLLS);
+    // thread of the group alike); then the chain still in flight is waited for
+    // once more, with the full default bound, before the TMEM is released
+    if (!ok) tc::mbar_wait(bars + group, phase, WAIT_POLLS);
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, TMEM_COLS);
+    if (warp == 0) tc::tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// Shared-memory bytes of the largest element's plan, or 0 when the networks
-// do not fit the tensor-core path (output layer wider than one neuron, no
-// hidden layer, a layer wider than 128, or shared memory above the CTA limit).
-int tc_smem_bytes(const Engine &E, bool split)
+// Bytes of a tile that keeps every layer's operands and f'(z) to itself.  A
+// network is computed in BF16 if those fit an SM's shared memory: larger ones
+// have always kept FP32 networks under every precision setting, and a result
+// that was FP32 stays so although the shared plan would hold more.
+static int64_t tc_plain_bytes(const DevType &T, const TcPlan &p)
 {
-    int big = 0;
+    int64_t tile = 0, slope = 0;
+    for (int h = 0; h + 1 < T.nlayer; ++h) {
+        tile += 2 * TILE * std::max(p.P[h], p.P[h + 1]);
+        slope += 4 * TILE * T.nodes[h + 1];
+    }
+    return HEADER + p.copies * (p.wbytes + tile) + slope + 4 * p.vfloats;
+}
+
+// Tiles in flight that the networks' largest shapes allow in one CTA (shared
+// memory, TMEM columns), at most `most`; 0 when they do not fit the tensor-core
+// path (output layer wider than one neuron, no hidden layer, a layer wider than
+// 128, a tile of more than an SM's shared memory).
+static int tc_groups(const Engine &E, bool split, int most, int *bytes)
+{
+    int groups = std::min(most, MAX_GROUPS), big = 0;
     for (int T = 0; T < E.dpot.ntypes; ++T) {
         const DevType &DT = E.dpot.t[T];
         if (DT.nlayer < 2 || DT.nodes[DT.nlayer] != 1) return 0;
         for (int l = 0; l < DT.nlayer; ++l)
-            if (pad16(DT.nodes[l]) > (int)TMEM_COLS) return 0;
+            if (pad16(DT.nodes[l]) > 128) return 0;
         TcPlan p;
-        make_plan(DT, split, p);
-        big = std::max(big, p.total);
+        make_plan(DT.nlayer, DT.nodes, split, p);
+        if (tc_plain_bytes(DT, p) > 227 * 1024) return 0;
+        groups = std::min(groups, (int)TMEM_COLS / p.cols);
+        while (groups > 0 && p.total(groups) > 227 * 1024) --groups;
     }
-    return big <= 227 * 1024 ? big : 0;
+    for (int T = 0; T < E.dpot.ntypes; ++T) {
+        TcPlan p;
+        make_plan(E.dpot.t[T].nlayer, E.dpot.t[T].nodes, split, p);
+        big = std::max(big, p.total(groups));
+    }
+    if (bytes) *bytes = big;
+    return groups;
 }
+
+int tc_fits(const Engine &E, bool split) { return tc_groups(E, split, 1, nullptr); }
 
 std::string run_nn_tc(Engine &E, bool split)
 {
     const int64_t N = E.n_atoms;
     if (N == 0) return "";
-    const int sm = tc_smem_bytes(E, split);
-    if (sm == 0) return "networks do not fit the tensor-core path";
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // at most 4 CTAs per SM: 4 x 128 TMEM columns is the SM's 512
-    int per_sm = std::max(1, std::min(4, (228 * 1024) / (sm + 1024)));
-    if (E.tune.tc_per_sm > 0) per_sm = std::min(per_sm, E.tune.tc_per_sm);   // autotuned (nnp_tune.cpp)
+    // a tile per SM before a second one on any
     const int64_t tiles = (N + TILE - 1) / TILE + E.dpot.ntypes;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)nsm * per_sm));
+    int most = (int)std::min<int64_t>(MAX_GROUPS, (tiles + nsm - 1) / nsm), sm = 0;
+    if (E.tune.tc_per_sm > 0) most = std::min(most, E.tune.tc_per_sm);   // autotuned (nnp_tune.cpp)
+    const int groups = tc_groups(E, split, most, &sm);
+    if (groups == 0) return "networks do not fit the tensor-core path";
+    const int grid = (int)std::min<int64_t>((tiles + groups - 1) / groups + E.dpot.ntypes, nsm);
     const uint32_t polls = E.mma_wait_polls > 0 ? E.mma_wait_polls : WAIT_POLLS;
-    if (split) {
-        cudaFuncSetAttribute(k_nn_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        k_nn_tc<true><<<grid, TILE, sm, E.stream>>>(E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride,
-                                                   E.e_atom.p, E.dEdG.p, E.err.p, polls);
-    } else {
-        cudaFuncSetAttribute(k_nn_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        k_nn_tc<false><<<grid, TILE, sm, E.stream>>>(E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride,
-                                                    E.e_atom.p, E.dEdG.p, E.err.p, polls);
-    }
+    int L = E.dpot.t[0].nlayer;
+    for (int T = 1; T < E.dpot.ntypes; ++T) L = E.dpot.t[T].nlayer == L ? L : 0;
+    auto kern = L == 3 ? (split ? k_nn_tc<true, 3> : k_nn_tc<false, 3>) : (split ? k_nn_tc<true, 0> : k_nn_tc<false, 0>);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    kern<<<grid, groups * TILE, sm, E.stream>>>(E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride,
+                                                E.e_atom.p, E.dEdG.p, E.err.p, polls);
     E.launches += 1;
     E.mark(3);
     cudaError_t e = cudaGetLastError();

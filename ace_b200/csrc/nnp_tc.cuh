@@ -122,6 +122,37 @@ __device__ __forceinline__ void tmem_ld8_raw(uint32_t taddr, uint32_t (&r)[8])
                  : "r"(taddr));
 }
 
+// 8 consecutive 32-bit columns of this thread's TMEM lane written (warp-collective),
+// visible to its later loads after tmem_wait_st
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+                 "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+                 "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// barrier over the 128 threads of one warpgroup (id 1 ..), and the same with
+// the conjunction of a predicate over them
+__device__ __forceinline__ void group_sync(int id) { asm volatile("barrier.cta.sync %0, 128;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ bool group_sync_and(int id, bool v)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %2, 0;\n\t"
+        "barrier.cta.red.and.pred q, %1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"(id), "r"(v ? 1u : 0u)
+        : "memory");
+    return r != 0;
+}
+
 // Waits for this thread's outstanding TMEM loads, with the registers of one
 // x8 load as operands, so that no use of them is scheduled before the wait
 __device__ __forceinline__ void tmem_wait_tie(uint32_t (&r)[8])

@@ -3,7 +3,7 @@
 // The specialised symmetry-function and force kernels are compiled with
 // register budgets (resident blocks per SM), a pair-loop unroll factor and a
 // coefficient chunk size (TuneParams, nnp_engine.h); the tensor-core network
-// kernel runs a number of CTAs per SM.  Which values are fastest depends on
+// kernel has a number of tiles in flight per SM.  Which values are fastest depends on
 // the potential (block sizes, damping groups, network widths), on the
 // neighbour counts of the workload and on the GPU.  On the first call of a
 // neighbour-capacity class the tuner compiles a small set of candidates (in

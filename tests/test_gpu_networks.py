@@ -38,3 +38,28 @@ def test_network_tiles_match_oracle(tmp_path, hidden, counts):
     vac = sum(pot.types[t].energy for t in b.type[s])
     assert abs(nn.compute_energy(b.type[s], G[s]) - vac - E[2]) < 2e-6 * counts[2] + 1e-6 * abs(vac)
     nn.close()
+
+
+@pytest.mark.parametrize("hidden", [[[32, 32]], [[48, 48], [16]], [[64, 64], [20, 20], [7, 33, 9]]], ids=str)
+@pytest.mark.parametrize("n_struct", [1, 120, 330])
+def test_tensor_core_tiles_in_flight(tmp_path, hidden, n_struct):
+    """One to four tiles of 128 atoms in flight per SM, elements with different
+    layer counts, the last element's last tile ragged: BF16X3 against FP32
+    networks.  ~16 significant bits of operands of order 1 through two or three
+    layers: 2e-5 eV/atom, 2e-4 eV/A as against the reference's outputs."""
+    nt = len(hidden)
+    pot = synth.make_potential(nt, 4.5, 16, [8] * (nt * (nt + 1) // 2), [4], 3)
+    rng = np.random.default_rng(6)
+    for i, h in enumerate(hidden):
+        pot.nets[i] = synth.xavier_net(rng, [pot.n_input(i)] + h + [1], "TANH")
+        pot.nets[i].inpw = np.full(pot.n_input(i), 0.25)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    b = synth.batch_random(3, [201] * n_struct, nt)
+    nn = NNP.read(path)
+    E0, F0 = nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    nn.set_precision(2)
+    E, F = nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    assert (np.abs(E - E0) / 201).max() < 2e-5 and np.abs(F - F0).max() < 2e-4
+    assert np.abs(F - F0).max() > 0                             # the tensor cores ran
+    nn.close()
