@@ -125,7 +125,7 @@ void Engine::free_all()
 {
     rpar.release(); apar.release(); wpar.release(); vac.release();
     rpar64.release(); apar64.release(); cut64.release();
-    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release();
+    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release(); len_order.release();
     atom_off.release(); pos.release(); cell.release(); xw.release();
     type.release(); atom_struct.release(); atom_cell.release(); grid.release(); bbox.release();
     cell_cnt.release(); cell_start.release(); cell_fill.release(); cell_atoms.release(); scan_tmp.release();
@@ -347,12 +347,16 @@ void Engine::build_moments()
     std::vector<float> tab(mom_tab_floats(T, L, mom_fmax), 0.f);
     float *p = tab.data();
     const int NC = mom_comps(L), TT1 = L + 2;
+    mom_norm.assign(NC, 0.0);
+    mom_gnorm.assign(NC, 0.0);
     auto put = [&](int c, int l, int m) {
         double n = (m ? 2.0 : 1.0), lead = 1.0;
         for (int q = l - m + 1; q <= l + m; ++q) n /= q;               // (2 - delta) (l-m)!/(l+m)!
         for (int q = 1; q <= l; ++q) lead *= (2.0 * q - 1.0) / q;      // (2l)!/(2^l l!^2)
         for (int q = l - m + 1; q <= l; ++q) lead *= q;                // l!/(l-m)!
-        p[c] = (float)(std::sqrt(n) * lead);
+        mom_norm[c] = mom_gnorm[c] = std::sqrt(n) * lead;
+        for (int q = 2; q <= l - m; ++q) mom_gnorm[c] *= q;
+        p[c] = (float)mom_norm[c];
         p[NC + c] = (float)std::sqrt(n);
         std::memcpy(&p[2 * NC + c], &l, sizeof l);
     };
@@ -362,6 +366,7 @@ void Engine::build_moments()
             for (int s = 0; s < 2; ++s) put(mom_base(L, m) + 2 * (l - m) + s, l, m);
     p += 3 * NC;
     float *coef = p + T * NNP_MOM_MAXD, *fun = coef + (size_t)T * TT1 * mom_fmax;
+    float *dcoef = tab.data() + mom_tab_base(T, L, mom_fmax);
     for (int II = 0; II < T; ++II)
         for (int K = 0, tt = 0; K < T; ++K)
             for (int J = 0; J <= K; ++J, ++tt) {
@@ -380,6 +385,9 @@ void Engine::build_moments()
                     for (int l = 0; l <= L; ++l) cf[(size_t)l * mom_fmax] = (float)(half * c[l]);
                     cf[(size_t)(L + 1) * mom_fmax] = J == K ? (float)(0.5 * std::pow(0.5 + q.x, q.y)) : 0.f;
                     std::memcpy(&fun[(size_t)II * mom_fmax + o], &fu, sizeof fu);
+                    for (int l = 0; l < TT1; ++l)
+                        dcoef[2 * (((size_t)II * mom_fmax + o) * mom_dl(L) + l) + (dmp & 1)] =
+                            (J == K ? 2.f : 1.f) * cf[(size_t)l * mom_fmax];
                 }
             }
     mom_tab_host = tab;
@@ -989,7 +997,7 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
     if (graphs)
         key = {N, S, b->pbc, n_ghost, E.cap, (int64_t)flags, (int64_t)(atom_energy != nullptr), (int64_t)(virial != nullptr),
                E.precision, (int64_t)(intptr_t)(E.use_jit ? E.jit_module : nullptr), (int64_t)E.acc64 + 2 * E.symm64,
-               (int64_t)(intptr_t)E.mom.p, E.mom_rows,
+               (int64_t)(intptr_t)E.mom.p, E.mom_rows, (int64_t)(intptr_t)E.len_order.p,
                (int64_t)(intptr_t)E.atom_off.p,
                (int64_t)(intptr_t)E.pos.p, (int64_t)(intptr_t)E.type.p, (int64_t)(intptr_t)E.cell.p,
                (int64_t)(intptr_t)E.nbr.p, (int64_t)(intptr_t)E.G.p, (int64_t)(intptr_t)E.force.p,

@@ -100,7 +100,8 @@ struct Engine {
     void *jit_module = nullptr;   // cudaLibrary_t
     void *jit_symm = nullptr, *jit_force = nullptr, *jit_tangent = nullptr;   // cudaKernel_t
     // cudaKernel_t, moment form: warp or thread per atom; one or two atoms per warp
-    void *jit_symm_mom = nullptr, *jit_symm_momt = nullptr, *jit_force_mom1 = nullptr, *jit_force_mom2 = nullptr;
+    void *jit_symm_mom = nullptr, *jit_symm_momt = nullptr, *jit_force_mom1 = nullptr, *jit_force_mom2 = nullptr,
+         *jit_force_momt = nullptr, *jit_force_few = nullptr;
     void *jit_symm_few = nullptr;                                            // and the blocks of few pairs
     std::string jit_source, jit_error;
 
@@ -108,13 +109,17 @@ struct Engine {
     bool mom_ok = false;          // every angular block is GAUSS with integer zeta <= NNP_MOM_MAXL
     int mom_L = 1, mom_ND = 1, mom_NR = 1, mom_fmax = 1;
     std::vector<float> mom_tab_host;
+    std::vector<double> mom_norm, mom_gnorm;   // M::norm, M::gnorm (nnp_moments.cuh)
     float mom_a_lo(int II, int d) const { return mom_tab_host[3 * mom_comps(mom_L) + II * NNP_MOM_MAXD + d]; }
     DBuf<float> mom_tab;          // MomTab
-    DBuf<float2> mom;             // moments of atoms order[0 .. mom_rows) (mom_at)
+    DBuf<float2> mom;             // moments of atoms visit()[0 .. mom_rows) (mom_at)
     DBuf<unsigned short> mom_cnt; // their neighbour counts by element [row][8]
     DBuf<int2> mom_items;         // (row, block) of the blocks of few pairs (number: DevErr::few)
     int64_t mom_rows = 0;         // rows of `mom` the current batch uses (0: not reserved)
     bool mom_valid = false;       // they hold the whole batch's moments
+    DBuf<int> len_order;          // visiting order by neighbour counts, its keys and ranks, its bins (run_len_order)
+    bool len_sorted = false;      // the moment kernels visit the atoms in that order
+    int *visit() { return len_sorted ? len_order.p : order.p; }
 
     // stream / events
     cudaStream_t stream = nullptr;
@@ -204,6 +209,11 @@ struct Engine {
     {
         return dpot.ntypes <= NNP_MOM_THREAD_T && 2 * mom_comps(mom_L) + mom_NR <= 184 &&
                mom_thread_floats(dpot.ntypes, mom_ND, mom_L) * (int)sizeof(float) <= 110 * 1024;
+    }
+    bool mom_force_thread() const
+    {
+        return mom_thread() && mom_ND <= 2 &&
+               mom_force_thread_floats(dpot.ntypes, mom_L, gstride) * (int)sizeof(float) <= 110 * 1024;
     }
     std::string upload();
     void free_all();

@@ -415,6 +415,8 @@ std::string gen_moment_constants(const Engine &E)
     pick("float", "damp_a", E.mom_ND, [&](int k) { return flit(d.t[0].damp_a[k]); });
     pick("float", "damp_lo", E.mom_ND, [&](int k) { return flit(E.mom_a_lo(0, k)); });
     pick("int", "damp_cut", E.mom_ND, [&](int k) { return std::to_string(d.t[0].damp_cut[k]); });
+    pick("float", "norm", (int)E.mom_norm.size(), [&](int k) { return flit((float)E.mom_norm[k]); });
+    pick("float", "gnorm", (int)E.mom_gnorm.size(), [&](int k) { return flit((float)E.mom_gnorm[k]); });
     return os.str();
 }
 
@@ -556,7 +558,8 @@ std::string make_source(const Engine &E, const TuneParams &tp)
           "                                 int cap, int lane, const float *eb)\n"
           "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
        << group_cases(fo) << "        default: return false;\n        }\n    }\n";
-    os << "    __device__ static bool radial_force(int II, int t, float r, float fc, float fcd, const float *eb, float &out)\n"
+    os << "    template <class E>\n"
+          "    __device__ static bool radial_force(int II, int t, float r, float fc, float fcd, E eb, float &out)\n"
           "    {\n        switch (II * NNP_MAX_TYPES + t) {\n"
        << group_cases(ra) << "        default: return false;\n        }\n    }\n";
     // radial sums of the symmetry-function kernel with the form fixed per case
@@ -621,7 +624,7 @@ extern "C" __global__ void __launch_bounds__(NNP_MOM_FORCE_WARPS * 32) \
 name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, \
      const float2 *__restrict__ rpar, const int *__restrict__ type, const int *__restrict__ order, \
      const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride, \
-     const float *__restrict__ dEdG, const float2 *__restrict__ mom, const unsigned short *__restrict__ mom_cnt, \
+     const float *__restrict__ dEdG, const float2 *__restrict__ mom, int msh, const unsigned short *__restrict__ mom_cnt, \
      const int2 *__restrict__ items, const int *__restrict__ nitems, double *__restrict__ F, nnp::DevErr *err, \
      const int *__restrict__ atom_struct, double *__restrict__ vir) \
 { \
@@ -633,7 +636,7 @@ name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot,
             err, atom_struct, vir); \
     else \
         nnp::mom_force_body<nnp::JitMoments, na>((int)blockIdx.x - nfew, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr, nbr_cnt, cap, \
-            gstride, dEdG, mom, mom_cnt, F, err, atom_struct, vir, reinterpret_cast<float *>(smem4)); \
+            gstride, dEdG, mom, msh, mom_cnt, F, err, atom_struct, vir, reinterpret_cast<float *>(smem4)); \
 }
 NNP_FORCE_KERNEL(k_force_jit, 1)
 NNP_FORCE_KERNEL(k_force_jit2, 2)
@@ -657,6 +660,30 @@ k_symm_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, co
     extern __shared__ float4 smem4[];
     nnp::mom_symm_thread_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, items, nitems,
         reinterpret_cast<float *>(smem4));
+}
+)";
+    if (E.mom_ok && E.mom_force_thread())
+        os << R"(
+extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
+k_force_jit_t(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+     const float2 *__restrict__ rpar, const int *__restrict__ type, const int *__restrict__ order,
+     const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride,
+     const float *__restrict__ dEdG, const float2 *__restrict__ mom, const unsigned short *__restrict__ mom_cnt,
+     double *__restrict__ F, nnp::DevErr *err)
+{
+    extern __shared__ float4 smem4[];
+    nnp::mom_force_thread_body<nnp::JitMoments>((int)blockIdx.x, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr,
+        nbr_cnt, cap, gstride, dEdG, mom, mom_cnt, F, err, reinterpret_cast<float *>(smem4));
+}
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
+k_force_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
+            const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+            const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+            const unsigned short *__restrict__ mom_cnt, const float *__restrict__ dEdG, double *__restrict__ F,
+            nnp::DevErr *err, const int *__restrict__ atom_struct)
+{
+    nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x, (int)gridDim.x, NNP_MOM_FEW_THREADS, items, nitems, lo, pot, tab,
+        fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, nullptr);
 }
 )";
     if (!E.mom_ok)
@@ -710,7 +737,7 @@ void jit_release(Engine &E)
     if (E.jit_module) cudaLibraryUnload((cudaLibrary_t)E.jit_module);
     E.jit_module = nullptr;
     E.jit_symm = E.jit_force = E.jit_tangent = nullptr;
-    E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = nullptr;
+    E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = E.jit_force_momt = E.jit_force_few = nullptr;
     E.jit_symm_few = nullptr;
 }
 
@@ -845,6 +872,7 @@ std::string jit_build(Engine &E)
     if (E.mom_ok) {
         fns.push_back({"k_symm_jit", &E.jit_symm_mom});
         if (E.mom_thread()) fns.push_back({"k_symm_jit_t", &E.jit_symm_momt});
+        if (E.mom_force_thread()) fns.push_back({"k_force_jit_t", &E.jit_force_momt}), fns.push_back({"k_force_few", &E.jit_force_few});
         fns.push_back({"k_force_jit", &E.jit_force_mom1});
         fns.push_back({"k_force_jit2", &E.jit_force_mom2});
         fns.push_back({"k_symm_few", &E.jit_symm_few});

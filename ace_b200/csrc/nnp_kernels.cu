@@ -1732,12 +1732,12 @@ std::string run_neighbors(Engine &E, int pbc)
 static std::string mom_reserve(Engine &E)
 {
     const size_t vals = mom_vals(E.dpot.ntypes, E.mom_ND, E.mom_L);
-    const int64_t most = (int64_t)(NNP_MOM_BYTES / (vals * sizeof(float2))) & ~(int64_t)3;
-    int64_t rows = std::min<int64_t>((E.n_centre + 3) & ~(int64_t)3, most);
+    const int64_t most = (int64_t)(NNP_MOM_BYTES / (vals * sizeof(float2))) & ~(int64_t)31;
+    int64_t rows = std::min<int64_t>((E.n_centre + 31) & ~(int64_t)31, most);
     cudaError_t e = E.mom.reserve((size_t)rows * vals);
     while (e != cudaSuccess && rows > 4096) {
         cudaGetLastError();
-        rows = (rows / 4) & ~(int64_t)3;
+        rows = (rows / 4) & ~(int64_t)31;
         e = E.mom.reserve((size_t)rows * vals);
     }
     if (e == cudaSuccess) e = E.mom_cnt.reserve(8 * (size_t)rows);
@@ -1749,6 +1749,127 @@ static std::string mom_reserve(Engine &E)
 #define NNP_MOM_THREAD_MIN 40000   // atoms from which a thread per atom is faster than a warp
 #define NNP_MOM_PAIR_MIN 20000     // atoms from which two atoms per warp are faster than one
 
+// Visiting order of the thread-per-atom kernels: the lanes of a warp walk their
+// neighbour lists element by element together, so a warp takes as long as its
+// longest segment of each element.  A counting sort puts atoms of one element
+// with about the same numbers of neighbours of each element next to each other
+// (1.09 M atoms: 0.14 ms, mostly the counts' loads, against 0.3 ms of the symmetry
+// functions and 0.7 ms of the forces).
+//
+// Bins of a centre element: the counts in steps of `width`, `bits` bits each,
+// the longest first.  scratch: order, key, rank of each of the n centres, then
+// the bins of all elements and a cursor per element.
+struct LenBins {
+    int bits, width, bins;
+};
+static LenBins len_bins(int ntypes)
+{
+    static const LenBins b[] = {{7, 1, 1 << 7}, {6, 2, 1 << 12}, {5, 3, 1 << 15}, {4, 5, 1 << 16}};
+    return b[ntypes - 1];
+}
+static_assert(NNP_MOM_THREAD_T == 4, "bins for each number of elements");
+
+__global__ void k_len_key(int64_t n, const int *__restrict__ order, const int *__restrict__ type, int ntypes,
+                          const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, LenBins lb,
+                          int *__restrict__ key, int *__restrict__ rank, int *__restrict__ hist)
+{
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int k = -1;                                       // no centre, or a type out of range: keeps its place
+    if (p < n) {
+        const int i = order[p], t = type[i];
+        if (t >= 0 && t < ntypes) {
+            const float4 *l = nbr + (int64_t)i * cap;
+            const int c = nbr_cnt[i], most = (1 << lb.bits) - 1;
+            int from = 0;
+            k = t;
+            for (int J = 0; J < ntypes; ++J) {
+                int to = c, lo = from;
+                while (J + 1 < ntypes && lo < to) {   // first neighbour of a later element
+                    const int mid = (lo + to) >> 1;
+                    if ((int)((unsigned)__float_as_int(l[mid].w) >> 28) > J) to = mid;
+                    else lo = mid + 1;
+                }
+                k = (k << lb.bits) | (most - min((to - from) / lb.width, most));
+                from = to;
+            }
+        }
+    }
+    const unsigned same = __match_any_sync(FULL, k), below = same & ((1u << (threadIdx.x & 31)) - 1u);
+    int r = 0;
+    if (k >= 0 && !below) r = atomicAdd(&hist[k], __popc(same));
+    r = __shfl_sync(FULL, r, __ffs(same) - 1) + __popc(below);
+    if (p < n) {
+        key[p] = k;
+        rank[p] = r;
+    }
+}
+
+// counts of the bins of element blockIdx.y -> places in the order; the blocks'
+// bins follow one another in any sequence
+__global__ void __launch_bounds__(256) k_len_base(LenBins lb, const int *__restrict__ type_count, int *__restrict__ hist,
+                                                  int *__restrict__ cursor)
+{
+    __shared__ int part[8], first;
+    const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, b0 = (blockIdx.x * 256 + tid) * 4;
+    int4 v = make_int4(0, 0, 0, 0);
+    int4 *h = reinterpret_cast<int4 *>(hist + (size_t)t * lb.bins + b0);
+    if (b0 < lb.bins) v = *h;
+    const int sum = v.x + v.y + v.z + v.w;
+    int inc = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(FULL, inc, d);
+        if (lane >= d) inc += u;
+    }
+    if (lane == 31) part[tid >> 5] = inc;
+    __syncthreads();
+    if (tid == 0) {
+        int run = 0, start = 0;
+        for (int w = 0; w < 8; ++w) {
+            const int c = part[w];
+            part[w] = run;
+            run += c;
+        }
+        for (int u = 0; u < t; ++u) start += type_count[u];
+        first = start + (run ? atomicAdd(&cursor[t], run) : 0);
+    }
+    __syncthreads();
+    if (b0 >= lb.bins) return;
+    const int at = first + part[tid >> 5] + inc - sum;
+    *h = make_int4(at, at + v.x, at + v.x + v.y, at + v.x + v.y + v.z);
+}
+
+__global__ void k_len_scatter(int64_t n, const int *__restrict__ order, const int *__restrict__ key,
+                              const int *__restrict__ rank, const int *__restrict__ base, int *__restrict__ out)
+{
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int k = key[p];
+    out[k < 0 ? p : base[k] + rank[p]] = order[p];
+}
+
+static void run_len_order(Engine &E)
+{
+    const int64_t n = E.n_centre, n4 = (n + 3) & ~(int64_t)3;
+    const int T = E.dpot.ntypes;
+    const LenBins lb = len_bins(T);
+    const size_t bins = (size_t)T * lb.bins;
+    if (E.len_order.reserve(3 * n4 + bins + T) != cudaSuccess) {     // the order by element serves as well
+        cudaGetLastError();
+        return;
+    }
+    int *out = E.len_order.p, *key = out + n4, *rank = key + n4, *hist = rank + n4;
+    cudaMemsetAsync(hist, 0, (bins + T) * sizeof(int), E.stream);
+    const int g = grid_for(n, 256, 1 << 30);
+    k_len_key<<<g, 256, 0, E.stream>>>(n, E.order.p, E.type.p, T, E.nbr.p, E.nbr_cnt.p, E.cap, lb, key, rank, hist);
+    k_len_base<<<dim3((lb.bins + 1023) / 1024, T), 256, 0, E.stream>>>(lb, E.type_fill.p, hist, hist + bins);
+    k_len_scatter<<<g, 256, 0, E.stream>>>(n, E.order.p, key, rank, hist, out);
+    E.launches += 3;
+    E.len_sorted = true;
+}
+
+static bool mom_by_thread(const Engine &E, int64_t n) { return E.jit_symm_momt && n >= NNP_MOM_THREAD_MIN; }
+
 // Moments of atoms order[lo .. hi) and, unless G is NULL, symmetry functions.
 // first: the list of few-pair blocks is empty (cleared with the error record).
 static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, bool first)
@@ -1756,12 +1877,12 @@ static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, 
     const int T = E.dpot.ntypes;
     long long l = lo, h = hi;
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
-    int *nitems = &E.err.p->few;
+    int *nitems = &E.err.p->few, *ord = E.visit();
     if (!first) cudaMemsetAsync(nitems, 0, sizeof(int), E.stream);
-    void *args[] = {&l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &E.order.p, &E.nbr.p, &E.nbr_cnt.p,
+    void *args[] = {&l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
                     &cap, &gs, &G, &E.mom.p, &E.mom_cnt.p, &E.mom_items.p, &nitems};
     E.launches += 1;
-    if (!E.jit_symm_momt || hi - lo < NNP_MOM_THREAD_MIN) {
+    if (!mom_by_thread(E, hi - lo)) {
         const size_t sm = (size_t)NNP_MOM_SYMM_WARPS * mom_symm_floats(T, E.mom_ND, E.mom_L, E.mom_NR, E.gstride) * sizeof(float);
         return jit_launch(E.jit_symm_mom, grid_for(hi - lo, NNP_MOM_SYMM_WARPS, num_sms() * 64), NNP_MOM_SYMM_WARPS * 32, sm,
                           E.stream, args);
@@ -1769,7 +1890,7 @@ static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, 
     std::string msg = jit_launch(E.jit_symm_momt, grid_for(hi - lo, NNP_MOM_THREADS, 1 << 30), NNP_MOM_THREADS,
                                  mom_thread_floats(T, E.mom_ND, E.mom_L) * sizeof(float), E.stream, args);
     if (!msg.empty() || !G) return msg;
-    void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &E.order.p, &E.nbr.p, &cap, &gs,
+    void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,
                    &E.mom_cnt.p, &G};
     E.launches += 1;
     return jit_launch(E.jit_symm_few, num_sms() * 8, NNP_MOM_FEW_THREADS, 0, E.stream, few);
@@ -1777,15 +1898,31 @@ static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, 
 
 static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *vir)
 {
-    const int T = E.dpot.ntypes, na = (!vir && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
-    const size_t sm = (size_t)na * NNP_MOM_FORCE_WARPS * mom_force_floats(T, E.mom_ND, E.mom_L, E.gstride) * sizeof(float);
+    const int T = E.dpot.ntypes;
     long long l = lo, h = hi;
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
+    const int *nitems = &E.err.p->few, *ord = E.visit();
+    if (E.jit_force_momt && !vir && mom_by_thread(E, hi - lo)) {
+        // the blocks of few pairs in a launch of their own: at the thread
+        // form's 8 warps per SM they took 1.2 ms of 1.09 M atoms' forces
+        void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,
+                       &E.mom_cnt.p, &E.dEdG.p, &E.force.p, &E.err.p, &E.atom_struct.p};
+        const std::string msg = jit_launch(E.jit_force_few, num_sms() * 16, NNP_MOM_FEW_THREADS, 0, E.stream, few);
+        if (!msg.empty()) return msg;
+        int nmain = grid_for(hi - lo, NNP_MOM_THREADS, 1 << 30);
+        void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
+                        &cap, &gs, &E.dEdG.p, &E.mom.p, &E.mom_cnt.p, &E.force.p, &E.err.p};
+        E.launches += 2;
+        return jit_launch(E.jit_force_momt, nmain, NNP_MOM_THREADS,
+                          sizeof(float) * mom_force_thread_floats(T, E.mom_L, E.gstride), E.stream, args);
+    }
+    const int na = (!vir && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
+    int msh = mom_by_thread(E, hi - lo) ? NNP_MOM_SH_T : NNP_MOM_SH_W;   // as launch_symm_mom wrote them
+    const size_t sm = (size_t)na * NNP_MOM_FORCE_WARPS * mom_force_floats(T, E.mom_ND, E.mom_L, E.gstride) * sizeof(float);
     int nmain = grid_for(hi - lo, na * NNP_MOM_FORCE_WARPS, num_sms() * 32);
     const int nfew = grid_for((hi - lo) * T * (T + 1) / 2, NNP_MOM_FORCE_WARPS * 2, num_sms() * 4);
-    const int *nitems = &E.err.p->few;
-    void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &E.order.p, &E.nbr.p, &E.nbr_cnt.p,
-                    &cap, &gs, &E.dEdG.p, &E.mom.p, &E.mom_cnt.p, &E.mom_items.p, &nitems, &E.force.p, &E.err.p,
+    void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
+                    &cap, &gs, &E.dEdG.p, &E.mom.p, &msh, &E.mom_cnt.p, &E.mom_items.p, &nitems, &E.force.p, &E.err.p,
                     &E.atom_struct.p, &vir};
     E.launches += 1;
     return jit_launch(na == 2 ? E.jit_force_mom2 : E.jit_force_mom1, nmain + nfew, NNP_MOM_FORCE_WARPS * 32, sm, E.stream, args);
@@ -1794,10 +1931,11 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
 std::string run_symm(Engine &E)
 {
     const int64_t N = E.n_centre;      // centres: the first n_centre entries of `order`
-    E.mom_valid = false;
+    E.mom_valid = E.len_sorted = false;
     if (N == 0) return "";
     if (E.use_jit && E.jit_symm_mom && !E.acc64 && !E.symm64) {
         std::string msg = mom_reserve(E);
+        if (mom_by_thread(E, std::min(N, E.mom_rows))) run_len_order(E);
         for (int64_t lo = 0; lo < N && msg.empty(); lo += E.mom_rows)
             msg = launch_symm_mom(E, lo, std::min(N, lo + E.mom_rows), E.G.p, lo == 0);
         E.mom_valid = E.mom_rows >= N;

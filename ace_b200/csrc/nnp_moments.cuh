@@ -41,6 +41,7 @@
 //   cut(c), rci_lo(c): cutoff c and the low part of its 1/rc,
 //   SAME: every centre element has the same damping factors, and then
 //   damp_a(d), damp_lo(d), damp_cut(d): exponent (high and low part) and cutoff,
+//   norm(c): factor of the monic Y_lm of component c, gnorm(c): times (l - m)!,
 //   radial_row(II, t, r, fc, row): values of the radial functions of a
 //   neighbour of element t, radial_force(II, t, r, fc, fcd, eb, out): sum of
 //   eb_f dG_f/dr, few_symm(II, tt, cs, w, acc): acc_f += x_f^zeta w_d,
@@ -73,12 +74,17 @@ NNP_HD constexpr int mom_comps(int L) { return mom_base(L, L) + 2; }
 
 // Moments in memory: component k = ((element * pairs of damping factors) + pair)
 // * comps + component of row r (the r-th atom of the visiting order) is the
-// float2 at mom_at(r, k): four rows interleaved, so that a thread per row writes
-// whole 32-byte sectors and so does a warp that reads one row's components
-// next to its neighbours'.  mom_cnt holds 8 neighbour counts (by element) per
-// row, mom_items the (row, block) entries of few pairs (their number: DevErr::few).
+// float2 at mom_at(r, k, vals, sh): 2^sh rows interleaved.  Written with a thread
+// per row sh = NNP_MOM_SH_T: a warp's access is two whole lines (with 4 rows it
+// touched 8 lines, and the tag lookups bounded both kernels: symmetry functions
+// of 1.09 M atoms 2.27 -> 2.13 ms, forces 3.51 -> 3.19 ms); written with a warp
+// per row sh = NNP_MOM_SH_W: it writes one row's components next to its
+// neighbours'.  mom_cnt holds 8 neighbour counts (by element) per row,
+// mom_items the (row, block) entries of few pairs (their number: DevErr::few).
+#define NNP_MOM_SH_T 5
+#define NNP_MOM_SH_W 2
 NNP_HD constexpr int mom_vals(int T, int ND, int L) { return T * ((ND + 1) / 2) * mom_comps(L); }
-NNP_HD inline i64 mom_at(i64 r, int k, int vals) { return ((r >> 2) * vals + k) * 4 + (r & 3); }
+NNP_HD inline i64 mom_at(i64 r, int k, int vals, int sh) { return (((r >> sh) * vals + k) << sh) + (r & ((1 << sh) - 1)); }
 
 // pairs of block (J, K) of an atom
 NNP_HD inline int mom_pairs(const unsigned short *cnt, int J, int K)
@@ -92,24 +98,35 @@ NNP_HD inline int mom_pairs(const unsigned short *cnt, int J, int K)
 //   per element: low parts of the damping exponents [NNP_MOM_MAXD],
 //   per element and angular function f, [L + 2][fmax]: coefficients c_0 .. c_L
 //   (halved for J == K), then f(1)/2 for J == K and 0 otherwise,
-//   per element and function, as int: tt | d << 8 | J << 16 | K << 24
+//   per element and function, as int: tt | d << 8 | J << 16 | K << 24,
+//   then, 16-byte aligned, per element and function mom_dl(L) float2: its
+//   coefficients in dE/dA (those above, twice for J == K) in .x for an even
+//   damping factor, in .y for an odd one
 struct MomTab {
     const float *norm, *fnorm;
     const int *deg;
     const float *a_lo;
     const float *coef;
     const int *fun;
+    const float2 *dcoef;
     int fmax;
 };
 
+NNP_HD constexpr int mom_dl(int L) { return (L + 3) & ~1; }
+NNP_HD inline int mom_tab_base(int T, int L, int fmax)       // floats before dcoef
+{
+    return (3 * mom_comps(L) + T * NNP_MOM_MAXD + T * fmax * (L + 3) + 3) & ~3;
+}
+
 NNP_HD inline int mom_tab_floats(int T, int L, int fmax)
 {
-    return 3 * mom_comps(L) + T * NNP_MOM_MAXD + T * fmax * (L + 3);
+    return mom_tab_base(T, L, fmax) + 2 * T * fmax * mom_dl(L);
 }
 
 NNP_HD inline MomTab mom_tab(const float *p, int T, int L, int fmax)
 {
     MomTab t;
+    t.dcoef = reinterpret_cast<const float2 *>(p + mom_tab_base(T, L, fmax));
     t.norm = p; p += mom_comps(L);
     t.fnorm = p; p += mom_comps(L);
     t.deg = reinterpret_cast<const int *>(p); p += mom_comps(L);
@@ -130,6 +147,12 @@ NNP_HD constexpr int mom_symm_floats(int T, int ND, int L, int NR, int gstride)
     return ((32 * mom_stage(L, NR, ND) + 3) & ~3) + 64 * ((ND + 1) / 2) + 2 * mom_vals(T, ND, L) + T * NNP_MOM_MAXD +
            ((2 * mom_s_vals(T, ND, L) + 3) & ~3) + gstride + 4;
 }
+// Forces, one thread per atom: D of one neighbour element, dE/dG.
+NNP_HD inline int mom_force_thread_floats(int T, int L, int gstride)
+{
+    return NNP_MOM_THREADS * (2 * T * (L + 1) + gstride);
+}
+
 // One thread per atom: S and the sums of w_d^2 of its NNP_MOM_THREADS threads.
 NNP_HD constexpr int mom_thread_floats(int T, int ND, int L)
 {
@@ -175,6 +198,12 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
+}
+
+// the line of a record that is read some iterations later
+__device__ __forceinline__ void mom_prefetch(const float4 *p)
+{
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
 NNP_HD constexpr float mom_beta(int l, int m) { return (float)((double)(l * l - m * m) / (double)(4 * l * l - 1)); }
@@ -717,7 +746,7 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
         }
         {
             const i64 r = idx - lo;
-            for (int k = lane; k < NV; k += 32) mom[mom_at(r, k, NV)] = reinterpret_cast<const float2 *>(A)[k];
+            for (int k = lane; k < NV; k += 32) mom[mom_at(r, k, NV, NNP_MOM_SH_W)] = reinterpret_cast<const float2 *>(A)[k];
             if (lane < 8) mom_cnt[8 * r + lane] = cnt[lane];
             for (int tt = lane; tt < TT; tt += 32) mom_push<T>(items, nitems, r, tt, cnt);
         }
@@ -730,10 +759,14 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
 // walks that element's segment of its list, so nothing is staged, exchanged or
 // reduced; the finished moments go to mom, from which the thread forms S
 // (through shared memory, entry-major) and G.  Lanes differ in the length of a
-// segment, which costs ~1.4x on the batched workload, against the staging,
-// flushes and partly filled 32-row chunks of the warp form.
+// segment (on average 21 of 32 worked on the batched workload), so the atoms are
+// visited in the order of their neighbour counts (run_len_order: 29 of 32).
 // Y_00's sum keeps its rounding errors in a second register (see above).
-// Bound: FP32 issue at 8 warps per SM (registers).
+// Bound: latency of the phases between the segments and FP32 issue at 8 warps
+// per SM (registers).  1.09 M atoms: 2.66 ms; lines of the list prefetched 2.43;
+// sorted visits 2.28; moments 32 rows interleaved 2.13; G from contiguous
+// coefficients, norms as literals 1.97 (the sort and the blocks of few pairs
+// included).
 template <class M>
 __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab,
                                      int fmax, const int *__restrict__ type, const int *__restrict__ order,
@@ -742,7 +775,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                                      unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems, float *smem)
 {
     constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
-                  NR = M::NR, NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), BT = NNP_MOM_THREADS;
+                  NR = M::NR, NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), DL = mom_dl(L), BT = NNP_MOM_THREADS;
     f32x2 *S = reinterpret_cast<f32x2 *>(smem) + threadIdx.x;    // [NS][BT]
     f32x2 *W2 = S + NS * BT;                                     // [T][NDP][BT]
     const DevPot &P = *pot;
@@ -774,6 +807,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                     MomNbr<M, false> v;
                     v.set(e, Ty, tb.a_lo + II * NNP_MOM_MAXD);
                     ++k;
+                    mom_prefetch(src + min(k + 6, n - 1));
                     e = k < n ? src[k] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
                     f32x2 cw = pk2(v.w[0], ND > 1 ? v.w[ND > 1 ? 1 : 0] : 0.f);
                     if (NDP > 1 && p > 0) cw = pk2(v.w[ND > 2 ? 2 : 0], ND > 3 ? v.w[ND > 3 ? 3 : 0] : 0.f);
@@ -818,9 +852,9 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                 }
                 cnt[J] = (unsigned short)(k - k0);
                 acc[0] = add2(acc[0], c00);
-                f32x2 *dst = reinterpret_cast<f32x2 *>(mom) + mom_at(r, (J * NDP + p) * NC, NV);
+                f32x2 *dst = reinterpret_cast<f32x2 *>(mom) + mom_at(r, (J * NDP + p) * NC, NV, NNP_MOM_SH_T);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) dst[4 * c] = mul2(acc[c], dup2(tb.norm[c]));
+                for (int c = 0; c < NC; ++c) dst[c << NNP_MOM_SH_T] = mul2(acc[c], dup2(M::norm(c)));
                 W2[(J * NDP + p) * BT] = ww;
                 if (G && p == 0) {
                     const DevBlockR B = Ty.br[J];
@@ -833,7 +867,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
 #pragma unroll
         for (int tt = 0; tt < TT; ++tt) mom_push<T>(items, nitems, r, tt, cnt);
         if (!G) continue;
-        const f32x2 *a = reinterpret_cast<const f32x2 *>(mom) + mom_at(r, 0, NV);
+        const f32x2 *a = reinterpret_cast<const f32x2 *>(mom) + mom_at(r, 0, NV, NNP_MOM_SH_T);
 #pragma unroll 1
         for (int p = 0; p < NDP; ++p)
 #pragma unroll
@@ -846,7 +880,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                         const int c = m == 0 ? l : mom_base(L, m > 0 ? m : 1) + 2 * (l - m) + h;
                         f32x2 v[T];
 #pragma unroll
-                        for (int J = 0; J < T; ++J) v[J] = a[4 * ((J * NDP + p) * NC + c)];
+                        for (int J = 0; J < T; ++J) v[J] = a[((J * NDP + p) * NC + c) << NNP_MOM_SH_T];
 #pragma unroll
                         for (int K = 0; K < T; ++K)
 #pragma unroll
@@ -858,14 +892,41 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
 #pragma unroll
                 for (int tt = 0; tt < TT; ++tt) S[((tt * NDP + p) * (L + 1) + l) * BT] = s[tt];
             }
-        const int na = Ty.n_input - Ty.n_input_r;
+        // G_f = sum_l c_l S_l - self (c and self as in dE/dA: half of them for J == K)
 #pragma unroll 1
-        for (int f = 0; f < na; ++f) {
-            const int fu = tb.fun[II * fmax + f], d = (fu >> 8) & 0xff;
-            const float *w2 = reinterpret_cast<const float *>(W2 + ((((fu >> 16) & 0xff) * NDP + (d >> 1)) * BT)) + (d & 1);
-            Gi[Ty.n_input_r + f] = mom_function<L, NDP>(tb, fu, tb.coef + (i64)II * (L + 2) * fmax + f,
-                                                         reinterpret_cast<const float2 *>(S), BT, w2, cnt);
-        }
+        for (int K = 0, tt = 0; K < T; ++K)
+#pragma unroll 1
+            for (int J = 0; J <= K; ++J, ++tt) {
+                const bool few = mom_pairs(cnt, J, K) <= NNP_MOM_FEW;    // added by the blocks of few pairs
+                const int off = Ty.ba[tt].off_g, bn = Ty.ba[tt].n, f0 = II * fmax + off - Ty.n_input_r;
+                const ulonglong2 *cf = reinterpret_cast<const ulonglong2 *>(tb.dcoef + (i64)f0 * DL);
+                const float h = J == K ? 0.5f : 1.f;
+                f32x2 st[DL];                                    // S, -sum of w_d^2
+#pragma unroll
+                for (int l = 0; l < DL; ++l) st[l] = 0ull;
+#pragma unroll 2
+                for (int f = 0; f < bn; ++f) {
+                    const int p = NDP > 1 ? (tb.fun[f0 + f] >> 9) & 0x7f : 0;
+                    if (NDP > 1 || f == 0) {
+#pragma unroll
+                        for (int l = 0; l <= L; ++l) st[l] = S[((tt * NDP + p) * (L + 1) + l) * BT];
+                        st[L + 1] = mul2(W2[(J * NDP + p) * BT], dup2(-1.f));
+                    }
+                    f32x2 c[DL], g = 0ull;
+#pragma unroll
+                    for (int l = 0; l < DL; l += 2) {
+                        const ulonglong2 v = __ldg(cf + f * (DL / 2) + l / 2);
+                        c[l] = v.x;
+                        c[l + 1] = v.y;
+                    }
+#pragma unroll
+                    for (int l = L; l >= 0; --l) g = fma2(c[l], st[l], g);
+                    g = fma2(c[L + 1], st[L + 1], g);
+                    float g0, g1;
+                    up2(g, g0, g1);
+                    Gi[off + f] = few ? 0.f : h * (g0 + g1);
+                }
+            }
         for (int f = Ty.n_input; f < gstride; ++f) Gi[f] = 0.f;
     }
 }
@@ -889,7 +950,7 @@ __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevP
                                const float2 *__restrict__ rpar, const int *__restrict__ type,
                                const int *__restrict__ order, const float4 *__restrict__ nbr,
                                const int *__restrict__ nbr_cnt, int cap, int gstride, const float *__restrict__ dEdG,
-                               const float2 *__restrict__ mom, const unsigned short *__restrict__ mom_cnt,
+                               const float2 *__restrict__ mom, int msh, const unsigned short *__restrict__ mom_cnt,
                                double *__restrict__ F, DevErr *err, const int *__restrict__ atom_struct,
                                double *__restrict__ vir, float *smem)
 {
@@ -965,7 +1026,7 @@ __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevP
         __syncwarp();
         if (II_l < T) {
             float *mine = base + al * per;
-            const f32x2 *src = reinterpret_cast<const f32x2 *>(mom) + mom_at(row + al, 0, NV);
+            const f32x2 *src = reinterpret_cast<const f32x2 *>(mom) + mom_at(row + al, 0, NV, msh);
 #pragma unroll 2
             for (int c = lane >> LA; c < NC; c += 32 / NA) {
                 const int l = tb.deg[c];
@@ -974,7 +1035,7 @@ __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevP
                 for (int p = 0; p < NDP; ++p) {
                     f32x2 a[T];
 #pragma unroll
-                    for (int K = 0; K < T; ++K) a[K] = __ldg(src + 4 * ((K * NDP + p) * NC + c));
+                    for (int K = 0; K < T; ++K) a[K] = __ldg(src + ((i64)((K * NDP + p) * NC + c) << msh));
 #pragma unroll
                     for (int J = 0; J < T; ++J) {
                         f32x2 b = 0ull;
@@ -1100,6 +1161,216 @@ __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevP
         }
         if (__any_sync(NNP_FULL, bad) && lane == 0) atomicMax(&err->nonfinite, 1);
         __syncwarp();
+    }
+}
+
+// dE/dG of a segment's radial functions in the threads' columns of shared memory
+struct MomStrided {
+    const float *p;
+    __device__ __forceinline__ float operator[](int f) const { return p[f * NNP_MOM_THREADS]; }
+};
+
+// One neighbour's sum_lm B Y_lm and its gradient with B in registers (b, scaled
+// by gnorm), both damping factors side by side.  r_n^m = d^m P_l / dz^m up to a
+// factor, n = l - m, scaled so that dr_n^m/dz = r_(n-1)^(m+1):
+//   r_(n+1) = z / (n + 1) r_n - beta / (n (n + 1)) r_(n-1),  r_0 = 1.
+// Row m serves the values of order m and the z slopes of order m - 1; the sums
+// over m are Horner's scheme in x - i y (f, its derivative g, and h for z).
+template <int L, int m>
+__device__ __forceinline__ void mom_gradient_regs(const f32x2 *b, float z, const float *zn, f32x2 x2, f32x2 y2, f32x2 ny2,
+                                                  f32x2 &fr, f32x2 &fi, f32x2 &gr, f32x2 &gi, f32x2 &hr, f32x2 &hi)
+{
+    f32x2 C = 0ull, S = 0ull, Cz = 0ull, Sz = 0ull;
+    float q0 = 1.f, q1 = 0.f;
+#pragma unroll
+    for (int l = m; l <= L; ++l) {
+        const f32x2 q2 = dup2(q0);
+        const int n = l - m;
+        if constexpr (m == 0) {
+            C = n == 0 ? b[0] : fma2(q2, b[l], C);
+        } else {
+            const f32x2 *bm = b + mom_base(L, m) + 2 * n;
+            C = n == 0 ? bm[0] : fma2(q2, bm[0], C);
+            S = n == 0 ? bm[1] : fma2(q2, bm[1], S);
+            if constexpr (m == 1) {
+                Cz = n == 0 ? b[l] : fma2(q2, b[l], Cz);
+            } else {
+                const f32x2 *bp = b + mom_base(L, m - 1) + 2 * (n + 1);
+                Cz = n == 0 ? bp[0] : fma2(q2, bp[0], Cz);
+                Sz = n == 0 ? bp[1] : fma2(q2, bp[1], Sz);
+            }
+        }
+        const float t = n == 0 ? z : fmaf(zn[n], q0, (-mom_beta(l, m) / (float)(n * (n + 1) > 0 ? n * (n + 1) : 1)) * q1);
+        q1 = q0;
+        q0 = t;
+    }
+    if constexpr (m == L) {
+        fr = C;
+        fi = S;
+        gr = gi = 0ull;
+        hr = Cz;
+        hi = Sz;
+    } else {
+        f32x2 t = fma2(gr, x2, fma2(gi, y2, fr));
+        gi = fma2(gi, x2, fma2(gr, ny2, fi));
+        gr = t;
+        t = fma2(fr, x2, fma2(fi, y2, C));
+        if constexpr (m > 0) fi = fma2(fi, x2, fma2(fr, ny2, S));
+        fr = t;
+        if constexpr (m > 0) {
+            t = fma2(hr, x2, fma2(hi, y2, Cz));
+            if constexpr (m > 1) hi = fma2(hi, x2, fma2(hr, ny2, Sz));
+            hr = t;
+        }
+    }
+    if constexpr (m > 0) mom_gradient_regs<L, m - 1>(b, z, zn, x2, y2, ny2, fr, fi, gr, gi, hr, hi);
+}
+
+// Forces with one thread per atom (at most two damping factors): B of one
+// neighbour element is the thread's registers while it walks that element's
+// segment of its list, so nothing of it is read again per neighbour (the warp
+// form's loads of B kept the shared-memory pipe 77 % busy).  Before each segment
+// the thread forms D^{JK} from its dE/dG, which a few 16-byte loads put into its
+// column of shared memory, and B from D and the moments.
+// Bound: issue and latency at 8 warps per SM (registers).  Forces of 1.09 M atoms
+// 3.29 (two atoms per warp) -> 2.41 ms, 354 k atoms of four elements 1.38 -> 1.16,
+// 131 k of a two-element crystal 0.46 -> 0.36.
+template <class M>
+__device__ void mom_force_thread_body(int block, int nblock, i64 lo, i64 hi, const DevPot *__restrict__ pot,
+                                      const float *__restrict__ tab, int fmax, const float2 *__restrict__ rpar,
+                                      const int *__restrict__ type, const int *__restrict__ order,
+                                      const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride,
+                                      const float *__restrict__ dEdG, const float2 *__restrict__ mom,
+                                      const unsigned short *__restrict__ mom_cnt, double *__restrict__ F, DevErr *err,
+                                      float *smem)
+{
+    constexpr int T = M::T, L = M::L, ND = M::ND, NC = mom_comps(L),
+                  NV = mom_vals(T, ND, L), DL = mom_dl(L), BT = NNP_MOM_THREADS;
+    f32x2 *D = reinterpret_cast<f32x2 *>(smem) + threadIdx.x;    // [T][L + 1][BT]: of one element
+    float *e = reinterpret_cast<float *>(reinterpret_cast<f32x2 *>(smem) + T * (L + 1) * BT) + threadIdx.x;   // [gstride][BT]: dE/dG
+    const DevPot &P = *pot;
+    const MomTab tb = mom_tab(tab, T, L, fmax);
+    for (i64 idx = lo + block * (i64)BT + threadIdx.x; idx < hi; idx += (i64)nblock * BT) {
+        const i64 i = order[idx], row = idx - lo;
+        const int II = type[i];
+        if ((unsigned)II >= (unsigned)T) continue;               // type out of range (reported by the call)
+        const int n = nbr_cnt[i];
+        const DevType &Ty = P.t[II];
+        const float4 *src = nbr + i * cap;
+        const unsigned short *cnt = mom_cnt + 8 * row;
+        const float *ei = dEdG + i * gstride;
+#pragma unroll 8
+        for (int k = 0; 4 * k < gstride; ++k) {
+            const float4 e4 = __ldg(reinterpret_cast<const float4 *>(ei) + k);
+            e[(4 * k) * BT] = e4.x;
+            e[(4 * k + 1) * BT] = e4.y;
+            e[(4 * k + 2) * BT] = e4.z;
+            e[(4 * k + 3) * BT] = e4.w;
+        }
+        double f0[3] = {0, 0, 0};
+        bool bad = false;
+        int k = 0;
+        float4 rec = n > 0 ? src[0] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+#pragma unroll 1
+        for (int J = 0; J < T; ++J) {
+            const DevBlockR Br = Ty.br[J];
+            // D^{JK}_{l,d} = sum_f e_f c_{f,l} [1 + (J == K)], and the self terms
+            float d0 = 0.f, d1 = 0.f;
+#pragma unroll 1
+            for (int K = 0; K < T; ++K) {
+                const int tt = J > K ? J * (J + 1) / 2 + K : K * (K + 1) / 2 + J;
+                const bool few = mom_pairs(cnt, J, K) <= NNP_MOM_FEW;
+                const int off = Ty.ba[tt].off_g, bn = Ty.ba[tt].n;
+                const ulonglong2 *cf =
+                    reinterpret_cast<const ulonglong2 *>(tb.dcoef + (i64)(II * fmax + off - Ty.n_input_r) * DL);
+                f32x2 acc[DL];
+#pragma unroll
+                for (int l = 0; l < DL; ++l) acc[l] = 0ull;
+#pragma unroll 4
+                for (int f = 0; f < bn; ++f) {
+                    const f32x2 e2 = dup2(few ? 0.f : e[(off + f) * BT]);
+#pragma unroll
+                    for (int l = 0; l < DL; l += 2) {
+                        const ulonglong2 c = __ldg(cf + f * (DL / 2) + l / 2);
+                        acc[l] = fma2(e2, c.x, acc[l]);
+                        acc[l + 1] = fma2(e2, c.y, acc[l + 1]);
+                    }
+                }
+#pragma unroll
+                for (int l = 0; l <= L; ++l) D[(K * (L + 1) + l) * BT] = acc[l];
+                if (J == K) up2(acc[L + 1], d0, d1);
+            }
+            // B^J = norm sum_K D^{JK} A^K
+            f32x2 b[NC];
+            {
+                const f32x2 *a = reinterpret_cast<const f32x2 *>(mom) + mom_at(row, 0, NV, NNP_MOM_SH_T);
+#pragma unroll
+                for (int l = 0; l <= L; ++l) {
+                    f32x2 dk[T];
+#pragma unroll
+                    for (int K = 0; K < T; ++K) dk[K] = D[(K * (L + 1) + l) * BT];
+#pragma unroll
+                    for (int m = 0; m <= l; ++m) {
+                        const int c0 = m == 0 ? l : mom_base(L, m > 0 ? m : 1) + 2 * (l - m);
+#pragma unroll
+                        for (int h = 0; h < (m ? 2 : 1); ++h) {
+                            f32x2 v = 0ull;
+#pragma unroll
+                            for (int K = 0; K < T; ++K) v = fma2(dk[K], __ldg(a + ((K * NC + c0 + h) << NNP_MOM_SH_T)), v);
+                            b[c0 + h] = mul2(v, dup2(M::gnorm(c0)));
+                        }
+                    }
+                }
+            }
+#pragma unroll 1
+            while ((int)((unsigned)__float_as_int(rec.w) >> 28) == J) {
+                MomNbr<M, true> v;
+                v.set(rec, Ty, tb.a_lo + II * NNP_MOM_MAXD);
+                const i64 j = __float_as_int(rec.w) & 0x0fffffff;
+                ++k;
+                mom_prefetch(src + min(k + 6, n - 1));
+                rec = k < n ? src[k] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+                f32x2 fr, fi, gr2, gi2, hr, hi2;
+                {
+                    float zn[L + 1];
+#pragma unroll
+                    for (int q = 1; q <= L; ++q) zn[q] = v.uz * (1.f / (float)(q + 1));
+                    mom_gradient_regs<L, L>(b, v.uz, zn, dup2(v.ux), dup2(v.uy), dup2(-v.uy), fr, fi, gr2, gi2, hr, hi2);
+                }
+                float fc = v.fc[0], fd = v.fd[0];
+#pragma unroll
+                for (int c = 1; c < M::NCUT; ++c)
+                    if (Br.cut == c) {
+                        fc = v.fc[c];
+                        fd = v.fd[c];
+                    }
+                float gr = 0.f;
+                M::radial_force(II, J, v.r, fc, fd, MomStrided{e + Br.off_g * BT}, gr);
+                float a0, a1, gx, gy, gz;
+                up2(fr, a0, a1);
+                gr = fmaf(fmaf(-d0, v.w[0], a0), v.wd[0], gr);
+                if (ND > 1) gr = fmaf(fmaf(-d1, v.w[ND > 1 ? 1 : 0], a1), v.wd[ND > 1 ? 1 : 0], gr);
+                const float w0 = v.w[0], w1 = ND > 1 ? v.w[ND > 1 ? 1 : 0] : 0.f;
+                up2(gr2, a0, a1);
+                gx = fmaf(w1, a1, w0 * a0);
+                up2(gi2, a0, a1);
+                gy = fmaf(w1, a1, w0 * a0);
+                up2(hr, a0, a1);
+                gz = fmaf(w1, a1, w0 * a0);
+                // dE/dd = u dE/dr + (I - u u^T) dE/du / r
+                const float pr = gr - v.ir * (gx * v.ux + gy * v.uy + gz * v.uz);
+                const float q[3] = {fmaf(gx, v.ir, pr * v.ux), fmaf(gy, v.ir, pr * v.uy), fmaf(gz, v.ir, pr * v.uz)};
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    bad |= !(fabsf(q[x]) <= 3.402823466e38f);
+                    atomicAdd(&F[3 * j + x], (double)q[x]);
+                    f0[x] += (double)q[x];
+                }
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 3; ++x) atomicAdd(&F[3 * i + x], -f0[x]);
+        if (bad) atomicMax(&err->nonfinite, 1);
     }
 }
 

@@ -229,3 +229,37 @@ def test_forms_for_many_atoms_match_the_small_call(tmp_path, shape):
     assert (np.abs(G[at] - Gs).max(1) / np.maximum(np.abs(Gs).max(1), 1e-30)).max() < 1e-6
     assert (np.abs(E[some] - Es) / np.diff(sub.atom_off)).max() < 1e-6
     assert np.abs(F[at] - Fs).max() < 5e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [40000, 40033])
+@pytest.mark.parametrize("shape", [(1, 20, [8], [9.0]), (2, 3, [3, 8], [7.0]), (3, 5, [1, 8], [7.0, 14.0]), (4, 4, [2, 8], [7.0, 14.0])],
+                         ids=lambda s: "T%d" % s[0])
+def test_thread_forms_at_their_limits(tmp_path, shape, n):
+    """The fewest atoms of the thread-per-atom kernels and a last group of one
+    row, elements in every proportion (blocks without pairs, of few pairs, lists
+    of one element), forces also with the virial (a warp per atom reads what a
+    thread per atom wrote); tolerances as above."""
+    nt, nrad, zetas, etas = shape
+    pot = basis(nt, nrad, zetas, etas, ["COS"], 6.0)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    rng = np.random.default_rng(2)
+    counts = [1, 2, 5] + list(rng.integers(20, 300, 400))
+    counts = counts[:int(np.searchsorted(np.cumsum(counts), n))]
+    counts.append(n - sum(counts))
+    b = synth.batch_random(8, counts, nt, density=0.05)
+    assert b.n_atoms == n
+    some = [0, 1, 2, 9, len(counts) - 2, len(counts) - 1]
+    sub = b.subset(some)
+    nn = NNP.read(path)
+    E, F, G = nn.compute_batch(b.atom_off, b.pos, b.type, b.cell, symm=True)
+    Em, Fm, _, Wm = nn.compute_md(b.atom_off, b.pos, b.type, b.cell)
+    Es, Fs, Gs = nn.compute_batch(sub.atom_off, sub.pos, sub.type, sub.cell, symm=True)
+    _, _, _, Ws = nn.compute_md(sub.atom_off, sub.pos, sub.type, sub.cell)
+    nn.close()
+    at = np.concatenate([np.arange(b.atom_off[s], b.atom_off[s + 1]) for s in some])
+    assert (np.abs(G[at] - Gs).max(1) / np.maximum(np.abs(Gs).max(1), 1e-30)).max() < 1e-6
+    assert (np.abs(E[some] - Es) / np.diff(sub.atom_off)).max() < 1e-6
+    assert np.abs(F[at] - Fs).max() < 5e-6 and np.abs(F - Fm).max() < 5e-6
+    assert (np.abs(Wm[some] - Ws).reshape(len(some), -1).max(1) / np.diff(sub.atom_off)).max() < 5e-5
