@@ -1746,8 +1746,17 @@ static std::string mom_reserve(Engine &E)
     return e == cudaSuccess ? "" : std::string("device allocation failed: ") + cudaGetErrorString(e);
 }
 
-#define NNP_MOM_THREAD_MIN 40000   // atoms from which a thread per atom is faster than a warp
-#define NNP_MOM_PAIR_MIN 20000     // atoms from which two atoms per warp are faster than one
+// Atoms from which a thread per atom is faster than a warp.  Symmetry functions,
+// warp and thread form (us): three elements 12 k atoms 71, 91; 15 k 86, 91; 22 k
+// 121, 102; two-element crystal 9 k 71, 87; 13.5 k 100, 88; four elements 16 k
+// 111, 102.  Forces, two atoms per warp and thread form: three elements 32 k 125,
+// 133; 40 k 152, 158; 50 k 187, 180; crystal 20 k 91, 115; 27 k 121, 119; 37 k
+// 157, 129; four elements 50 k 222, 237; 354 k 1380, 1110.
+#define NNP_MOM_THREAD_MIN 16000
+#define NNP_MOM_FORCE_THREAD_MIN 40000
+// atoms from which two atoms per warp are faster than one (forces, one and two:
+// crystal of 9 k atoms 55, 50 us; three elements 12 k 61, 55; below, too few blocks)
+#define NNP_MOM_PAIR_MIN 8000
 
 // Visiting order of the thread-per-atom kernels: the lanes of a warp walk their
 // neighbour lists element by element together, so a warp takes as long as its
@@ -1767,6 +1776,7 @@ static LenBins len_bins(int ntypes)
     static const LenBins b[] = {{7, 1, 1 << 7}, {6, 2, 1 << 12}, {5, 3, 1 << 15}, {4, 5, 1 << 16}};
     return b[ntypes - 1];
 }
+static_assert(NNP_MOM_FORCE_THREAD_MIN >= NNP_MOM_THREAD_MIN, "its moments are interleaved by a thread per row");
 static_assert(NNP_MOM_THREAD_T == 4, "bins for each number of elements");
 
 __global__ void k_len_key(int64_t n, const int *__restrict__ order, const int *__restrict__ type, int ntypes,
@@ -1902,7 +1912,7 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
     long long l = lo, h = hi;
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
     const int *nitems = &E.err.p->few, *ord = E.visit();
-    if (E.jit_force_momt && !vir && mom_by_thread(E, hi - lo)) {
+    if (E.jit_force_momt && !vir && hi - lo >= NNP_MOM_FORCE_THREAD_MIN) {
         // the blocks of few pairs in a launch of their own: at the thread
         // form's 8 warps per SM they took 1.2 ms of 1.09 M atoms' forces
         void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,

@@ -232,12 +232,12 @@ def test_forms_for_many_atoms_match_the_small_call(tmp_path, shape):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [40000, 40033])
+@pytest.mark.parametrize("n", [16000, 16033, 40000, 40033])
 @pytest.mark.parametrize("shape", [(1, 20, [8], [9.0]), (2, 3, [3, 8], [7.0]), (3, 5, [1, 8], [7.0, 14.0]), (4, 4, [2, 8], [7.0, 14.0])],
                          ids=lambda s: "T%d" % s[0])
 def test_thread_forms_at_their_limits(tmp_path, shape, n):
-    """The fewest atoms of the thread-per-atom kernels and a last group of one
-    row, elements in every proportion (blocks without pairs, of few pairs, lists
+    """The fewest atoms of the thread-per-atom kernels (symmetry functions, then
+    forces too) and a last group of one row, elements in every proportion (blocks without pairs, of few pairs, lists
     of one element), forces also with the virial (a warp per atom reads what a
     thread per atom wrote); tolerances as above."""
     nt, nrad, zetas, etas = shape
