@@ -137,3 +137,28 @@ def test_thin_and_skewed_cells(tmp_path):
     nn.close()
     want = np.concatenate([brute_counts(pot.rc, *b.structure(s), 3, m) for s, m in ((0, (4, 2, 2)), (1, (3, 3, 3)))])
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n, side", [(38, 6.0), (96, 8.2), (150, 9.5), (9, 3.7)])
+def test_candidate_lists_longer_than_the_buffers(tmp_path, n, side):
+    """Dense cells one cell wide: candidate lists that end inside a round of 256, longer
+    than the segment window (1024) and with more kept candidates than the list
+    holds (640), segments short and long.  In the 6 A cell every atom's own images
+    lie at the cutoff itself, where the rounding of either side decides: counts
+    between those at rc -+ 1e-10, which are equal for the other cells."""
+    pot = synth.potential_config(2)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    rng = np.random.default_rng(5)
+    cells = np.array([np.eye(3) * side, np.eye(3) * side])
+    pos = rng.uniform(0, side, (2 * n, 3))
+    typ = np.concatenate([rng.integers(0, 3, n), np.zeros(n)]).astype(np.int32)
+    b = synth.Batch(np.array([0, n, 2 * n]), pos, typ, cells, True)
+    low, high = (np.concatenate([brute_counts(pot.rc + d, *b.structure(s), 3, (3, 3, 3)) for s in (0, 1)])
+                 for d in (-1e-10, 1e-10))
+    assert np.array_equal(low, high) == (side != pot.rc)
+    nn = NNP.read(path)
+    nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    got = nn.neighbor_counts(b.n_atoms)
+    nn.close()
+    assert (low <= got).all() and (got <= high).all()
