@@ -125,7 +125,7 @@ void Engine::free_all()
 {
     rpar.release(); apar.release(); wpar.release(); vac.release();
     rpar64.release(); apar64.release(); cut64.release();
-    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release(); len_order.release();
+    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release(); momd.release(); len_order.release();
     atom_off.release(); pos.release(); cell.release(); xw.release();
     type.release(); atom_struct.release(); atom_cell.release(); grid.release(); bbox.release();
     cell_cnt.release(); cell_start.release(); cell_fill.release(); cell_atoms.release(); scan_tmp.release();

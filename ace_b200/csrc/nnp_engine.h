@@ -101,7 +101,7 @@ struct Engine {
     void *jit_symm = nullptr, *jit_force = nullptr, *jit_tangent = nullptr;   // cudaKernel_t
     // cudaKernel_t, moment form: warp or thread per atom; one or two atoms per warp
     void *jit_symm_mom = nullptr, *jit_symm_momt = nullptr, *jit_force_mom1 = nullptr, *jit_force_mom2 = nullptr,
-         *jit_force_momt = nullptr, *jit_force_few = nullptr;
+         *jit_force_momt = nullptr, *jit_force_few = nullptr, *jit_tangent_momt = nullptr, *jit_tangent_few = nullptr;
     void *jit_symm_few = nullptr;                                            // and the blocks of few pairs
     std::string jit_source, jit_error;
 
@@ -113,6 +113,7 @@ struct Engine {
     float mom_a_lo(int II, int d) const { return mom_tab_host[3 * mom_comps(mom_L) + II * NNP_MOM_MAXD + d]; }
     DBuf<float> mom_tab;          // MomTab
     DBuf<float2> mom;             // moments of atoms visit()[0 .. mom_rows) (mom_at)
+    DBuf<float2> momd;            // derivatives of the moments along the training step's displacements
     DBuf<unsigned short> mom_cnt; // their neighbour counts by element [row][8]
     DBuf<int2> mom_items;         // (row, block) of the blocks of few pairs (number: DevErr::few)
     int64_t mom_rows = 0;         // rows of `mom` the current batch uses (0: not reserved)
@@ -229,6 +230,8 @@ std::string run_energy(Engine &E, bool vacuum);
 std::string run_symm_to_double(Engine &E, double *out);
 std::string run_atom_energy(Engine &E, bool vacuum, double *out);
 std::string run_outputs(Engine &E, double *energy, double *forces);
+// tangent symmetry functions from the moments; false when the batch does not take that path
+bool run_tangent_mom(Engine &E, std::string &msg);
 std::string run_nn_from_symm(Engine &E, const double *symm_d, int gstride_in);
 std::string run_neighbor_counts(Engine &E, int *d_counts);
 std::string run_train_grad(Engine &E, bool with_force);

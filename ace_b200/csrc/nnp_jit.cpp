@@ -357,6 +357,46 @@ std::string gen_few_symm_body(const Engine &E, const DevBlockA &B)
     return os.str();
 }
 
+// One pair's share of the block's tangents: acc[f] += dx^zeta/dcos w[d] + x^zeta dw[d].
+std::string gen_few_tangent_body(const Engine &E, const DevBlockA &B)
+{
+    std::ostringstream os, body;
+    const std::vector<Fn> fs = block_fns(E, B);
+    std::vector<float> bases;
+    gen_bases(body, fs, bases);
+    Powers P(body);
+    for (size_t f = 0; f < fs.size(); ++f) {
+        const int b = base_of(bases, fs[f].lf);
+        const std::string d = std::to_string(fs[f].damp), F = std::to_string(f), pz = P.pw(b, fs[f].iz);
+        body << "            acc[" << F << "] = fmaf(" << pz << ", dw[" << d << "], acc[" << F << "]);\n";
+        if (fs[f].iz >= 1) {
+            const std::string pm1 = P.pw(b, fs[f].iz - 1);
+            body << "            acc[" << F << "] = fmaf(" << flit(fs[f].zeta * fs[f].lf) << " * " << pm1 << ", w[" << d << "], acc["
+                 << F << "]);\n";
+        }
+    }
+    os << "        {\n" << body.str() << "            return;\n        }\n";
+    return os.str();
+}
+
+// Slopes of one radial block's functions at a neighbour: row[f] = dG_f/dr.
+std::string gen_radial_drow_body(const Engine &E, const DevBlockR &B)
+{
+    std::ostringstream os;
+    os << "        {\n            const float c = fc[" << B.cut << "], cd = fd[" << B.cut << "];\n";
+    for (int f = 0; f < B.n; ++f) {
+        const float2 q = E.rpar_host[B.par + f];
+        if (B.form == RAD_GAUSSIAN)
+            os << "            { const float g = " << flit(q.y) << " * (r - " << flit(q.x) << "); row[" << f
+               << "] = expf(-g * g) * fmaf(" << flit(-2.f * q.y) << " * g, c, cd); }\n";
+        else
+            os << "            { float val; radial_fd(" << B.form << ", r, " << flit(q.x) << ", " << flit(q.y)
+               << ", c, cd, val, row[" << f << "]); }\n";
+    }
+    os << "            return;\n        }\n";
+    return os.str();
+}
+
 // One pair's dE/dcos and dE/dr of both neighbours from e = dE/dG of the block.
 std::string gen_few_force_body(const Engine &E, const DevBlockA &B)
 {
@@ -527,7 +567,7 @@ std::string make_source(const Engine &E, const TuneParams &tp)
     // between many chunks (used by a test)
     if (tp.force_chunk != NNP_PCH) os << "#define NNP_FORCE_CHUNK " << tp.force_chunk << "\n";
     os << "#include \"nnp_moments.cuh\"\nnamespace nnp {\nstruct JitBlocks {\n";
-    std::vector<std::pair<int, std::string>> sy, fo, ta, ra, rr, fy, ff;
+    std::vector<std::pair<int, std::string>> sy, fo, ta, ra, rr, rd, fy, ff, ft;
     int na = 1;   // angular functions of the largest block
     const int T = E.dpot.ntypes, TT = T * (T + 1) / 2;
     for (int II = 0; II < T; ++II)
@@ -535,6 +575,7 @@ std::string make_source(const Engine &E, const TuneParams &tp)
             const DevBlockR &B = E.dpot.t[II].br[J];
             if (B.n > 0) ra.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_force_body(E, B));
             if (B.n > 0 && E.mom_ok) rr.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_row_body(E, B));
+            if (B.n > 0 && E.mom_ok) rd.emplace_back(II * NNP_MAX_TYPES + J, gen_radial_drow_body(E, B));
         }
     for (int II = 0; II < T; ++II)
         for (int tt = 0; tt < TT; ++tt) {
@@ -544,6 +585,7 @@ std::string make_source(const Engine &E, const TuneParams &tp)
             if (E.mom_ok) {
                 fy.emplace_back(II * NNP_MAX_TT + tt, gen_few_symm_body(E, B));
                 ff.emplace_back(II * NNP_MAX_TT + tt, gen_few_force_body(E, B));
+                ft.emplace_back(II * NNP_MAX_TT + tt, gen_few_tangent_body(E, B));
             } else {
                 sy.emplace_back(II * NNP_MAX_TT + tt, gen_symm_body(E, B));
                 fo.emplace_back(II * NNP_MAX_TT + tt, gen_force_body(E, B));
@@ -599,6 +641,12 @@ std::string make_source(const Engine &E, const TuneParams &tp)
            << "    __device__ static void radial_row(int II, int t, float r, const float *fc, float *row)\n"
               "    {\n        switch (II * NNP_MAX_TYPES + t) {\n"
            << group_cases(rr) << "        default: return;\n        }\n    }\n"
+              "    __device__ static void radial_drow(int II, int t, float r, const float *fc, const float *fd, float *row)\n"
+              "    {\n        switch (II * NNP_MAX_TYPES + t) {\n"
+           << group_cases(rd) << "        default: return;\n        }\n    }\n"
+              "    __device__ static void few_tangent(int II, int tt, float cs, const float *w, const float *dw, float *acc)\n"
+              "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
+           << group_cases(ft) << "        default: return;\n        }\n    }\n"
               "    __device__ static void few_symm(int II, int tt, float cs, const float *w, float *acc)\n"
               "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
            << group_cases(fy) << "        default: return;\n        }\n    }\n"
@@ -675,6 +723,24 @@ k_force_jit_t(int nmain, long long lo, long long hi, const nnp::DevPot *__restri
     nnp::mom_force_thread_body<nnp::JitMoments>((int)blockIdx.x, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr,
         nbr_cnt, cap, gstride, dEdG, mom, mom_cnt, F, err, reinterpret_cast<float *>(smem4));
 }
+extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
+k_tangent_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+     const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
+     const int *__restrict__ nbr_cnt, int cap, int gstride, const float4 *__restrict__ V, const float2 *__restrict__ mom,
+     float2 *momd, const unsigned short *__restrict__ mom_cnt, float *__restrict__ Cout)
+{
+    extern __shared__ float4 smem4[];
+    nnp::mom_tangent_thread_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, V, mom, momd,
+        mom_cnt, Cout, reinterpret_cast<float *>(smem4));
+}
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
+k_tangent_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
+              const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+              const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+              const unsigned short *__restrict__ mom_cnt, const float4 *__restrict__ V, float *__restrict__ Cout)
+{
+    nnp::mom_few_tangent_body<nnp::JitMoments>(items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, V, Cout);
+}
 extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
 k_force_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
             const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
@@ -738,6 +804,7 @@ void jit_release(Engine &E)
     E.jit_module = nullptr;
     E.jit_symm = E.jit_force = E.jit_tangent = nullptr;
     E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = E.jit_force_momt = E.jit_force_few = nullptr;
+    E.jit_tangent_momt = E.jit_tangent_few = nullptr;
     E.jit_symm_few = nullptr;
 }
 
@@ -872,7 +939,8 @@ std::string jit_build(Engine &E)
     if (E.mom_ok) {
         fns.push_back({"k_symm_jit", &E.jit_symm_mom});
         if (E.mom_thread()) fns.push_back({"k_symm_jit_t", &E.jit_symm_momt});
-        if (E.mom_force_thread()) fns.push_back({"k_force_jit_t", &E.jit_force_momt}), fns.push_back({"k_force_few", &E.jit_force_few});
+        if (E.mom_force_thread()) fns.push_back({"k_force_jit_t", &E.jit_force_momt}), fns.push_back({"k_force_few", &E.jit_force_few}),
+            fns.push_back({"k_tangent_jit_t", &E.jit_tangent_momt}), fns.push_back({"k_tangent_few", &E.jit_tangent_few});
         fns.push_back({"k_force_jit", &E.jit_force_mom1});
         fns.push_back({"k_force_jit2", &E.jit_force_mom2});
         fns.push_back({"k_symm_few", &E.jit_symm_few});

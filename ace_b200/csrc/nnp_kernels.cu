@@ -2010,6 +2010,29 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
     return jit_launch(na == 2 ? E.jit_force_mom2 : E.jit_force_mom1, nmain + nfew, NNP_MOM_FORCE_WARPS * 32, sm, E.stream, args);
 }
 
+bool run_tangent_mom(Engine &E, std::string &msg)
+{
+    const int64_t N = E.n_centre;
+    if (!E.use_jit || !E.jit_tangent_momt || !E.mom_valid || !mom_by_thread(E, N)) return false;
+    const int T = E.dpot.ntypes;
+    if (E.momd.reserve((size_t)E.mom_rows * mom_vals(T, E.mom_ND, E.mom_L)) != cudaSuccess) {
+        cudaGetLastError();                                       // the pair loops need no such buffer
+        return false;
+    }
+    long long l = 0, h = N;
+    int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
+    const int *nitems = &E.err.p->few, *ord = E.visit();
+    void *args[] = {&l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p, &cap, &gs, &E.tvec.p,
+                    &E.mom.p, &E.momd.p, &E.mom_cnt.p, &E.tang.p};
+    void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,
+                   &E.mom_cnt.p, &E.tvec.p, &E.tang.p};
+    E.launches += 2;
+    msg = jit_launch(E.jit_tangent_momt, grid_for(N, NNP_MOM_THREADS, 1 << 30), NNP_MOM_THREADS,
+                     mom_thread_floats(T, E.mom_ND, E.mom_L) * sizeof(float), E.stream, args);
+    if (msg.empty()) msg = jit_launch(E.jit_tangent_few, num_sms() * 16, NNP_MOM_FEW_THREADS, 0, E.stream, few);
+    return true;
+}
+
 std::string run_symm(Engine &E)
 {
     const int64_t N = E.n_centre;      // centres: the first n_centre entries of `order`

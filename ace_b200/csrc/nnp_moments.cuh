@@ -46,7 +46,9 @@
 //   neighbour of element t, radial_force(II, t, r, fc, fcd, eb, out): sum of
 //   eb_f dG_f/dr, few_symm(II, tt, cs, w, acc): acc_f += x_f^zeta w_d,
 //   few_force(II, tt, cs, e, wa, wda, wb, wdb, hc, ha, hb): dE/dcos, dE/dr_a and
-//   dE/dr_b of one pair.
+//   dE/dr_b of one pair, radial_drow(II, t, r, fc, fd, row): slopes of the radial
+//   functions, few_tangent(II, tt, cs, w, dw, acc): acc_f += dx_f^zeta/dcos w_d +
+//   x_f^zeta dw_d.
 #pragma once
 
 #include "nnp_device.cuh"
@@ -786,6 +788,51 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
     }
 }
 
+// Angular functions of a thread's atom from S and the sums of w_d^2 (entries
+// BT apart): G_f = sum_l c_l S_l - self (c and self as in dE/dA: half of them
+// for J == K), self = -wscale sum w_d^2.  Blocks of few pairs are 0 here.
+template <class M>
+__device__ __forceinline__ void mom_functions_thread(const MomTab &tb, int fmax, int II, const DevType &Ty,
+                                                     const unsigned short *cnt, const f32x2 *S, const f32x2 *W2,
+                                                     float wscale, float *Gi)
+{
+    constexpr int T = M::T, L = M::L, NDP = (M::ND + 1) / 2, DL = mom_dl(L), BT = NNP_MOM_THREADS;
+#pragma unroll 1
+    for (int K = 0, tt = 0; K < T; ++K)
+#pragma unroll 1
+        for (int J = 0; J <= K; ++J, ++tt) {
+            const bool few = mom_pairs(cnt, J, K) <= NNP_MOM_FEW;    // added by the blocks of few pairs
+            const int off = Ty.ba[tt].off_g, bn = Ty.ba[tt].n, f0 = II * fmax + off - Ty.n_input_r;
+            const ulonglong2 *cf = reinterpret_cast<const ulonglong2 *>(tb.dcoef + (i64)f0 * DL);
+            const float h = J == K ? 0.5f : 1.f;
+            f32x2 st[DL];                                    // S, -sum of w_d^2
+#pragma unroll
+            for (int l = 0; l < DL; ++l) st[l] = 0ull;
+#pragma unroll 2
+            for (int f = 0; f < bn; ++f) {
+                const int p = NDP > 1 ? (tb.fun[f0 + f] >> 9) & 0x7f : 0;
+                if (NDP > 1 || f == 0) {
+#pragma unroll
+                    for (int l = 0; l <= L; ++l) st[l] = S[((tt * NDP + p) * (L + 1) + l) * BT];
+                    st[L + 1] = mul2(W2[(J * NDP + p) * BT], dup2(wscale));
+                }
+                f32x2 c[DL], g = 0ull;
+#pragma unroll
+                for (int l = 0; l < DL; l += 2) {
+                    const ulonglong2 v = __ldg(cf + f * (DL / 2) + l / 2);
+                    c[l] = v.x;
+                    c[l + 1] = v.y;
+                }
+#pragma unroll
+                for (int l = L; l >= 0; --l) g = fma2(c[l], st[l], g);
+                g = fma2(c[L + 1], st[L + 1], g);
+                float g0, g1;
+                up2(g, g0, g1);
+                Gi[off + f] = few ? 0.f : h * (g0 + g1);
+            }
+        }
+}
+
 // The same with one thread per atom: the moments of one neighbour element and
 // damping pair are the thread's registers (81 packed pairs for L = 8) while it
 // walks that element's segment of its list, so nothing is staged, exchanged or
@@ -807,7 +854,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                                      unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems, float *smem)
 {
     constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
-                  NR = M::NR, NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), DL = mom_dl(L), BT = NNP_MOM_THREADS;
+                  NR = M::NR, NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), BT = NNP_MOM_THREADS;
     f32x2 *S = reinterpret_cast<f32x2 *>(smem) + threadIdx.x;    // [NS][BT]
     f32x2 *W2 = S + NS * BT;                                     // [T][NDP][BT]
     const DevPot &P = *pot;
@@ -924,41 +971,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
 #pragma unroll
                 for (int tt = 0; tt < TT; ++tt) S[((tt * NDP + p) * (L + 1) + l) * BT] = s[tt];
             }
-        // G_f = sum_l c_l S_l - self (c and self as in dE/dA: half of them for J == K)
-#pragma unroll 1
-        for (int K = 0, tt = 0; K < T; ++K)
-#pragma unroll 1
-            for (int J = 0; J <= K; ++J, ++tt) {
-                const bool few = mom_pairs(cnt, J, K) <= NNP_MOM_FEW;    // added by the blocks of few pairs
-                const int off = Ty.ba[tt].off_g, bn = Ty.ba[tt].n, f0 = II * fmax + off - Ty.n_input_r;
-                const ulonglong2 *cf = reinterpret_cast<const ulonglong2 *>(tb.dcoef + (i64)f0 * DL);
-                const float h = J == K ? 0.5f : 1.f;
-                f32x2 st[DL];                                    // S, -sum of w_d^2
-#pragma unroll
-                for (int l = 0; l < DL; ++l) st[l] = 0ull;
-#pragma unroll 2
-                for (int f = 0; f < bn; ++f) {
-                    const int p = NDP > 1 ? (tb.fun[f0 + f] >> 9) & 0x7f : 0;
-                    if (NDP > 1 || f == 0) {
-#pragma unroll
-                        for (int l = 0; l <= L; ++l) st[l] = S[((tt * NDP + p) * (L + 1) + l) * BT];
-                        st[L + 1] = mul2(W2[(J * NDP + p) * BT], dup2(-1.f));
-                    }
-                    f32x2 c[DL], g = 0ull;
-#pragma unroll
-                    for (int l = 0; l < DL; l += 2) {
-                        const ulonglong2 v = __ldg(cf + f * (DL / 2) + l / 2);
-                        c[l] = v.x;
-                        c[l + 1] = v.y;
-                    }
-#pragma unroll
-                    for (int l = L; l >= 0; --l) g = fma2(c[l], st[l], g);
-                    g = fma2(c[L + 1], st[L + 1], g);
-                    float g0, g1;
-                    up2(g, g0, g1);
-                    Gi[off + f] = few ? 0.f : h * (g0 + g1);
-                }
-            }
+        mom_functions_thread<M>(tb, fmax, II, Ty, cnt, S, W2, -1.f, Gi);
         for (int f = Ty.n_input; f < gstride; ++f) Gi[f] = 0.f;
     }
 }
@@ -1403,6 +1416,218 @@ __device__ void mom_force_thread_body(int block, int nblock, i64 lo, i64 hi, con
 #pragma unroll
         for (int x = 0; x < 3; ++x) atomicAdd(&F[3 * i + x], -f0[x]);
         if (bad) atomicMax(&err->nonfinite, 1);
+    }
+}
+
+// ---------------------------------------------------------------- tangents
+
+// C_i = sum_k dG_i/dx_k V_k of the training gradient (see tangent_body), one
+// thread per atom with at most two damping factors: the moments' derivatives
+//   A' = sum_k w'_k rr_k Y(u_k) + w_k (u'_k . grad) Y,
+//   rr = u . dv, u' = (dv - rr u) / r, dv = V_i - V_k,
+// are the thread's registers as in mom_symm_thread_body, and S' = A'^J A^K +
+// A^J A'^K replaces S.  r_n^m and its slope r_(n-1)^(m+1) as in
+// mom_gradient_regs; (C, S) = w (x + i y)^m and (Cd, Sd) its derivative.
+// Bound: issue and latency at 8 warps per SM (registers).  41 k atoms of two
+// elements: training step 909 us (a warp per atom over the pairs) -> 794 us.
+template <class M>
+__device__ void mom_tangent_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab,
+                                        int fmax, const int *__restrict__ type, const int *__restrict__ order,
+                                        const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap,
+                                        int gstride, const float4 *__restrict__ V, const float2 *__restrict__ mom,
+                                        float2 *momd, const unsigned short *__restrict__ mom_cnt,
+                                        float *__restrict__ Cout, float *smem)
+{
+    constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NC = mom_comps(L), NR = M::NR,
+                  NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), BT = NNP_MOM_THREADS;
+    f32x2 *S = reinterpret_cast<f32x2 *>(smem) + threadIdx.x;    // [NS][BT]
+    f32x2 *W2 = S + NS * BT;                                     // [T][BT]: sums of w w' rr
+    const DevPot &P = *pot;
+    const MomTab tb = mom_tab(tab, T, L, fmax);
+    for (i64 idx = lo + blockIdx.x * (i64)BT + threadIdx.x; idx < hi; idx += (i64)gridDim.x * BT) {
+        const i64 i = order[idx], r = idx - lo;
+        const int II = type[i];
+        if ((unsigned)II >= (unsigned)T) continue;               // type out of range (reported by the call)
+        const int n = nbr_cnt[i];
+        const DevType &Ty = P.t[II];
+        const float4 *src = nbr + i * cap;
+        float *Ci = Cout + i * gstride;
+        const unsigned short *cnt = mom_cnt + 8 * r;
+        const float4 vi = V[i];
+        int k = 0;
+        const float4 none = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+        float4 e = n > 0 ? src[0] : none, ve = vi;
+        if (n > 0) ve = V[__float_as_int(e.w) & 0x0fffffff];
+#pragma unroll 1
+        for (int J = 0; J < T; ++J) {
+            f32x2 acc[NC], ww = 0ull;
+            float rad[NR];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) acc[c] = 0ull;
+#pragma unroll
+            for (int f = 0; f < NR; ++f) rad[f] = 0.f;
+#pragma unroll 1
+            while ((int)((unsigned)__float_as_int(e.w) >> 28) == J) {
+                MomNbr<M, true> v;
+                v.set(e, Ty, tb.a_lo + II * NNP_MOM_MAXD);
+                const float dx = vi.x - ve.x, dy = vi.y - ve.y, dz = vi.z - ve.z;
+                ++k;
+                mom_prefetch(src + min(k + 6, n - 1));
+                e = k < n ? src[k] : none;
+                if (k < n) ve = V[__float_as_int(e.w) & 0x0fffffff];
+                const float rr = v.ux * dx + v.uy * dy + v.uz * dz;
+                const float xd = (dx - rr * v.ux) * v.ir, yd = (dy - rr * v.uy) * v.ir, zd = (dz - rr * v.uz) * v.ir;
+                const f32x2 w2 = pk2(v.w[0], ND > 1 ? v.w[ND > 1 ? 1 : 0] : 0.f);
+                f32x2 C = w2, Sn = 0ull, Sd = 0ull, Cd = pk2(v.wd[0] * rr, ND > 1 ? v.wd[ND > 1 ? 1 : 0] * rr : 0.f);
+                ww = fma2(C, Cd, ww);
+                const f32x2 x2 = dup2(v.ux), y2 = dup2(v.uy), ny2 = dup2(-v.uy), xd2 = dup2(xd), yd2 = dup2(yd),
+                            nyd2 = dup2(-yd), zd2 = dup2(zd);
+                float zn[L + 1];
+#pragma unroll
+                for (int q = 1; q <= L; ++q) zn[q] = v.uz * (1.f / (float)(q + 1));
+#pragma unroll
+                for (int m = 0; m <= L; ++m) {
+                    const f32x2 Cz = mul2(C, zd2), Sz = mul2(Sn, zd2);
+                    float q0 = 1.f, q1 = 0.f, p0 = 0.f, p1 = 0.f;   // r_n^m, its slope
+#pragma unroll
+                    for (int l = m; l <= L; ++l) {
+                        const int n1 = l - m;
+                        const f32x2 q2 = dup2(q0), p2 = dup2(p0);
+                        if (m == 0) {
+                            acc[l] = fma2(q2, Cd, acc[l]);
+                            if (n1 > 0) acc[l] = fma2(p2, Cz, acc[l]);
+                        } else {
+                            const int c = mom_base(L, m > 0 ? m : 1) + 2 * n1;
+                            acc[c] = fma2(q2, Cd, acc[c]);
+                            acc[c + 1] = fma2(q2, Sd, acc[c + 1]);
+                            if (n1 > 0) {
+                                acc[c] = fma2(p2, Cz, acc[c]);
+                                acc[c + 1] = fma2(p2, Sz, acc[c + 1]);
+                            }
+                        }
+                        const float t = n1 == 0 ? v.uz
+                                                : fmaf(zn[n1 > 0 ? n1 : 1], q0,
+                                                       (-mom_beta(l, m) / (float)(n1 > 0 ? n1 * (n1 + 1) : 1)) * q1);
+                        q1 = q0;
+                        q0 = t;
+                        // r_(n1)^(m+1) from its two before (n1 - 1 of order m + 1 is l of m + 1)
+                        const float s = n1 == 0 ? 1.f
+                                        : n1 == 1 ? v.uz
+                                                  : fmaf(zn[n1 > 1 ? n1 - 1 : 1], p0,
+                                                         (-mom_beta(l, m + 1) / (float)(n1 > 1 ? (n1 - 1) * n1 : 1)) * p1);
+                        p1 = p0;
+                        p0 = s;
+                    }
+                    const f32x2 c = C, cd = Cd;
+                    Cd = fma2(Sd, ny2, fma2(Sn, nyd2, fma2(cd, x2, mul2(c, xd2))));
+                    Sd = fma2(Sd, x2, fma2(Sn, xd2, fma2(cd, y2, mul2(c, yd2))));
+                    C = fma2(Sn, ny2, mul2(c, x2));
+                    Sn = fma2(Sn, x2, mul2(c, y2));
+                }
+                {
+                    float rv[NR];
+#pragma unroll
+                    for (int f = 0; f < NR; ++f) rv[f] = 0.f;
+                    M::radial_drow(II, J, v.r, v.fc, v.fd, rv);
+#pragma unroll
+                    for (int f = 0; f < NR; ++f) rad[f] = fmaf(rv[f], rr, rad[f]);
+                }
+            }
+            f32x2 *dst = reinterpret_cast<f32x2 *>(momd) + mom_at(r, J * NC, NV, NNP_MOM_SH_T);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) dst[c << NNP_MOM_SH_T] = mul2(acc[c], dup2(M::gnorm(c)));
+            W2[J * BT] = ww;
+            const DevBlockR B = Ty.br[J];
+#pragma unroll
+            for (int f = 0; f < NR; ++f)
+                if (f < B.n) Ci[B.off_g + f] = rad[f];
+        }
+        const f32x2 *a = reinterpret_cast<const f32x2 *>(mom) + mom_at(r, 0, NV, NNP_MOM_SH_T);
+        const f32x2 *d = reinterpret_cast<const f32x2 *>(momd) + mom_at(r, 0, NV, NNP_MOM_SH_T);
+#pragma unroll
+        for (int l = 0; l <= L; ++l) {
+            f32x2 s[TT];
+#pragma unroll
+            for (int tt = 0; tt < TT; ++tt) s[tt] = 0ull;
+#pragma unroll
+            for (int m = 0; m <= l; ++m)
+#pragma unroll
+                for (int h = 0; h < (m ? 2 : 1); ++h) {
+                    const int c = m == 0 ? l : mom_base(L, m > 0 ? m : 1) + 2 * (l - m) + h;
+                    f32x2 va[T], vd[T];
+#pragma unroll
+                    for (int J = 0; J < T; ++J) {
+                        va[J] = a[(J * NC + c) << NNP_MOM_SH_T];
+                        vd[J] = d[(J * NC + c) << NNP_MOM_SH_T];
+                    }
+#pragma unroll
+                    for (int K = 0; K < T; ++K)
+#pragma unroll
+                        for (int J = 0; J <= K; ++J) {
+                            const int tt = K * (K + 1) / 2 + J;
+                            s[tt] = fma2(va[J], vd[K], fma2(vd[J], va[K], s[tt]));
+                        }
+                }
+#pragma unroll
+            for (int tt = 0; tt < TT; ++tt) S[(tt * (L + 1) + l) * BT] = s[tt];
+        }
+        mom_functions_thread<M>(tb, fmax, II, Ty, cnt, S, W2, -2.f, Ci);
+        for (int f = Ty.n_input; f < gstride; ++f) Ci[f] = 0.f;
+    }
+}
+
+// Tangents of the listed blocks, 16 lanes each, a lane per pair.
+template <class M>
+__device__ void mom_few_tangent_body(const int2 *__restrict__ items, const int *__restrict__ nitems, i64 lo,
+                                     const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+                                     const int *__restrict__ type, const int *__restrict__ order,
+                                     const float4 *__restrict__ nbr, int cap, int gstride,
+                                     const unsigned short *__restrict__ mom_cnt, const float4 *__restrict__ V,
+                                     float *__restrict__ Cout)
+{
+    const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
+    const int nit = *nitems, h = threadIdx.x & 15;
+    const unsigned mask = 0xffffu << (threadIdx.x & 16);
+    for (int q = (blockIdx.x * NNP_MOM_FEW_THREADS + threadIdx.x) >> 4; q < nit; q += gridDim.x * (NNP_MOM_FEW_THREADS / 16)) {
+        const int2 it = items[q];
+        const i64 i = order[lo + it.x];
+        const int II = type[i], tt = it.y;
+        const DevType &Ty = pot->t[II];
+        const MomFew b = mom_few(mom_cnt + 8 * (i64)it.x, M::T, tt, h);
+        MomNbr<M, true> v;
+        const float4 rec = nbr[i * cap + mom_few_slot(b, h)], vi = V[i], vk = V[__float_as_int(rec.w) & 0x0fffffff];
+        v.set(rec, Ty, tb.a_lo + II * NNP_MOM_MAXD);
+        const float dv[3] = {vi.x - vk.x, vi.y - vk.y, vi.z - vk.z}, u[3] = {v.ux, v.uy, v.uz};
+        const float rr = u[0] * dv[0] + u[1] * dv[1] + u[2] * dv[2];
+        float cs = 0.f, cd = 0.f, w[M::ND], dw[M::ND], acc[M::NA];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            const float ud = (dv[x] - rr * u[x]) * v.ir;
+            const float ua = __shfl_sync(mask, u[x], b.a, 16), ub = __shfl_sync(mask, u[x], b.b, 16);
+            const float da = __shfl_sync(mask, ud, b.a, 16), db = __shfl_sync(mask, ud, b.b, 16);
+            cs = fmaf(ua, ub, cs);
+            cd = fmaf(da, ub, fmaf(ua, db, cd));
+        }
+#pragma unroll
+        for (int d = 0; d < M::ND; ++d) {
+            const float wr = v.wd[d] * rr;
+            const float wa = __shfl_sync(mask, v.w[d], b.a, 16), wb = __shfl_sync(mask, v.w[d], b.b, 16);
+            const float ra = __shfl_sync(mask, wr, b.a, 16), rb = __shfl_sync(mask, wr, b.b, 16);
+            w[d] = wa * wb * cd;
+            dw[d] = fmaf(ra, wb, wa * rb);
+        }
+#pragma unroll
+        for (int f = 0; f < M::NA; ++f) acc[f] = 0.f;
+        if (h < b.pairs) M::few_tangent(II, tt, cs, w, dw, acc);
+        const int n = Ty.ba[tt].n;
+        float *Cb = Cout + i * gstride + Ty.ba[tt].off_g;
+#pragma unroll
+        for (int f = 0; f < M::NA; ++f) {
+            float s = acc[f];
+#pragma unroll
+            for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(mask, s, o, 16);
+            if (h == 0 && f < n) Cb[f] = s;
+        }
     }
 }
 

@@ -433,15 +433,18 @@ std::string run_train_grad(Engine &E, bool with_force)
         const size_t sm = (size_t)WARPS * ((per + 3) & ~3) * sizeof(float);
         if (sm > 227 * 1024) return "neighbour capacity too large for the tangent kernel";
         const int grid = grid_for(N, WARPS, nsm * 16);
-        E.launches += 1;
-        if (E.use_jit && E.jit_tangent) {
+        std::string tmsg;
+        const bool done = run_tangent_mom(E, tmsg);
+        if (!tmsg.empty()) return tmsg;
+        E.launches += done ? 0 : 1;
+        if (!done && E.use_jit && E.jit_tangent) {
             long long n = N;
             int cap = E.cap, gs = E.gstride;
             void *args[] = {&n, &E.d_pot, &E.rpar.p, &E.apar.p, &E.type.p, &E.order.p, &E.nbr.p, &E.nbr_cnt.p,
                             &cap, &ncut, &ndamp, &gs, &E.tvec.p, &E.tang.p};
             std::string msg = jit_launch(E.jit_tangent, grid, WARPS * 32, sm, E.stream, args);
             if (!msg.empty()) return msg;
-        } else {
+        } else if (!done) {
             cudaFuncSetAttribute(k_tangent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_tangent<<<grid, WARPS * 32, sm, E.stream>>>(N, E.d_pot, E.rpar.p, E.apar.p, E.type.p, E.order.p, E.nbr.p,
                                                           E.nbr_cnt.p, E.cap, ncut, ndamp, E.gstride, E.tvec.p, E.tang.p);

@@ -263,3 +263,30 @@ def test_thread_forms_at_their_limits(tmp_path, shape, n):
     assert (np.abs(E[some] - Es) / np.diff(sub.atom_off)).max() < 1e-6
     assert np.abs(F[at] - Fs).max() < 5e-6 and np.abs(F - Fm).max() < 5e-6
     assert (np.abs(Wm[some] - Ws).reshape(len(some), -1).max(1) / np.diff(sub.atom_off)).max() < 5e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 20, [8], [9.0]), (2, 3, [3, 8], [7.0]), (3, 5, [1, 8], [7.0, 14.0]), (4, 4, [2, 8], [7.0, 14.0])],
+                         ids=lambda s: "T%d" % s[0])
+def test_training_gradient_from_moments(tmp_path, shape):
+    """Tangent symmetry functions of a thread per atom (16033 atoms, blocks of no
+    and of few pairs) against the generic pair loops: the gradient within 1e-5 of
+    its largest entry (FP32 rows to 2e-5 of their largest value, summed over
+    atoms)."""
+    nt, nrad, zetas, etas = shape
+    pot = basis(nt, nrad, zetas, etas, ["COS"], 6.0)
+    path = str(tmp_path / "pot.nnp")
+    potential.write(path, pot)
+    rng = np.random.default_rng(2)
+    counts = [1, 2, 5] + list(rng.integers(20, 300, 400))
+    counts = counts[:int(np.searchsorted(np.cumsum(counts), 16033))]
+    counts.append(16033 - sum(counts))
+    b = synth.batch_random(8, counts, nt, density=0.05)
+    e_ref, f_ref = rng.normal(0, 1, len(counts)), rng.normal(0, 1, (b.n_atoms, 3))
+    nn = NNP.read(path)
+    loss, g, _, _ = nn.train_grad(b.atom_off, b.pos, b.type, b.cell, e_ref, f_ref, 0.5)
+    nn.set_specialization(False)
+    loss0, g0, _, _ = nn.train_grad(b.atom_off, b.pos, b.type, b.cell, e_ref, f_ref, 0.5)
+    nn.close()
+    assert abs(loss - loss0) < 1e-5 * abs(loss0)
+    assert np.abs(g - g0).max() < 1e-5 * np.abs(g0).max()
