@@ -12,12 +12,17 @@
 //                  most 2048 atoms and 32 structures
 //   k_neigh        one block per cell or part of a cell: candidates from the
 //                  (2m+1)^3 cells gathered in shared memory, one warp per atom,
-//                  exact FP64 displacement test, neighbours grouped by type
+//                  FP32 test with a margin, exact FP64 displacement test of
+//                  what passes, neighbours grouped by type
 //                  (replaces NeighborList::build, struc/neighbor.cpp:46-87)
+//   k_len_*        visiting order by neighbour counts (thread-per-atom kernels)
 //   k_symm         one warp per atom: radial + angular symmetry functions
-//                  (NNP::compute_symm, nnp/nnp.cpp:350-392)
+//                  (NNP::compute_symm, nnp/nnp.cpp:350-392); compiled at run
+//                  time for the potential, a warp or a thread per atom from
+//                  moments of the neighbours (nnp_moments.cuh) or over pairs
 //   k_nn_fp32      one warp per atom: network forward + input gradient dE/dG
-//                  (ANN::fpbp + DODZ::grad, ml/nn.cpp:1402-1420,1836-1859)
+//                  (ANN::fpbp + DODZ::grad, ml/nn.cpp:1402-1420,1836-1859);
+//                  k_nn_tile in tiles of 32 atoms, k_nn_tc on the tensor cores
 //   k_force        one warp per atom: adjoint of the symmetry functions,
 //                  per-neighbour gradients, FP64 force scatter
 //                  (NNP::compute_force, nnp/nnp.cpp:412-476)

@@ -118,13 +118,31 @@ def build_potential(name: str, path: str, seed: int = 1234):
     return pot
 
 
+def moment_degree(pot):
+    """Largest zeta of a potential whose angular functions the library forms
+    from moments (GAUSS, integer zeta of at most 8), else 0."""
+    L = 0
+    for row in pot.basis_a:
+        for B in row:
+            z = np.asarray(B.zeta, dtype=np.float64)
+            if B.size and (B.form != "GAUSS" or (z != np.round(z)).any() or z.max() > 8 or z.min() < 0):
+                return 0
+            L = max(L, int(z.max()) if B.size else 0)
+    return L
+
+
 def flops_per_stage(pot, types: np.ndarray, counts: np.ndarray):
     """Algorithmic FLOPs (FMA = 2) of the symmetry-function and force kernels
-    and the networks, from the per-atom neighbour counts by type: the per-atom
-    count P(20 + 20 nR) + T(57 + 24 nA) + 4 sum n_{l-1} n_l, split as
-    symm P(10 + 8 nR) + T(25 + 10 nA), force P(10 + 12 nR) + T(32 + 14 nA)."""
+    and the networks, from the per-atom neighbour counts by type.  Moment form
+    (L = largest zeta, M = (L + 1)^2 moments, D damping factors per element):
+    symm P(40 + 8 nR + 2 D M + 3 (L+1)(L+2)/2) per neighbour and 2 D M per block
+    and atom, forces P(60 + 12 nR + 4 D M + 3 (L+1)(L+2)/2 + 24 D L) and
+    4 D M per ordered pair of elements and atom.  Pair loops (other
+    potentials): symm P(10 + 8 nR) + T(25 + 10 nA), force P(10 + 12 nR) +
+    T(32 + 14 nA).  Networks 4 sum n_{l-1} n_l."""
     from ace_b200.potential import tt_index
     Tn = pot.ntypes
+    L = moment_degree(pot)
     f_symm = f_force = f_nn = 0.0
     pairs = trip = 0.0
     for II in range(Tn):
@@ -132,27 +150,30 @@ def flops_per_stage(pot, types: np.ndarray, counts: np.ndarray):
         c = counts[sel].astype(np.float64)          # [n_II, T]
         if len(c) == 0:
             continue
+        D = len({(B.rc, B.cut, e) for B in pot.basis_a[II] for e in np.asarray(B.eta)}) if L else 0
+        M, rec = (L + 1) ** 2, 3 * (L + 1) * (L + 2) / 2
         for J in range(Tn):
             nR = pot.basis_r[II][J].size
             P = c[:, J].sum()
             pairs += P
-            f_symm += P * (10 + 8 * nR)
-            f_force += P * (10 + 12 * nR)
+            f_symm += P * (40 + 8 * nR + 2 * D * M + rec if L else 10 + 8 * nR)
+            f_force += P * (60 + 12 * nR + 4 * D * M + rec + 24 * D * L if L else 10 + 12 * nR)
         for J in range(Tn):
             for K in range(J, Tn):
                 nA = pot.basis_a[II][tt_index(J, K)].size
                 t = (c[:, J] * (c[:, J] - 1) / 2).sum() if J == K else (c[:, J] * c[:, K]).sum()
                 trip += t
-                f_symm += t * (25 + 10 * nA)
-                f_force += t * (32 + 14 * nA)
+                f_symm += len(c) * 2 * D * M if L else t * (25 + 10 * nA)
+                f_force += len(c) * (4 if J == K else 8) * D * M if L else t * (32 + 14 * nA)
         nodes = pot.nets[II].nodes
         f_nn += len(c) * 4 * sum(nodes[l] * nodes[l + 1] for l in range(len(nodes) - 1))
     return {"symm": f_symm, "forces": f_force, "networks": f_nn, "pairs": pairs, "triplets": trip}
 
 
 # DRAM bytes per atom of one launch, from the ncu capture of the 512-structure
-# case of the batched workload (dram__bytes_read.sum + dram__bytes_write.sum / atoms)
-DRAM_BYTES_PER_ATOM = {"k_force_jit": 146.598144e6 / 134400, "k_symm_jit": 119.099648e6 / 134400}
+# case of the batched workload (dram__bytes.sum.per_second x duration / atoms); the
+# moments (2 KB per atom) are written by one and read by the other
+DRAM_BYTES_PER_ATOM = {"k_force_jit_t": 492.8e6 / 134400, "k_symm_jit_t": 392.0e6 / 134400}
 
 
 def traffic_bytes(kernel: str, atoms: int):
@@ -471,13 +492,15 @@ def time_inference(args, name, nn, pot, b, world, dist, clocks, dev, stream):
     achieved = fl[kern] / (per_step[kern] / 1e3) / 1e12
     jit = bool(nn.specialization()[0])
     kname = ("k_symm" if kern == "symm" else "k_force") + ("_jit" if jit else "")
+    if jit and moment_degree(pot) and N >= {"symm": 16000, "forces": 40000}[kern]:
+        kname += "_t"                               # a thread per atom
     roofline = {"bound": "fp32", "kernel": kname, "achieved": round(achieved, 3), "peak": round(peak_fp32, 2),
                 "unit": "TFLOP/s", "frac": round(achieved / peak_fp32, 4),
                 "peak_source": "%d SMs x 128 FP32 FMA/clk x 2 x measured %.0f MHz (no FP32 figure in "
                                "MEASURED_PEAKS.json)" % (n_sm, sm_mhz),
                 "traffic": traffic_bytes(kname, N) if name == "batched" else None}
     if roofline["traffic"] is not None:
-        roofline["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one %s launch on the "
+        roofline["traffic_source"] = ("ncu DRAM bytes (read + write) of one %s launch on the "
                                       "first 512 structures (134,400 atoms), scaled by atoms" % kname)
     line = {
         "metric": METRIC, "value": round(value, 1), "unit": UNIT, "n_gpus": world, "steps": args.steps,

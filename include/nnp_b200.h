@@ -142,8 +142,10 @@ int nnp_specialization_check(const char *potential_path, char *log, int32_t log_
  * Choices (params[0..4]): blocks per SM the symmetry-function kernel's
  * registers are budgeted for, the same for the force kernel, the force
  * kernel's pair-loop unroll, its pair coefficients per chunk (a smaller
- * chunk needs less shared memory, so more blocks may be resident), and CTAs
- * per SM of the tensor-core network kernel (0 = as many as fit).
+ * chunk needs less shared memory, so more blocks may be resident), and tiles
+ * in flight per SM of the tensor-core network kernel (0 = as many as fit).
+ * The kernels of potentials whose angular functions are formed from moments
+ * (GAUSS, integer zeta of at most 8) have only the last of these.
  * nnp_tune_params returns the handle's current choices, where they came from
  * (*source: 0 defaults, 1 tuning cache, 2 tuned on this handle) and the last
  * tuning's measurements (*log).  nnp_tune_cache_key / _store / _load read and
