@@ -164,6 +164,16 @@ void Engine::graph_release()
     graph_launches = 0;
 }
 
+// Every buffer of the handle that a step uses: a graph holds their addresses,
+// and another call may have replaced one.  With the sizes, since a larger
+// buffer can get the address of the one that was freed for it.
+void Engine::buffer_key(std::vector<int64_t> &key) const
+{
+    auto add = [&](const auto &...b) { (..., (key.push_back((int64_t)(intptr_t)b.p), key.push_back((int64_t)b.n))); };
+    add(xw, atom_struct, atom_cell, grid, bbox, scan_tmp, cell_cnt, cell_start, cell_fill, cell_tcnt, cell_atoms, cell_pos, order,
+        type_fill, neigh_items, nbr, nbr_cnt, G, dEdG, e_atom, e_struct, force, err, vir, mom, mom_cnt, mom_items, len_order);
+}
+
 // Build the device potential.  Angular functions of one BasisA that form a
 // run of equal eta (BasisA::init, basis_angular.cpp:178-205) share the run's
 // first eta for their damping factor, as the reference does.
@@ -994,17 +1004,20 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
     bool graphs = E.use_graphs && !E.timing && E.stream != nullptr && E.stream != cudaStreamLegacy &&
                   E.stream != cudaStreamPerThread;
     std::vector<int64_t> key;
-    if (graphs)
+    if (graphs) {
         key = {N, S, b->pbc, n_ghost, E.cap, (int64_t)flags, (int64_t)(atom_energy != nullptr), (int64_t)(virial != nullptr),
-               E.precision, (int64_t)(intptr_t)(E.use_jit ? E.jit_module : nullptr), (int64_t)E.acc64 + 2 * E.symm64,
-               (int64_t)(intptr_t)E.mom.p, E.mom_rows, (int64_t)(intptr_t)E.len_order.p,
-               (int64_t)(intptr_t)E.atom_off.p,
-               (int64_t)(intptr_t)E.pos.p, (int64_t)(intptr_t)E.type.p, (int64_t)(intptr_t)E.cell.p,
-               (int64_t)(intptr_t)E.nbr.p, (int64_t)(intptr_t)E.G.p, (int64_t)(intptr_t)E.force.p,
-               (int64_t)(intptr_t)E.e_struct.p, (int64_t)(intptr_t)E.e_atom.p, (int64_t)(intptr_t)E.vir.p};
+               E.precision, (int64_t)(intptr_t)(E.use_jit ? E.jit_module : nullptr), (int64_t)E.acc64 + 2 * E.symm64, E.mom_rows,
+               (int64_t)(intptr_t)E.atom_off.p, (int64_t)(intptr_t)E.pos.p, (int64_t)(intptr_t)E.type.p,
+               (int64_t)(intptr_t)E.cell.p};
+        E.buffer_key(key);
+    }
     for (int attempt = 0; attempt < 4; ++attempt) {
         std::string msg;
         if (graphs && E.graph_exec && key == E.graph_key) {
+            // the replayed step leaves behind what the captured one did
+            E.set_batch(N, S);
+            E.mom_valid = E.graph_mom_valid;
+            E.len_sorted = E.graph_len_sorted;
             chk(cudaGraphLaunch((cudaGraphExec_t)E.graph_exec, E.stream));
             E.launches += E.graph_launches;
         } else if (graphs && key == E.graph_key) {
@@ -1022,6 +1035,8 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
             if (g == cudaSuccess && msg.empty() && exec) {
                 E.graph_exec = exec;
                 E.graph_launches = E.launches - l0;
+                E.graph_mom_valid = E.mom_valid;
+                E.graph_len_sorted = E.len_sorted;
                 E.launches = l0;
                 chk(cudaGraphLaunch(exec, E.stream));
                 E.launches += E.graph_launches;
@@ -1059,7 +1074,7 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
             if (virial) out.add(virial, E.vir.p, sizeof(double) * 9 * S);
             if (ce == cudaSuccess) chk(out.enqueue(E));
         } else if (plain && (energy || forces)) {
-            nnp::run_outputs(E, (flags & NNP_ENERGY) ? energy : nullptr, (flags & NNP_FORCES) ? forces : nullptr);
+            nnp::run_outputs(E, S, N, (flags & NNP_ENERGY) ? energy : nullptr, (flags & NNP_FORCES) ? forces : nullptr);
         }
         chk(cudaMemcpyAsync(E.h_err, E.err.p, sizeof(nnp::DevErr), cudaMemcpyDeviceToHost, E.stream));
         chk(cudaStreamSynchronize(E.stream));

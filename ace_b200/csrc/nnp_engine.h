@@ -7,6 +7,7 @@
 
 #include <cstdint>
 #include <functional>
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -193,7 +194,16 @@ struct Engine {
     void *graph_exec = nullptr;     // cudaGraphExec_t
     std::vector<int64_t> graph_key;
     int64_t graph_launches = 0;     // kernels in the graph
+    bool graph_mom_valid = false, graph_len_sorted = false;   // mom_valid, len_sorted behind the captured step
     void graph_release();
+    // sizes of the batch that the buffers hold
+    void set_batch(int64_t atoms, int structs)
+    {
+        n_atoms = atoms;
+        n_centre = atoms - std::min<int64_t>(std::max<int64_t>(n_ghost, 0), atoms);
+        n_struct = structs;
+    }
+    void buffer_key(std::vector<int64_t> &key) const;
     cudaEvent_t ev[6] = {};
     int64_t launches = 0;
     void mark(int k)
@@ -229,7 +239,7 @@ std::string run_force(Engine &E);
 std::string run_energy(Engine &E, bool vacuum);
 std::string run_symm_to_double(Engine &E, double *out);
 std::string run_atom_energy(Engine &E, bool vacuum, double *out);
-std::string run_outputs(Engine &E, double *energy, double *forces);
+std::string run_outputs(Engine &E, int S, int64_t N, double *energy, double *forces);
 // tangent symmetry functions from the moments; false when the batch does not take that path
 bool run_tangent_mom(Engine &E, std::string &msg);
 std::string run_nn_from_symm(Engine &E, const double *symm_d, int gstride_in);

@@ -1696,9 +1696,7 @@ static size_t view_bytes(const Engine &E, bool force, bool jit)
 std::string run_prepare(Engine &E, int64_t n_atoms, int n_struct, int pbc)
 {
     (void)pbc;
-    E.n_atoms = n_atoms;
-    E.n_centre = n_atoms - std::min<int64_t>(std::max<int64_t>(E.n_ghost, 0), n_atoms);
-    E.n_struct = n_struct;
+    E.set_batch(n_atoms, n_struct);
     const size_t N = (size_t)std::max<int64_t>(n_atoms, 1), S = (size_t)std::max(n_struct, 1);
     const size_t cell_bound = 64 * S + 2 * N + 64;
     cudaError_t e = cudaSuccess;
@@ -2211,9 +2209,9 @@ __global__ void k_outputs(const DevErr *__restrict__ err, int cap, int64_t ne, c
     for (int64_t i = t; i < ne; i += step) energy[i] = es[i];
 }
 
-std::string run_outputs(Engine &E, double *energy, double *forces)
+std::string run_outputs(Engine &E, int S, int64_t N, double *energy, double *forces)
 {
-    const int64_t ne = energy ? E.n_struct : 0, nf = forces ? 3 * E.n_atoms : 0;
+    const int64_t ne = energy ? S : 0, nf = forces ? 3 * N : 0;
     k_outputs<<<grid_for(std::max(ne, nf), 512, num_sms() * 8), 256, 0, E.stream>>>(E.err.p, E.cap, ne, E.e_struct.p, energy,
                                                                                  nf, E.force.p, forces);
     E.launches += 1;
