@@ -1064,18 +1064,19 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
             if (flags & NNP_FORCES) out.add(forces, E.force.p, sizeof(double) * 3 * N);
             if (flags & NNP_SYMM) {
                 chk(E.symm_d.reserve((size_t)N * E.gstride + 1));
-                if (ce == cudaSuccess) nnp::run_symm_to_double(E, E.symm_d.p);
+                if (ce == cudaSuccess) msg = nnp::run_symm_to_double(E, E.symm_d.p);
                 out.add(symm_out, E.symm_d.p, sizeof(double) * N * E.gstride);
             }
             if (atom_energy) {
-                nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, E.eatom_d.p);
+                if (msg.empty()) msg = nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, E.eatom_d.p);
                 out.add(atom_energy, E.eatom_d.p, sizeof(double) * (N - n_ghost));
             }
             if (virial) out.add(virial, E.vir.p, sizeof(double) * 9 * S);
-            if (ce == cudaSuccess) chk(out.enqueue(E));
+            if (ce == cudaSuccess && msg.empty()) chk(out.enqueue(E));
         } else if (plain && (energy || forces)) {
-            nnp::run_outputs(E, S, N, (flags & NNP_ENERGY) ? energy : nullptr, (flags & NNP_FORCES) ? forces : nullptr);
+            msg = nnp::run_outputs(E, S, N, (flags & NNP_ENERGY) ? energy : nullptr, (flags & NNP_FORCES) ? forces : nullptr);
         }
+        if (!msg.empty()) { rc = fail(h, NNP_ERR_CUDA, msg); break; }
         chk(cudaMemcpyAsync(E.h_err, E.err.p, sizeof(nnp::DevErr), cudaMemcpyDeviceToHost, E.stream));
         chk(cudaStreamSynchronize(E.stream));
         if (ce != cudaSuccess) { rc = fail(h, NNP_ERR_CUDA, std::string("kernel failure: ") + cudaGetErrorString(ce)); break; }
@@ -1116,8 +1117,9 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
         } else if (!plain) {
             if ((flags & NNP_ENERGY) && energy) chk(cudaMemcpyAsync(energy, E.e_struct.p, sizeof(double) * S, cudaMemcpyDeviceToDevice, E.stream));
             if ((flags & NNP_FORCES) && forces) chk(cudaMemcpyAsync(forces, E.force.p, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, E.stream));
-            if (flags & NNP_SYMM) nnp::run_symm_to_double(E, symm_out);
-            if (atom_energy) nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, atom_energy);
+            if (flags & NNP_SYMM) msg = nnp::run_symm_to_double(E, symm_out);
+            if (atom_energy && msg.empty()) msg = nnp::run_atom_energy(E, (flags & NNP_VACUUM) != 0, atom_energy);
+            if (!msg.empty()) { rc = fail(h, NNP_ERR_CUDA, msg); break; }
             if (virial) chk(cudaMemcpyAsync(virial, E.vir.p, sizeof(double) * 9 * S, cudaMemcpyDeviceToDevice, E.stream));
             chk(cudaStreamSynchronize(E.stream));
         }
