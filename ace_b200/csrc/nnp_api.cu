@@ -125,7 +125,7 @@ void Engine::free_all()
 {
     rpar.release(); apar.release(); wpar.release(); vac.release();
     rpar64.release(); apar64.release(); cut64.release();
-    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release(); momd.release(); len_order.release();
+    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release(); mom_mask.release(); momd.release(); len_order.release();
     atom_off.release(); pos.release(); cell.release(); xw.release();
     type.release(); atom_struct.release(); atom_cell.release(); grid.release(); bbox.release();
     cell_cnt.release(); cell_start.release(); cell_fill.release(); cell_atoms.release(); scan_tmp.release();
@@ -171,7 +171,7 @@ void Engine::buffer_key(std::vector<int64_t> &key) const
 {
     auto add = [&](const auto &...b) { (..., (key.push_back((int64_t)(intptr_t)b.p), key.push_back((int64_t)b.n))); };
     add(xw, atom_struct, atom_cell, grid, bbox, scan_tmp, cell_cnt, cell_start, cell_fill, cell_tcnt, cell_atoms, cell_pos, order,
-        type_fill, neigh_items, nbr, nbr_cnt, G, dEdG, e_atom, e_struct, force, err, vir, mom, mom_cnt, mom_items, len_order);
+        type_fill, neigh_items, nbr, nbr_cnt, G, dEdG, e_atom, e_struct, force, err, vir, mom, mom_cnt, mom_items, mom_mask, len_order);
 }
 
 // Build the device potential.  Angular functions of one BasisA that form a

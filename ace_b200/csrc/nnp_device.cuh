@@ -103,7 +103,7 @@ struct DevErr {
     int bad_type;     // an atom type was outside [0, ntypes)
     int bad_cell;     // a periodic cell had no volume (1) or was thinner than rc / NNP_MAX_IMAGES (2)
     int nonfinite;    // a non-finite energy or force
-    int few;          // (atom, angular block) entries of few pairs (nnp_moments.cuh); not an error
+    int few, wide;    // (atom, angular block) entries of few pairs and of many (nnp_moments.cuh); not errors
 };
 
 #if defined(__CUDACC__)

@@ -102,8 +102,9 @@ struct Engine {
     void *jit_symm = nullptr, *jit_force = nullptr, *jit_tangent = nullptr;   // cudaKernel_t
     // cudaKernel_t, moment form: warp or thread per atom; one or two atoms per warp
     void *jit_symm_mom = nullptr, *jit_symm_momt = nullptr, *jit_force_mom1 = nullptr, *jit_force_mom2 = nullptr,
-         *jit_force_momt = nullptr, *jit_force_few = nullptr, *jit_tangent_momt = nullptr, *jit_tangent_few = nullptr;
-    void *jit_symm_few = nullptr;                                            // and the blocks of few pairs
+         *jit_force_momt = nullptr, *jit_tangent_momt = nullptr;
+    // and the blocks that are summed over pairs
+    void *jit_symm_list = nullptr, *jit_force_list = nullptr, *jit_tangent_list = nullptr;
     std::string jit_source, jit_error;
 
     // moment form of the angular functions (nnp_moments.cuh)
@@ -116,7 +117,8 @@ struct Engine {
     DBuf<float2> mom;             // moments of atoms visit()[0 .. mom_rows) (mom_at)
     DBuf<float2> momd;            // derivatives of the moments along the training step's displacements
     DBuf<unsigned short> mom_cnt; // their neighbour counts by element [row][8]
-    DBuf<int2> mom_items;         // (row, block) of the blocks of few pairs (number: DevErr::few)
+    DBuf<int2> mom_items;         // (row, block) of the blocks that are summed over pairs (MomLists)
+    DBuf<unsigned long long> mom_mask;   // their bits [row]
     int64_t mom_rows = 0;         // rows of `mom` the current batch uses (0: not reserved)
     bool mom_valid = false;       // they hold the whole batch's moments
     DBuf<int> len_order;          // visiting order by neighbour counts, its keys and ranks, its bins (run_len_order)

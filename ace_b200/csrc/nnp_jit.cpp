@@ -657,56 +657,70 @@ std::string make_source(const Engine &E, const TuneParams &tp)
     os << "}  // namespace nnp\n";
     if (E.mom_ok)
         os << R"(
-extern "C" __global__ void __launch_bounds__(NNP_MOM_SYMM_WARPS * 32)
+extern "C" __global__ void __launch_bounds__(NNP_MOM_SYMM_WARPS * 32, 7)
 k_symm_jit(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
    const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
    const int *__restrict__ nbr_cnt, int cap, int gstride, float *__restrict__ G, float2 *mom,
-   unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems)
+   unsigned short *__restrict__ mom_cnt, const nnp::MomLists ls)
 {
     extern __shared__ float4 smem4[];
-    nnp::mom_symm_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, items, nitems,
+    nnp::mom_symm_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, ls,
         reinterpret_cast<float *>(smem4));
 }
-#define NNP_FORCE_KERNEL(name, na) \
-extern "C" __global__ void __launch_bounds__(NNP_MOM_FORCE_WARPS * 32) \
+#define NNP_FORCE_KERNEL(name, na, ...) \
+extern "C" __global__ void __launch_bounds__(__VA_ARGS__) \
 name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, \
      const float2 *__restrict__ rpar, const int *__restrict__ type, const int *__restrict__ order, \
      const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride, \
      const float *__restrict__ dEdG, const float2 *__restrict__ mom, int msh, const unsigned short *__restrict__ mom_cnt, \
-     const int2 *__restrict__ items, const int *__restrict__ nitems, double *__restrict__ F, nnp::DevErr *err, \
+     const nnp::MomLists ls, double *__restrict__ F, nnp::DevErr *err, \
      const int *__restrict__ atom_struct, double *__restrict__ vir) \
 { \
     extern __shared__ float4 smem4[]; \
     const int nfew = (int)gridDim.x - nmain; \
-    if ((int)blockIdx.x < nfew) \
-        nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x, nfew, \
-            NNP_MOM_FORCE_WARPS * 32, items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, \
-            err, atom_struct, vir); \
-    else \
+    if ((int)blockIdx.x >= nfew) \
         nnp::mom_force_body<nnp::JitMoments, na>((int)blockIdx.x - nfew, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr, nbr_cnt, cap, \
-            gstride, dEdG, mom, msh, mom_cnt, F, err, atom_struct, vir, reinterpret_cast<float *>(smem4)); \
+            gstride, dEdG, mom, msh, ls.mask, F, err, atom_struct, vir, reinterpret_cast<float *>(smem4)); \
+    else if (na == 1) { \
+        nnp::mom_wide_force_body<nnp::JitMoments>((int)blockIdx.x, nfew, NNP_MOM_FORCE_WARPS * 32, ls, lo, pot, tab, fmax, \
+            type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, vir); \
+        nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x, nfew, NNP_MOM_FORCE_WARPS * 32, ls, lo, pot, tab, fmax, \
+            type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, vir); \
+    } \
 }
-NNP_FORCE_KERNEL(k_force_jit, 1)
-NNP_FORCE_KERNEL(k_force_jit2, 2)
-extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
-k_symm_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
-           const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
-           const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
-           const unsigned short *__restrict__ mom_cnt, float *__restrict__ G)
+NNP_FORCE_KERNEL(k_force_jit, 1, NNP_MOM_FORCE_WARPS * 32, 5)
+NNP_FORCE_KERNEL(k_force_jit2, 2, NNP_MOM_FORCE_WARPS * 32)
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS, NNP_MOM_LIST_BLOCKS)
+k_force_list(const nnp::MomLists ls, long long lo,
+             const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+             const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+             const unsigned short *__restrict__ mom_cnt, const float *__restrict__ dEdG, double *__restrict__ F,
+             nnp::DevErr *err, const int *__restrict__ atom_struct)
 {
-    nnp::mom_few_symm_body<nnp::JitMoments>(items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, G);
+    nnp::mom_wide_force_body<nnp::JitMoments>((int)blockIdx.x, (int)gridDim.x, NNP_MOM_FEW_THREADS, ls, lo, pot, tab,
+        fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, nullptr);
+    nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x, (int)gridDim.x, NNP_MOM_FEW_THREADS, ls, lo, pot, tab,
+        fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, nullptr);
 }
 )";
     if (E.mom_ok && E.mom_thread())
         os << R"(
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS, NNP_MOM_LIST_BLOCKS)
+k_symm_list(const nnp::MomLists ls, long long lo,
+     const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+     const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+     const unsigned short *__restrict__ mom_cnt, float *__restrict__ G)
+{
+    nnp::mom_list_symm_body<nnp::JitMoments>(ls, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, G);
+}
 extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
 k_symm_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
    const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
    const int *__restrict__ nbr_cnt, int cap, int gstride, float *__restrict__ G, float2 *mom,
-   unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems)
+   unsigned short *__restrict__ mom_cnt, const nnp::MomLists ls)
 {
     extern __shared__ float4 smem4[];
-    nnp::mom_symm_thread_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, items, nitems,
+    nnp::mom_symm_thread_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, ls,
         reinterpret_cast<float *>(smem4));
 }
 )";
@@ -716,40 +730,30 @@ extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
 k_force_jit_t(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
      const float2 *__restrict__ rpar, const int *__restrict__ type, const int *__restrict__ order,
      const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride,
-     const float *__restrict__ dEdG, const float2 *__restrict__ mom, const unsigned short *__restrict__ mom_cnt,
+     const float *__restrict__ dEdG, const float2 *__restrict__ mom, const unsigned long long *__restrict__ mom_mask,
      double *__restrict__ F, nnp::DevErr *err)
 {
     extern __shared__ float4 smem4[];
     nnp::mom_force_thread_body<nnp::JitMoments>((int)blockIdx.x, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr,
-        nbr_cnt, cap, gstride, dEdG, mom, mom_cnt, F, err, reinterpret_cast<float *>(smem4));
+        nbr_cnt, cap, gstride, dEdG, mom, mom_mask, F, err, reinterpret_cast<float *>(smem4));
 }
 extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
 k_tangent_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
      const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
      const int *__restrict__ nbr_cnt, int cap, int gstride, const float4 *__restrict__ V, const float2 *__restrict__ mom,
-     float2 *momd, const unsigned short *__restrict__ mom_cnt, float *__restrict__ Cout)
+     float2 *momd, const unsigned long long *__restrict__ mom_mask, float *__restrict__ Cout)
 {
     extern __shared__ float4 smem4[];
     nnp::mom_tangent_thread_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, V, mom, momd,
-        mom_cnt, Cout, reinterpret_cast<float *>(smem4));
+        mom_mask, Cout, reinterpret_cast<float *>(smem4));
 }
-extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
-k_tangent_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
-              const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
-              const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
-              const unsigned short *__restrict__ mom_cnt, const float4 *__restrict__ V, float *__restrict__ Cout)
+extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS, NNP_MOM_LIST_BLOCKS)
+k_tangent_list(const nnp::MomLists ls, long long lo,
+     const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+     const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+     const unsigned short *__restrict__ mom_cnt, const float4 *__restrict__ V, float *__restrict__ Cout)
 {
-    nnp::mom_few_tangent_body<nnp::JitMoments>(items, nitems, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, V, Cout);
-}
-extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS)
-k_force_few(const int2 *__restrict__ items, const int *__restrict__ nitems, long long lo,
-            const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, const int *__restrict__ type,
-            const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
-            const unsigned short *__restrict__ mom_cnt, const float *__restrict__ dEdG, double *__restrict__ F,
-            nnp::DevErr *err, const int *__restrict__ atom_struct)
-{
-    nnp::mom_few_force_body<nnp::JitMoments>((int)blockIdx.x, (int)gridDim.x, NNP_MOM_FEW_THREADS, items, nitems, lo, pot, tab,
-        fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, nullptr);
+    nnp::mom_list_tangent_body<nnp::JitMoments>(ls, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, V, Cout);
 }
 )";
     if (!E.mom_ok)
@@ -803,9 +807,8 @@ void jit_release(Engine &E)
     if (E.jit_module) cudaLibraryUnload((cudaLibrary_t)E.jit_module);
     E.jit_module = nullptr;
     E.jit_symm = E.jit_force = E.jit_tangent = nullptr;
-    E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = E.jit_force_momt = E.jit_force_few = nullptr;
-    E.jit_tangent_momt = E.jit_tangent_few = nullptr;
-    E.jit_symm_few = nullptr;
+    E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = E.jit_force_momt = nullptr;
+    E.jit_tangent_momt = E.jit_symm_list = E.jit_force_list = E.jit_tangent_list = nullptr;
 }
 
 std::string &jit_last_log()
@@ -938,12 +941,18 @@ std::string jit_build(Engine &E)
     std::vector<std::pair<const char *, void **>> fns = {{"k_tangent_jit", &E.jit_tangent}};
     if (E.mom_ok) {
         fns.push_back({"k_symm_jit", &E.jit_symm_mom});
-        if (E.mom_thread()) fns.push_back({"k_symm_jit_t", &E.jit_symm_momt});
-        if (E.mom_force_thread()) fns.push_back({"k_force_jit_t", &E.jit_force_momt}), fns.push_back({"k_force_few", &E.jit_force_few}),
-            fns.push_back({"k_tangent_jit_t", &E.jit_tangent_momt}), fns.push_back({"k_tangent_few", &E.jit_tangent_few});
+        if (E.mom_thread()) {
+            fns.push_back({"k_symm_jit_t", &E.jit_symm_momt});
+            fns.push_back({"k_symm_list", &E.jit_symm_list});
+        }
+        if (E.mom_force_thread()) {
+            fns.push_back({"k_force_jit_t", &E.jit_force_momt});
+            fns.push_back({"k_tangent_jit_t", &E.jit_tangent_momt});
+            fns.push_back({"k_tangent_list", &E.jit_tangent_list});
+        }
         fns.push_back({"k_force_jit", &E.jit_force_mom1});
         fns.push_back({"k_force_jit2", &E.jit_force_mom2});
-        fns.push_back({"k_symm_few", &E.jit_symm_few});
+        fns.push_back({"k_force_list", &E.jit_force_list});
     } else {
         fns.push_back({"k_symm_jit", &E.jit_symm});
         fns.push_back({"k_force_jit", &E.jit_force});

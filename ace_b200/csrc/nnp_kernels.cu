@@ -1808,6 +1808,7 @@ static std::string mom_reserve(Engine &E)
         e = E.mom.reserve((size_t)rows * vals);
     }
     if (e == cudaSuccess) e = E.mom_cnt.reserve(8 * (size_t)rows);
+    if (e == cudaSuccess) e = E.mom_mask.reserve((size_t)rows);
     if (e == cudaSuccess) e = E.mom_items.reserve((size_t)rows * (E.dpot.ntypes * (E.dpot.ntypes + 1) / 2));
     E.mom_rows = rows;
     return e == cudaSuccess ? "" : std::string("device allocation failed: ") + cudaGetErrorString(e);
@@ -1955,17 +1956,26 @@ static void run_len_order(Engine &E)
 
 static bool mom_by_thread(const Engine &E, int64_t n) { return E.jit_symm_momt && n >= NNP_MOM_THREAD_MIN; }
 
+// the lists of blocks that are summed over pairs, of a part of E.mom_rows rows
+static MomLists mom_lists(Engine &E)
+{
+    const int64_t all = E.mom_rows * (E.dpot.ntypes * (E.dpot.ntypes + 1) / 2);
+    return {E.mom_items.p, E.mom_items.p + all - 1, &E.err.p->few, E.mom_mask.p};
+}
+static_assert(offsetof(DevErr, wide) == offsetof(DevErr, few) + sizeof(int), "MomLists::n");
+
 // Moments of atoms order[lo .. hi) and, unless G is NULL, symmetry functions.
-// first: the list of few-pair blocks is empty (cleared with the error record).
+// first: the lists of blocks are empty (cleared with the error record).
 static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, bool first)
 {
     const int T = E.dpot.ntypes;
     long long l = lo, h = hi;
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
-    int *nitems = &E.err.p->few, *ord = E.visit();
-    if (!first) cudaMemsetAsync(nitems, 0, sizeof(int), E.stream);
+    int *ord = E.visit();
+    MomLists ls = mom_lists(E);
+    if (!first) cudaMemsetAsync(ls.n, 0, 2 * sizeof(int), E.stream);
     void *args[] = {&l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
-                    &cap, &gs, &G, &E.mom.p, &E.mom_cnt.p, &E.mom_items.p, &nitems};
+                    &cap, &gs, &G, &E.mom.p, &E.mom_cnt.p, &ls};
     E.launches += 1;
     if (!mom_by_thread(E, hi - lo)) {
         const size_t sm = (size_t)NNP_MOM_SYMM_WARPS * mom_symm_floats(T, E.mom_ND, E.mom_L, E.mom_NR, E.gstride) * sizeof(float);
@@ -1975,10 +1985,9 @@ static std::string launch_symm_mom(Engine &E, int64_t lo, int64_t hi, float *G, 
     std::string msg = jit_launch(E.jit_symm_momt, grid_for(hi - lo, NNP_MOM_THREADS, 1 << 30), NNP_MOM_THREADS,
                                  mom_thread_floats(T, E.mom_ND, E.mom_L) * sizeof(float), E.stream, args);
     if (!msg.empty() || !G) return msg;
-    void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,
-                   &E.mom_cnt.p, &G};
+    void *list[] = {&ls, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs, &E.mom_cnt.p, &G};
     E.launches += 1;
-    return jit_launch(E.jit_symm_few, num_sms() * 8, NNP_MOM_FEW_THREADS, 0, E.stream, few);
+    return jit_launch(E.jit_symm_list, num_sms() * NNP_MOM_LIST_BLOCKS, NNP_MOM_FEW_THREADS, 0, E.stream, list);
 }
 
 static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *vir)
@@ -1986,28 +1995,33 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
     const int T = E.dpot.ntypes;
     long long l = lo, h = hi;
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
-    const int *nitems = &E.err.p->few, *ord = E.visit();
-    if (E.jit_force_momt && !vir && hi - lo >= NNP_MOM_FORCE_THREAD_MIN) {
-        // the blocks of few pairs in a launch of their own: at the thread
-        // form's 8 warps per SM they took 1.2 ms of 1.09 M atoms' forces
-        void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,
-                       &E.mom_cnt.p, &E.dEdG.p, &E.force.p, &E.err.p, &E.atom_struct.p};
-        const std::string msg = jit_launch(E.jit_force_few, num_sms() * 16, NNP_MOM_FEW_THREADS, 0, E.stream, few);
+    const int *ord = E.visit();
+    MomLists ls = mom_lists(E);
+    const int na = (!vir && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
+    if (na == 2) {
+        // the listed blocks in a launch of their own: at the thread form's 8 warps
+        // per SM they took 1.2 ms of 1.09 M atoms' forces.  A small call, a chain of
+        // launches, takes them in the same one.
+        void *list[] = {&ls, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs, &E.mom_cnt.p, &E.dEdG.p,
+                        &E.force.p, &E.err.p, &E.atom_struct.p};
+        const std::string msg = jit_launch(E.jit_force_list, num_sms() * NNP_MOM_LIST_BLOCKS, NNP_MOM_FEW_THREADS, 0, E.stream, list);
         if (!msg.empty()) return msg;
+        E.launches += 1;
+    }
+    if (na == 2 && E.jit_force_momt && hi - lo >= NNP_MOM_FORCE_THREAD_MIN) {
         int nmain = grid_for(hi - lo, NNP_MOM_THREADS, 1 << 30);
         void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
-                        &cap, &gs, &E.dEdG.p, &E.mom.p, &E.mom_cnt.p, &E.force.p, &E.err.p};
-        E.launches += 2;
+                        &cap, &gs, &E.dEdG.p, &E.mom.p, &ls.mask, &E.force.p, &E.err.p};
+        E.launches += 1;
         return jit_launch(E.jit_force_momt, nmain, NNP_MOM_THREADS,
                           sizeof(float) * mom_force_thread_floats(T, E.mom_L, E.gstride), E.stream, args);
     }
-    const int na = (!vir && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
     int msh = mom_by_thread(E, hi - lo) ? NNP_MOM_SH_T : NNP_MOM_SH_W;   // as launch_symm_mom wrote them
     const size_t sm = (size_t)na * NNP_MOM_FORCE_WARPS * mom_force_floats(T, E.mom_ND, E.mom_L, E.gstride) * sizeof(float);
     int nmain = grid_for(hi - lo, na * NNP_MOM_FORCE_WARPS, num_sms() * 32);
-    const int nfew = grid_for((hi - lo) * T * (T + 1) / 2, NNP_MOM_FORCE_WARPS * 2, num_sms() * 4);
+    const int nfew = na == 2 ? 0 : grid_for((hi - lo) * T * (T + 1) / 2, NNP_MOM_FORCE_WARPS * 2, num_sms() * 4);
     void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
-                    &cap, &gs, &E.dEdG.p, &E.mom.p, &msh, &E.mom_cnt.p, &E.mom_items.p, &nitems, &E.force.p, &E.err.p,
+                    &cap, &gs, &E.dEdG.p, &E.mom.p, &msh, &E.mom_cnt.p, &ls, &E.force.p, &E.err.p,
                     &E.atom_struct.p, &vir};
     E.launches += 1;
     return jit_launch(na == 2 ? E.jit_force_mom2 : E.jit_force_mom1, nmain + nfew, NNP_MOM_FORCE_WARPS * 32, sm, E.stream, args);
@@ -2024,15 +2038,17 @@ bool run_tangent_mom(Engine &E, std::string &msg)
     }
     long long l = 0, h = N;
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
-    const int *nitems = &E.err.p->few, *ord = E.visit();
+    const int *ord = E.visit();
+    MomLists ls = mom_lists(E);
     void *args[] = {&l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p, &cap, &gs, &E.tvec.p,
-                    &E.mom.p, &E.momd.p, &E.mom_cnt.p, &E.tang.p};
-    void *few[] = {&E.mom_items.p, &nitems, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs,
-                   &E.mom_cnt.p, &E.tvec.p, &E.tang.p};
+                    &E.mom.p, &E.momd.p, &ls.mask, &E.tang.p};
+    void *list[] = {&ls, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs, &E.mom_cnt.p, &E.tvec.p,
+                   &E.tang.p};
     E.launches += 2;
     msg = jit_launch(E.jit_tangent_momt, grid_for(N, NNP_MOM_THREADS, 1 << 30), NNP_MOM_THREADS,
                      mom_thread_floats(T, E.mom_ND, E.mom_L) * sizeof(float), E.stream, args);
-    if (msg.empty()) msg = jit_launch(E.jit_tangent_few, num_sms() * 16, NNP_MOM_FEW_THREADS, 0, E.stream, few);
+    if (msg.empty())
+        msg = jit_launch(E.jit_tangent_list, num_sms() * NNP_MOM_LIST_BLOCKS, NNP_MOM_FEW_THREADS, 0, E.stream, list);
     return true;
 }
 

@@ -20,14 +20,20 @@
 // force pass and an atom of the batched workload has 1000 pairs; a neighbour
 // (45 per atom) costs ~500 there and ~400 in the symmetry functions.
 //
-// The moment form's rounding error is ~1e-7 of (sum w)^2, a pair sum's ~1e-7 of
-// the sum itself.  With few pairs the sum can be any fraction of (sum w)^2 (two
-// neighbours on opposite sides of the centre: ((1 + cos)/2)^8 ~ 0); above 15
-// pairs (six neighbours of one element) it is below 1/64 of it for under 10 %
-// of the blocks of the batched workloads and never below 1/1000.  So blocks of
-// at most NNP_MOM_FEW pairs are summed pair by pair (mom_few_symm,
-// mom_few_force_body), 16 lanes each, from a list that the symmetry functions
-// append to.
+// The moment form's rounding error is ~1e-7 of sum_l |c_l S_l| + f(1) sum w^2, a
+// pair sum's ~1e-7 of the sum itself.  The two differ where neighbours lie to one
+// side of the centre (an adatom, a tip) or are few: ((1 - cos)/2)^8 of neighbours
+// in a cone, ((1 + cos)/2)^8 of two on opposite sides are 1e-4 to 1e-8 of it.  So a
+// block is summed pair by pair when one of its functions comes out below
+// NNP_MOM_CANCEL of that sum, at any number of pairs.  The symmetry functions
+// decide, from the sums that they form anyway, and leave a bit per block in
+// mom_mask, which the forces and tangents follow; lists of the (row, block)
+// entries are worked off by groups of lanes (mom_few_*: at most NNP_MOM_FEW pairs,
+// mom_wide_*: more).  In random cells of 0.05 atoms per cubic A of three elements
+// 9 % of the blocks are listed as few and 3.5 % as wide, in crystals none.
+// With 1/16 the errors of G and of the forces are those of pair sums, function by
+// function (rms), over adatoms, tips, surfaces and random cells; with 1/32 functions
+// of zeta = 8 at a free surface had 4.5 times the pair sum's.
 //
 // Y_lm(u) = Q_lm(z) Re/Im (x + i y)^m with Q_lm the monic polynomial
 // proportional to d^m P_l / dz^m: Q_{l+1,m} = z Q_lm - beta_lm Q_{l-1,m},
@@ -59,8 +65,10 @@
 #define NNP_MOM_THREADS 128   // threads per block, symmetry functions with a thread per atom
 #define NNP_MOM_THREAD_T 4    // most elements of that form (its sums of pairs of elements are unrolled)
 #define NNP_MOM_FORCE_WARPS 4 // warps per block, forces
-#define NNP_MOM_FEW 15        // blocks of at most this many pairs are summed pair by pair
+#define NNP_MOM_CANCEL 0.0625f // blocks with a function below this part of its terms' absolute sum are summed pair by pair
+#define NNP_MOM_FEW 15        // 16 lanes take such a block if it has at most this many pairs
 #define NNP_MOM_FEW_THREADS 128
+#define NNP_MOM_LIST_BLOCKS 8 // blocks per SM of the list kernels (64 registers), all resident
 
 namespace nnp {
 
@@ -81,12 +89,22 @@ NNP_HD constexpr int mom_comps(int L) { return mom_base(L, L) + 2; }
 // touched 8 lines, and the tag lookups bounded both kernels: symmetry functions
 // of 1.09 M atoms 2.27 -> 2.13 ms, forces 3.51 -> 3.19 ms); written with a warp
 // per row sh = NNP_MOM_SH_W: it writes one row's components next to its
-// neighbours'.  mom_cnt holds 8 neighbour counts (by element) per row,
-// mom_items the (row, block) entries of few pairs (their number: DevErr::few).
+// neighbours'.  mom_cnt holds 8 neighbour counts (by element) per row, mom_mask
+// the row's blocks that are summed over pairs.
 #define NNP_MOM_SH_T 5
 #define NNP_MOM_SH_W 2
 NNP_HD constexpr int mom_vals(int T, int ND, int L) { return T * ((ND + 1) / 2) * mom_comps(L); }
 NNP_HD inline i64 mom_at(i64 r, int k, int vals, int sh) { return (((r >> sh) * vals + k) << sh) + (r & ((1 << sh) - 1)); }
+
+// Blocks that are summed over pairs (or have none): a bit per block of each row, and
+// the (row, block) entries, those of few pairs from the start of one array, the
+// others from its end backwards (an entry is in one of the two, so rows x blocks
+// hold both).
+struct MomLists {
+    int2 *few, *wide;             // the first entry of either
+    int *n;                       // their numbers (DevErr::few, DevErr::wide)
+    unsigned long long *mask;
+};
 
 // pairs of block (J, K) of an atom
 NNP_HD inline int mom_pairs(const unsigned short *cnt, int J, int K)
@@ -372,18 +390,39 @@ struct MomFew {
     int J, K, so, no, sp, np, nn, pairs, a, b;
 };
 
-__device__ __forceinline__ MomFew mom_few(const unsigned short *cnt, int T, int tt, int p)
+// Elements of block tt, the first slots and numbers of their neighbours (cnt: an
+// atom's eight counts, 16-byte aligned).
+template <int T>
+__device__ __forceinline__ void mom_block(const unsigned short *cnt, int tt, int &J, int &K, int &sJ, int &nJ, int &sK, int &nK)
+{
+    const uint4 v = *reinterpret_cast<const uint4 *>(cnt);
+    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+    K = 0;
+#pragma unroll
+    for (int k = 1; k < T; ++k) K += tt >= k * (k + 1) / 2;
+    J = tt - K * (K + 1) / 2;
+    sJ = nJ = sK = nK = 0;
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        const int c = (int)((w[k / 2] >> (k & 1 ? 16 : 0)) & 0xffffu);
+        sJ += k < J ? c : 0;
+        nJ = k == J ? c : nJ;
+        sK += k < K ? c : 0;
+        nK = k == K ? c : nK;
+    }
+}
+
+template <int T>
+__device__ __forceinline__ MomFew mom_few(const unsigned short *cnt, int tt, int p)
 {
     MomFew f;
-    f.K = 0;
-    for (int k = 1; k < T; ++k) f.K += tt >= k * (k + 1) / 2;
-    f.J = tt - f.K * (f.K + 1) / 2;
-    const int big = cnt[f.J] >= cnt[f.K] ? f.J : f.K, other = f.J + f.K - big;
-    f.so = f.sp = 0;
-    for (int k = 0; k < big; ++k) f.so += cnt[k];
-    for (int k = 0; k < other; ++k) f.sp += cnt[k];
-    f.no = cnt[big];
-    f.np = cnt[other];
+    int sJ, nJ, sK, nK;
+    mom_block<T>(cnt, tt, f.J, f.K, sJ, nJ, sK, nK);
+    const bool j = nJ >= nK;
+    f.so = j ? sJ : sK;
+    f.sp = j ? sK : sJ;
+    f.no = j ? nJ : nK;
+    f.np = j ? nK : nJ;
     if (f.J == f.K) {                                            // at most 6 neighbours: a < b, p = b (b - 1) / 2 + a
         f.nn = f.no;
         f.pairs = f.no * (f.no - 1) / 2;
@@ -412,7 +451,7 @@ __device__ __forceinline__ void mom_few_symm(unsigned mask, int h, const float4 
                                              const unsigned short *cnt, const DevType &Ty, int II, int tt,
                                              const float *a_lo, float *Gb)
 {
-    const MomFew b = mom_few(cnt, M::T, tt, h);
+    const MomFew b = mom_few<M::T>(cnt, tt, h);
     MomNbr<M, false> v;
     v.set(src[mom_few_slot(b, h)], Ty, a_lo);
     float cs = 0.f, w[M::ND], acc[M::NA];
@@ -434,19 +473,196 @@ __device__ __forceinline__ void mom_few_symm(unsigned mask, int h, const float4 
     }
 }
 
-// Symmetry functions of the listed blocks (thread-per-atom form), 16 lanes each.
+// ---------------------------------------------------------------- blocks of many pairs
+//
+// A warp per block.  The block's neighbours (of J, then of K; J == K: of the
+// element) are loaded a lane each, 32 at a time (such blocks have mostly 7 to 16).
+// For sums over pairs a lane then takes a pair, with the values of both ends by
+// shuffles (mom_wide_pairs); for the forces it takes a neighbour a (as many lanes each
+// as fit, a's partners divided among them) and walks the partners, so that it gets
+// the gradient at a without a second exchange, at two evaluations a pair
+// (mom_wide_walk).
+// Bound: latency of the chain from the list entry to the neighbours (entry and atom
+// are fetched one turn ahead), then issue.
+
+struct MomWide {
+    int sJ, nJ, sK, nn;           // first slots, neighbours of J and of the block
+    bool one;                     // J == K
+    __device__ __forceinline__ int slot(int k) const { return k < nJ ? sJ + k : sK + k - nJ; }
+};
+
+template <int T>
+__device__ __forceinline__ MomWide mom_wide(const unsigned short *cnt, int tt)
+{
+    MomWide w;
+    int J, K, nK;
+    mom_block<T>(cnt, tt, J, K, w.sJ, w.nJ, w.sK, nK);
+    w.one = J == K;
+    w.nn = w.nJ + (w.one ? 0 : nK);
+    return w;
+}
+
+// Entries q, q + step, .. of the list, the next entry and its atom on the way.
+struct MomQueue {
+    const int2 *p;
+    const int *order;
+    int q, n, step, i, ni;
+    int2 it, nx;
+    __device__ __forceinline__ MomQueue(const int2 *list, int count, const int *ord, int first, int stride)
+        : p(list), order(ord), q(first), n(count), step(stride), i(0), ni(0)
+    {
+        if (q < n) {
+            it = at(q);
+            nx = at(q + step);
+            i = order[it.x];
+        }
+    }
+    __device__ __forceinline__ int2 at(int k) const { return p[-(i64)min(k, n - 1)]; }
+    __device__ __forceinline__ void ahead() { ni = order[nx.x]; }
+    __device__ __forceinline__ void next()
+    {
+        q += step;
+        it = nx;
+        i = ni;
+        nx = at(q + step);
+    }
+};
+
+// First entry of the few-pair list for a group of 16 lanes, of `all` groups: the
+// round goes on where that of the other list, a warp each, ended.
+__device__ __forceinline__ int mom_few_first(const MomLists &ls, int group, int all)
+{
+    const int f = group - 2 * (ls.n[1] % (all / 2));
+    return f < 0 ? f + all : f;
+}
+
+// load(slot) -> a neighbour's values; pair(A, la, B, lb, ok) for every pair of the
+// block: its ends are the values of lanes la in A and lb in B (ok: the lane has one)
+template <class Load, class Pair>
+__device__ __forceinline__ void mom_wide_pairs(const MomWide &w, Load load, Pair pair)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int a0 = 0; a0 < (w.one ? w.nn : w.nJ); a0 += 32) {
+        const int ca = min(32, w.nn - a0);
+        const auto A = load(w.slot(a0 + min(lane, ca - 1)));
+#pragma unroll 1
+        for (int b0 = a0; b0 < w.nn; b0 += 32) {
+            const int cb = min(32, w.nn - b0);
+            auto B = A;
+            if (b0 != a0) B = load(w.slot(b0 + min(lane, cb - 1)));
+            // a's are lanes [0, na) of A, b's lanes [fb, cb) of B
+            const int na = w.one ? ca : min(ca, w.nJ - a0), fb = w.one ? 0 : max(w.nJ - b0, 0);
+            const bool tri = w.one && a0 == b0;
+            const int np = tri ? na * (na - 1) / 2 : na * max(cb - fb, 0);
+#pragma unroll 1
+            for (int p0 = 0; p0 < np; p0 += 32) {
+                const int p = min(p0 + lane, np - 1);
+                // p = b (b - 1) / 2 + a, a < b, or (b - fb) na + a (exact in FP32: p < 1024)
+                const int b = tri ? (int)(0.5f + sqrtf(0.25f + 2.f * (float)p)) : fb + (int)__fdividef((float)p + 0.5f, (float)na);
+                const int a = tri ? p - b * (b - 1) / 2 : p - (b - fb) * na;
+                pair(A, a, B, b, p0 + lane < np);
+            }
+        }
+    }
+}
+
+// take(v, lane) -> the values that a lane holds; pair(a, B, q, ok) for each step: b is
+// the value of lane q in B (ok: the lane has a pair); end(A, a, lane that loaded a,
+// first lane of a, lanes per a)
+template <class Load, class Take, class Pair, class End>
+__device__ __forceinline__ void mom_wide_walk(const MomWide &w, Load load, Take take, Pair pair, End end)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int a0 = 0; a0 < w.nn; a0 += 32) {
+        const int ca = min(32, w.nn - a0);
+        const int sh = 31 - __clz(32 / ca);                      // 1 << sh lanes per a
+        const int la = min(lane >> sh, ca - 1), ia = a0 + la, part = lane & ((1 << sh) - 1);
+        const bool act = (lane >> sh) < ca;
+        const auto A = load(w.slot(a0 + min(lane, ca - 1)));
+        const auto a = take(A, la);
+#pragma unroll 1
+        for (int b0 = 0; b0 < w.nn; b0 += 32) {
+            const int cb = min(32, w.nn - b0);
+            auto B = A;
+            if (b0 != a0) B = load(w.slot(b0 + min(lane, cb - 1)));
+            // partners of a, and the most that any a has
+            const int lo = w.one || ia >= w.nJ ? b0 : max(b0, w.nJ), hi = w.one || ia < w.nJ ? b0 + cb : min(b0 + cb, w.nJ);
+            const int most = w.one ? cb : max(b0 + cb - max(b0, w.nJ), min(b0 + cb, w.nJ) - b0);
+#pragma unroll 1
+            for (int t = 0; t < most; t += 1 << sh) {
+                const int q = lo + part + t;
+                pair(a, B, min(q - b0, cb - 1), act && q < hi && !(w.one && q == ia));
+            }
+        }
+        end(A, a, la, act && part == 0, 1 << sh);
+    }
+}
+
+// Symmetry functions of block tt by a warp, to Gb.
 template <class M>
-__device__ void mom_few_symm_body(const int2 *__restrict__ items, const int *__restrict__ nitems, i64 lo,
-                                  const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
-                                  const int *__restrict__ type, const int *__restrict__ order,
-                                  const float4 *__restrict__ nbr, int cap, int gstride,
-                                  const unsigned short *__restrict__ mom_cnt, float *__restrict__ G)
+__device__ __noinline__ void mom_wide_symm(const float4 *__restrict__ src, const unsigned short *cnt, const DevType &Ty,
+                                           int II, int tt, const float *a_lo, float *Gb)
+{
+    struct Nbr {
+        float u[3], w[M::ND];
+    };
+    float acc[M::NA];
+#pragma unroll
+    for (int f = 0; f < M::NA; ++f) acc[f] = 0.f;
+    mom_wide_pairs(
+        mom_wide<M::T>(cnt, tt),
+        [&](int k) {
+            MomNbr<M, false> v;
+            v.set(src[k], Ty, a_lo);
+            Nbr o;
+            o.u[0] = v.ux;
+            o.u[1] = v.uy;
+            o.u[2] = v.uz;
+#pragma unroll
+            for (int d = 0; d < M::ND; ++d) o.w[d] = v.w[d];
+            return o;
+        },
+        [&](const Nbr &A, int a, const Nbr &B, int b, bool ok) {
+            float cs = 0.f, w[M::ND];
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+                cs = fmaf(__shfl_sync(NNP_FULL, A.u[x], a), __shfl_sync(NNP_FULL, B.u[x], b), cs);
+#pragma unroll
+            for (int d = 0; d < M::ND; ++d) w[d] = __shfl_sync(NNP_FULL, A.w[d], a) * __shfl_sync(NNP_FULL, B.w[d], b);
+            if (ok) M::few_symm(II, tt, cs, w, acc);
+        });
+    const int n = Ty.ba[tt].n;
+#pragma unroll
+    for (int f = 0; f < M::NA; ++f) {
+        const float s = warp_sum(acc[f]);
+        if ((threadIdx.x & 31) == 0 && f < n) Gb[f] = s;
+    }
+}
+
+// Symmetry functions of the listed blocks (thread-per-atom form).
+template <class M>
+__device__ void mom_list_symm_body(const MomLists ls, i64 lo, const DevPot *__restrict__ pot,
+                                   const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+                                   const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+                                   const unsigned short *__restrict__ mom_cnt, float *__restrict__ G)
 {
     const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
-    const int n = *nitems, h = threadIdx.x & 15;
+    const int id = blockIdx.x * NNP_MOM_FEW_THREADS + threadIdx.x, all = gridDim.x * (NNP_MOM_FEW_THREADS / 16);
+    for (MomQueue u(ls.wide, ls.n[1], order + lo, id >> 5, all / 2); u.q < u.n; u.next()) {
+        const i64 i = u.i;
+        const int II = type[i], tt = u.it.y;
+        const DevType &Ty = pot->t[II];
+        u.ahead();
+        mom_wide_symm<M>(nbr + i * cap, mom_cnt + 8 * (i64)u.it.x, Ty, II, tt, tb.a_lo + II * NNP_MOM_MAXD,
+                         G + i * gstride + Ty.ba[tt].off_g);
+    }
+    __syncwarp();
+    const int n = ls.n[0], h = threadIdx.x & 15;
     const unsigned mask = 0xffffu << (threadIdx.x & 16);
-    for (int q = (blockIdx.x * NNP_MOM_FEW_THREADS + threadIdx.x) >> 4; q < n; q += gridDim.x * (NNP_MOM_FEW_THREADS / 16)) {
-        const int2 it = items[q];
+    for (int q = mom_few_first(ls, id >> 4, all); q < n; q += all) {
+        const int2 it = ls.few[q];
         const i64 i = order[lo + it.x];
         const int II = type[i];
         const DevType &Ty = pot->t[II];
@@ -455,11 +671,124 @@ __device__ void mom_few_symm_body(const int2 *__restrict__ items, const int *__r
     }
 }
 
-// Forces of the listed blocks, 16 lanes each: lane p evaluates pair p, then lane
-// h gathers the gradient at neighbour h from the pairs that it is in.
+// Forces of the listed blocks of many pairs: per pair the gradient at a.
 template <class M>
-__device__ void mom_few_force_body(int block, int nblock, int threads, const int2 *__restrict__ items,
-                                   const int *__restrict__ nitems, i64 lo, const DevPot *__restrict__ pot,
+__device__ __noinline__ void mom_wide_force_body(int block, int nblock, int threads, const MomLists ls, i64 lo,
+                                                 const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
+                                                 const int *__restrict__ type, const int *__restrict__ order,
+                                                 const float4 *__restrict__ nbr, int cap, int gstride,
+                                                 const unsigned short *__restrict__ mom_cnt,
+                                                 const float *__restrict__ dEdG, double *__restrict__ F, DevErr *err,
+                                                 const int *__restrict__ atom_struct, double *__restrict__ vir)
+{
+    struct Nbr {
+        float u[3], ir, w[M::ND], wd[M::ND];
+        float4 rec;
+    };
+    const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (MomQueue u(ls.wide, ls.n[1], order + lo, (block * threads + (int)threadIdx.x) >> 5, nblock * (threads / 32)); u.q < u.n;
+         u.next()) {
+        const i64 i = u.i;
+        const int II = type[i], tt = u.it.y;
+        const DevType &Ty = pot->t[II];
+        u.ahead();
+        const float *a_lo = tb.a_lo + II * NNP_MOM_MAXD, *e = dEdG + i * gstride + Ty.ba[tt].off_g;
+        const float4 *src = nbr + i * cap;
+        double f[3] = {0, 0, 0}, wv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        float g[3] = {0.f, 0.f, 0.f};
+        bool bad = false;
+        mom_wide_walk(
+            mom_wide<M::T>(mom_cnt + 8 * (i64)u.it.x, tt),
+            [&](int k) {
+                Nbr o;
+                o.rec = src[k];
+                MomNbr<M, true> v;
+                v.set(o.rec, Ty, a_lo);
+                o.u[0] = v.ux;
+                o.u[1] = v.uy;
+                o.u[2] = v.uz;
+                o.ir = v.ir;
+#pragma unroll
+                for (int d = 0; d < M::ND; ++d) {
+                    o.w[d] = v.w[d];
+                    o.wd[d] = v.wd[d];
+                }
+                return o;
+            },
+            [](const Nbr &v, int q) {
+                Nbr o;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) o.u[x] = __shfl_sync(NNP_FULL, v.u[x], q);
+                o.ir = __shfl_sync(NNP_FULL, v.ir, q);
+#pragma unroll
+                for (int d = 0; d < M::ND; ++d) {
+                    o.w[d] = __shfl_sync(NNP_FULL, v.w[d], q);
+                    o.wd[d] = __shfl_sync(NNP_FULL, v.wd[d], q);
+                }
+                o.rec = make_float4(0.f, 0.f, 0.f, __shfl_sync(NNP_FULL, v.rec.w, q));
+                return o;
+            },
+            [&](const Nbr &a, const Nbr &B, int q, bool ok) {
+                float b[3], wb[M::ND], none[M::ND];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) b[x] = __shfl_sync(NNP_FULL, B.u[x], q);
+#pragma unroll
+                for (int d = 0; d < M::ND; ++d) {
+                    wb[d] = __shfl_sync(NNP_FULL, B.w[d], q);
+                    none[d] = 0.f;
+                }
+                const float cs = fmaf(a.u[2], b[2], fmaf(a.u[1], b[1], a.u[0] * b[0]));
+                float hc = 0.f, ha = 0.f, hb = 0.f;              // dE/dcos, dE/dr_a
+                if (ok) M::few_force(II, tt, cs, e, a.w, a.wd, wb, none, hc, ha, hb);
+                const float ta = hc * a.ir, sa = ha - ta * cs;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) g[x] += fmaf(sa, a.u[x], ta * b[x]);
+            },
+            [&](const Nbr &A, const Nbr &a, int la, bool first, int lanes) {
+                const i64 j = __float_as_int(a.rec.w) & 0x0fffffff;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    for (int o = lanes >> 1; o; o >>= 1) g[x] += __shfl_xor_sync(NNP_FULL, g[x], o);
+                    if (first) {
+                        bad |= !(fabsf(g[x]) <= 3.402823466e38f);
+                        atomicAdd(&F[3 * j + x], (double)g[x]);
+                        f[x] += (double)g[x];
+                    }
+                }
+                if (vir) {
+                    const double d3[3] = {__shfl_sync(NNP_FULL, A.rec.x, la), __shfl_sync(NNP_FULL, A.rec.y, la),
+                                          __shfl_sync(NNP_FULL, A.rec.z, la)};
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+#pragma unroll
+                        for (int y = 0; y < 3; ++y) wv[3 * x + y] -= first ? (double)g[x] * d3[y] : 0.0;
+                }
+#pragma unroll
+                for (int x = 0; x < 3; ++x) g[x] = 0.f;
+            });
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            const double s = warp_sum(f[x]);
+            if (lane == x) atomicAdd(&F[3 * i + x], -s);
+        }
+        if (vir) {
+            double *ws = vir + 9 * (i64)atom_struct[i];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                const double s = warp_sum(wv[q]);
+                if (lane == 0) atomicAdd(ws + q, s);
+            }
+        }
+        if (bad) atomicMax(&err->nonfinite, 1);
+    }
+}
+
+// Forces of the listed blocks of few pairs, 16 lanes each: lane p evaluates pair p,
+// then lane h gathers the gradient at neighbour h from the pairs that it is in.
+template <class M>
+__device__ void mom_few_force_body(int block, int nblock, int threads, const MomLists ls, i64 lo, const DevPot *__restrict__ pot,
                                    const float *__restrict__ tab, int fmax, const int *__restrict__ type,
                                    const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
                                    const unsigned short *__restrict__ mom_cnt, const float *__restrict__ dEdG,
@@ -467,14 +796,14 @@ __device__ void mom_few_force_body(int block, int nblock, int threads, const int
                                    double *__restrict__ vir)
 {
     const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
-    const int n = *nitems, h = threadIdx.x & 15;
+    const int n = ls.n[0], h = threadIdx.x & 15, all = nblock * (threads / 16);
     const unsigned mask = 0xffffu << (threadIdx.x & 16);
-    for (int q = (block * threads + (int)threadIdx.x) >> 4; q < n; q += nblock * (threads / 16)) {
-        const int2 it = items[q];
+    for (int q = mom_few_first(ls, (block * threads + (int)threadIdx.x) >> 4, all); q < n; q += all) {
+        const int2 it = ls.few[q];
         const i64 i = order[lo + it.x];
         const int II = type[i], tt = it.y;
         const DevType &Ty = pot->t[II];
-        const MomFew b = mom_few(mom_cnt + 8 * (i64)it.x, M::T, tt, h);
+        const MomFew b = mom_few<M::T>(mom_cnt + 8 * (i64)it.x, tt, h);
         const float *a_lo = tb.a_lo + II * NNP_MOM_MAXD, *e = dEdG + i * gstride + Ty.ba[tt].off_g;
         MomNbr<M, true> v;
         const float4 rv = nbr[i * cap + mom_few_slot(b, h)];
@@ -561,30 +890,40 @@ __device__ void mom_few_force_body(int block, int nblock, int threads, const int
 
 // ---------------------------------------------------------------- symmetry functions
 
-// G_f of one angular function from S (float2 [tt][pair][l], stride ss between
-// entries) and the sum of w_d^2; a block of few pairs is 0 here.
+// G_f of one angular function from S (float2 [tt][pair][l]) and the sum of
+// w_d^2, and whether its terms cancel.
 template <int L, int NDP>
-__device__ __forceinline__ float mom_function(const MomTab &tb, int fu, const float *cf, const float2 *S, int ss,
-                                             const float *w2, const unsigned short *cnt)
+__device__ __forceinline__ float mom_function(const MomTab &tb, int fu, const float *cf, const float2 *S, const float *w2,
+                                             bool &cancels)
 {
     const int tt = fu & 0xff, d = (fu >> 8) & 0xff;
-    if (mom_pairs(cnt, (fu >> 16) & 0xff, (fu >> 24) & 0xff) <= NNP_MOM_FEW) return 0.f;
-    const float2 *s = S + (i64)((tt * NDP + (d >> 1)) * (L + 1)) * ss;
-    float g = 0.f;
+    const float2 *s = S + (tt * NDP + (d >> 1)) * (L + 1);
+    float g = 0.f, most = 0.f;
 #pragma unroll
-    for (int l = L; l >= 0; --l) g = fmaf(cf[l * tb.fmax], (d & 1) ? s[l * ss].y : s[l * ss].x, g);
-    return fmaf(-cf[(L + 1) * tb.fmax], *w2, g);
+    for (int l = L; l >= 0; --l) {
+        const float c = cf[l * tb.fmax], v = (d & 1) ? s[l].y : s[l].x;
+        g = fmaf(c, v, g);
+        most = fmaf(fabsf(c), fabsf(v), most);
+    }
+    const float self = cf[(L + 1) * tb.fmax];
+    g = fmaf(-self, *w2, g);
+    cancels = g < NNP_MOM_CANCEL * fmaf(self, *w2, most);
+    return g;
 }
 
-// appends block tt of row r to the list when it has few pairs
+// block tt of row r goes to one of the lists
 template <int T>
-__device__ __forceinline__ void mom_push(int2 *items, int *nitems, i64 r, int tt, const unsigned short *cnt)
+__device__ __forceinline__ void mom_push(const MomLists &ls, i64 r, int tt, const unsigned short *cnt)
 {
     int K = 0;
 #pragma unroll
     for (int k = 1; k < T; ++k) K += tt >= k * (k + 1) / 2;
     const int np = mom_pairs(cnt, tt - K * (K + 1) / 2, K);
-    if (np > 0 && np <= NNP_MOM_FEW) items[atomicAdd(nitems, 1)] = make_int2((int)r, tt);
+    if (np <= NNP_MOM_FEW) {
+        if (np > 0) ls.few[atomicAdd(ls.n, 1)] = make_int2((int)r, tt);
+    } else {
+        ls.wide[-(i64)atomicAdd(ls.n + 1, 1)] = make_int2((int)r, tt);
+    }
 }
 
 // Symmetry functions of atoms order[lo .. hi) and their moments (row idx - lo),
@@ -603,7 +942,7 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
                               const int *__restrict__ type, const int *__restrict__ order,
                               const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride,
                               float *__restrict__ G, float2 *__restrict__ mom, unsigned short *__restrict__ mom_cnt,
-                              int2 *__restrict__ items, int *__restrict__ nitems, float *smem)
+                              const MomLists ls, float *smem)
 {
     constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
                   NR = M::NR, ROW = mom_stage(L, NR, ND), NQ = (NC + NR + ND + 31) / 32,
@@ -725,7 +1064,8 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
             __syncwarp();
         }
         __syncwarp();
-        if (G) {
+        unsigned long long mask;                                 // blocks that are summed over pairs
+        {
             // S^{JK}_{l,d}: lane = (l, pair of damping factors, element pair), largest l first
             for (int s = lane; s < NS; s += 32) {
                 const int l = L - s / (TT * NDP), rem = s % (TT * NDP), p = rem / TT, tt = rem % TT;
@@ -751,20 +1091,35 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
             __syncwarp();
             // G: lane = angular function
             const int na = Ty.n_input - Ty.n_input_r;
+            unsigned long long list = 0, few = 0, none = 0;
             for (int f = lane; f < na; f += 32) {
                 const int fu = tb.fun[II * fmax + f];
+                bool cancels;
                 Gs[Ty.n_input_r + f] = mom_function<L, NDP>(tb, fu, tb.coef + (i64)II * (L + 2) * fmax + f,
-                                                             reinterpret_cast<const float2 *>(S), 1,
-                                                             W2 + ((fu >> 16) & 0xff) * NNP_MOM_MAXD + ((fu >> 8) & 0xff), cnt);
+                                                             reinterpret_cast<const float2 *>(S),
+                                                             W2 + ((fu >> 16) & 0xff) * NNP_MOM_MAXD + ((fu >> 8) & 0xff),
+                                                             cancels);
+                if (cancels) list |= 1ull << (fu & 0xff);
             }
+            list = (unsigned long long)__reduce_or_sync(NNP_FULL, (unsigned)(list >> 32)) << 32 |
+                   __reduce_or_sync(NNP_FULL, (unsigned)list);
             __syncwarp();
-            // blocks of few pairs, one per half warp
-            unsigned long long few = 0;
             for (int K = 0, tt = 0; K < T; ++K)
                 for (int J = 0; J <= K; ++J, ++tt) {
                     const int np = mom_pairs(cnt, J, K);
-                    if (np > 0 && np <= NNP_MOM_FEW && Ty.ba[tt].n > 0) few |= 1ull << tt;
+                    if (np == 0) none |= 1ull << tt;
+                    else if (np <= NNP_MOM_FEW) few |= 1ull << tt;
                 }
+            mask = none | list;
+            for (unsigned long long m = G ? list & ~none & ~few : 0; m; m &= m - 1) {
+                const int tt = __ffsll(m) - 1;
+                mom_wide_symm<M>(src, cnt, Ty, II, tt, tb.a_lo + II * NNP_MOM_MAXD, Gs + Ty.ba[tt].off_g);
+            }
+            if (none)
+                for (int f = lane; f < na; f += 32)
+                    if (none >> (tb.fun[II * fmax + f] & 0xff) & 1) Gs[Ty.n_input_r + f] = 0.f;
+            // blocks of few pairs, one per half warp
+            few = G ? few & list : 0;
             while (few) {
                 const int t0 = __ffsll(few) - 1;
                 few &= few - 1;
@@ -775,14 +1130,15 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
                                     Gs + Ty.ba[tt].off_g);
             }
             __syncwarp();
-            for (int k = lane; 4 * k < gstride; k += 32)
+            for (int k = lane; G && 4 * k < gstride; k += 32)
                 reinterpret_cast<float4 *>(G + i * gstride)[k] = reinterpret_cast<const float4 *>(Gs)[k];
         }
         {
             const i64 r = idx - lo;
             for (int k = lane; k < NV; k += 32) mom[mom_at(r, k, NV, NNP_MOM_SH_W)] = reinterpret_cast<const float2 *>(A)[k];
             if (lane < 8) mom_cnt[8 * r + lane] = cnt[lane];
-            for (int tt = lane; tt < TT; tt += 32) mom_push<T>(items, nitems, r, tt, cnt);
+            if (lane == 0) ls.mask[r] = mask;
+            for (int tt = lane; tt < TT; tt += 32) if (mask >> tt & 1) mom_push<T>(ls, r, tt, cnt);
         }
         __syncwarp();
     }
@@ -790,21 +1146,26 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
 
 // Angular functions of a thread's atom from S and the sums of w_d^2 (entries
 // BT apart): G_f = sum_l c_l S_l - self (c and self as in dE/dA: half of them
-// for J == K), self = -wscale sum w_d^2.  Blocks of few pairs are 0 here.
-template <class M>
-__device__ __forceinline__ void mom_functions_thread(const MomTab &tb, int fmax, int II, const DevType &Ty,
-                                                     const unsigned short *cnt, const f32x2 *S, const f32x2 *W2,
-                                                     float wscale, float *Gi)
+// for J == K), self = -wscale sum w_d^2.  Blocks that are summed over pairs are
+// written too and replaced.  `mask` has those without pairs (0 here); with MARK it
+// gets those whose terms cancel.  The coefficients' signs are those of lambda^l, so the
+// absolute sum needs only the sums over even and odd l of c_l |S_l|: one more
+// multiply-add per term, 1 % of the symmetry functions.
+template <class M, bool MARK>
+__device__ __forceinline__ unsigned long long mom_functions_thread(const MomTab &tb, int fmax, int II, const DevType &Ty,
+                                                                   unsigned long long mask, const f32x2 *S, const f32x2 *W2,
+                                                                   float wscale, float *Gi)
 {
     constexpr int T = M::T, L = M::L, NDP = (M::ND + 1) / 2, DL = mom_dl(L), BT = NNP_MOM_THREADS;
 #pragma unroll 1
     for (int K = 0, tt = 0; K < T; ++K)
 #pragma unroll 1
         for (int J = 0; J <= K; ++J, ++tt) {
-            const bool few = mom_pairs(cnt, J, K) <= NNP_MOM_FEW;    // added by the blocks of few pairs
+            const bool none = mask >> tt & 1;
             const int off = Ty.ba[tt].off_g, bn = Ty.ba[tt].n, f0 = II * fmax + off - Ty.n_input_r;
             const ulonglong2 *cf = reinterpret_cast<const ulonglong2 *>(tb.dcoef + (i64)f0 * DL);
             const float h = J == K ? 0.5f : 1.f;
+            bool cancels = false;
             f32x2 st[DL];                                    // S, -sum of w_d^2
 #pragma unroll
             for (int l = 0; l < DL; ++l) st[l] = 0ull;
@@ -816,7 +1177,7 @@ __device__ __forceinline__ void mom_functions_thread(const MomTab &tb, int fmax,
                     for (int l = 0; l <= L; ++l) st[l] = S[((tt * NDP + p) * (L + 1) + l) * BT];
                     st[L + 1] = mul2(W2[(J * NDP + p) * BT], dup2(wscale));
                 }
-                f32x2 c[DL], g = 0ull;
+                f32x2 c[DL], g = 0ull, a[2] = {0ull, 0ull};
 #pragma unroll
                 for (int l = 0; l < DL; l += 2) {
                     const ulonglong2 v = __ldg(cf + f * (DL / 2) + l / 2);
@@ -824,13 +1185,25 @@ __device__ __forceinline__ void mom_functions_thread(const MomTab &tb, int fmax,
                     c[l + 1] = v.y;
                 }
 #pragma unroll
-                for (int l = L; l >= 0; --l) g = fma2(c[l], st[l], g);
+                for (int l = L; l >= 0; --l) {
+                    g = fma2(c[l], st[l], g);
+                    if (MARK) a[l & 1] = fma2(c[l], st[l] & 0x7fffffff7fffffffull, a[l & 1]);
+                }
                 g = fma2(c[L + 1], st[L + 1], g);
                 float g0, g1;
                 up2(g, g0, g1);
-                Gi[off + f] = few ? 0.f : h * (g0 + g1);
+                if (MARK) {
+                    float e0, e1, o0, o1, s0, s1;
+                    up2(a[0], e0, e1);
+                    up2(a[1], o0, o1);
+                    up2(mul2(c[L + 1], st[L + 1]), s0, s1);      // at most 0
+                    cancels |= g0 + g1 < NNP_MOM_CANCEL * (e0 + e1 + fabsf(o0 + o1) - (s0 + s1));
+                }
+                if (Gi) Gi[off + f] = none ? 0.f : h * (g0 + g1);
             }
+            if (MARK && cancels) mask |= 1ull << tt;
         }
+    return mask;
 }
 
 // The same with one thread per atom: the moments of one neighbour element and
@@ -851,7 +1224,7 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                                      int fmax, const int *__restrict__ type, const int *__restrict__ order,
                                      const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap,
                                      int gstride, float *__restrict__ G, float2 *mom,
-                                     unsigned short *__restrict__ mom_cnt, int2 *__restrict__ items, int *__restrict__ nitems, float *smem)
+                                     unsigned short *__restrict__ mom_cnt, const MomLists ls, float *smem)
 {
     constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NDP = (ND + 1) / 2, NC = mom_comps(L),
                   NR = M::NR, NV = mom_vals(T, ND, L), NS = mom_s_vals(T, ND, L), BT = NNP_MOM_THREADS;
@@ -943,9 +1316,6 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
                 }
             }
         }
-#pragma unroll
-        for (int tt = 0; tt < TT; ++tt) mom_push<T>(items, nitems, r, tt, cnt);
-        if (!G) continue;
         const f32x2 *a = reinterpret_cast<const f32x2 *>(mom) + mom_at(r, 0, NV, NNP_MOM_SH_T);
 #pragma unroll 1
         for (int p = 0; p < NDP; ++p)
@@ -971,8 +1341,15 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
 #pragma unroll
                 for (int tt = 0; tt < TT; ++tt) S[((tt * NDP + p) * (L + 1) + l) * BT] = s[tt];
             }
-        mom_functions_thread<M>(tb, fmax, II, Ty, cnt, S, W2, -1.f, Gi);
-        for (int f = Ty.n_input; f < gstride; ++f) Gi[f] = 0.f;
+        unsigned long long mask = 0;
+        for (int K = 0, tt = 0; K < T; ++K)
+            for (int J = 0; J <= K; ++J, ++tt)
+                if (mom_pairs(cnt, J, K) == 0) mask |= 1ull << tt;
+        mask = mom_functions_thread<M, true>(tb, fmax, II, Ty, mask, S, W2, -1.f, Gi);
+        ls.mask[r] = mask;
+#pragma unroll 1
+        for (unsigned long long m = mask; m; m &= m - 1) mom_push<T>(ls, r, __ffsll(m) - 1, cnt);
+        for (int f = Ty.n_input; G && f < gstride; ++f) Gi[f] = 0.f;
     }
 }
 
@@ -987,15 +1364,15 @@ __device__ void mom_symm_thread_body(i64 lo, i64 hi, const DevPot *__restrict__ 
 // damping factors per 8-byte half, cos and sin parts per 16-byte load, packed
 // FP32 arithmetic), adds the radial terms and scatters dE_i/dd_j in FP64 as
 // force_body does.  Here Q_lm = d^m P_l / dz^m, so that dQ_lm/dz = Q_{l,m+1}
-// needs no factor.  The launch's first blocks take the blocks of few pairs
-// (behind the others they were a tail of 0.10 of 3.39 ms).
+// needs no factor.  With NA = 1 the launch's first thread blocks take the listed blocks
+// of pairs (a small call is a chain of launches; behind the others they were a tail).
 // Bound: instruction issue (FP32 pipe).
 template <class M, int NA>
 __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
                                const float2 *__restrict__ rpar, const int *__restrict__ type,
                                const int *__restrict__ order, const float4 *__restrict__ nbr,
                                const int *__restrict__ nbr_cnt, int cap, int gstride, const float *__restrict__ dEdG,
-                               const float2 *__restrict__ mom, int msh, const unsigned short *__restrict__ mom_cnt,
+                               const float2 *__restrict__ mom, int msh, const unsigned long long *__restrict__ mom_mask,
                                double *__restrict__ F, DevErr *err, const int *__restrict__ atom_struct,
                                double *__restrict__ vir, float *smem)
 {
@@ -1036,7 +1413,7 @@ __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevP
             float *mine = base + al * per;
             const float *e = mine + oE;
             const DevType &Ty = P.t[II_l];
-            const unsigned short *cnt = mom_cnt + 8 * (row + al);
+            const unsigned long long mask = mom_mask[row + al];
             for (int s = lane >> LA; s < TT * NDP * (L + 2); s += 32 / NA) {
                 const int l = s % (L + 2), rem = s / (L + 2), p = rem % NDP, tt = rem / NDP;
                 int K = 0;
@@ -1045,7 +1422,7 @@ __device__ void mom_force_body(int block, int nblock, i64 lo, i64 hi, const DevP
                 const int J = tt - K * (K + 1) / 2;
                 const int bn = Ty.ba[tt].n, off = Ty.ba[tt].off_g, f0 = off - Ty.n_input_r;
                 float s0 = 0.f, s1 = 0.f;
-                if (mom_pairs(cnt, J, K) > NNP_MOM_FEW) {
+                if (!(mask >> tt & 1)) {
                     const float *cf = tb.coef + ((i64)II_l * (L + 2) + l) * fmax + f0;
                     const int *fu = tb.fun + II_l * fmax + f0;
 #pragma unroll 2
@@ -1286,8 +1663,8 @@ __device__ void mom_force_thread_body(int block, int nblock, i64 lo, i64 hi, con
                                       const int *__restrict__ type, const int *__restrict__ order,
                                       const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap, int gstride,
                                       const float *__restrict__ dEdG, const float2 *__restrict__ mom,
-                                      const unsigned short *__restrict__ mom_cnt, double *__restrict__ F, DevErr *err,
-                                      float *smem)
+                                      const unsigned long long *__restrict__ mom_mask, double *__restrict__ F,
+                                      DevErr *err, float *smem)
 {
     constexpr int T = M::T, L = M::L, ND = M::ND, NC = mom_comps(L),
                   NV = mom_vals(T, ND, L), DL = mom_dl(L), BT = NNP_MOM_THREADS;
@@ -1302,7 +1679,7 @@ __device__ void mom_force_thread_body(int block, int nblock, i64 lo, i64 hi, con
         const int n = nbr_cnt[i];
         const DevType &Ty = P.t[II];
         const float4 *src = nbr + i * cap;
-        const unsigned short *cnt = mom_cnt + 8 * row;
+        const unsigned long long mask = mom_mask[row];
         const float *ei = dEdG + i * gstride;
 #pragma unroll 8
         for (int k = 0; 4 * k < gstride; ++k) {
@@ -1324,7 +1701,7 @@ __device__ void mom_force_thread_body(int block, int nblock, i64 lo, i64 hi, con
 #pragma unroll 1
             for (int K = 0; K < T; ++K) {
                 const int tt = J > K ? J * (J + 1) / 2 + K : K * (K + 1) / 2 + J;
-                const bool few = mom_pairs(cnt, J, K) <= NNP_MOM_FEW;
+                const bool few = mask >> tt & 1;
                 const int off = Ty.ba[tt].off_g, bn = Ty.ba[tt].n;
                 const ulonglong2 *cf =
                     reinterpret_cast<const ulonglong2 *>(tb.dcoef + (i64)(II * fmax + off - Ty.n_input_r) * DL);
@@ -1435,7 +1812,7 @@ __device__ void mom_tangent_thread_body(i64 lo, i64 hi, const DevPot *__restrict
                                         int fmax, const int *__restrict__ type, const int *__restrict__ order,
                                         const float4 *__restrict__ nbr, const int *__restrict__ nbr_cnt, int cap,
                                         int gstride, const float4 *__restrict__ V, const float2 *__restrict__ mom,
-                                        float2 *momd, const unsigned short *__restrict__ mom_cnt,
+                                        float2 *momd, const unsigned long long *__restrict__ mom_mask,
                                         float *__restrict__ Cout, float *smem)
 {
     constexpr int T = M::T, TT = T * (T + 1) / 2, L = M::L, ND = M::ND, NC = mom_comps(L), NR = M::NR,
@@ -1452,7 +1829,6 @@ __device__ void mom_tangent_thread_body(i64 lo, i64 hi, const DevPot *__restrict
         const DevType &Ty = P.t[II];
         const float4 *src = nbr + i * cap;
         float *Ci = Cout + i * gstride;
-        const unsigned short *cnt = mom_cnt + 8 * r;
         const float4 vi = V[i];
         int k = 0;
         const float4 none = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
@@ -1571,29 +1947,92 @@ __device__ void mom_tangent_thread_body(i64 lo, i64 hi, const DevPot *__restrict
 #pragma unroll
             for (int tt = 0; tt < TT; ++tt) S[(tt * (L + 1) + l) * BT] = s[tt];
         }
-        mom_functions_thread<M>(tb, fmax, II, Ty, cnt, S, W2, -2.f, Ci);
+        mom_functions_thread<M, false>(tb, fmax, II, Ty, mom_mask[r], S, W2, -2.f, Ci);
         for (int f = Ty.n_input; f < gstride; ++f) Ci[f] = 0.f;
     }
 }
 
-// Tangents of the listed blocks, 16 lanes each, a lane per pair.
+// Tangents of the listed blocks: of many pairs, a warp each, a lane per pair; of few,
+// 16 lanes each, a lane per pair.
 template <class M>
-__device__ void mom_few_tangent_body(const int2 *__restrict__ items, const int *__restrict__ nitems, i64 lo,
-                                     const DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
-                                     const int *__restrict__ type, const int *__restrict__ order,
-                                     const float4 *__restrict__ nbr, int cap, int gstride,
-                                     const unsigned short *__restrict__ mom_cnt, const float4 *__restrict__ V,
-                                     float *__restrict__ Cout)
+__device__ void mom_list_tangent_body(const MomLists ls, i64 lo, const DevPot *__restrict__ pot,
+                                      const float *__restrict__ tab, int fmax, const int *__restrict__ type,
+                                      const int *__restrict__ order, const float4 *__restrict__ nbr, int cap, int gstride,
+                                      const unsigned short *__restrict__ mom_cnt, const float4 *__restrict__ V,
+                                      float *__restrict__ Cout)
 {
+    struct Nbr {
+        float u[3], ud[3], w[M::ND], wr[M::ND];   // direction and damping factors, and their derivatives
+    };
     const MomTab tb = mom_tab(tab, M::T, M::L, fmax);
-    const int nit = *nitems, h = threadIdx.x & 15;
+    const int id = blockIdx.x * NNP_MOM_FEW_THREADS + threadIdx.x, all = gridDim.x * (NNP_MOM_FEW_THREADS / 16);
+    for (MomQueue u(ls.wide, ls.n[1], order + lo, id >> 5, all / 2); u.q < u.n; u.next()) {
+        const i64 i = u.i;
+        const int II = type[i], tt = u.it.y;
+        const DevType &Ty = pot->t[II];
+        u.ahead();
+        const float *a_lo = tb.a_lo + II * NNP_MOM_MAXD;
+        const float4 *src = nbr + i * cap;
+        const float4 vi = V[i];
+        float acc[M::NA];
+#pragma unroll
+        for (int f = 0; f < M::NA; ++f) acc[f] = 0.f;
+        mom_wide_pairs(
+            mom_wide<M::T>(mom_cnt + 8 * (i64)u.it.x, tt),
+            [&](int k) {
+                const float4 rec = src[k], vk = V[__float_as_int(rec.w) & 0x0fffffff];
+                MomNbr<M, true> v;
+                v.set(rec, Ty, a_lo);
+                const float dv[3] = {vi.x - vk.x, vi.y - vk.y, vi.z - vk.z};
+                const float rr = v.ux * dv[0] + v.uy * dv[1] + v.uz * dv[2];
+                Nbr o;
+                o.u[0] = v.ux;
+                o.u[1] = v.uy;
+                o.u[2] = v.uz;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) o.ud[x] = (dv[x] - rr * o.u[x]) * v.ir;
+#pragma unroll
+                for (int d = 0; d < M::ND; ++d) {
+                    o.w[d] = v.w[d];
+                    o.wr[d] = v.wd[d] * rr;
+                }
+                return o;
+            },
+            [&](const Nbr &A, int a, const Nbr &B, int b, bool ok) {
+                float cs = 0.f, cd = 0.f, w[M::ND], dw[M::ND];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    const float ua = __shfl_sync(NNP_FULL, A.u[x], a), ub = __shfl_sync(NNP_FULL, B.u[x], b);
+                    const float da = __shfl_sync(NNP_FULL, A.ud[x], a), db = __shfl_sync(NNP_FULL, B.ud[x], b);
+                    cs = fmaf(ua, ub, cs);
+                    cd = fmaf(da, ub, fmaf(ua, db, cd));
+                }
+#pragma unroll
+                for (int d = 0; d < M::ND; ++d) {
+                    const float wa = __shfl_sync(NNP_FULL, A.w[d], a), wb = __shfl_sync(NNP_FULL, B.w[d], b);
+                    const float ra = __shfl_sync(NNP_FULL, A.wr[d], a), rb = __shfl_sync(NNP_FULL, B.wr[d], b);
+                    w[d] = wa * wb * cd;
+                    dw[d] = fmaf(ra, wb, wa * rb);
+                }
+                if (ok) M::few_tangent(II, tt, cs, w, dw, acc);
+            });
+        const int n = Ty.ba[tt].n;
+        float *Cb = Cout + i * gstride + Ty.ba[tt].off_g;
+#pragma unroll
+        for (int f = 0; f < M::NA; ++f) {
+            const float v = warp_sum(acc[f]);
+            if ((threadIdx.x & 31) == 0 && f < n) Cb[f] = v;
+        }
+    }
+    __syncwarp();
+    const int nit = ls.n[0], h = threadIdx.x & 15;
     const unsigned mask = 0xffffu << (threadIdx.x & 16);
-    for (int q = (blockIdx.x * NNP_MOM_FEW_THREADS + threadIdx.x) >> 4; q < nit; q += gridDim.x * (NNP_MOM_FEW_THREADS / 16)) {
-        const int2 it = items[q];
+    for (int q = mom_few_first(ls, id >> 4, all); q < nit; q += all) {
+        const int2 it = ls.few[q];
         const i64 i = order[lo + it.x];
         const int II = type[i], tt = it.y;
         const DevType &Ty = pot->t[II];
-        const MomFew b = mom_few(mom_cnt + 8 * (i64)it.x, M::T, tt, h);
+        const MomFew b = mom_few<M::T>(mom_cnt + 8 * (i64)it.x, tt, h);
         MomNbr<M, true> v;
         const float4 rec = nbr[i * cap + mom_few_slot(b, h)], vi = V[i], vk = V[__float_as_int(rec.w) & 0x0fffffff];
         v.set(rec, Ty, tb.a_lo + II * NNP_MOM_MAXD);
