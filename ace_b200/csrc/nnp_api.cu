@@ -791,6 +791,22 @@ int nnp_set_graphs(nnp_handle *h, int32_t enable)
     return NNP_OK;
 }
 
+int nnp_set_moment_memory(nnp_handle *h, int64_t limit, int64_t available)
+{
+    if (!h) return NNP_ERR_ARG;
+    if (limit < 0 || available < 0) return fail(h, NNP_ERR_ARG, "negative size");
+    nnp::Engine &E = h->E;
+    cudaStreamSynchronize(E.stream);
+    E.graph_release();
+    E.mom.release(); E.mom_cnt.release(); E.mom_mask.release(); E.mom_items.release(); E.momd.release();
+    E.mom_limit = (size_t)limit;
+    E.mom_avail = (size_t)available;
+    E.mom_want = E.momd_failed = E.len_failed = -1;
+    E.mom_rows = 0;
+    E.mom_valid = false;
+    return NNP_OK;
+}
+
 int nnp_set_accumulation(nnp_handle *h, int32_t acc)
 {
     if (!h) return NNP_ERR_ARG;

@@ -30,13 +30,14 @@ template <class T>
 struct DBuf {
     T *p = nullptr;
     size_t n = 0;
-    cudaError_t reserve(size_t count)
+    // a quarter more than asked for, but not above `most`
+    cudaError_t reserve(size_t count, size_t most = ~(size_t)0)
     {
         if (count <= n) return cudaSuccess;
         if (p) cudaFree(p);
         p = nullptr;
         n = 0;
-        size_t c = count + count / 4 + 16;
+        size_t c = std::min(count + count / 4 + 16, std::max(count, most));
         cudaError_t e = cudaMalloc((void **)&p, c * sizeof(T));
         if (e == cudaSuccess) n = c;
         return e;
@@ -121,6 +122,11 @@ struct Engine {
     DBuf<unsigned long long> mom_mask;   // their bits [row]
     int64_t mom_rows = 0;         // rows of `mom` the current batch uses (0: not reserved)
     bool mom_valid = false;       // they hold the whole batch's moments
+    // bytes of the buffers above at most (and as many again for momd), and the size
+    // above which an allocation counts as failed (0: the device decides)
+    size_t mom_limit = (size_t)8 << 30, mom_avail = 0;
+    int64_t mom_want = -1;        // rows asked for when the buffers were last made, of which they hold mom_rows
+    int64_t momd_failed = -1, len_failed = -1;   // batch sizes for which these could not be had
     DBuf<int> len_order;          // visiting order by neighbour counts, its keys and ranks, its bins (run_len_order)
     bool len_sorted = false;      // the moment kernels visit the atoms in that order
     int *visit() { return len_sorted ? len_order.p : order.p; }

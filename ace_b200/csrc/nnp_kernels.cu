@@ -1792,26 +1792,39 @@ std::string run_neighbors(Engine &E, int pbc)
     return cuda_msg("neighbour list");
 }
 
-// Moments of the batch: rows for all its centres when they fit NNP_MOM_BYTES
-// (and the device's free memory), else for as many as do; the force stage then
-// recomputes them part by part.
-#define NNP_MOM_BYTES ((size_t)8 << 30)
-static std::string mom_reserve(Engine &E)
+// Moments of the batch: rows for all its centres when they fit mom_limit (and the
+// device's free memory), else for as many as do; the force stage then recomputes
+// them part by part.  What could be had is kept for the batch size that asked: no
+// call asks again for what failed, and none allocates while its step is captured
+// (the eager call before has).  false: no room for a useful number of rows; the
+// pair kernels need none.
+#define NNP_MOM_MIN_ROWS 1024
+static size_t mom_row_bytes(const Engine &E)
 {
-    const size_t vals = mom_vals(E.dpot.ntypes, E.mom_ND, E.mom_L);
-    const int64_t most = (int64_t)(NNP_MOM_BYTES / (vals * sizeof(float2))) & ~(int64_t)31;
-    int64_t rows = std::min<int64_t>((E.n_centre + 31) & ~(int64_t)31, most);
-    cudaError_t e = E.mom.reserve((size_t)rows * vals);
-    while (e != cudaSuccess && rows > 4096) {
+    return mom_vals(E.dpot.ntypes, E.mom_ND, E.mom_L) * sizeof(float2) + 8 * sizeof(short) + sizeof(unsigned long long) +
+           E.dpot.ntypes * (E.dpot.ntypes + 1) / 2 * sizeof(int2);
+}
+static int64_t mom_most(const Engine &E) { return (int64_t)(E.mom_limit / mom_row_bytes(E)) & ~(int64_t)31; }
+
+static bool mom_reserve(Engine &E)
+{
+    const size_t vals = mom_vals(E.dpot.ntypes, E.mom_ND, E.mom_L), TT = E.dpot.ntypes * (E.dpot.ntypes + 1) / 2;
+    const int64_t want = (E.n_centre + 31) & ~(int64_t)31, most = mom_most(E);
+    if (want == E.mom_want) return E.mom_rows > 0;
+    E.mom_want = want;
+    int64_t rows = std::min(want, most);
+    for (; rows >= std::min<int64_t>(want, NNP_MOM_MIN_ROWS); rows = (rows / 4) & ~(int64_t)31) {
+        cudaError_t e = E.mom_avail && rows * mom_row_bytes(E) > E.mom_avail ? cudaErrorMemoryAllocation : cudaSuccess;
+        if (e == cudaSuccess) e = E.mom.reserve(rows * vals, most * vals);
+        if (e == cudaSuccess) e = E.mom_cnt.reserve(8 * rows, 8 * most);
+        if (e == cudaSuccess) e = E.mom_mask.reserve(rows, most);
+        if (e == cudaSuccess) e = E.mom_items.reserve(rows * TT, most * TT);
+        if (e == cudaSuccess) break;
         cudaGetLastError();
-        rows = (rows / 4) & ~(int64_t)31;
-        e = E.mom.reserve((size_t)rows * vals);
+        E.mom.release(); E.mom_cnt.release(); E.mom_mask.release(); E.mom_items.release();
     }
-    if (e == cudaSuccess) e = E.mom_cnt.reserve(8 * (size_t)rows);
-    if (e == cudaSuccess) e = E.mom_mask.reserve((size_t)rows);
-    if (e == cudaSuccess) e = E.mom_items.reserve((size_t)rows * (E.dpot.ntypes * (E.dpot.ntypes + 1) / 2));
-    E.mom_rows = rows;
-    return e == cudaSuccess ? "" : std::string("device allocation failed: ") + cudaGetErrorString(e);
+    E.mom_rows = rows >= std::min<int64_t>(want, NNP_MOM_MIN_ROWS) && E.mom.p ? rows : 0;
+    return E.mom_rows > 0;
 }
 
 // Atoms from which a thread per atom is faster than a warp.  Symmetry functions,
@@ -1940,8 +1953,10 @@ static void run_len_order(Engine &E)
     const int T = E.dpot.ntypes;
     const LenBins lb = len_bins(T);
     const size_t bins = (size_t)T * lb.bins;
-    if (E.len_order.reserve(3 * n4 + bins + T) != cudaSuccess) {     // the order by element serves as well
+    if (n == E.len_failed) return;                                   // the order by element serves as well
+    if (E.len_order.reserve(3 * n4 + bins + T) != cudaSuccess) {
         cudaGetLastError();
+        E.len_failed = n;
         return;
     }
     int *out = E.len_order.p, *key = out + n4, *rank = key + n4, *hist = rank + n4;
@@ -2032,8 +2047,11 @@ bool run_tangent_mom(Engine &E, std::string &msg)
     const int64_t N = E.n_centre;
     if (!E.use_jit || !E.jit_tangent_momt || !E.mom_valid || !mom_by_thread(E, N)) return false;
     const int T = E.dpot.ntypes;
-    if (E.momd.reserve((size_t)E.mom_rows * mom_vals(T, E.mom_ND, E.mom_L)) != cudaSuccess) {
-        cudaGetLastError();                                       // the pair loops need no such buffer
+    const size_t vals = mom_vals(T, E.mom_ND, E.mom_L);
+    if (N == E.momd_failed) return false;                         // the pair loops need no such buffer
+    if (E.momd.reserve(E.mom_rows * vals, mom_most(E) * vals) != cudaSuccess) {
+        cudaGetLastError();
+        E.momd_failed = N;
         return false;
     }
     long long l = 0, h = N;
@@ -2057,8 +2075,8 @@ std::string run_symm(Engine &E)
     const int64_t N = E.n_centre;      // centres: the first n_centre entries of `order`
     E.mom_valid = E.len_sorted = false;
     if (N == 0) return "";
-    if (E.use_jit && E.jit_symm_mom && !E.acc64 && !E.symm64) {
-        std::string msg = mom_reserve(E);
+    if (E.use_jit && E.jit_symm_mom && !E.acc64 && !E.symm64 && mom_reserve(E)) {
+        std::string msg;
         if (mom_by_thread(E, std::min(N, E.mom_rows))) run_len_order(E);
         for (int64_t lo = 0; lo < N && msg.empty(); lo += E.mom_rows)
             msg = launch_symm_mom(E, lo, std::min(N, lo + E.mom_rows), E.G.p, lo == 0);
@@ -2143,13 +2161,12 @@ std::string run_force(Engine &E)
     cudaMemsetAsync(E.force.p, 0, 3 * (size_t)E.n_atoms * sizeof(double), E.stream);
     double *vir = E.want_virial ? E.vir.p : nullptr;
     if (vir) cudaMemsetAsync(vir, 0, 9 * (size_t)E.n_struct * sizeof(double), E.stream);
-    if (E.use_jit && E.jit_force_mom1) {
+    if (E.use_jit && E.jit_force_mom1 && N > 0 && (E.mom_valid || mom_reserve(E))) {
         std::string msg;
         if (E.mom_valid) {
             msg = launch_force_mom(E, 0, N, vir);
-        } else if (N > 0) {
+        } else {
             // moments not kept by the symmetry functions (FP64 ones, or more rows than memory): part by part
-            msg = mom_reserve(E);
             for (int64_t lo = 0; lo < N && msg.empty(); lo += E.mom_rows) {
                 const int64_t hi = std::min(N, lo + E.mom_rows);
                 msg = launch_symm_mom(E, lo, hi, nullptr, false);

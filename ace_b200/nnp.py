@@ -90,6 +90,7 @@ def lib():
             "nnp_tune_cache_key": ([C.c_char_p, C.c_char_p, i, i, C.c_char_p, i], i),
             "nnp_tune_cache_store": ([C.c_char_p, p, i], i),
             "nnp_tune_cache_load": ([C.c_char_p, p, i], i),
+            "nnp_set_moment_memory": ([p, C.c_int64, C.c_int64], i),
             "nnp_set_accumulation": ([p, i], i),
             "nnp_set_specialization": ([p, i], i),
             "nnp_specialization": ([p, C.POINTER(i), C.POINTER(C.c_char_p)], i),
@@ -300,6 +301,10 @@ class NNP:
     def set_graphs(self, on: bool = True):
         """Replay the device-side step as a CUDA graph while calls repeat their shape."""
         self._check(lib().nnp_set_graphs(self._h, 1 if on else 0))
+
+    def set_moment_memory(self, limit: int = 8 << 30, available: int = 0):
+        """Device memory for the moments of the angular functions, bytes (see nnp_set_moment_memory)."""
+        self._check(lib().nnp_set_moment_memory(self._h, limit, available))
 
     def set_accumulation(self, mode=1):
         """Precision of the symmetry functions: ACC_FP32 (0, or False), ACC_FP64

@@ -100,6 +100,15 @@ int nnp_set_precision(nnp_handle *h, int32_t precision);
  * tensor memory, so the handle stays usable. */
 int nnp_set_mma_wait(nnp_handle *h, int64_t polls);
 
+/* Device memory for the moments of the angular functions (GAUSS, integer zeta):
+ * at most `limit` bytes (default 8 GiB), and as many again for their derivatives
+ * in training steps.  A batch whose moments need more is worked off part by part
+ * (the forces then form them again); with too little for 1024 atoms the pair
+ * kernels run.  `available`: an allocation above this many bytes counts as failed
+ * without asking the device (0: the device decides).  What the handle holds is
+ * given back. */
+int nnp_set_moment_memory(nnp_handle *h, int64_t limit, int64_t available);
+
 /* Precision of the symmetry functions: NNP_ACC_FP32 (default) computes every
  * pair/triplet term and running sum in FP32; NNP_ACC_FP64 adds the FP32 terms
  * into FP64 sums (~sqrt(T/32) ulp less error for T triplets per atom);
