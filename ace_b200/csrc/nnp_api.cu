@@ -774,12 +774,10 @@ int nnp_specialization_check(const char *potential_path, char *log, int32_t log_
         put(msg);
         return NNP_ERR_UNSUPPORTED;
     }
-    std::string src;
-    std::vector<char> cubin;
-    nnp::jit_last_log().clear();
     nnp::tune_from_env(E.tune);
-    msg = nnp::jit_compile(E, src, cubin);
-    put(msg.empty() ? nnp::jit_last_log() + "\n" + src : msg);
+    std::string text_log;
+    msg = nnp::jit_check(E, text_log);
+    put(msg.empty() ? text_log : msg);
     return msg.empty() ? NNP_OK : NNP_ERR_CUDA;
 }
 
@@ -1006,6 +1004,8 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
     // the handle's buffers, so it can be captured as one CUDA graph
     auto step = [&]() -> std::string {
         std::string msg = nnp::run_prepare(E, N, S, b->pbc);
+        if (E.use_jit && E.jit_module)     // what fails to compile is done by the other kernels
+            nnp::jit_need(E, nnp::jit_parts(E, E.n_centre, (flags & NNP_FORCES) || virial, virial != nullptr));
         if (msg.empty()) msg = nnp::run_neighbors(E, b->pbc);
         if (msg.empty()) msg = nnp::run_symm(E);
         if (msg.empty() && ((flags & (NNP_ENERGY | NNP_FORCES)) || atom_energy || virial)) msg = nnp::run_nn(E);

@@ -66,6 +66,13 @@ struct TuneParams {
     }
 };
 
+// The specialised kernels are compiled and loaded in parts, each when a call first
+// needs it (jit_need): with the handle those that any call runs (a warp per atom),
+// then by the number of atoms two atoms per warp, a thread per atom for the symmetry
+// functions, for the forces, and those of training steps.  All at once they took two
+// to four times the compile time of the first alone.
+enum JitPart { JIT_BASE, JIT_PAIR, JIT_SYMM_T, JIT_FORCE_T, JIT_TANGENT, JIT_TANGENT_T, JIT_PARTS };
+
 struct Engine {
     // potential
     HostPot host;
@@ -99,7 +106,9 @@ struct Engine {
     int tune_source = 0;          // 0 defaults, 1 loaded from the tuning cache, 2 tuned on this handle's data
     std::string tune_log;         // the last tuning's measurements
     bool use_jit = true;
-    void *jit_module = nullptr;   // cudaLibrary_t
+    void *jit_module = nullptr;   // cudaLibrary_t of JIT_BASE, null without specialised kernels
+    void *jit_part[JIT_PARTS] = {};
+    unsigned jit_tried = 0;       // parts that were loaded, or failed to be
     void *jit_symm = nullptr, *jit_force = nullptr, *jit_tangent = nullptr;   // cudaKernel_t
     // cudaKernel_t, moment form: warp or thread per atom; one or two atoms per warp
     void *jit_symm_mom = nullptr, *jit_symm_momt = nullptr, *jit_force_mom1 = nullptr, *jit_force_mom2 = nullptr,
@@ -278,8 +287,10 @@ bool tune_params_valid(const TuneParams &p);
 void tune_from_env(TuneParams &p);
 
 // run-time specialised kernels (nnp_jit.cpp)
-std::string jit_compile(const Engine &E, std::string &source, std::vector<char> &cubin);
-std::string jit_compile_params(const Engine &E, const TuneParams &tp, std::string &source, std::vector<char> &cubin);
+std::string jit_compile_params(const Engine &E, const TuneParams &tp, int part, std::string &source, std::vector<char> &cubin);
+std::string jit_check(Engine &E, std::string &log);     // compiles every part; compiler messages and sources
+std::string jit_need(Engine &E, unsigned want);
+unsigned jit_parts(const Engine &E, int64_t centres, bool forces, bool virial);
 std::string jit_source(const Engine &E, const TuneParams &p);
 uint64_t source_hash(const std::string &s);
 std::string cache_dir();

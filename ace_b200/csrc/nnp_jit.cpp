@@ -27,6 +27,7 @@
 #include <set>
 #include <sstream>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "nnp_engine.h"
@@ -550,7 +551,7 @@ std::string group_cases(const std::vector<std::pair<int, std::string>> &cases)
     return os.str();
 }
 
-std::string make_source(const Engine &E, const TuneParams &tp)
+std::string make_source(const Engine &E, const TuneParams &tp, int part)
 {
     std::ostringstream os;
     // Launch-bound, unroll and chunk choices, as macros at the top of the
@@ -655,7 +656,7 @@ std::string make_source(const Engine &E, const TuneParams &tp)
               "    {\n        switch (II * NNP_MAX_TT + tt) {\n"
            << group_cases(ff) << "        default: return;\n        }\n    }\n};\n";
     os << "}  // namespace nnp\n";
-    if (E.mom_ok)
+    if (E.mom_ok && part == JIT_BASE)
         os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_MOM_SYMM_WARPS * 32, 7)
 k_symm_jit(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
@@ -667,6 +668,9 @@ k_symm_jit(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, cons
     nnp::mom_symm_body<nnp::JitMoments>(lo, hi, pot, tab, fmax, type, order, nbr, nbr_cnt, cap, gstride, G, mom, mom_cnt, ls,
         reinterpret_cast<float *>(smem4));
 }
+)";
+    if (E.mom_ok && (part == JIT_BASE || part == JIT_PAIR))
+        os << R"(
 #define NNP_FORCE_KERNEL(name, na, ...) \
 extern "C" __global__ void __launch_bounds__(__VA_ARGS__) \
 name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax, \
@@ -688,7 +692,10 @@ name(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot,
             type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, vir); \
     } \
 }
-NNP_FORCE_KERNEL(k_force_jit, 1, NNP_MOM_FORCE_WARPS * 32, 5)
+)";
+    if (E.mom_ok && part == JIT_BASE) os << "NNP_FORCE_KERNEL(k_force_jit, 1, NNP_MOM_FORCE_WARPS * 32, 5)\n";
+    if (E.mom_ok && part == JIT_PAIR)
+        os << R"(
 NNP_FORCE_KERNEL(k_force_jit2, 2, NNP_MOM_FORCE_WARPS * 32)
 extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS, NNP_MOM_LIST_BLOCKS)
 k_force_list(const nnp::MomLists ls, long long lo,
@@ -703,7 +710,7 @@ k_force_list(const nnp::MomLists ls, long long lo,
         fmax, type, order, nbr, cap, gstride, mom_cnt, dEdG, F, err, atom_struct, nullptr);
 }
 )";
-    if (E.mom_ok && E.mom_thread())
+    if (part == JIT_SYMM_T)
         os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_MOM_FEW_THREADS, NNP_MOM_LIST_BLOCKS)
 k_symm_list(const nnp::MomLists ls, long long lo,
@@ -724,7 +731,7 @@ k_symm_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, co
         reinterpret_cast<float *>(smem4));
 }
 )";
-    if (E.mom_ok && E.mom_force_thread())
+    if (part == JIT_FORCE_T)
         os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
 k_force_jit_t(int nmain, long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
@@ -737,6 +744,9 @@ k_force_jit_t(int nmain, long long lo, long long hi, const nnp::DevPot *__restri
     nnp::mom_force_thread_body<nnp::JitMoments>((int)blockIdx.x, nmain, lo, hi, pot, tab, fmax, rpar, type, order, nbr,
         nbr_cnt, cap, gstride, dEdG, mom, mom_mask, F, err, reinterpret_cast<float *>(smem4));
 }
+)";
+    if (part == JIT_TANGENT_T)
+        os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_MOM_THREADS, 2)
 k_tangent_jit_t(long long lo, long long hi, const nnp::DevPot *__restrict__ pot, const float *__restrict__ tab, int fmax,
      const int *__restrict__ type, const int *__restrict__ order, const float4 *__restrict__ nbr,
@@ -756,7 +766,7 @@ k_tangent_list(const nnp::MomLists ls, long long lo,
     nnp::mom_list_tangent_body<nnp::JitMoments>(ls, lo, pot, tab, fmax, type, order, nbr, cap, gstride, mom_cnt, V, Cout);
 }
 )";
-    if (!E.mom_ok)
+    if (!E.mom_ok && part == JIT_BASE)
         os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_WARPS * 32, NNP_SYMM_MINB)
 k_symm_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__restrict__ rpar,
@@ -783,7 +793,8 @@ k_force_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__re
 }
 
 )";
-    os << R"(
+    if (part == JIT_TANGENT)
+        os << R"(
 extern "C" __global__ void __launch_bounds__(NNP_WARPS * 32, 1)
 k_tangent_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__restrict__ rpar,
               const float4 *__restrict__ apar, const int *__restrict__ type, const int *__restrict__ order,
@@ -800,15 +811,43 @@ k_tangent_jit(long long N, const nnp::DevPot *__restrict__ pot, const float2 *__
 
 }  // namespace
 
-std::string jit_source(const Engine &E, const TuneParams &p) { return make_source(E, p); }
+std::string jit_source(const Engine &E, const TuneParams &p) { return make_source(E, p, JIT_BASE); }
+
+// The kernels of each part, with the handle's places for them; empty when the
+// potential has none.
+static std::vector<std::pair<const char *, void **>> part_kernels(Engine &E, int part)
+{
+    switch (part) {
+    case JIT_BASE:
+        if (E.mom_ok) return {{"k_symm_jit", &E.jit_symm_mom}, {"k_force_jit", &E.jit_force_mom1}};
+        return {{"k_symm_jit", &E.jit_symm}, {"k_force_jit", &E.jit_force}};
+    case JIT_PAIR:
+        if (!E.mom_ok) return {};
+        return {{"k_force_jit2", &E.jit_force_mom2}, {"k_force_list", &E.jit_force_list}};
+    case JIT_SYMM_T:
+        if (!E.mom_ok || !E.mom_thread()) return {};
+        return {{"k_symm_jit_t", &E.jit_symm_momt}, {"k_symm_list", &E.jit_symm_list}};
+    case JIT_FORCE_T:
+        if (!E.mom_ok || !E.mom_force_thread()) return {};
+        return {{"k_force_jit_t", &E.jit_force_momt}};
+    case JIT_TANGENT:
+        return {{"k_tangent_jit", &E.jit_tangent}};
+    case JIT_TANGENT_T:
+        if (!E.mom_ok || !E.mom_force_thread()) return {};
+        return {{"k_tangent_jit_t", &E.jit_tangent_momt}, {"k_tangent_list", &E.jit_tangent_list}};
+    }
+    return {};
+}
 
 void jit_release(Engine &E)
 {
-    if (E.jit_module) cudaLibraryUnload((cudaLibrary_t)E.jit_module);
+    for (int p = 0; p < JIT_PARTS; ++p) {
+        if (E.jit_part[p]) cudaLibraryUnload((cudaLibrary_t)E.jit_part[p]);
+        E.jit_part[p] = nullptr;
+        for (auto &f : part_kernels(E, p)) *f.second = nullptr;
+    }
     E.jit_module = nullptr;
-    E.jit_symm = E.jit_force = E.jit_tangent = nullptr;
-    E.jit_symm_mom = E.jit_symm_momt = E.jit_force_mom1 = E.jit_force_mom2 = E.jit_force_momt = nullptr;
-    E.jit_tangent_momt = E.jit_symm_list = E.jit_force_list = E.jit_tangent_list = nullptr;
+    E.jit_tried = 0;
 }
 
 std::string &jit_last_log()
@@ -847,20 +886,14 @@ std::string cache_path(uint64_t h)
     return d + name;
 }
 
-// Compiles the specialised kernels with the handle's launch choices.
-std::string jit_compile(const Engine &E, std::string &source, std::vector<char> &cubin)
-{
-    return jit_compile_params(E, E.tune, source, cubin);
-}
-
-// Compiles the specialised kernels with launch choices tp; cubins are kept
-// per process and on disk (cache_dir()) by a hash of the source.  Safe to call
+// Compiles a part of the specialised kernels with launch choices tp; cubins are
+// kept per process and on disk (cache_dir()) by a hash of the source.  Safe to call
 // from several host threads at once.
-std::string jit_compile_params(const Engine &E, const TuneParams &tp, std::string &source, std::vector<char> &cubin)
+std::string jit_compile_params(const Engine &E, const TuneParams &tp, int part, std::string &source, std::vector<char> &cubin)
 {
     static std::mutex mu;
     static std::map<uint64_t, std::vector<char>> memo;
-    source = make_source(E, tp);
+    source = make_source(E, tp, part);
     const uint64_t key = source_hash(source + kDeviceHeaderSource + kMomentsHeaderSource);
     {
         std::lock_guard<std::mutex> lk(mu);
@@ -926,54 +959,102 @@ std::string jit_compile_params(const Engine &E, const TuneParams &tp, std::strin
     return "";
 }
 
+// Compiles every part in `parts` that the potential has, side by side: NVRTC takes
+// seconds for each, and the call waits for the longest.
+static std::vector<std::string> compile_parts(const Engine &E, const std::vector<int> &parts, std::vector<std::string> &src,
+                                              std::vector<std::vector<char>> &cubin, std::vector<std::string> &log)
+{
+    const size_t n = parts.size();
+    std::vector<std::string> msg(n);
+    src.resize(n);
+    cubin.resize(n);
+    log.resize(n);
+    auto one = [&](size_t k) {
+        jit_last_log().clear();
+        msg[k] = jit_compile_params(E, E.tune, parts[k], src[k], cubin[k]);
+        log[k] = jit_last_log();
+    };
+    std::vector<std::thread> th;
+    for (size_t k = 1; k < n; ++k) th.emplace_back(one, k);
+    if (n) one(0);
+    for (auto &t : th) t.join();
+    return msg;
+}
+
+std::string jit_check(Engine &E, std::string &log)
+{
+    std::vector<int> parts;
+    for (int p = 0; p < JIT_PARTS; ++p)
+        if (!part_kernels(E, p).empty()) parts.push_back(p);
+    std::vector<std::string> src, logs;
+    std::vector<std::vector<char>> cubin;
+    const std::vector<std::string> msg = compile_parts(E, parts, src, cubin, logs);
+    for (size_t k = 0; k < parts.size(); ++k) {
+        if (!msg[k].empty()) return msg[k];
+        log += logs[k] + "\n" + src[k];
+    }
+    return "";
+}
+
+// Loads the parts of the bit set `want` that the handle has not loaded yet.  A part
+// that fails is not tried again: its kernels stay null, and the calls take the other
+// ones.  Not while a stream is captured (the eager call before has them loaded).
+std::string jit_need(Engine &E, unsigned want)
+{
+    want &= ~E.jit_tried;
+    if (!want) return "";
+    E.jit_tried |= want;
+    std::vector<int> parts;
+    for (int p = 0; p < JIT_PARTS; ++p)
+        if ((want >> p & 1) && !part_kernels(E, p).empty()) parts.push_back(p);
+    std::vector<std::string> src, log;
+    std::vector<std::vector<char>> cubin;
+    std::vector<std::string> msg = compile_parts(E, parts, src, cubin, log);
+    std::string first;
+    for (size_t k = 0; k < parts.size(); ++k) {
+        cudaLibrary_t lib;
+        if (msg[k].empty() &&
+            cudaLibraryLoadData(&lib, cubin[k].data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
+            cudaGetLastError();
+            msg[k] = "cudaLibraryLoadData failed";
+        }
+        if (msg[k].empty()) {
+            E.jit_part[parts[k]] = (void *)lib;
+            if (parts[k] == JIT_BASE) E.jit_source = src[k];
+            for (auto &f : part_kernels(E, parts[k])) {
+                cudaKernel_t q;
+                if (cudaLibraryGetKernel(&q, lib, f.first) != cudaSuccess) {
+                    cudaGetLastError();
+                    msg[k] = "run-time kernels not found";
+                    break;
+                }
+                *f.second = (void *)q;
+                if (std::getenv("NNP_JIT_VERBOSE")) {    // registers and local memory of the compiled kernels
+                    cudaFuncAttributes a;
+                    if (cudaFuncGetAttributes(&a, (const void *)q) == cudaSuccess)
+                        std::fprintf(stderr, "nnp jit: %s %d registers, %zu bytes local memory\n", f.first, a.numRegs,
+                                     a.localSizeBytes);
+                    else
+                        cudaGetLastError();
+                }
+            }
+            if (!msg[k].empty())
+                for (auto &f : part_kernels(E, parts[k])) *f.second = nullptr;
+        }
+        if (first.empty()) first = msg[k];
+    }
+    return first;
+}
+
 std::string jit_build(Engine &E)
 {
     jit_release(E);
-    std::vector<char> cubin;
-    std::string msg = jit_compile(E, E.jit_source, cubin);
-    if (!msg.empty()) return msg;
-    cudaLibrary_t lib;
-    if (cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
-        cudaGetLastError();
-        return "cudaLibraryLoadData failed";
+    const std::string msg = jit_need(E, 1u << JIT_BASE);
+    if (!msg.empty()) {
+        jit_release(E);
+        return msg;
     }
-    E.jit_module = (void *)lib;
-    std::vector<std::pair<const char *, void **>> fns = {{"k_tangent_jit", &E.jit_tangent}};
-    if (E.mom_ok) {
-        fns.push_back({"k_symm_jit", &E.jit_symm_mom});
-        if (E.mom_thread()) {
-            fns.push_back({"k_symm_jit_t", &E.jit_symm_momt});
-            fns.push_back({"k_symm_list", &E.jit_symm_list});
-        }
-        if (E.mom_force_thread()) {
-            fns.push_back({"k_force_jit_t", &E.jit_force_momt});
-            fns.push_back({"k_tangent_jit_t", &E.jit_tangent_momt});
-            fns.push_back({"k_tangent_list", &E.jit_tangent_list});
-        }
-        fns.push_back({"k_force_jit", &E.jit_force_mom1});
-        fns.push_back({"k_force_jit2", &E.jit_force_mom2});
-        fns.push_back({"k_force_list", &E.jit_force_list});
-    } else {
-        fns.push_back({"k_symm_jit", &E.jit_symm});
-        fns.push_back({"k_force_jit", &E.jit_force});
-    }
-    for (auto &f : fns) {
-        cudaKernel_t k;
-        if (cudaLibraryGetKernel(&k, lib, f.first) != cudaSuccess) {
-            cudaGetLastError();
-            jit_release(E);
-            return "run-time kernels not found";
-        }
-        *f.second = (void *)k;
-        if (std::getenv("NNP_JIT_VERBOSE")) {    // registers and local memory of the compiled kernels
-            cudaFuncAttributes a;
-            if (cudaFuncGetAttributes(&a, (const void *)k) == cudaSuccess)
-                std::fprintf(stderr, "nnp jit: %s %d registers, %zu bytes local memory\n", f.first, a.numRegs,
-                             a.localSizeBytes);
-            else
-                cudaGetLastError();
-        }
-    }
+    E.jit_module = E.jit_part[JIT_BASE];
     return "";
 }
 

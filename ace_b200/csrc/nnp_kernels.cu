@@ -1969,7 +1969,18 @@ static void run_len_order(Engine &E)
     E.len_sorted = true;
 }
 
-static bool mom_by_thread(const Engine &E, int64_t n) { return E.jit_symm_momt && n >= NNP_MOM_THREAD_MIN; }
+// parts of the specialised kernels that a step on so many centres uses
+unsigned jit_parts(const Engine &E, int64_t centres, bool forces, bool virial)
+{
+    if (!E.mom_ok) return 0;
+    unsigned p = 0;
+    if (forces && !virial && centres >= NNP_MOM_PAIR_MIN) p |= 1u << JIT_PAIR;
+    if (centres >= NNP_MOM_THREAD_MIN) p |= 1u << JIT_SYMM_T;
+    if (forces && !virial && centres >= NNP_MOM_FORCE_THREAD_MIN) p |= 1u << JIT_FORCE_T;
+    return p;
+}
+
+static bool mom_by_thread(const Engine &E, int64_t n) { return E.jit_symm_momt && E.jit_symm_list && n >= NNP_MOM_THREAD_MIN; }
 
 // the lists of blocks that are summed over pairs, of a part of E.mom_rows rows
 static MomLists mom_lists(Engine &E)
@@ -2012,7 +2023,7 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
     int cap = E.cap, gs = E.gstride, fm = E.mom_fmax;
     const int *ord = E.visit();
     MomLists ls = mom_lists(E);
-    const int na = (!vir && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
+    const int na = (!vir && E.jit_force_mom2 && E.jit_force_list && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
     if (na == 2) {
         // the listed blocks in a launch of their own: at the thread form's 8 warps
         // per SM they took 1.2 ms of 1.09 M atoms' forces.  A small call, a chain of
@@ -2023,7 +2034,7 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
         if (!msg.empty()) return msg;
         E.launches += 1;
     }
-    if (na == 2 && E.jit_force_momt && hi - lo >= NNP_MOM_FORCE_THREAD_MIN) {
+    if (na == 2 && E.jit_force_momt && hi - lo >= NNP_MOM_FORCE_THREAD_MIN && mom_by_thread(E, hi - lo)) {
         int nmain = grid_for(hi - lo, NNP_MOM_THREADS, 1 << 30);
         void *args[] = {&nmain, &l, &h, &E.d_pot, &E.mom_tab.p, &fm, &E.rpar.p, &E.type.p, &ord, &E.nbr.p, &E.nbr_cnt.p,
                         &cap, &gs, &E.dEdG.p, &E.mom.p, &ls.mask, &E.force.p, &E.err.p};
@@ -2045,7 +2056,9 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
 bool run_tangent_mom(Engine &E, std::string &msg)
 {
     const int64_t N = E.n_centre;
-    if (!E.use_jit || !E.jit_tangent_momt || !E.mom_valid || !mom_by_thread(E, N)) return false;
+    if (!E.use_jit || !E.mom_valid || !mom_by_thread(E, N)) return false;
+    jit_need(E, 1u << JIT_TANGENT_T);
+    if (!E.jit_tangent_momt || !E.jit_tangent_list) return false;
     const int T = E.dpot.ntypes;
     const size_t vals = mom_vals(T, E.mom_ND, E.mom_L);
     if (N == E.momd_failed) return false;                         // the pair loops need no such buffer

@@ -447,16 +447,21 @@ std::string run_train_grad(Engine &E, bool with_force)
     }
     maxn = (maxn + 3) & ~3;
     if (with_force) {
-        const int per = nbr_view_floats(E.cap, ncut, ndamp, E.gstride, true,
-                                        (E.use_jit && E.jit_tangent) ? E.tune.force_chunk : NNP_PCH);
-        const size_t sm = (size_t)WARPS * ((per + 3) & ~3) * sizeof(float);
-        if (sm > 227 * 1024) return "neighbour capacity too large for the tangent kernel";
+        auto view = [&](bool jit) {
+            const int per = nbr_view_floats(E.cap, ncut, ndamp, E.gstride, true, jit ? E.tune.force_chunk : NNP_PCH);
+            return (size_t)WARPS * ((per + 3) & ~3) * sizeof(float);
+        };
+        const bool spec = E.use_jit && E.jit_module;
+        if (view(spec) > 227 * 1024) return "neighbour capacity too large for the tangent kernel";
         const int grid = grid_for(N, WARPS, nsm * 16);
         std::string tmsg;
         const bool done = run_tangent_mom(E, tmsg);
         if (!tmsg.empty()) return tmsg;
         E.launches += done ? 0 : 1;
-        if (!done && E.use_jit && E.jit_tangent) {
+        if (!done && spec) jit_need(E, 1u << JIT_TANGENT);
+        const size_t sm = view(spec && E.jit_tangent);
+        if (!done && sm > 227 * 1024) return "neighbour capacity too large for the tangent kernel";
+        if (!done && spec && E.jit_tangent) {
             long long n = N;
             int cap = E.cap, gs = E.gstride;
             void *args[] = {&n, &E.d_pot, &E.rpar.p, &E.apar.p, &E.type.p, &E.order.p, &E.nbr.p, &E.nbr_cnt.p,

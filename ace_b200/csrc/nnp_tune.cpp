@@ -250,7 +250,7 @@ std::string autotune(Engine &E, int cap, const std::function<std::string()> &run
             th.emplace_back([&, k] {
                 std::string src;
                 std::vector<char> cubin;
-                errs[k] = jit_compile_params(E, cand[k], src, cubin);
+                errs[k] = jit_compile_params(E, cand[k], JIT_BASE, src, cubin);
             });
         for (auto &t : th) t.join();
         for (const auto &e : errs)
