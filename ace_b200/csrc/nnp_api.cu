@@ -26,7 +26,10 @@ namespace {
 
 thread_local std::string g_create_error;
 
-constexpr size_t H_COUNT_OFF = 64;    // of the atom count behind the pinned error record
+// The handle's pinned memory: the error record, the atom count of device-pointer
+// calls, then room for the inputs and the results of small calls, so that a handle's
+// first call pins none (two allocations of ~0.1 ms).
+constexpr size_t H_COUNT_OFF = 64, H_STAGE_OFF = 256, H_STAGE_BYTES = 124 << 10;
 static_assert(sizeof(nnp::DevErr) <= H_COUNT_OFF, "error record");
 
 int fail(nnp_handle *h, int code, const std::string &msg)
@@ -125,7 +128,7 @@ void Engine::free_all()
 {
     rpar.release(); apar.release(); wpar.release(); vac.release();
     rpar64.release(); apar64.release(); cut64.release();
-    mom_tab.release(); mom.release(); mom_cnt.release(); mom_items.release(); mom_mask.release(); momd.release(); len_order.release();
+    mom_tab.release(); mom_mem.release(); momd.release(); len_order.release();
     atom_off.release(); pos.release(); cell.release(); xw.release();
     type.release(); atom_struct.release(); atom_cell.release(); grid.release(); bbox.release();
     cell_cnt.release(); cell_start.release(); cell_fill.release(); cell_atoms.release(); scan_tmp.release();
@@ -142,10 +145,10 @@ void Engine::free_all()
     d_pot = nullptr;
     if (h_err) cudaFreeHost(h_err);
     h_err = nullptr;
-    if (h_stage) cudaFreeHost(h_stage);
+    if (h_stage && own_stage) cudaFreeHost(h_stage);
     h_stage = nullptr;
     h_stage_bytes = 0;
-    if (h_out) cudaFreeHost(h_out);
+    if (h_out && own_out) cudaFreeHost(h_out);
     h_out = nullptr;
     h_out_bytes = 0;
     if (own_stream && stream) cudaStreamDestroy(stream);
@@ -171,7 +174,7 @@ void Engine::buffer_key(std::vector<int64_t> &key) const
 {
     auto add = [&](const auto &...b) { (..., (key.push_back((int64_t)(intptr_t)b.p), key.push_back((int64_t)b.n))); };
     add(xw, atom_struct, atom_cell, grid, bbox, scan_tmp, cell_cnt, cell_start, cell_fill, cell_tcnt, cell_atoms, cell_pos, order,
-        type_fill, neigh_items, nbr, nbr_cnt, G, dEdG, e_atom, e_struct, force, err, vir, mom, mom_cnt, mom_items, mom_mask, len_order);
+        type_fill, neigh_items, nbr, nbr_cnt, G, dEdG, e_atom, e_struct, force, err, vir, mom_mem, len_order);
 }
 
 // Build the device potential.  Angular functions of one BasisA that form a
@@ -466,11 +469,14 @@ int finish_create(nnp_handle *h, nnp_handle **out)
         return fail(nullptr, NNP_ERR_CUDA, "cudaStreamCreate failed");
     }
     E.own_stream = true;
-    if (cudaMallocHost((void **)&E.h_err, H_COUNT_OFF + sizeof(int64_t)) != cudaSuccess) {
+    if (cudaMallocHost((void **)&E.h_err, H_STAGE_OFF + 2 * H_STAGE_BYTES) != cudaSuccess) {
         E.free_all();
         delete h;
         return fail(nullptr, NNP_ERR_CUDA, "cudaMallocHost failed");
     }
+    E.h_stage = reinterpret_cast<char *>(E.h_err) + H_STAGE_OFF;
+    E.h_out = reinterpret_cast<char *>(E.h_stage) + H_STAGE_BYTES;
+    E.h_stage_bytes = E.h_out_bytes = H_STAGE_BYTES;
     std::string msg = E.upload();
     if (!msg.empty()) {
         E.free_all();
@@ -498,9 +504,10 @@ int finish_create(nnp_handle *h, nnp_handle **out)
 int stage_bytes(nnp::Engine &E, size_t bytes)
 {
     if (bytes <= E.h_stage_bytes) return NNP_OK;
-    if (E.h_stage) cudaFreeHost(E.h_stage);
+    if (E.h_stage && E.own_stage) cudaFreeHost(E.h_stage);
     E.h_stage = nullptr;
     E.h_stage_bytes = 0;
+    E.own_stage = true;
     const size_t want = bytes + bytes / 4 + 4096;
     if (cudaMallocHost(&E.h_stage, want) != cudaSuccess) return NNP_ERR_CUDA;
     E.h_stage_bytes = want;
@@ -541,9 +548,10 @@ struct OutCopies {
         staged = !list.empty() && bytes <= most;
         if (!staged) return cudaSuccess;
         if (bytes > E.h_out_bytes) {
-            if (E.h_out) cudaFreeHost(E.h_out);
+            if (E.h_out && E.own_out) cudaFreeHost(E.h_out);
             E.h_out = nullptr;
             E.h_out_bytes = 0;
+            E.own_out = true;
             const size_t want = std::min(most, 2 * bytes + 4096);
             const cudaError_t e = cudaMallocHost(&E.h_out, want);
             if (e != cudaSuccess) return e;
@@ -796,7 +804,7 @@ int nnp_set_moment_memory(nnp_handle *h, int64_t limit, int64_t available)
     nnp::Engine &E = h->E;
     cudaStreamSynchronize(E.stream);
     E.graph_release();
-    E.mom.release(); E.mom_cnt.release(); E.mom_mask.release(); E.mom_items.release(); E.momd.release();
+    E.mom_mem.release(); E.momd.release();
     E.mom_limit = (size_t)limit;
     E.mom_avail = (size_t)available;
     E.mom_want = E.momd_failed = E.len_failed = -1;

@@ -124,11 +124,20 @@ struct Engine {
     std::vector<double> mom_norm, mom_gnorm;   // M::norm, M::gnorm (nnp_moments.cuh)
     float mom_a_lo(int II, int d) const { return mom_tab_host[3 * mom_comps(mom_L) + II * NNP_MOM_MAXD + d]; }
     DBuf<float> mom_tab;          // MomTab
-    DBuf<float2> mom;             // moments of atoms visit()[0 .. mom_rows) (mom_at)
+    DBuf<unsigned char> mom_mem;  // the four arrays below, one allocation
+    struct {
+        float2 *p = nullptr;
+    } mom;                        // moments of atoms visit()[0 .. mom_rows) (mom_at)
+    struct {
+        unsigned short *p = nullptr;
+    } mom_cnt;                    // their neighbour counts by element [row][8]
+    struct {
+        int2 *p = nullptr;
+    } mom_items;                  // (row, block) of the blocks that are summed over pairs (MomLists)
+    struct {
+        unsigned long long *p = nullptr;
+    } mom_mask;                   // their bits [row]
     DBuf<float2> momd;            // derivatives of the moments along the training step's displacements
-    DBuf<unsigned short> mom_cnt; // their neighbour counts by element [row][8]
-    DBuf<int2> mom_items;         // (row, block) of the blocks that are summed over pairs (MomLists)
-    DBuf<unsigned long long> mom_mask;   // their bits [row]
     int64_t mom_rows = 0;         // rows of `mom` the current batch uses (0: not reserved)
     bool mom_valid = false;       // they hold the whole batch's moments
     // bytes of the buffers above at most (and as many again for momd), and the size
@@ -199,6 +208,7 @@ struct Engine {
     size_t h_stage_bytes = 0;
     void *h_out = nullptr;          // the same for their results (OutCopies)
     size_t h_out_bytes = 0;
+    bool own_stage = false, own_out = false;   // not parts of h_err's allocation
 
     std::string last_error;
 

@@ -839,10 +839,54 @@ static std::vector<std::pair<const char *, void **>> part_kernels(Engine &E, int
     return {};
 }
 
+// Loaded libraries, shared by the process's handles of one potential: loading and
+// the first launch of each kernel take ~0.5 ms per handle.  A library is unloaded
+// with the last handle that uses it.
+struct SharedLibrary {
+    cudaLibrary_t lib;
+    int users;
+};
+static std::mutex lib_mu;
+static std::map<uint64_t, SharedLibrary> &libraries()
+{
+    static std::map<uint64_t, SharedLibrary> m;
+    return m;
+}
+
+static std::string library_acquire(const std::string &source, const std::vector<char> &cubin, cudaLibrary_t &lib)
+{
+    const uint64_t key = source_hash(source);
+    std::lock_guard<std::mutex> lk(lib_mu);
+    auto it = libraries().find(key);
+    if (it == libraries().end()) {
+        if (cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
+            cudaGetLastError();
+            return "cudaLibraryLoadData failed";
+        }
+        it = libraries().insert({key, {lib, 0}}).first;
+    }
+    ++it->second.users;
+    lib = it->second.lib;
+    return "";
+}
+
+static void library_release(cudaLibrary_t lib)
+{
+    std::lock_guard<std::mutex> lk(lib_mu);
+    for (auto it = libraries().begin(); it != libraries().end(); ++it)
+        if (it->second.lib == lib) {
+            if (--it->second.users == 0) {
+                cudaLibraryUnload(lib);
+                libraries().erase(it);
+            }
+            return;
+        }
+}
+
 void jit_release(Engine &E)
 {
     for (int p = 0; p < JIT_PARTS; ++p) {
-        if (E.jit_part[p]) cudaLibraryUnload((cudaLibrary_t)E.jit_part[p]);
+        if (E.jit_part[p]) library_release((cudaLibrary_t)E.jit_part[p]);
         E.jit_part[p] = nullptr;
         for (auto &f : part_kernels(E, p)) *f.second = nullptr;
     }
@@ -1012,12 +1056,8 @@ std::string jit_need(Engine &E, unsigned want)
     std::vector<std::string> msg = compile_parts(E, parts, src, cubin, log);
     std::string first;
     for (size_t k = 0; k < parts.size(); ++k) {
-        cudaLibrary_t lib;
-        if (msg[k].empty() &&
-            cudaLibraryLoadData(&lib, cubin[k].data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess) {
-            cudaGetLastError();
-            msg[k] = "cudaLibraryLoadData failed";
-        }
+        cudaLibrary_t lib = nullptr;
+        if (msg[k].empty()) msg[k] = library_acquire(src[k], cubin[k], lib);
         if (msg[k].empty()) {
             E.jit_part[parts[k]] = (void *)lib;
             if (parts[k] == JIT_BASE) E.jit_source = src[k];
@@ -1029,6 +1069,8 @@ std::string jit_need(Engine &E, unsigned want)
                     break;
                 }
                 *f.second = (void *)q;
+                // one value for all: handles in several threads launch the shared kernels
+                cudaFuncSetAttribute((const void *)q, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
                 if (std::getenv("NNP_JIT_VERBOSE")) {    // registers and local memory of the compiled kernels
                     cudaFuncAttributes a;
                     if (cudaFuncGetAttributes(&a, (const void *)q) == cudaSuccess)
@@ -1061,8 +1103,6 @@ std::string jit_build(Engine &E)
 std::string jit_launch(void *fn, int grid, int block, size_t smem, cudaStream_t stream, void **args)
 {
     const void *k = (const void *)fn;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(cudaGetLastError());
     const cudaError_t r = cudaLaunchKernel(k, dim3(grid), dim3(block), args, smem, stream);
     if (r != cudaSuccess) return std::string("cudaLaunchKernel: ") + cudaGetErrorString(r);
     return "";

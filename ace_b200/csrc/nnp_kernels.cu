@@ -1809,21 +1809,22 @@ static int64_t mom_most(const Engine &E) { return (int64_t)(E.mom_limit / mom_ro
 static bool mom_reserve(Engine &E)
 {
     const size_t vals = mom_vals(E.dpot.ntypes, E.mom_ND, E.mom_L), TT = E.dpot.ntypes * (E.dpot.ntypes + 1) / 2;
+    const size_t row = mom_row_bytes(E);
     const int64_t want = (E.n_centre + 31) & ~(int64_t)31, most = mom_most(E);
     if (want == E.mom_want) return E.mom_rows > 0;
     E.mom_want = want;
     int64_t rows = std::min(want, most);
     for (; rows >= std::min<int64_t>(want, NNP_MOM_MIN_ROWS); rows = (rows / 4) & ~(int64_t)31) {
-        cudaError_t e = E.mom_avail && rows * mom_row_bytes(E) > E.mom_avail ? cudaErrorMemoryAllocation : cudaSuccess;
-        if (e == cudaSuccess) e = E.mom.reserve(rows * vals, most * vals);
-        if (e == cudaSuccess) e = E.mom_cnt.reserve(8 * rows, 8 * most);
-        if (e == cudaSuccess) e = E.mom_mask.reserve(rows, most);
-        if (e == cudaSuccess) e = E.mom_items.reserve(rows * TT, most * TT);
+        cudaError_t e = E.mom_avail && rows * row > E.mom_avail ? cudaErrorMemoryAllocation : cudaSuccess;
+        if (e == cudaSuccess) e = E.mom_mem.reserve(rows * row, most * row);
         if (e == cudaSuccess) break;
         cudaGetLastError();
-        E.mom.release(); E.mom_cnt.release(); E.mom_mask.release(); E.mom_items.release();
     }
-    E.mom_rows = rows >= std::min<int64_t>(want, NNP_MOM_MIN_ROWS) && E.mom.p ? rows : 0;
+    E.mom_rows = rows >= std::min<int64_t>(want, NNP_MOM_MIN_ROWS) ? rows : 0;
+    E.mom.p = reinterpret_cast<float2 *>(E.mom_mem.p);
+    E.mom_items.p = reinterpret_cast<int2 *>(E.mom.p + E.mom_rows * vals);
+    E.mom_mask.p = reinterpret_cast<unsigned long long *>(E.mom_items.p + E.mom_rows * TT);
+    E.mom_cnt.p = reinterpret_cast<unsigned short *>(E.mom_mask.p + E.mom_rows);   // rows: multiple of 32, so 16-byte aligned
     return E.mom_rows > 0;
 }
 
