@@ -66,6 +66,11 @@ struct TuneParams {
     }
 };
 
+// Dynamic shared memory that every kernel is allowed, whatever a launch takes: the
+// attribute belongs to the kernel, and one set to a launch's own size would fail the
+// launch of another thread's handle that needs more.
+constexpr int NNP_SMEM_MAX = 227 * 1024;
+
 // The specialised kernels are compiled and loaded in parts, each when a call first
 // needs it (jit_need): with the handle those that any call runs (a warp per atom),
 // then by the number of atoms two atoms per warp, a thread per atom for the symmetry

@@ -1069,8 +1069,7 @@ std::string jit_need(Engine &E, unsigned want)
                     break;
                 }
                 *f.second = (void *)q;
-                // one value for all: handles in several threads launch the shared kernels
-                cudaFuncSetAttribute((const void *)q, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+                cudaFuncSetAttribute((const void *)q, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
                 if (std::getenv("NNP_JIT_VERBOSE")) {    // registers and local memory of the compiled kernels
                     cudaFuncAttributes a;
                     if (cudaFuncGetAttributes(&a, (const void *)q) == cudaSuccess)

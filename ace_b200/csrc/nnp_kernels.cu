@@ -2112,7 +2112,7 @@ std::string run_symm(Engine &E)
     }
     if (E.symm64) {
         const size_t sm64 = (size_t)WARPS * (symm64_floats(E.cap) / 2 + 4) * sizeof(double);
-        cudaFuncSetAttribute(k_symm_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm64);
+        cudaFuncSetAttribute(k_symm_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
         k_symm_f64<<<grid, WARPS * 32, sm64, E.stream>>>(N, E.d_pot, E.rpar64.p, E.apar64.p, E.cut64.p, E.type.p,
                                                          E.order.p, E.nbr.p, E.nbr_cnt.p, E.cap, E.xw.p,
                                                          E.atom_struct.p, E.grid.p, E.gstride, E.G.p);
@@ -2120,7 +2120,7 @@ std::string run_symm(Engine &E)
         return cuda_msg("symmetry functions (FP64)");
     }
     auto kern = E.acc64 ? k_symm<double> : k_symm<float>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
     kern<<<grid, WARPS * 32, sm, E.stream>>>(N, E.d_pot, E.rpar.p, E.apar.p, E.type.p, E.order.p, E.nbr.p, E.nbr_cnt.p, E.cap,
                                              ncut_max(E), ndamp_max(E), E.gstride, E.G.p);
     E.mark(2);
@@ -2149,7 +2149,7 @@ std::string run_nn(Engine &E)
         const int nt = tiles <= num_sms() + E.dpot.ntypes ? 256 : 128;
         auto kern = nt == 256 ? (L == 2 ? k_nn_tile<256, 2> : L == 3 ? k_nn_tile<256, 3> : k_nn_tile<256, 0>)
                               : (L == 2 ? k_nn_tile<128, 2> : L == 3 ? k_nn_tile<128, 3> : k_nn_tile<128, 0>);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
         const int per_sm = (int)std::min<size_t>(8, std::max<size_t>(1, (228 * 1024) / (smt + 1024)));
         kern<<<grid_for(tiles, 1, num_sms() * per_sm), nt, smt, E.stream>>>(
             E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride, E.e_atom.p, E.dEdG.p);
@@ -2160,7 +2160,7 @@ std::string run_nn(Engine &E)
     const int maxn = max_nodes(E);
     const size_t sm = (size_t)(((E.wfloats + 3) & ~3) + WARPS * (NNP_MAX_LAYERS + 2) * maxn) * sizeof(float);
     if (sm > 220 * 1024) return "networks too large for the shared-memory FP32 path";
-    cudaFuncSetAttribute(k_nn_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_nn_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
     k_nn_fp32<<<grid_for(N, WARPS * 8, num_sms() * 2), WARPS * 32, sm, E.stream>>>(
         E.n_centre, E.d_pot, E.wpar.p, E.wfloats, E.type.p, E.G.p, E.gstride, maxn, E.e_atom.p, E.dEdG.p);
     E.launches += 1;
@@ -2202,7 +2202,7 @@ std::string run_force(Engine &E)
         E.mark(4);
         return msg;
     }
-    cudaFuncSetAttribute(k_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_force, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
     k_force<<<grid, WARPS * 32, sm, E.stream>>>(N, E.d_pot, E.rpar.p, E.apar.p, E.type.p, E.order.p, E.nbr.p, E.nbr_cnt.p, E.cap,
                                                 ncut_max(E), ndamp_max(E), E.gstride, E.dEdG.p, E.force.p, E.err.p,
                                                 E.atom_struct.p, vir);
@@ -2406,7 +2406,7 @@ std::string run_energy_symm_noalloc(Engine &E, int S, int64_t N, const int64_t *
     const size_t sm = (size_t)(((E.wfloats + 3) & ~3) + WARPS * 2 * maxn) * sizeof(float);
     if (sm > 220 * 1024) return "networks too large for the shared-memory FP32 path";
     if (N > 0) {
-        cudaError_t e = cudaFuncSetAttribute(k_nn_energy_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = cudaFuncSetAttribute(k_nn_energy_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
         if (e != cudaSuccess) return std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
         k_nn_energy_fp32<<<grid_for(N, WARPS * 8, num_sms() * 2), WARPS * 32, sm, E.stream>>>(
             N, E.d_pot, E.wpar.p, E.wfloats, type, G, gstride, maxn, e_atom);

@@ -488,7 +488,7 @@ std::string run_nn_tc(Engine &E, bool split)
     int L = E.dpot.t[0].nlayer;
     for (int T = 1; T < E.dpot.ntypes; ++T) L = E.dpot.t[T].nlayer == L ? L : 0;
     auto kern = L == 3 ? (split ? k_nn_tc<true, 3> : k_nn_tc<false, 3>) : (split ? k_nn_tc<true, 0> : k_nn_tc<false, 0>);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
     kern<<<grid, groups * TILE, sm, E.stream>>>(E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride,
                                                 E.e_atom.p, E.dEdG.p, E.err.p, polls);
     E.launches += 1;

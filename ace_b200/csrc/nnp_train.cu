@@ -469,7 +469,7 @@ std::string run_train_grad(Engine &E, bool with_force)
             std::string msg = jit_launch(E.jit_tangent, grid, WARPS * 32, sm, E.stream, args);
             if (!msg.empty()) return msg;
         } else if (!done) {
-            cudaFuncSetAttribute(k_tangent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            cudaFuncSetAttribute(k_tangent, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
             k_tangent<<<grid, WARPS * 32, sm, E.stream>>>(N, E.d_pot, E.rpar.p, E.apar.p, E.type.p, E.order.p, E.nbr.p,
                                                           E.nbr_cnt.p, E.cap, ncut, ndamp, E.gstride, E.tvec.p, E.tang.p);
             std::string msg = cuda_msg("tangent symmetry functions");
@@ -491,7 +491,7 @@ std::string run_train_grad(Engine &E, bool with_force)
     const size_t smt = train_tile_floats(dims) * sizeof(float);
     const char *tile_env = std::getenv("NNP_TRAIN_TILE");
     if (smt <= 227 * 1024 && !(tile_env && tile_env[0] == '0')) {
-        cudaFuncSetAttribute(k_nn_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
+        cudaFuncSetAttribute(k_nn_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
         const int per_sm = std::max(1, std::min(4, (int)((228 * 1024) / (smt + 1024))));
         const int grid = grid_for(N / TT_ROWS + E.dpot.ntypes, 1, nsm * per_sm);
         k_nn_train_tile<<<grid, WARPS * 32, smt, E.stream>>>(E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p,
@@ -502,7 +502,7 @@ std::string run_train_grad(Engine &E, bool with_force)
     }
     const size_t sm = (size_t)(2 * ((E.wfloats + 3) & ~3) + WARPS * train_warp_floats(maxl, maxn)) * sizeof(float);
     if (sm > 227 * 1024) return "networks too large for the shared-memory training kernel";
-    cudaFuncSetAttribute(k_nn_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_nn_train, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
     k_nn_train<<<grid_for(N, WARPS * 16, nsm * 2), WARPS * 32, sm, E.stream>>>(
         N, E.d_pot, E.wpar.p, E.wfloats, E.type.p, E.order.p, E.G.p, with_force ? E.tang.p : nullptr, E.gstride, maxn,
         maxl, E.gE.p, E.pgrad.p);
