@@ -23,6 +23,10 @@
 // template parameter (plan and widths in registers) and TMEM read 16 columns at
 // a time: 1,088,749 atoms of three elements (56-32-32-1) 768 -> 433 us, 353,589
 // of four (64-48-48-1) 562 -> 251 us, 131,072 of two (80-64-64-1) 301 -> 175 us.
+// Other counts, split BF16, with weights and f'(z) in every tile's shared memory /
+// the count at run time / as a template parameter, 4000 and 400,000 atoms: one hidden
+// layer of 32: 24.5, 187 / 24.6, 127 / 20.5, 115 us; three: 43, 609 / 47, 293 / 41,
+// 254; elements with two and three (always at run time): 43, 529 / 46, 254.
 // Bound: the serial chain of MMAs and epilogues of a tile.
 // Thread r of a warpgroup owns row r of its tile (TMEM lane r).  Tiles are taken
 // in groups of one per warpgroup, all of one element, element by element over
@@ -487,7 +491,8 @@ std::string run_nn_tc(Engine &E, bool split)
     const uint32_t polls = E.mma_wait_polls > 0 ? E.mma_wait_polls : WAIT_POLLS;
     int L = E.dpot.t[0].nlayer;
     for (int T = 1; T < E.dpot.ntypes; ++T) L = E.dpot.t[T].nlayer == L ? L : 0;
-    auto kern = L == 3 ? (split ? k_nn_tc<true, 3> : k_nn_tc<false, 3>) : (split ? k_nn_tc<true, 0> : k_nn_tc<false, 0>);
+    auto kern = split ? (L == 2 ? k_nn_tc<true, 2> : L == 3 ? k_nn_tc<true, 3> : L == 4 ? k_nn_tc<true, 4> : k_nn_tc<true, 0>)
+                      : (L == 2 ? k_nn_tc<false, 2> : L == 3 ? k_nn_tc<false, 3> : L == 4 ? k_nn_tc<false, 4> : k_nn_tc<false, 0>);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NNP_SMEM_MAX);
     kern<<<grid, groups * TILE, sm, E.stream>>>(E.d_pot, E.wpar.p, E.type_fill.p, E.order.p, E.G.p, E.gstride,
                                                 E.e_atom.p, E.dEdG.p, E.err.p, polls);
