@@ -27,6 +27,7 @@
 #include <set>
 #include <sstream>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -1019,7 +1020,13 @@ static std::vector<std::string> compile_parts(const Engine &E, const std::vector
         log[k] = jit_last_log();
     };
     std::vector<std::thread> th;
-    for (size_t k = 1; k < n; ++k) th.emplace_back(one, k);
+    for (size_t k = 1; k < n; ++k) {
+        try {
+            th.emplace_back(one, k);
+        } catch (const std::system_error &) {        // no thread to be had
+            one(k);
+        }
+    }
     if (n) one(0);
     for (auto &t : th) t.join();
     return msg;
