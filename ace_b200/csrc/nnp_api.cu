@@ -1091,7 +1091,9 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
         if (!msg.empty()) { rc = fail(h, NNP_ERR_CUDA, msg); break; }
         // results: behind the step where their arrays stay untouched if it failed
         OutCopies out;
-        const bool plain = devp && !(flags & NNP_SYMM) && !atom_energy && !virial;
+        // (k_outputs stores doubles; arrays at other addresses are copied)
+        const bool plain = devp && !(flags & NNP_SYMM) && !atom_energy && !virial &&
+                           !(((uintptr_t)energy | (uintptr_t)forces) & (sizeof(double) - 1));
         if (!devp) {
             if (flags & NNP_ENERGY) out.add(energy, E.e_struct.p, sizeof(double) * S);
             if (flags & NNP_FORCES) out.add(forces, E.force.p, sizeof(double) * 3 * N);

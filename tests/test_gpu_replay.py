@@ -96,3 +96,22 @@ def test_gradient_of_a_replayed_step(tmp_path):
         assert np.abs(e - e0).max() < 1e-9 and np.abs(f - f0).max() < 1e-9
     nn.close()
     ref.close()
+
+
+@pytest.mark.parametrize("shift", [1, 4])
+def test_result_arrays_at_any_address(tmp_path, shift):
+    """device results into arrays that are not aligned to doubles"""
+    path = make(tmp_path)
+    b = synth.batch_random(5, [30, 50], 3)
+    nn = NNP.read(path)
+    e0, f0 = nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    d = Device(b)
+    e = torch.zeros(8 * b.n_struct + 16, dtype=torch.uint8, device="cuda")
+    f = torch.zeros(24 * b.n_atoms + 16, dtype=torch.uint8, device="cuda")
+    for _ in range(4):
+        nn.compute_device(d.off.data_ptr(), d.pos.data_ptr(), d.typ.data_ptr(), d.cell.data_ptr(), b.n_struct,
+                          e.data_ptr() + shift, f.data_ptr() + shift)
+        e1 = e.cpu().numpy()[shift:shift + 8 * b.n_struct].copy().view(np.float64)
+        f1 = f.cpu().numpy()[shift:shift + 24 * b.n_atoms].copy().view(np.float64).reshape(-1, 3)
+        assert np.abs(e1 - e0).max() < 1e-9 and np.abs(f1 - f0).max() < 1e-9
+    nn.close()
