@@ -1168,9 +1168,11 @@ __device__ void mom_symm_body(i64 lo, i64 hi, const DevPot *__restrict__ pot, co
 // BT apart): G_f = sum_l c_l S_l - self (c and self as in dE/dA: half of them
 // for J == K), self = -wscale sum w_d^2.  Blocks that are summed over pairs are
 // written too and replaced.  `mask` has those without pairs (0 here); with MARK it
-// gets those whose terms cancel.  The coefficients' signs are those of lambda^l, so the
-// absolute sum needs only the sums over even and odd l of c_l |S_l|: one more
-// multiply-add per term, 1 % of the symmetry functions.
+// gets those whose terms cancel.  The absolute sum of the terms is taken as that of
+// the sums over even and over odd l (with J == K, S_l >= 0 and the coefficients'
+// signs are those of lambda^l, so it is the absolute sum; J and K to one side or
+// opposite sides likewise), and at least the term of l = 0 (J and K at right angles):
+// no further sums.  With sums of |c_l S_l|, 1.09 M atoms: 1.63 ms instead of 1.55.
 template <class M, bool MARK>
 __device__ __forceinline__ unsigned long long mom_functions_thread(const MomTab &tb, int fmax, int II, const DevType &Ty,
                                                                    unsigned long long mask, const f32x2 *S, const f32x2 *W2,
@@ -1197,7 +1199,7 @@ __device__ __forceinline__ unsigned long long mom_functions_thread(const MomTab 
                     for (int l = 0; l <= L; ++l) st[l] = S[((tt * NDP + p) * (L + 1) + l) * BT];
                     st[L + 1] = mul2(W2[(J * NDP + p) * BT], dup2(wscale));
                 }
-                f32x2 c[DL], g = 0ull, a[2] = {0ull, 0ull};
+                f32x2 c[DL], ge = 0ull, go = 0ull;               // even and odd l
 #pragma unroll
                 for (int l = 0; l < DL; l += 2) {
                     const ulonglong2 v = __ldg(cf + f * (DL / 2) + l / 2);
@@ -1206,18 +1208,19 @@ __device__ __forceinline__ unsigned long long mom_functions_thread(const MomTab 
                 }
 #pragma unroll
                 for (int l = L; l >= 0; --l) {
-                    g = fma2(c[l], st[l], g);
-                    if (MARK) a[l & 1] = fma2(c[l], st[l] & 0x7fffffff7fffffffull, a[l & 1]);
+                    if (l & 1) go = fma2(c[l], st[l], go);
+                    else ge = fma2(c[l], st[l], ge);
                 }
-                g = fma2(c[L + 1], st[L + 1], g);
-                float g0, g1;
-                up2(g, g0, g1);
+                const f32x2 self = mul2(c[L + 1], st[L + 1]);    // at most 0
+                float e0, e1, g0, g1;
+                up2(ge, e0, e1);
+                up2(add2(fma2(c[L + 1], st[L + 1], ge), go), g0, g1);
                 if (MARK) {
-                    float e0, e1, o0, o1, s0, s1;
-                    up2(a[0], e0, e1);
-                    up2(a[1], o0, o1);
-                    up2(mul2(c[L + 1], st[L + 1]), s0, s1);      // at most 0
-                    cancels |= g0 + g1 < NNP_MOM_CANCEL * (e0 + e1 + fabsf(o0 + o1) - (s0 + s1));
+                    float o0, o1, s0, s1, z0, z1;
+                    up2(go, o0, o1);
+                    up2(self, s0, s1);
+                    up2(mul2(c[0], st[0]), z0, z1);
+                    cancels |= g0 + g1 < NNP_MOM_CANCEL * (fmaxf(fabsf(e0 + e1) + fabsf(o0 + o1), z0 + z1) - (s0 + s1));
                 }
                 if (Gi) Gi[off + f] = none ? 0.f : h * (g0 + g1);
             }
