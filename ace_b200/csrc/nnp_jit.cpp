@@ -850,8 +850,8 @@ struct SharedLibrary {
 static std::mutex lib_mu;
 static std::map<uint64_t, SharedLibrary> &libraries()
 {
-    static std::map<uint64_t, SharedLibrary> m;
-    return m;
+    static auto *m = new std::map<uint64_t, SharedLibrary>;   // outlives handles that are closed at exit
+    return *m;
 }
 
 static std::string library_acquire(const std::string &source, const std::vector<char> &cubin, cudaLibrary_t &lib)

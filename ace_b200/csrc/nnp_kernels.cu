@@ -2027,7 +2027,8 @@ static std::string launch_force_mom(Engine &E, int64_t lo, int64_t hi, double *v
     const int na = (!vir && E.jit_force_mom2 && E.jit_force_list && hi - lo >= NNP_MOM_PAIR_MIN) ? 2 : 1;
     if (na == 2) {
         // the listed blocks in a launch of their own: at the thread form's 8 warps
-        // per SM they took 1.2 ms of 1.09 M atoms' forces.  A small call, a chain of
+        // per SM they took 1.2 ms of 1.09 M atoms' forces, and with them the form of two
+        // atoms per warp has 96 registers instead of 72.  A small call, a chain of
         // launches, takes them in the same one.
         void *list[] = {&ls, &l, &E.d_pot, &E.mom_tab.p, &fm, &E.type.p, &ord, &E.nbr.p, &cap, &gs, &E.mom_cnt.p, &E.dEdG.p,
                         &E.force.p, &E.err.p, &E.atom_struct.p};
