@@ -1044,6 +1044,7 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
                (int64_t)(intptr_t)E.cell.p};
         E.buffer_key(key);
     }
+    E.nbr_atoms = -1;
     for (int attempt = 0; attempt < 4; ++attempt) {
         std::string msg;
         if (graphs && E.graph_exec && key == E.graph_key) {
@@ -1089,6 +1090,7 @@ int compute_impl(nnp_handle *h, const nnp_batch *b, double *energy, double *forc
             msg = step();
         }
         if (!msg.empty()) { rc = fail(h, NNP_ERR_CUDA, msg); break; }
+        E.nbr_atoms = N;
         // results: behind the step where their arrays stay untouched if it failed
         OutCopies out;
         // (k_outputs stores doubles; arrays at other addresses are copied)
@@ -1426,7 +1428,10 @@ int nnp_compute_energy_symm(nnp_handle *h, int32_t n_struct, const int64_t *atom
     cudaError_t ce = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (x != cudaSuccess && ce == cudaSuccess) ce = x; };
     E.n_ghost = 0;
+    const void *lists = E.nbr.p, *counts = E.nbr_cnt.p;
+    const size_t ln = E.nbr.n, cn = E.nbr_cnt.n;
     std::string msg = nnp::run_prepare(E, N, n_struct, 0);
+    if (E.nbr.p != lists || E.nbr.n != ln || E.nbr_cnt.p != counts || E.nbr_cnt.n != cn) E.nbr_atoms = -1;
     if (!msg.empty()) return fail(h, NNP_ERR_CUDA, msg);
     chk(E.atom_off.reserve(n_struct + 1));
     chk(E.type.reserve(std::max<int64_t>(N, 1)));
@@ -1479,7 +1484,8 @@ int nnp_neighbor_counts(nnp_handle *h, int32_t *counts)
 {
     if (!h || !counts) return NNP_ERR_ARG;
     nnp::Engine &E = h->E;
-    const size_t n = (size_t)E.n_atoms * E.dpot.ntypes;
+    if (E.nbr_atoms < 0) return fail(h, NNP_ERR_ARG, "the neighbour lists of the last compute call are gone");
+    const size_t n = (size_t)E.nbr_atoms * E.dpot.ntypes;
     if (n == 0) return NNP_OK;
     int *d = nullptr;
     if (cudaMalloc((void **)&d, n * sizeof(int)) != cudaSuccess) return fail(h, NNP_ERR_CUDA, "cudaMalloc failed");

@@ -178,6 +178,7 @@ struct Engine {
     DBuf<int4> neigh_items;       // neighbour-search work items {cell, structure, first atom, end atom}
     DBuf<float4> nbr;
     DBuf<int> nbr_cnt;
+    int64_t nbr_atoms = 0;        // atoms that they hold the lists of (-1: lost to another call's buffers)
     DBuf<float> G, dEdG, e_atom;
     DBuf<double> e_struct, force, symm_d;
     DBuf<DevErr> err;

@@ -1643,8 +1643,8 @@ __global__ void k_nbr_types(int64_t N, const float4 *__restrict__ nbr, const int
 
 std::string run_neighbor_counts(Engine &E, int *d_counts)
 {
-    if (E.n_atoms == 0) return "";
-    k_nbr_types<<<grid_for(E.n_atoms, 256, 1 << 30), 256, 0, E.stream>>>(E.n_atoms, E.nbr.p, E.nbr_cnt.p, E.cap,
+    if (E.nbr_atoms <= 0) return "";
+    k_nbr_types<<<grid_for(E.nbr_atoms, 256, 1 << 30), 256, 0, E.stream>>>(E.nbr_atoms, E.nbr.p, E.nbr_cnt.p, E.cap,
                                                                          E.dpot.ntypes, d_counts);
     return cuda_msg("neighbour counts");
 }

@@ -447,7 +447,8 @@ int nnp_stage_times(const nnp_handle *h, float *ms, int32_t n);
 
 /* Neighbour counts of the last nnp_compute, split by neighbour type:
  * counts[i*ntypes + t] is the number of type-t neighbours of atom i (host
- * array of N*ntypes).  The pair and triplet counts per atom follow from these
+ * array of N*ntypes; NNP_ERR_ARG if the lists are gone: the buffers of a larger
+ * nnp_compute_energy_symm replaced them).  The pair and triplet counts per atom follow from these
  * (NeighborList::size, struc/neighbor.hpp:35). */
 int nnp_neighbor_counts(nnp_handle *h, int32_t *counts);
 

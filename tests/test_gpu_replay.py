@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from ace_b200 import NNP, potential, synth
+from ace_b200.nnp import NNPError
 
 pytestmark = pytest.mark.gpu
 
@@ -114,4 +115,25 @@ def test_result_arrays_at_any_address(tmp_path, shift):
         e1 = e.cpu().numpy()[shift:shift + 8 * b.n_struct].copy().view(np.float64)
         f1 = f.cpu().numpy()[shift:shift + 24 * b.n_atoms].copy().view(np.float64).reshape(-1, 3)
         assert np.abs(e1 - e0).max() < 1e-9 and np.abs(f1 - f0).max() < 1e-9
+    nn.close()
+
+
+@pytest.mark.parametrize("other", [10, 5000])
+def test_neighbour_counts_are_the_last_compute_calls(tmp_path, other):
+    """after energies of another structure: the same counts, or an error when its larger
+    buffers replaced the lists"""
+    path = make(tmp_path)
+    b = synth.batch_random(5, [30, 50], 3)
+    nn = NNP.read(path)
+    nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    want = nn.neighbor_counts(b.n_atoms)
+    rng = np.random.default_rng(4)
+    nn.compute_energy(rng.integers(0, 3, other).astype(np.int32), rng.uniform(0.0, 1.0, (other, nn.gstride)))
+    if other < b.n_atoms:
+        assert (nn.neighbor_counts(b.n_atoms) == want).all()
+    else:
+        with pytest.raises(NNPError):
+            nn.neighbor_counts(b.n_atoms)
+    nn.compute_batch(b.atom_off, b.pos, b.type, b.cell)
+    assert (nn.neighbor_counts(b.n_atoms) == want).all()
     nn.close()
